@@ -56,6 +56,13 @@ int pcx_exp_f32(float* p, int64_t n, void* stream);
  * 0 = they hold linear flows (PyJuice's logspace_flows=False).  Arithmetic is done in log space either way;
  * the flag only changes how flows are read and written. */
 
+/* data[v, b] = category of variable v in sample b, int32, samples padded to W columns with category 0:
+ * x[b * stride_b + v * stride_v], element size elsize in {1,2,4,8} (unsigned 8-bit or signed wider; 64-bit values
+ * outside the int32 range saturate, so that they stay outside every table).  Takes the place of the transpose of
+ * model/tensorcircuit.py:355-356. */
+int pcx_load_inputs(int32_t* data, const void* x, int elsize, int64_t B, int64_t V, int64_t stride_b,
+                    int64_t stride_v, int64_t W, void* stream);
+
 /* node_flows[root rows, b] = w (linear) or log w (log space), w = weights ? weights[r*B+b] : 1
  * (model/tensorcircuit.py:537-552). */
 int pcx_set_root_flows(float* node_flows, const float* weights, int64_t root_start, int64_t num_roots,

@@ -27,6 +27,7 @@ SIGNATURES = {
     "pcx_fill_f32": [P, L, F],
     "pcx_scale_f32": [P, L, F],
     "pcx_exp_f32": [P, L],
+    "pcx_load_inputs": [P, P, I, L, L, L, L, L],
     "pcx_set_root_flows": [P, P, L, L, I, I],
     "pcx_input_cat_fwd": [P, P, P, I, P, P, P, I, L, L, I],
     "pcx_input_cat_bwd": [P, P, P, I, P, P, P, I, L, L, I, I],

@@ -45,6 +45,36 @@ __global__ void root_flows_kernel(float* __restrict__ node_flows, const float* _
     node_flows[root_start + i] = logspace ? logf(w) : w;              // root rows are contiguous: [num_roots, B]
 }
 
+// The batch, [B, V] in the caller's integer type, as [V, W] int32: 32 x 32 tiles through shared memory, so that both
+// sides are read and written in whole lines (a [784, 512] batch: 3 us, and the leaf kernels that read the result have
+// one element type and 16-byte loads of four categories).
+__global__ void __launch_bounds__(256)
+load_inputs_kernel(int32_t* __restrict__ data, const void* __restrict__ x, int elsize, int64_t B, int64_t V,
+                   int64_t stride_b, int64_t stride_v, int64_t W) {
+    __shared__ int32_t tile[32][33];
+    const int64_t b0 = (int64_t)blockIdx.x * 32, v0 = (int64_t)blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int k = ty; k < 32; k += 8) {
+        const int64_t b = b0 + k, v = v0 + tx;
+        int32_t c = 0;
+        if (b < B && v < V) {
+            const int64_t at = b * stride_b + v * stride_v;
+            if (elsize == 8) {
+                const int64_t q = ((const int64_t*)x)[at];
+                c = (int32_t)min(max(q, (int64_t)INT32_MIN), (int64_t)INT32_MAX);
+            } else {
+                c = pcx_load_cat(x, elsize, at);
+            }
+        }
+        tile[k][tx] = c;
+    }
+    __syncthreads();
+    for (int k = ty; k < 32; k += 8) {
+        const int64_t v = v0 + k, b = b0 + tx;
+        if (v < V && b < W) data[v * W + b] = tile[tx][k];
+    }
+}
+
 // Categorical leaves, general form: one CTA per node, threads walk the batch.  Used when the batch is not a multiple
 // of four or a node has too many categories to stage its table in shared memory.  A category id outside the node's
 // table (invalid data) must not address outside it: the forward kernel clamps it, the backward kernel adds no flow.
@@ -483,6 +513,17 @@ int pcx_exp_f32(float* p, int64_t n, void* stream) {
     int64_t g = pcx_cdiv(n, kThreads);
     if (g > 148 * 16) g = 148 * 16;
     exp_kernel<<<(int)g, kThreads, 0, (cudaStream_t)stream>>>(p, n);
+    PCX_LAUNCH_CHECK();
+    return 0;
+}
+
+int pcx_load_inputs(int32_t* data, const void* x, int elsize, int64_t B, int64_t V, int64_t stride_b, int64_t stride_v,
+                    int64_t W, void* stream) {
+    if (elsize != 1 && elsize != 2 && elsize != 4 && elsize != 8) return -1;
+    if (B <= 0 || V <= 0) return 0;
+    if (W < B || pcx_cdiv(V, 32) > 65535) return -1;
+    dim3 grid((unsigned)pcx_cdiv(W, 32), (unsigned)pcx_cdiv(V, 32));
+    load_inputs_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(data, x, elsize, B, V, stride_b, stride_v, W);
     PCX_LAUNCH_CHECK();
     return 0;
 }

@@ -30,6 +30,18 @@ def _dev_i32(t: torch.Tensor, device) -> torch.Tensor:
     return t.to(device=device, dtype=torch.int32).contiguous()
 
 
+def _rows(*bufs):
+    """Value buffers as the kernels address them.  A circuit's public buffers are views of the first B columns of rows
+    padded to a multiple of eight samples; the kernels work on whole rows."""
+    return tuple(t if t is None or t.stride(0) == t.size(1) or t.size(0) <= 1
+                 else t.as_strided((t.size(0), t.stride(0)), (t.stride(0), 1)) for t in bufs)
+
+
+def _pad_data(data: torch.Tensor, width: int) -> torch.Tensor:
+    """``[V, B]`` categories, padded with category 0 to the row width of the value buffers."""
+    return data.contiguous() if data.size(1) == width else nn.functional.pad(data, (0, width - data.size(1)))
+
+
 ALG_IDS = {"LL": 0, "MPE": 1, "GeneralLL": 2}
 
 
@@ -310,8 +322,9 @@ class InputLayer(Layer, nn.Module):
         """``data`` is ``[num_vars, B]`` (variables outermost), integer."""
         _unsupported(params=params is not None, missing_mask=missing_mask is not None)
         self._require_cuda()
-        data = data.contiguous()
+        node_mars, = _rows(node_mars)
         B = node_mars.size(1)
+        data = _pad_data(data, B)
         if self._shadow_ok(B):
             sh = self._shadow
             stamp = (self.params.data_ptr(), self.params._version, self._param_epoch)
@@ -334,8 +347,9 @@ class InputLayer(Layer, nn.Module):
         self._require_cuda()
         if self._param_flows is None:
             self.init_param_flows()
-        data = data.contiguous()
+        node_flows, = _rows(node_flows)
         B = node_flows.size(1)
+        data = _pad_data(data, B)
         if self._shadow_ok(B):
             sh = self._shadow
             if sh["flows"] is None:
@@ -457,6 +471,7 @@ class ProdLayer(Layer, nn.Module):
     def forward(self, node_mars: torch.Tensor, element_mars: torch.Tensor, _for_backward: bool = False, **kwargs):
         if self._dev is None:
             raise NotImplementedError("product layers run on CUDA only (no CPU path)")
+        node_mars, element_mars = _rows(node_mars, element_mars)
         B = node_mars.size(1)
         for nids, cids in self._dev["fw"]:
             _lib.call("pcx_prod_fwd", element_mars, node_mars, nids, cids, nids.numel(), cids.size(1), self.block_size, B)
@@ -466,6 +481,7 @@ class ProdLayer(Layer, nn.Module):
     def backward(self, node_flows: torch.Tensor, element_flows: torch.Tensor, logspace_flows: bool = False, **kwargs):
         if self._dev is None:
             raise NotImplementedError("product layers run on CUDA only (no CPU path)")
+        node_flows, element_flows = _rows(node_flows, element_flows)
         B = node_flows.size(1)
         raw = getattr(self, "_raw_backward_tables", False) and "bk_raw" in self._dev
         for u_cids, parids in self._dev["bk_raw" if raw else "bk"]:
@@ -664,6 +680,7 @@ class SumLayer(Layer, nn.Module):
                 propagation_alg: str = "LL", pflow_temperature: float = 1.0, **kwargs):
         self._require_cuda()
         _unsupported(pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6)
+        node_mars, element_mars = _rows(node_mars, element_mars)
         B = node_mars.size(1)
         alg, alpha = _alg_of(propagation_alg, kwargs)
         if alg != 0:                                      # "MPE" / "GeneralLL": plain fp32 kernels
@@ -751,6 +768,7 @@ class SumLayer(Layer, nn.Module):
         _unsupported(allow_modify_flows=allow_modify_flows,
                      negate_pflows=negate_pflows, accumulate_ch_flows=accumulate_ch_flows, allow_neg_flows=allow_neg_flows,
                      pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6, temper_eflow=temper_eflow)
+        node_flows, element_flows, node_mars, element_mars = _rows(node_flows, element_flows, node_mars, element_mars)
         B = node_flows.size(1)
         ls = int(bool(logspace_flows))
         alg, alpha = _alg_of(propagation_alg, kwargs)

@@ -85,7 +85,8 @@ class TensorCircuit(nn.Module):
         scope = as_bitset(root_ns.scope).to_list()
         self.num_vars = (max(scope) + 1) if scope else 0
 
-        self.node_mars = self.element_mars = self.node_flows = self.element_flows = None
+        self._nm = self._em = self._nf = self._ef = None
+        self._batch = 0
         self.param_flows = None
         self._init_layers(layer_sparsity_tol, max_num_partitions, max_tied_ns_per_parflow_block)
 
@@ -250,7 +251,7 @@ class TensorCircuit(nn.Module):
     def _reset_parentless(self, prod_gi: int, logspace_flows: bool):
         rng = self._parentless.get(prod_gi)
         if rng is not None:
-            _fill(self.element_flows[rng[0]:rng[1]], NEG_INF if logspace_flows else 0.0)
+            _fill(self._ef[rng[0]:rng[1]], NEG_INF if logspace_flows else 0.0)
 
     def _mask_parentless_in_device_tables(self):
         """The kernels' copies of the product layers' backward tables skip parentless products (id 0 = padding), so
@@ -330,8 +331,8 @@ class TensorCircuit(nn.Module):
         self._em_dev = {k: (v.to(device) if isinstance(v, torch.Tensor) else v) for k, v in self._em_blocks.items()}
         self._fusing_dev = [(start, n, torch.tensor(accs, dtype=torch.int64, device=device))
                             for start, n, accs in self._tied_sum_groups]
-        for name in ("node_mars", "element_mars", "node_flows", "element_flows", "param_flows"):
-            setattr(self, name, None)
+        self._nm = self._em = self._nf = self._ef = self.param_flows = None
+        self._data_buf = None
         if device.type == "cuda":
             self._mask_parentless_in_device_tables()
         self._setup_fusion()
@@ -455,17 +456,46 @@ class TensorCircuit(nn.Module):
             raise NotImplementedError("the compiled circuit runs on CUDA only; call `pc.to('cuda:0')` first "
                                       "(there is no CPU path)")
 
+    # ---- value buffers ---------------------------------------------------------------------------------------------
+    # The buffers hold a multiple of eight columns (`_PAD`): eight fp32 samples are one 32-byte sector, and every fast
+    # kernel (vector loads, folded products, dense operands, tensor-core parameter flows) reads whole groups of them.  A
+    # ragged batch used to fall back to the general kernels as a whole (an HMM with 512 states, 64 tokens and 77
+    # samples: 3.87 ms per training step, 2.78 ms padded to 80; 196-variable tree, 256 states, 100 samples: 1.85, 1.34 ms).  Padding columns evaluate category 0 and get the
+    # root flow 0, so they add nothing to any parameter flow.  The public attributes are views of the first B columns.
+    _PAD = 8
+
+    def _columns(self, t):
+        return t if t is None or t.size(1) == self._batch else t[:, :self._batch]
+
+    @property
+    def node_mars(self):
+        return self._columns(self._nm)
+
+    @property
+    def element_mars(self):
+        return self._columns(self._em)
+
+    @property
+    def node_flows(self):
+        return self._columns(self._nf)
+
+    @property
+    def element_flows(self):
+        return self._columns(self._ef)
+
     def _ensure_buffers(self, B: int, backward: bool = False):
-        """(Re)allocate the value buffers when the batch size changes.  Dummy rows are written here once:
+        """(Re)allocate the value buffers when the padded batch size changes.  Dummy rows are written here once:
         every other row is fully overwritten by the layer that owns it on each pass."""
-        if self.node_mars is None or self.node_mars.size(1) != B:
-            self.node_mars = torch.zeros(self.num_nodes, B, device=self.device)
-            self.element_mars = torch.full((self.num_elements, B), NEG_INF, device=self.device)
-            self.node_flows = self.element_flows = None
+        self._batch = B
+        W = -(-B // self._PAD) * self._PAD
+        if self._nm is None or self._nm.size(1) != W:
+            self._nm = torch.zeros(self.num_nodes, W, device=self.device)
+            self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
+            self._nf = self._ef = None
             self._graphs = {}
-        if backward and (self.node_flows is None or self.node_flows.size(1) != B):
-            self.node_flows = torch.empty(self.num_nodes, B, device=self.device)
-            self.element_flows = torch.full((self.num_elements, B), NEG_INF, device=self.device)
+        if backward and (self._nf is None or self._nf.size(1) != W):
+            self._nf = torch.empty(self.num_nodes, W, device=self.device)
+            self._ef = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             self._eflow_mode = 1
             self._graphs = {k: g for k, g in self._graphs.items() if k[0] != "bk"}
 
@@ -480,13 +510,21 @@ class TensorCircuit(nn.Module):
     # ------------------------------------------------------------------------------------------
     # forward
     # ------------------------------------------------------------------------------------------
-    def _prepare_inputs(self, inputs: torch.Tensor) -> torch.Tensor:
+    def _prepare_inputs(self, inputs: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """The batch as ``[V, W]`` int32 (variables outermost, batch padded with category 0), the layout every leaf
+        kernel reads.  ``out`` is written when it fits."""
         assert inputs.dim() == 2 and inputs.size(1) >= self.num_vars
         if inputs.is_floating_point():
             raise TypeError("categorical inputs must be an integer tensor")
         if inputs.dtype not in (torch.uint8, torch.int16, torch.int32, torch.int64):
             inputs = inputs.long()
-        return inputs.to(self.device, non_blocking=True).t().contiguous()       # [V, B]
+        x = inputs.to(self.device, non_blocking=True)
+        B, V = x.size(0), x.size(1)
+        W = -(-B // self._PAD) * self._PAD
+        if out is None or out.size(0) != V or out.size(1) != W:
+            out = torch.empty(V, W, dtype=torch.int32, device=self.device)
+        _lib.call("pcx_load_inputs", out, x, x.element_size(), B, V, x.stride(0), x.stride(1), W)
+        return out
 
     def _run_inner(self, key, fn):
         """Run ``fn`` (a sequence of launches on the current stream) — from a CUDA graph after the first call."""
@@ -516,9 +554,9 @@ class TensorCircuit(nn.Module):
         if backward and self._reference_compat:
             return False
         if self._fused[gi].get("dense") and not (SumLayer.use_dense_kernels and SumLayer.use_wide_dense
-                                                 and self.node_mars is not None and self.node_mars.size(1) % 8 == 0):
+                                                 and self._nm is not None and self._nm.size(1) % 8 == 0):
             return False
-        return (not backward) or self.node_mars.size(1) % 8 == 0
+        return (not backward) or self._nm.size(1) % 8 == 0
 
     def _launch_cfg(self):
         """Everything that changes which kernels a pass launches (part of the key of a captured graph)."""
@@ -595,13 +633,13 @@ class TensorCircuit(nn.Module):
         return plan
 
     def _launch_chain(self, plan, mode: int, logspace_flows: bool = True):
-        _lib.call("pcx_sum_chain", mode, self.node_mars, self.node_flows if mode == 1 else None, plan["jobs"],
-                  plan["n_jobs"], plan["n_items"], plan["n_levels"], plan["tn"], plan["fc"], self.node_mars.size(1),
+        _lib.call("pcx_sum_chain", mode, self._nm, self._nf if mode == 1 else None, plan["jobs"],
+                  plan["n_jobs"], plan["n_items"], plan["n_levels"], plan["tn"], plan["fc"], self._nm.size(1),
                   int(bool(logspace_flows)), plan["ctrl"], plan["ctrl"].numel())
 
     def _forward_inner(self):
         groups = self.inner_layer_groups
-        plan = self._chain_plan(self.node_mars.size(1), 0)
+        plan = self._chain_plan(self._nm.size(1), 0)
         for gi, group in enumerate(groups):
             if plan is not None and plan["lo"] - 1 <= gi <= plan["hi"]:
                 if gi == plan["lo"]:
@@ -609,12 +647,12 @@ class TensorCircuit(nn.Module):
                 continue
             if group.is_prod():
                 if not self._fusion_on(gi + 1):
-                    group.forward(self.node_mars, self.element_mars)
+                    group.forward(self._nm, self._em)
             elif self._fusion_on(gi):
                 for layer in group:
-                    layer.forward_fused(self.node_mars)
+                    layer.forward_fused(self._nm)
             else:
-                group.forward(self.node_mars, self.element_mars, self.params.data, **self._alg_kwargs())
+                group.forward(self._nm, self._em, self.params.data, **self._alg_kwargs())
 
     def _alg_kwargs(self) -> dict:
         names = ("LL", "MPE", "GeneralLL")
@@ -649,8 +687,9 @@ class TensorCircuit(nn.Module):
             B = inputs.size(0)
             data = self._prepare_inputs(inputs)
             self._ensure_buffers(B)
+            W = self._nm.size(1)
             if self.debug_poison:               # every row must be rewritten by the layer that owns it
-                _fill(self.node_mars[self.num_dummy_nodes:], float("nan"))
+                _fill(self._nm[self.num_dummy_nodes:], float("nan"))
             self._last_data, self._last_inputs = data, origin_inputs
             # the operand tiles of the tensor-core kernels are re-packed (when the parameters changed) on a second
             # stream, beside the input layer: neither reads what the other writes
@@ -664,12 +703,12 @@ class TensorCircuit(nn.Module):
                 self._packer.refresh(self.params.data)
             with self._nvtx("pcx forward: input layers"):
                 for layer in self.input_layer_group:
-                    layer.forward(data, self.node_mars)
+                    layer.forward(data, self._nm)
             if forked:
                 cur.wait_stream(self._side_stream)
             with self._nvtx("pcx forward: inner layers"):
-                self._run_inner(("fw", B, self._launch_cfg(), self.params.data_ptr()), self._forward_inner)
-            lls = self.node_mars[self._root_node_range[0]:self._root_node_range[1], :].permute(1, 0).clone()
+                self._run_inner(("fw", W, self._launch_cfg(), self.params.data_ptr()), self._forward_inner)
+            lls = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t().clone()
         if torch.is_grad_enabled():
             lls.requires_grad = True
             lls.register_hook(partial(_pc_model_backward_hook, pc=self, inputs=origin_inputs, **self._alg_kwargs()))
@@ -779,7 +818,7 @@ class TensorCircuit(nn.Module):
         pf = self.param_flows if compute_param_flows else None
         groups = self.inner_layer_groups
         any_fused = False
-        dense = self._dense_par_plan(self.node_mars.size(1)) if (pf is not None and self._alg[0] == 0) else None
+        dense = self._dense_par_plan(self._nm.size(1)) if (pf is not None and self._alg[0] == 0) else None
 
         def dense_stage(layer, p, node_flows, node_mars, element_mars, ls):
             hit = dense["where"].get((id(layer), p))
@@ -799,7 +838,7 @@ class TensorCircuit(nn.Module):
                           slot, ls)
             return True
 
-        plan = self._chain_plan(self.node_mars.size(1), 1)
+        plan = self._chain_plan(self._nm.size(1), 1)
         cur = torch.cuda.current_stream(self.device)
         side = self._side_stream if self.use_side_stream else None
         forked = False
@@ -812,7 +851,7 @@ class TensorCircuit(nn.Module):
                 continue
             if group.is_prod():
                 if not (self._fusion_on(gi + 1, True) and self._fused[gi + 1]["direct"]):
-                    group.backward(self.node_flows, self.element_flows, logspace_flows=logspace_flows)
+                    group.backward(self._nf, self._ef, logspace_flows=logspace_flows)
             elif self._fusion_on(gi, True) and self._fused[gi].get("dense"):
                 # The operands of the (tied) parameter-flow product only read this depth's node flows and values, which
                 # are final by now; the element flows below read the same rows and write the children's.  The two are
@@ -824,22 +863,22 @@ class TensorCircuit(nn.Module):
                     with torch.cuda.stream(side if side is not None else cur):
                         for layer in group:
                             for p in range(layer.num_fw_partitions):
-                                ok = dense is not None and dense_stage(layer, p, self.node_flows, self.node_mars, None,
+                                ok = dense is not None and dense_stage(layer, p, self._nf, self._nm, None,
                                                                        int(bool(logspace_flows)))
                                 assert ok, "a dense-folded table must have a slot in the dense parameter-flow product"
                     forked = forked or side is not None
                 for layer in group:
-                    layer.backward_ele_fused(self.node_flows, self.element_flows, self.node_mars, logspace_flows)
+                    layer.backward_ele_fused(self._nf, self._ef, self._nm, logspace_flows)
             elif self._fusion_on(gi, True):
                 any_fused = any_fused or not self._fused[gi]["sm"]
                 for layer in group:
                     if self._fused[gi]["sm"] and pf is not None:       # (the 128-row kernels do this in one launch below)
-                        layer.backward_par_fused(self.node_flows, self.node_mars, self.params.data, pf, logspace_flows)
-                    layer.backward_ele_fused(self.node_flows, self.element_flows, self.node_mars, logspace_flows)
+                        layer.backward_par_fused(self._nf, self._nm, self.params.data, pf, logspace_flows)
+                    layer.backward_ele_fused(self._nf, self._ef, self._nm, logspace_flows)
             else:
                 # the shared element buffer holds another depth by now: recompute this depth's products
-                groups[gi - 1].forward(self.node_mars, self.element_mars, _for_backward=True)
-                group.backward(self.node_flows, self.element_flows, self.node_mars, self.element_mars,
+                groups[gi - 1].forward(self._nm, self._em, _for_backward=True)
+                group.backward(self._nf, self._ef, self._nm, self._em,
                                self.params.data, param_flows=pf, logspace_flows=logspace_flows,
                                dense_par_stage=dense_stage if dense is not None else None, **self._alg_kwargs())
         if dense is not None:
@@ -855,9 +894,9 @@ class TensorCircuit(nn.Module):
         self._batched_par_pending = any_fused and pf is not None     # launched by `backward`, after this sweep
 
     def _launch_batched_par(self, logspace_flows: bool):
-        B = self.node_flows.size(1)
+        B = self._nf.size(1)
         for fc, jobs, n_jobs, n_items, chunks_per_cta in self._par_jobs(B):
-            _lib.call("pcx_sum_bwd_par_batched", self.param_flows, self.node_flows, self.node_mars, self.params.data,
+            _lib.call("pcx_sum_bwd_par_batched", self.param_flows, self._nf, self._nm, self.params.data,
                       jobs, n_jobs, n_items, fc, B, chunks_per_cta, int(bool(logspace_flows)))
 
     @_in_own_mode
@@ -877,10 +916,10 @@ class TensorCircuit(nn.Module):
         _unsupported(input_layer_fn=input_layer_fn is not None, cache=cache is not None, return_cache=return_cache,
                      negate_pflows=negate_pflows, pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6,
                      missing_mask=kwargs.get("missing_mask") is not None)
-        assert self.node_mars is not None and self.element_mars is not None, "Should run forward path first."
+        assert self._nm is not None and self._em is not None, "Should run forward path first."
         self._run_params = dict(logspace_flows=logspace_flows, propagation_alg=propagation_alg)
         with torch.no_grad():
-            B = self.node_mars.size(1)
+            B, W = self._batch, self._nm.size(1)
             if inputs is None or inputs is getattr(self, "_last_inputs", None):
                 data = self._last_data
             else:
@@ -890,45 +929,47 @@ class TensorCircuit(nn.Module):
             ls = int(bool(logspace_flows))
             reset = NEG_INF if logspace_flows else 0.0
             if self.debug_poison:               # rows outside the reset ranges must be rewritten by direct stores
-                _fill(self.node_flows, float("nan"))
+                _fill(self._nf, float("nan"))
             # the partial reset is only valid while every depth that was counted as "stores flows directly" does so
-            rkey = (B, self._launch_cfg())
+            rkey = (W, self._launch_cfg())
             if getattr(self, "_reset_key", None) != rkey:            # (a hundred depths: decided once per configuration)
                 self._reset_key = rkey
-                self._reset_partial = (B % 8 == 0 and not self._reference_compat
+                self._reset_partial = (not self._reference_compat
                                        and all(self._fusion_on(gi, True) for gi in self._fused))
             ranges = self._flow_reset_ranges if self._reset_partial else None
             if ranges is None:
-                _fill(self.node_flows, reset)
+                _fill(self._nf, reset)
             else:                                            # every other row is rewritten by a direct store
                 for a0, a1 in ranges:
-                    _fill(self.node_flows[a0:a1], reset)
+                    _fill(self._nf[a0:a1], reset)
             if self._eflow_mode != ls or self._reference_compat:
                 # dummy / parentless element rows: -inf in log space, 0 linearly (`reference_compat`: the buffer is
                 # cleared once per pass, as the reference does, and rows without a writer keep an earlier depth's flow)
-                _fill(self.element_flows, NEG_INF if logspace_flows else 0.0)
+                _fill(self._ef, NEG_INF if logspace_flows else 0.0)
                 self._eflow_mode = ls
 
             if compute_param_flows:                          # decay (or clear) the accumulators and the flow total first
                 self.init_param_flows(flows_memory=flows_memory)
             r0, r1 = self._root_node_range
-            if ll_weights is None:
-                _lib.call("pcx_set_root_flows", self.node_flows, None, r0, r1 - r0, B, ls)
-                if compute_param_flows:
-                    self._cum_flow_host += (r1 - r0) * B
-            else:
-                w = ll_weights.to(self.device, torch.float32)
+            w = ll_weights
+            if w is not None:
+                w = w.to(self.device, torch.float32)
                 w = w.unsqueeze(0) if w.dim() == 1 else w
                 assert w.size(0) == self.num_root_nodes and w.size(1) == B
-                w = w.contiguous()
-                _lib.call("pcx_set_root_flows", self.node_flows, w, r0, r1 - r0, B, ls)
                 if compute_param_flows:
                     s = w.sum(dtype=torch.float64)
                     self._cum_flow_dev = s if self._cum_flow_dev is None else self._cum_flow_dev + s
+            elif compute_param_flows:
+                self._cum_flow_host += (r1 - r0) * B
+            if W != B:                                        # padding columns carry no flow
+                full = torch.zeros(r1 - r0, W, device=self.device)
+                full[:, :B] = 1.0 if w is None else w
+                w = full
+            _lib.call("pcx_set_root_flows", self._nf, None if w is None else w.contiguous(), r0, r1 - r0, W, ls)
 
             if _lib.sum_mode() != 0:
                 self._packer.refresh(self.params.data)
-            key = ("bk", B, bool(compute_param_flows), ls, self._launch_cfg(), self.params.data_ptr(),
+            key = ("bk", W, bool(compute_param_flows), ls, self._launch_cfg(), self.params.data_ptr(),
                    self.param_flows.data_ptr() if compute_param_flows else 0)
             self._batched_par_pending = self._bk_par_pending.get(key, False)
             with self._nvtx("pcx backward: inner layers"):
@@ -945,12 +986,12 @@ class TensorCircuit(nn.Module):
                     self._side_stream.wait_stream(cur)
                     with torch.cuda.stream(self._side_stream):
                         for layer in self.input_layer_group:
-                            layer.backward(data, self.node_flows, self.node_mars, logspace_flows=bool(logspace_flows))
+                            layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
                     self._launch_batched_par(logspace_flows)
                     cur.wait_stream(self._side_stream)
                 else:
                     for layer in self.input_layer_group:
-                        layer.backward(data, self.node_flows, self.node_mars, logspace_flows=bool(logspace_flows))
+                        layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
                     self._start_early_flow_sync()
                     if self._batched_par_pending:
                         self._launch_batched_par(logspace_flows)
@@ -1117,14 +1158,14 @@ class TensorCircuit(nn.Module):
                 self._tdp = t
             if self.param_flows is None:
                 self.init_param_flows()
-            saved = (self.node_mars, self.element_mars, self.node_flows, self.element_flows, self._eflow_mode)
-            self.node_mars, self.element_mars, self.node_flows, self.element_flows = t["nm"], t["em"], t["nf"], t["ef"]
+            saved = (self._nm, self._em, self._nf, self._ef, self._eflow_mode)
+            self._nm, self._em, self._nf, self._ef = t["nm"], t["em"], t["nf"], t["ef"]
             try:
-                _fill(self.node_flows, 0.0)
-                _fill(self.element_flows, 0.0)
+                _fill(self._nf, 0.0)
+                _fill(self._ef, 0.0)
                 t["w"].fill_(float(scale) / COLS)
                 r0, r1 = self._root_node_range
-                _lib.call("pcx_set_root_flows", self.node_flows, t["w"], r0, r1 - r0, COLS, 0)
+                _lib.call("pcx_set_root_flows", self._nf, t["w"], r0, r1 - r0, COLS, 0)
                 if _lib.sum_mode() != 0:
                     self._packer.refresh(self.params.data)
                 key = ("bk-tdp", COLS, bool(update_pflow), 0, self._launch_cfg(), self.params.data_ptr(),
@@ -1134,12 +1175,12 @@ class TensorCircuit(nn.Module):
                 self._bk_par_pending[key] = self._batched_par_pending
                 if update_pflow and self._batched_par_pending:
                     self._launch_batched_par(False)
-                td = self.node_flows.sum(dim=1)
+                td = self._nf.sum(dim=1)
                 if update_pflow:
                     for layer in self.input_layer_group:
                         layer.add_missing_flows(td, scale=1.0)       # `td` already carries the scale
             finally:
-                self.node_mars, self.element_mars, self.node_flows, self.element_flows, self._eflow_mode = saved
+                self._nm, self._em, self._nf, self._ef, self._eflow_mode = saved
         return td
 
     @_in_own_mode
@@ -1274,7 +1315,7 @@ class TensorCircuit(nn.Module):
         """With ``debug_poison`` on, the value buffer (and, after a backward pass, the flow buffer) was NaN before the
         pass: a NaN that is still there marks a row no kernel wrote — a tile skipped by a grid computation, a
         wrong range.  Raises with the number of such values and the first rows."""
-        bufs = [("node_mars", self.node_mars)] + ([("node_flows", self.node_flows)] if backward else [])
+        bufs = [("node_mars", self._nm)] + ([("node_flows", self._nf)] if backward else [])
         for name, buf in bufs:
             bad = torch.isnan(buf[self.num_dummy_nodes:])
             if bool(bad.any()):
@@ -1368,7 +1409,7 @@ class TensorCircuit(nn.Module):
         if ns.is_sum() or ns.is_input():
             return self.node_mars[s:e, :].detach()
         gi = self._prod_layer_of(ns)
-        self.inner_layer_groups[gi].forward(self.node_mars, self.element_mars)
+        self.inner_layer_groups[gi].forward(self._nm, self._em)
         return self.element_mars[s:e, :].detach()
 
     def get_node_flows(self, ns, **kwargs):
@@ -1376,9 +1417,9 @@ class TensorCircuit(nn.Module):
         if ns.is_sum() or ns.is_input():
             return self.node_flows[s:e, :].detach()
         gi = self._prod_layer_of(ns)
-        self.inner_layer_groups[gi].forward(self.node_mars, self.element_mars, _for_backward=True)
+        self.inner_layer_groups[gi].forward(self._nm, self._em, _for_backward=True)
         self._reset_parentless(gi, self._run_params.get("logspace_flows", True))
-        self.inner_layer_groups[gi + 1].backward(self.node_flows, self.element_flows, self.node_mars, self.element_mars,
+        self.inner_layer_groups[gi + 1].backward(self._nf, self._ef, self._nm, self._em,
                                                  self.params.data, param_flows=None,
                                                  logspace_flows=self._run_params.get("logspace_flows", True))
         return self.element_flows[s:e, :].detach()
