@@ -63,6 +63,12 @@ int pcx_exp_f32(float* p, int64_t n, void* stream);
 int pcx_load_inputs(int32_t* data, const void* x, int elsize, int64_t B, int64_t V, int64_t stride_b,
                     int64_t stride_v, int64_t W, void* stream);
 
+/* Weights of the root flows, w[r, b] for b < W (0 where b >= B): grad[b * stride_b + r * stride_r], or 1 where grad is
+ * NULL; with `normalise`, grad / sum(grad) * B (model/tensorcircuit.py:28-41).  total (may be NULL): their sum is
+ * written to it, or added with `accumulate`. */
+int pcx_root_weights(float* w, const float* grad, int64_t stride_b, int64_t stride_r, int B, int num_roots, int W,
+                     int normalise, double* total, int accumulate, void* stream);
+
 /* node_flows[root rows, b] = w (linear) or log w (log space), w = weights ? weights[r*B+b] : 1
  * (model/tensorcircuit.py:537-552). */
 int pcx_set_root_flows(float* node_flows, const float* weights, int64_t root_start, int64_t num_roots,

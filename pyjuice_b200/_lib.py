@@ -28,6 +28,7 @@ SIGNATURES = {
     "pcx_scale_f32": [P, L, F],
     "pcx_exp_f32": [P, L],
     "pcx_load_inputs": [P, P, I, L, L, L, L, L],
+    "pcx_root_weights": [P, P, L, L, I, I, I, I, P, I],
     "pcx_set_root_flows": [P, P, L, L, I, I],
     "pcx_input_cat_fwd": [P, P, P, I, P, P, P, I, L, L, I],
     "pcx_input_cat_bwd": [P, P, P, I, P, P, P, I, L, L, I, I],
@@ -147,36 +148,40 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)      # absent from builds without CUDA
+
+
 def call(name: str, *args) -> None:
     """Invoke one entry point; tensors are passed as device pointers.  The launch goes to the device of the first
     tensor argument, on torch's current stream OF THAT DEVICE (which need not be the current device)."""
-    lib = load()
+    lib = _lib if _lib is not None else load()
     conv = []
     dev = None
     for a in args:
         if isinstance(a, torch.Tensor):
-            if not a.is_cuda:
-                raise PcxError(f"{name}: tensor argument is not on a CUDA device (no CPU path exists)")
             if dev is None:
                 dev = a.device
+            if not a.is_cuda:
+                raise PcxError(f"{name}: tensor argument is not on a CUDA device (no CPU path exists)")
             conv.append(a.data_ptr())
-        elif a is None:
-            conv.append(None)
         else:
             conv.append(a)
     global COUNT
     COUNT += 1
     _sync_mode(lib)
-    if dev is not None and dev.index != torch.cuda.current_device():
+    if dev is not None and dev.index != torch._C._cuda_getDevice():
         with torch.cuda.device(dev):             # the C side reads per-device state (SM count, built-in scratch)
             rc = _invoke(lib, name, conv, args, dev)
+    elif PROFILE is None:
+        rc = getattr(lib, name)(*conv, _raw_stream(dev.index if dev is not None else torch._C._cuda_getDevice()))
     else:
         rc = _invoke(lib, name, conv, args, dev)
+    if rc == 0:
+        return
     if rc == -2 and name == "pcx_sum_fwd_noalloc":
         raise PcxError(f"{name}: the table needs more pre-split parameter tiles than the library's built-in scratch "
                        "holds (256 tiles of 32 KB); use the packed entry points with a caller-owned buffer instead")
-    if rc != 0:
-        raise PcxError(f"{name} failed with status {rc}")
+    raise PcxError(f"{name} failed with status {rc}")
 
 
 def _invoke(lib, name, conv, args, dev) -> int:

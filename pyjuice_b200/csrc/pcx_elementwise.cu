@@ -45,6 +45,42 @@ __global__ void root_flows_kernel(float* __restrict__ node_flows, const float* _
     node_flows[root_start + i] = logspace ? logf(w) : w;              // root rows are contiguous: [num_roots, B]
 }
 
+// Weights of the root flows from the gradient of the likelihoods, and their total: one block, since it is a handful of
+// values per sample (it takes the place of five tensor operations, 25 us of host time per backward pass).
+__global__ void __launch_bounds__(1024)
+root_weights_kernel(float* __restrict__ w, const float* __restrict__ grad, int64_t stride_b, int64_t stride_r, int B,
+                    int n_roots, int W, int normalise, double* __restrict__ total, int accumulate) {
+    __shared__ double s_part[32];
+    __shared__ double s_sum;
+    double part = 0.0;
+    if (grad != nullptr) {
+        for (int i = threadIdx.x; i < n_roots * B; i += 1024) {
+            const int r = i / B, b = i - r * B;
+            part += (double)grad[b * stride_b + r * stride_r];
+        }
+    } else {
+        for (int i = threadIdx.x; i < n_roots * B; i += 1024) part += 1.0;
+    }
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = part;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double t = s_part[threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) s_sum = t;
+    }
+    __syncthreads();
+    const double scale = normalise ? (double)B / s_sum : 1.0;
+    for (int i = threadIdx.x; i < n_roots * W; i += 1024) {
+        const int r = i / W, b = i - r * W;
+        w[i] = b < B ? (grad != nullptr ? (float)((double)grad[b * stride_b + r * stride_r] * scale) : 1.0f) : 0.0f;
+    }
+    if (threadIdx.x == 0 && total != nullptr) {
+        const double t = s_sum * scale;
+        *total = accumulate ? *total + t : t;
+    }
+}
+
 // The batch, [B, V] in the caller's integer type, as [V, W] int32: 32 x 32 tiles through shared memory, so that both
 // sides are read and written in whole lines (a [784, 512] batch: 3 us, and the leaf kernels that read the result have
 // one element type and 16-byte loads of four categories).
@@ -524,6 +560,15 @@ int pcx_load_inputs(int32_t* data, const void* x, int elsize, int64_t B, int64_t
     if (W < B || pcx_cdiv(V, 32) > 65535) return -1;
     dim3 grid((unsigned)pcx_cdiv(W, 32), (unsigned)pcx_cdiv(V, 32));
     load_inputs_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(data, x, elsize, B, V, stride_b, stride_v, W);
+    PCX_LAUNCH_CHECK();
+    return 0;
+}
+
+int pcx_root_weights(float* w, const float* grad, int64_t stride_b, int64_t stride_r, int B, int num_roots, int W,
+                     int normalise, double* total, int accumulate, void* stream) {
+    if (B <= 0 || num_roots <= 0) return 0;
+    if (W < B || (int64_t)num_roots * W > INT32_MAX) return -1;
+    root_weights_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(w, grad, stride_b, stride_r, B, num_roots, W, normalise, total, accumulate);
     PCX_LAUNCH_CHECK();
     return 0;
 }

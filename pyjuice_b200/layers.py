@@ -120,10 +120,14 @@ class ParamPacker:
             self._sm_jobs = None
         return entry["buf"]
 
-    def refresh(self, params: torch.Tensor):
-        stamp = (params.data_ptr(), params._version, self._epoch)
-        if stamp == self._stamp or not (self.entries or self.sm_entries):
-            return
+    def stale(self, params: torch.Tensor) -> bool:
+        """Whether the tiles lag behind ``params``."""
+        return bool(self.entries or self.sm_entries) and (params.data_ptr(), params._version, self._epoch) != self._stamp
+
+    def mark(self, params: torch.Tensor):
+        self._stamp = (params.data_ptr(), params._version, self._epoch)
+
+    def launch(self, params: torch.Tensor):
         if self.entries:
             if getattr(self, "_jobs", None) is None:
                 self._jobs = self._job_table()
@@ -134,7 +138,11 @@ class ParamPacker:
                 self._sm_jobs = self._sm_job_table()
             jobs, n_jobs, n_vec = self._sm_jobs
             _lib.call("pcx_pack_sm_jobs", jobs, n_jobs, n_vec, params)
-        self._stamp = stamp
+
+    def refresh(self, params: torch.Tensor):
+        if self.stale(params):
+            self.launch(params)
+            self.mark(params)
 
     def _sm_job_table(self):
         """Device array of PcxSmPackJob records (include/pcx_b200.h), one per sample-major table."""
@@ -214,6 +222,13 @@ class InputLayer(Layer, nn.Module):
         self._arena_zero = False                 # True while the [row, category] flow accumulators are known to be all zero
         self.param_flows = None
         self._dev = {}
+
+    def __setattr__(self, name, value):
+        # bookkeeping of a pass: plain private values skip `nn.Module`'s search through its tables
+        if name[0] == "_" and not isinstance(value, (nn.Module, nn.Parameter)):
+            object.__setattr__(self, name, value)
+        else:
+            nn.Module.__setattr__(self, name, value)
 
     def is_input(self):
         return True
@@ -325,14 +340,28 @@ class InputLayer(Layer, nn.Module):
         node_mars, = _rows(node_mars)
         B = node_mars.size(1)
         data = _pad_data(data, B)
+        stale = self._shadow_stale(B)
+        self._launch_forward(data, node_mars, stale)
+        if stale:
+            self._mark_shadow()
+
+    def _shadow_stamp(self):
+        return (self.params.data_ptr(), self.params._version, self._param_epoch)
+
+    def _shadow_stale(self, B: int) -> bool:
+        return self._shadow_ok(B) and self._shadow["stamp"] != self._shadow_stamp()
+
+    def _mark_shadow(self):
+        self._shadow["stamp"] = self._shadow_stamp()
+
+    def _launch_forward(self, data: torch.Tensor, node_mars: torch.Tensor, stale: bool):
+        B = node_mars.size(1)
         if self._shadow_ok(B):
             sh = self._shadow
-            stamp = (self.params.data_ptr(), self.params._version, self._param_epoch)
             if sh["logp"] is None:
                 sh["logp"] = torch.empty(sh["R"] * sh["C"], dtype=torch.float32, device=self.device)
-            if sh["stamp"] != stamp:                        # parameters changed: transpose and take logarithms once
+            if stale:                                       # parameters changed: transpose and take logarithms once
                 _lib.call("pcx_input_cat_shadow", sh["logp"], self.params.data, sh["R"], sh["C"])
-                sh["stamp"] = stamp
             _lib.call("pcx_input_cat_fwd_t", node_mars, sh["logp"], data, data.element_size(), self._dev["vids"],
                       sh["prow"], sh["R"], sh["C"], self.num_nodes, self._output_ind_range[0], B)
             return
@@ -350,6 +379,19 @@ class InputLayer(Layer, nn.Module):
         node_flows, = _rows(node_flows)
         B = node_flows.size(1)
         data = _pad_data(data, B)
+        self._launch_backward(data, node_flows, logspace_flows)
+        self._mark_backward(B)
+
+    def _mark_backward(self, B: int):
+        """What the host keeps track of when a backward pass has been launched."""
+        if self._shadow_ok(B):
+            self._shadow["dirty"] = True                  # every flow lands in its source row: replicas stay as they are
+        else:
+            self._tied_folded = False                     # replica accumulators receive new flows
+            self._arena_zero = False
+
+    def _launch_backward(self, data: torch.Tensor, node_flows: torch.Tensor, logspace_flows: bool):
+        B = node_flows.size(1)
         if self._shadow_ok(B):
             sh = self._shadow
             if sh["flows"] is None:
@@ -358,10 +400,7 @@ class InputLayer(Layer, nn.Module):
             _lib.call("pcx_input_cat_bwd_t", sh["flows"], sh["touched"], node_flows, data, data.element_size(), self._dev["vids"],
                       sh["prow"], sh["R"], sh["C"], self.num_nodes, self._output_ind_range[0], B,
                       int(bool(logspace_flows)))
-            sh["dirty"] = True                            # every flow lands in its source row: replicas stay as they are
             return
-        self._tied_folded = False                         # replica accumulators receive new flows
-        self._arena_zero = False
         _lib.call("pcx_input_cat_bwd", self._param_flows, node_flows, data, data.element_size(),
                   self._dev["vids"], self._dev["s_pfids"], self._dev["node_cats"], self.max_cats,
                   self.num_nodes, self._output_ind_range[0], B, int(bool(logspace_flows)))

@@ -39,10 +39,8 @@ def _pc_model_backward_hook(grad, pc, inputs, **kwargs):
     """Autograd hook on the returned log-likelihoods: ``lls.mean().backward()`` (or any other scalar
     loss) triggers the circuit's own backward pass with per-sample weights grad / sum(grad) * B
     (model/tensorcircuit.py:28-41)."""
-    grad = grad.permute(1, 0)
-    pc.backward(inputs=inputs, ll_weights=grad / grad.sum() * grad.size(1),
-                compute_param_flows=pc._optim_hyperparams["compute_param_flows"],
-                flows_memory=pc._optim_hyperparams["flows_memory"], **kwargs)
+    pc._backward(inputs=inputs, grad=grad, compute_param_flows=pc._optim_hyperparams["compute_param_flows"],
+                 flows_memory=pc._optim_hyperparams["flows_memory"], **kwargs)
     return None
 
 
@@ -53,7 +51,7 @@ def _in_own_mode(fn):
     @functools.wraps(fn)
     def wrapper(self, *args, **kwargs):
         mode, prev = self.sum_mode, self._alg
-        if fn.__name__ in ("forward", "backward"):
+        if fn.__name__ in ("forward", "backward", "_backward"):
             name = kwargs.get("propagation_alg")
             if name is None:
                 name = self.default_propagation_alg if fn.__name__ == "forward" else "LL"
@@ -108,6 +106,14 @@ class TensorCircuit(nn.Module):
         self._cum_flow_dev = None
         self._eflow_mode = 1
         self._reference_compat = False
+
+    def __setattr__(self, name, value):
+        # `nn.Module` searches its parameter, buffer and module tables on every assignment; the bookkeeping of a pass
+        # (a dozen private plain values) needs none of that
+        if name[0] == "_" and not isinstance(value, (nn.Module, nn.Parameter)):
+            object.__setattr__(self, name, value)
+        else:
+            nn.Module.__setattr__(self, name, value)
 
     @property
     def reference_compat(self) -> bool:
@@ -332,7 +338,7 @@ class TensorCircuit(nn.Module):
         self._fusing_dev = [(start, n, torch.tensor(accs, dtype=torch.int64, device=device))
                             for start, n, accs in self._tied_sum_groups]
         self._nm = self._em = self._nf = self._ef = self.param_flows = None
-        self._data_buf = None
+        self._data_buf = self._root_mars = self._root_w = self._cum_buf = None
         if device.type == "cuda":
             self._mask_parentless_in_device_tables()
         self._setup_fusion()
@@ -491,6 +497,7 @@ class TensorCircuit(nn.Module):
         if self._nm is None or self._nm.size(1) != W:
             self._nm = torch.zeros(self.num_nodes, W, device=self.device)
             self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
+            self._root_mars = self._nm[self._root_node_range[0]:self._root_node_range[1]]
             self._nf = self._ef = None
             self._graphs = {}
         if backward and (self._nf is None or self._nf.size(1) != W):
@@ -674,6 +681,29 @@ class TensorCircuit(nn.Module):
     def forward_general_ll(self, *args, **kwargs):
         return self.forward(*args, propagation_alg="GeneralLL", **kwargs)
 
+    def _param_ptrs(self):
+        return (self.params.data_ptr(),) + tuple(layer.params.data_ptr() for layer in self.input_layer_group)
+
+    def _forward_pass(self, data: torch.Tensor, pack: bool, shadows):
+        """All launches of a forward pass on the batch in ``data``, captured as one graph.  The operand tiles of the
+        tensor-core kernels are re-packed (when the parameters changed: ``pack``) on a second stream, beside the input
+        layer: neither reads what the other writes."""
+        cur = torch.cuda.current_stream(self.device)
+        forked = pack and self.use_side_stream
+        if forked:
+            self._side_stream.wait_stream(cur)
+            with torch.cuda.stream(self._side_stream):
+                self._packer.launch(self.params.data)
+        elif pack:
+            self._packer.launch(self.params.data)
+        with self._nvtx("pcx forward: input layers"):
+            for layer, stale in zip(self.input_layer_group, shadows):
+                layer._launch_forward(data, self._nm, stale)
+        if forked:
+            cur.wait_stream(self._side_stream)
+        with self._nvtx("pcx forward: inner layers"):
+            self._forward_inner()
+
     @_in_own_mode
     def forward(self, inputs: torch.Tensor, input_layer_fn=None, cache=None, return_cache: bool = False,
                 propagation_alg: Optional[str] = None, pflow_temperature: float = 1.0, **kwargs):
@@ -685,30 +715,22 @@ class TensorCircuit(nn.Module):
         origin_inputs = inputs
         with torch.no_grad():
             B = inputs.size(0)
-            data = self._prepare_inputs(inputs)
             self._ensure_buffers(B)
             W = self._nm.size(1)
+            data = self._data_buf = self._prepare_inputs(inputs, out=self._data_buf)
+            self._last_inputs = origin_inputs
             if self.debug_poison:               # every row must be rewritten by the layer that owns it
                 _fill(self._nm[self.num_dummy_nodes:], float("nan"))
-            self._last_data, self._last_inputs = data, origin_inputs
-            # the operand tiles of the tensor-core kernels are re-packed (when the parameters changed) on a second
-            # stream, beside the input layer: neither reads what the other writes
-            cur = torch.cuda.current_stream(self.device)
-            forked = _lib.sum_mode() != 0 and self.use_side_stream
-            if forked:
-                self._side_stream.wait_stream(cur)
-                with torch.cuda.stream(self._side_stream):
-                    self._packer.refresh(self.params.data)   # outside any graph capture
-            elif _lib.sum_mode() != 0:
-                self._packer.refresh(self.params.data)
-            with self._nvtx("pcx forward: input layers"):
-                for layer in self.input_layer_group:
-                    layer.forward(data, self._nm)
-            if forked:
-                cur.wait_stream(self._side_stream)
-            with self._nvtx("pcx forward: inner layers"):
-                self._run_inner(("fw", W, self._launch_cfg(), self.params.data_ptr()), self._forward_inner)
-            lls = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t().clone()
+            pack = _lib.sum_mode() != 0 and self._packer.stale(self.params.data)
+            shadows = tuple(layer._shadow_stale(W) for layer in self.input_layer_group)
+            key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
+            self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
+            if pack:
+                self._packer.mark(self.params.data)
+            for layer, stale in zip(self.input_layer_group, shadows):
+                if stale:
+                    layer._mark_shadow()
+            lls = self._root_mars[:, :B].t().clone()
         if torch.is_grad_enabled():
             lls.requires_grad = True
             lls.register_hook(partial(_pc_model_backward_hook, pc=self, inputs=origin_inputs, **self._alg_kwargs()))
@@ -916,86 +938,115 @@ class TensorCircuit(nn.Module):
         _unsupported(input_layer_fn=input_layer_fn is not None, cache=cache is not None, return_cache=return_cache,
                      negate_pflows=negate_pflows, pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6,
                      missing_mask=kwargs.get("missing_mask") is not None)
+        w = ll_weights
+        if w is not None:
+            assert self._nm is not None, "Should run forward path first."
+            w = w.to(self.device, torch.float32)
+            w = w.unsqueeze(0) if w.dim() == 1 else w
+            assert w.size(0) == self.num_root_nodes and w.size(1) == self._batch
+        self._backward_pass(inputs, w, False, compute_param_flows, flows_memory, propagation_alg, logspace_flows)
+        return None
+
+    @_in_own_mode
+    def _backward(self, inputs, grad, compute_param_flows, flows_memory, propagation_alg: str = "LL", **kwargs):
+        """`backward` with the per-sample weights ``grad / sum(grad) * B`` of an autograd gradient ``[B, num_roots]``."""
+        if grad.dtype != torch.float32:
+            grad = grad.float()
+        self._backward_pass(inputs, grad.permute(1, 0), True, compute_param_flows, flows_memory, propagation_alg, True)
+
+    def _backward_pass(self, inputs, w, normalise: bool, compute_param_flows: bool, flows_memory: float,
+                       propagation_alg: str, logspace_flows: bool):
+        """``w``: ``[num_roots, B]`` weights of the root flows (any strides), or None for ones."""
         assert self._nm is not None and self._em is not None, "Should run forward path first."
         self._run_params = dict(logspace_flows=logspace_flows, propagation_alg=propagation_alg)
         with torch.no_grad():
             B, W = self._batch, self._nm.size(1)
-            if inputs is None or inputs is getattr(self, "_last_inputs", None):
-                data = self._last_data
+            own = inputs is None or inputs is getattr(self, "_last_inputs", None)
+            if own:
+                data = self._data_buf
             else:
                 assert inputs.dim() == 2 and inputs.size(0) == B
                 data = self._prepare_inputs(inputs)
             self._ensure_buffers(B, backward=True)
             ls = int(bool(logspace_flows))
-            reset = NEG_INF if logspace_flows else 0.0
             if self.debug_poison:               # rows outside the reset ranges must be rewritten by direct stores
                 _fill(self._nf, float("nan"))
-            # the partial reset is only valid while every depth that was counted as "stores flows directly" does so
-            rkey = (W, self._launch_cfg())
-            if getattr(self, "_reset_key", None) != rkey:            # (a hundred depths: decided once per configuration)
-                self._reset_key = rkey
-                self._reset_partial = (not self._reference_compat
-                                       and all(self._fusion_on(gi, True) for gi in self._fused))
-            ranges = self._flow_reset_ranges if self._reset_partial else None
-            if ranges is None:
-                _fill(self._nf, reset)
-            else:                                            # every other row is rewritten by a direct store
-                for a0, a1 in ranges:
-                    _fill(self._nf[a0:a1], reset)
             if self._eflow_mode != ls or self._reference_compat:
                 # dummy / parentless element rows: -inf in log space, 0 linearly (`reference_compat`: the buffer is
                 # cleared once per pass, as the reference does, and rows without a writer keep an earlier depth's flow)
                 _fill(self._ef, NEG_INF if logspace_flows else 0.0)
                 self._eflow_mode = ls
-
             if compute_param_flows:                          # decay (or clear) the accumulators and the flow total first
                 self.init_param_flows(flows_memory=flows_memory)
             r0, r1 = self._root_node_range
-            w = ll_weights
-            if w is not None:
-                w = w.to(self.device, torch.float32)
-                w = w.unsqueeze(0) if w.dim() == 1 else w
-                assert w.size(0) == self.num_root_nodes and w.size(1) == B
-                if compute_param_flows:
-                    s = w.sum(dtype=torch.float64)
-                    self._cum_flow_dev = s if self._cum_flow_dev is None else self._cum_flow_dev + s
-            elif compute_param_flows:
-                self._cum_flow_host += (r1 - r0) * B
-            if W != B:                                        # padding columns carry no flow
-                full = torch.zeros(r1 - r0, W, device=self.device)
-                full[:, :B] = 1.0 if w is None else w
-                w = full
-            _lib.call("pcx_set_root_flows", self._nf, None if w is None else w.contiguous(), r0, r1 - r0, W, ls)
+            if self._root_w is None or self._root_w.size(1) != W:
+                self._root_w = torch.empty(r1 - r0, W, device=self.device)
+                self._graphs = {k: g for k, g in self._graphs.items() if k[0] != "bk"}
+            total = None
+            if compute_param_flows:
+                if w is None:
+                    self._cum_flow_host += (r1 - r0) * B
+                else:
+                    if self._cum_buf is None:
+                        self._cum_buf = torch.zeros((), dtype=torch.float64, device=self.device)
+                    total = self._cum_buf
+            _lib.call("pcx_root_weights", self._root_w, w, 0 if w is None else w.stride(1), 0 if w is None else w.stride(0),
+                      B, r1 - r0, W, int(normalise), total, int(self._cum_flow_dev is not None))
+            if total is not None:
+                self._cum_flow_dev = total
 
             if _lib.sum_mode() != 0:
                 self._packer.refresh(self.params.data)
-            key = ("bk", W, bool(compute_param_flows), ls, self._launch_cfg(), self.params.data_ptr(),
-                   self.param_flows.data_ptr() if compute_param_flows else 0)
+            # The parameter flows of the sum layers and of the input layer close the pass.  They belong to the captured
+            # pass too, unless data-parallel ranks overlap them with the all-reduce, or the leaves see another batch.
+            tail = compute_param_flows and own and not self._overlap_ready()
+            key = ("bk", W, bool(compute_param_flows), tail, ls, self._launch_cfg(), self._param_ptrs(),
+                   self.param_flows.data_ptr() if compute_param_flows else 0, data.data_ptr() if tail else 0)
             self._batched_par_pending = self._bk_par_pending.get(key, False)
-            with self._nvtx("pcx backward: inner layers"):
-                self._run_inner(key, partial(self._backward_inner, compute_param_flows, bool(logspace_flows)))
+            with self._nvtx("pcx backward"):
+                self._run_inner(key, partial(self._backward_sweep, data if tail else None, compute_param_flows,
+                                             bool(logspace_flows)))
             self._bk_par_pending[key] = self._batched_par_pending
-
-            if compute_param_flows:
-                # The parameter flows of the sum layers and of the input layer are independent once every node flow
-                # exists.  One rank: both run together, on two streams.  Data-parallel ranks with the overlapped
-                # all-reduce: the input layer first, then the all-reduce of its flows (the larger part of the
-                # arena) beside the sum layers' parameter-flow kernel.
-                cur = torch.cuda.current_stream(self.device)
-                if self._batched_par_pending and self.use_side_stream and not self._overlap_ready():
-                    self._side_stream.wait_stream(cur)
-                    with torch.cuda.stream(self._side_stream):
-                        for layer in self.input_layer_group:
-                            layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
+            if tail:
+                for layer in self.input_layer_group:
+                    layer._mark_backward(W)
+            elif compute_param_flows:
+                # the input layer first, then the all-reduce of its flows (the larger part of the arena) beside the sum
+                # layers' parameter-flow kernel
+                for layer in self.input_layer_group:
+                    layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
+                self._start_early_flow_sync()
+                if self._batched_par_pending:
                     self._launch_batched_par(logspace_flows)
-                    cur.wait_stream(self._side_stream)
-                else:
-                    for layer in self.input_layer_group:
-                        layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
-                    self._start_early_flow_sync()
-                    if self._batched_par_pending:
-                        self._launch_batched_par(logspace_flows)
-        return None
+
+    def _backward_sweep(self, data, compute_param_flows: bool, logspace_flows: bool):
+        """All launches of a backward pass from the root weights in ``_root_w``; ``data``: with the parameter flows
+        that close the pass."""
+        W = self._nf.size(1)
+        # the partial reset is only valid while every depth that was counted as "stores flows directly" does so
+        partial_reset = not self._reference_compat and all(self._fusion_on(gi, True) for gi in self._fused)
+        ranges = self._flow_reset_ranges if partial_reset else None
+        reset = NEG_INF if logspace_flows else 0.0
+        for a0, a1 in ([(0, self.num_nodes)] if ranges is None else ranges):
+            _fill(self._nf[a0:a1], reset)                    # every other row is rewritten by a direct store
+        r0, r1 = self._root_node_range
+        _lib.call("pcx_set_root_flows", self._nf, self._root_w, r0, r1 - r0, W, int(logspace_flows))
+        self._backward_inner(compute_param_flows, logspace_flows)
+        if data is None:
+            return
+        cur = torch.cuda.current_stream(self.device)
+        if self._batched_par_pending and self.use_side_stream:
+            self._side_stream.wait_stream(cur)
+            with torch.cuda.stream(self._side_stream):
+                for layer in self.input_layer_group:
+                    layer._launch_backward(data, self._nf, logspace_flows)
+            self._launch_batched_par(logspace_flows)
+            cur.wait_stream(self._side_stream)
+        else:
+            for layer in self.input_layer_group:
+                layer._launch_backward(data, self._nf, logspace_flows)
+            if self._batched_par_pending:
+                self._launch_batched_par(logspace_flows)
 
     # ---- data-parallel flow synchronisation overlapped with the tail of the step ---------------------------------
     def enable_flow_sync_overlap(self, group=None, dtype: Optional[torch.dtype] = None):
@@ -1183,6 +1234,10 @@ class TensorCircuit(nn.Module):
                 self._nm, self._em, self._nf, self._ef, self._eflow_mode = saved
         return td
 
+    # Below this many sum parameters the update of either kind takes a few microseconds, less than the host spends on
+    # sending work to a second stream and joining it again (35 us).
+    _EM_FORK_PARAMS = 1 << 21
+
     @_in_own_mode
     def mini_batch_em(self, step_size: float, pseudocount: float = 0.0, keep_zero_params: bool = False,
                       step_size_rescaling: bool = False, **kwargs):
@@ -1223,12 +1278,12 @@ class TensorCircuit(nn.Module):
                     layer.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
 
             # sum parameters and input-layer parameters are disjoint
-            cur = torch.cuda.current_stream(self.device)
             if getattr(self, "_late_sync", None) is not None:
                 input_update()                              # beside the all-reduce of the sum-layer flows
                 self._finish_late_sync()
                 sum_update()
-            elif self.use_side_stream:                      # the two updates run on two streams
+            elif self.use_side_stream and self.num_sum_params >= self._EM_FORK_PARAMS:    # on two streams
+                cur = torch.cuda.current_stream(self.device)
                 self._side_stream.wait_stream(cur)
                 with torch.cuda.stream(self._side_stream):
                     sum_update()
