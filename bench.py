@@ -184,7 +184,11 @@ def circuit_stats(pc, B):
 def family_of(name: str) -> str:
     """Launch family of a C-ABI entry point: the variants of one operator (product layer folded in, pre-split
     parameter tiles, all layers in one launch, built-in scratch) count as that operator."""
-    if name.startswith("pcx_sum_chain"):                  # the dataflow launch: forward or element flows of many layers
+    if name == "pcx_column_par":
+        return "pcx_sum_bwd_par"
+    if name == "pcx_column_pack":
+        return "pcx_pack_sum_params"
+    if name.startswith(("pcx_sum_chain", "pcx_column_run")):     # one launch: forward or element flows of many layers
         return "pcx_sum_fwd" if name.endswith("_fwd") else "pcx_sum_bwd_ele"
     if name.endswith("_dense2_prep"):                     # operand pre-pass of the wide dense kernels (fwd and element flows)
         return "pcx_sum_dense_prep"

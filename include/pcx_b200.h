@@ -463,6 +463,59 @@ int pcx_input_cat_missing(float* param_flows, const float* params, const float* 
                           const int32_t* source_nids, const int32_t* s_pids, const int32_t* s_pfids,
                           const int32_t* node_cats, int64_t n_source, float scale, void* stream);
 
+/* ---- column program: all levels of a circuit of small node blocks in one launch --------------------------------
+ * A cluster of `cluster` CTAs owns 8 * nt * tiles columns (nt 1 or 2; tiles a power of two) of the value buffers ([rows, W], W % 8 == 0) and walks the levels; a level is a
+ * list of tasks without dependencies among them.  Takes the place of the per-layer launches of
+ * model/tensorcircuit.py:377-441 (forward) and 556-674 (backward). */
+typedef struct {
+    int32_t kid_off;    /* first entry of the task in `kids` */
+    int32_t n_k;        /* MMA: 16-deep steps of the contraction; SIMT: its depth; product task: parent products */
+    int32_t n_kids;     /* forward: children per element; -1: the operand rows are stored element values */
+    int32_t width;      /* int32 per entry.  MMA forward: child rows [, row of the stored element value]; SIMT forward:
+                         * parameter offset, child rows [, row]; MMA element flows: parent row; SIMT: parameter offset,
+                         * parent row; product task: parent element row */
+    int32_t strip_off;  /* first record in `strips`; product task: the node row */
+    int32_t n_rows;     /* MMA: strips of 16 rows (at most 2); SIMT: rows (1, 2, 4, 8 or 16); product task: rows */
+    int32_t par_off;    /* MMA: first parameter fragment, [step][strip] */
+    int32_t kind;       /* 0 MMA, 1 SIMT, 2 SIMT with the contraction split over a CTA (one row), 3 product task */
+    int32_t sk, sr;     /* SIMT: parameter stride per child and per row; product task: sk = add to the row's flow */
+    int32_t lg_entry;   /* SIMT: 3 when an entry stands for eight consecutive children, 0 for one */
+    int32_t pad;
+} PcxColTask;
+/* strips: int32 x 4.  Forward: output row.  Element flows: element row, then by flag (the last word) -1: row of the stored
+ * value; 0 / 1: two child rows (the second may be 0); 2 / 3: offset of the child rows in `kids`, their number.  Flags 1 and
+ * 3: the flow goes to the children's rows, else to element_flows.
+ * wide > 0: ONE level over the whole machine (cluster 1, nt 4, tiles = all column tiles of the row): 1 any tasks, 2 MMA
+ * tasks of at most 32 operand entries and two children per element (operands staged through shared memory), 3 (element flows) product tasks only.
+ * levels: int32 x 4: first warp task, how many, first split task, how many.  terms: 3 (bf16 hi / lo) or 1. */
+int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,
+                   const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
+                   const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int tiles, int cluster,
+                   int wide, int logspace, int terms, void* stream);
+/* Clusters of `cluster` CTAs of that launch that the current device can hold at a time. */
+int pcx_column_clusters(int cluster);
+/* Parameter fragments (1 KB each: 16 rows x 16 children, bf16 high parts then low parts in the order of the A operand of
+ * mma.m16n8k16).  bases: int32 x 4: parameter of (row 0, child 0), stride per row, stride per child, unused. */
+int pcx_column_pack(void* frags, const int32_t* bases, int64_t n, const float* params, void* stream);
+
+/* Parameter flows of all levels.  kind 0: tensor-core tiles of up to 32 nodes (strips of 16 from row0 and row1) x n_k
+ * (at most 2) steps of 16 edges; kind 1: fp32 tiles of n_strips nodes (1, 2, 4, 8 or 16) x n_k
+ * edges; kinds 2 and 3: as kind 0 for elements of at most two children (or stored values), up to 2 x 2 / 4 x 4 strips x
+ * steps, operands staged through shared memory.  offsets: int32 x 2: (parameter,
+ * flow) of the first (node, edge) of every (step, strip) / entry; the next edge is bs further. */
+typedef struct {
+    int32_t row0, row1;
+    int32_t n_strips;
+    int32_t kid_off, n_k, n_kids, width;    /* n_kids -1: the entry is the row of a stored element value */
+    int32_t pp_off;
+    int32_t bs;
+    int32_t lg_entry;
+    int32_t row2, row3;
+} PcxColPar;
+int pcx_column_par(int kind, float* param_flows, const float* node_flows, const float* node_mars,
+                   const float* element_values, const float* params, const PcxColPar* jobs, const int32_t* kids,
+                   const int32_t* offsets, int n_jobs, int W, int logspace, int terms, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

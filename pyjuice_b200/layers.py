@@ -120,14 +120,27 @@ class ParamPacker:
             self._sm_jobs = None
         return entry["buf"]
 
-    def stale(self, params: torch.Tensor) -> bool:
+    # ``plan``: a plan of the column program; its parameter fragments then stand in for all tiles of the per-layer kernels.
+    def _stamp_of(self, params: torch.Tensor):
+        return (params.data_ptr(), params._version, self._epoch)
+
+    def stale(self, params: torch.Tensor, plan=None) -> bool:
         """Whether the tiles lag behind ``params``."""
-        return bool(self.entries or self.sm_entries) and (params.data_ptr(), params._version, self._epoch) != self._stamp
+        if plan is not None:
+            return plan.get("stamp") != self._stamp_of(params)
+        return bool(self.entries or self.sm_entries) and self._stamp_of(params) != self._stamp
 
-    def mark(self, params: torch.Tensor):
-        self._stamp = (params.data_ptr(), params._version, self._epoch)
+    def mark(self, params: torch.Tensor, plan=None):
+        if plan is not None:
+            plan["stamp"] = self._stamp_of(params)
+        else:
+            self._stamp = self._stamp_of(params)
 
-    def launch(self, params: torch.Tensor):
+    def launch(self, params: torch.Tensor, plan=None):
+        if plan is not None:
+            if plan["n_frag"]:
+                _lib.call("pcx_column_pack", plan["frags"], plan["bases"], plan["n_frag"], params)
+            return
         if self.entries:
             if getattr(self, "_jobs", None) is None:
                 self._jobs = self._job_table()
@@ -139,10 +152,10 @@ class ParamPacker:
             jobs, n_jobs, n_vec = self._sm_jobs
             _lib.call("pcx_pack_sm_jobs", jobs, n_jobs, n_vec, params)
 
-    def refresh(self, params: torch.Tensor):
-        if self.stale(params):
-            self.launch(params)
-            self.mark(params)
+    def refresh(self, params: torch.Tensor, plan=None):
+        if self.stale(params, plan):
+            self.launch(params, plan)
+            self.mark(params, plan)
 
     def _sm_job_table(self):
         """Device array of PcxSmPackJob records (include/pcx_b200.h), one per sample-major table."""

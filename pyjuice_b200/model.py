@@ -29,6 +29,7 @@ import torch.nn as nn
 from . import _lib
 from .compiler import _IdDict, compile_cum_par_flows, compile_par_update, create_node_layers
 from .layers import InputLayer, LayerGroup, ParamPacker, ProdLayer, SumLayer, _alg_of, _fill, _scale, _unsupported
+from .column import ColumnProgram, Unsupported
 from .flows import FlowArena
 from .nodes import as_bitset
 
@@ -91,7 +92,9 @@ class TensorCircuit(nn.Module):
         self._optim_hyperparams = {"compute_param_flows": True, "flows_memory": 1.0}
         self._graphs = {}
         self.use_cuda_graphs = True
+        self._column_program = None
         self.use_dataflow_launch = True       # runs of folded depths as one launch (tiles wait on counters)
+        self.use_column_program = True        # circuits of small node blocks: all levels in one launch
         self.use_side_stream = True           # independent kernels of a step share the device (two streams)
         self.debug_poison = False             # fill value / flow buffers with NaN before every pass (see `assert_no_poison`)
         self.use_nvtx = bool(os.environ.get("PCX_B200_NVTX"))     # NVTX ranges around the phases of a step (profilers)
@@ -348,6 +351,7 @@ class TensorCircuit(nn.Module):
         self._par_job_cache = {}
         self._chain_cache = {}
         self._dense_par_cache = {}
+        self._column_program = None
         self._cum_flow_dev = None
         return self
 
@@ -565,9 +569,23 @@ class TensorCircuit(nn.Module):
             return False
         return (not backward) or self._nm.size(1) % 8 == 0
 
+    def _column_plan(self):
+        """The column program's plan for the current row width, or None where the per-layer kernels run: a node block of
+        more than 64 nodes (their tables fill 128-row tensor-core tiles), fp32 or rule-based passes, `reference_compat`."""
+        if (not (self.use_column_program and self.fuse_product_layers and SumLayer.use_sample_major) or self._reference_compat
+                or self._alg[0] != 0 or _lib.sum_mode() == 0):
+            return None
+        if self._column_program is None:
+            try:
+                self._column_program = ColumnProgram(self)
+            except Unsupported:
+                self._column_program = False
+        return self._column_program.plan(self._nm.size(1)) if self._column_program else None
+
     def _launch_cfg(self):
         """Everything that changes which kernels a pass launches (part of the key of a captured graph)."""
         return (_lib.sum_mode(), self.fuse_product_layers, self.use_dataflow_launch, self.chain_tile,
+                self.use_column_program,
                 SumLayer.use_dense_kernels, SumLayer.use_wide_dense, SumLayer.use_sample_major,
                 getattr(self._packer, "grown", 0),
                 self._reference_compat, self._alg)
@@ -645,6 +663,10 @@ class TensorCircuit(nn.Module):
                   int(bool(logspace_flows)), plan["ctrl"], plan["ctrl"].numel())
 
     def _forward_inner(self):
+        plan = self._column_plan()
+        if plan is not None:
+            self._column_program.run(plan, 0, self._nm, None, None, self.params.data)
+            return
         groups = self.inner_layer_groups
         plan = self._chain_plan(self._nm.size(1), 0)
         for gi, group in enumerate(groups):
@@ -693,9 +715,9 @@ class TensorCircuit(nn.Module):
         if forked:
             self._side_stream.wait_stream(cur)
             with torch.cuda.stream(self._side_stream):
-                self._packer.launch(self.params.data)
+                self._packer.launch(self.params.data, self._column_plan())
         elif pack:
-            self._packer.launch(self.params.data)
+            self._packer.launch(self.params.data, self._column_plan())
         with self._nvtx("pcx forward: input layers"):
             for layer, stale in zip(self.input_layer_group, shadows):
                 layer._launch_forward(data, self._nm, stale)
@@ -721,12 +743,13 @@ class TensorCircuit(nn.Module):
             self._last_inputs = origin_inputs
             if self.debug_poison:               # every row must be rewritten by the layer that owns it
                 _fill(self._nm[self.num_dummy_nodes:], float("nan"))
-            pack = _lib.sum_mode() != 0 and self._packer.stale(self.params.data)
+            plan = self._column_plan()
+            pack = _lib.sum_mode() != 0 and self._packer.stale(self.params.data, plan)
             shadows = tuple(layer._shadow_stale(W) for layer in self.input_layer_group)
             key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
             self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
             if pack:
-                self._packer.mark(self.params.data)
+                self._packer.mark(self.params.data, plan)
             for layer, stale in zip(self.input_layer_group, shadows):
                 if stale:
                     layer._mark_shadow()
@@ -915,6 +938,13 @@ class TensorCircuit(nn.Module):
             cur.wait_stream(side)
         self._batched_par_pending = any_fused and pf is not None     # launched by `backward`, after this sweep
 
+    def _launch_par(self, logspace_flows: bool):
+        plan = self._column_plan()
+        if plan is None:
+            self._launch_batched_par(logspace_flows)
+        else:
+            self._column_program.param_flows(plan, self.param_flows, self._nf, self._nm, self.params.data, logspace_flows)
+
     def _launch_batched_par(self, logspace_flows: bool):
         B = self._nf.size(1)
         for fc, jobs, n_jobs, n_items, chunks_per_cta in self._par_jobs(B):
@@ -996,7 +1026,7 @@ class TensorCircuit(nn.Module):
                 self._cum_flow_dev = total
 
             if _lib.sum_mode() != 0:
-                self._packer.refresh(self.params.data)
+                self._packer.refresh(self.params.data, self._column_plan())
             # The parameter flows of the sum layers and of the input layer close the pass.  They belong to the captured
             # pass too, unless data-parallel ranks overlap them with the all-reduce, or the leaves see another batch.
             tail = compute_param_flows and own and not self._overlap_ready()
@@ -1017,21 +1047,27 @@ class TensorCircuit(nn.Module):
                     layer.backward(data, self._nf, self._nm, logspace_flows=bool(logspace_flows))
                 self._start_early_flow_sync()
                 if self._batched_par_pending:
-                    self._launch_batched_par(logspace_flows)
+                    self._launch_par(logspace_flows)
 
     def _backward_sweep(self, data, compute_param_flows: bool, logspace_flows: bool):
         """All launches of a backward pass from the root weights in ``_root_w``; ``data``: with the parameter flows
         that close the pass."""
         W = self._nf.size(1)
-        # the partial reset is only valid while every depth that was counted as "stores flows directly" does so
-        partial_reset = not self._reference_compat and all(self._fusion_on(gi, True) for gi in self._fused)
-        ranges = self._flow_reset_ranges if partial_reset else None
-        reset = NEG_INF if logspace_flows else 0.0
-        for a0, a1 in ([(0, self.num_nodes)] if ranges is None else ranges):
-            _fill(self._nf[a0:a1], reset)                    # every other row is rewritten by a direct store
         r0, r1 = self._root_node_range
-        _lib.call("pcx_set_root_flows", self._nf, self._root_w, r0, r1 - r0, W, int(logspace_flows))
-        self._backward_inner(compute_param_flows, logspace_flows)
+        plan = self._column_plan()
+        if plan is not None:                                 # the first level that touches a flow row writes it: no reset
+            _lib.call("pcx_set_root_flows", self._nf, self._root_w, r0, r1 - r0, W, int(logspace_flows))
+            self._column_program.run(plan, 1, self._nm, self._nf, self._ef, self.params.data, logspace_flows)
+            self._batched_par_pending = compute_param_flows
+        else:
+            # the partial reset is only valid while every depth that was counted as "stores flows directly" does so
+            partial_reset = not self._reference_compat and all(self._fusion_on(gi, True) for gi in self._fused)
+            ranges = self._flow_reset_ranges if partial_reset else None
+            reset = NEG_INF if logspace_flows else 0.0
+            for a0, a1 in ([(0, self.num_nodes)] if ranges is None else ranges):
+                _fill(self._nf[a0:a1], reset)                # every other row is rewritten by a direct store
+            _lib.call("pcx_set_root_flows", self._nf, self._root_w, r0, r1 - r0, W, int(logspace_flows))
+            self._backward_inner(compute_param_flows, logspace_flows)
         if data is None:
             return
         cur = torch.cuda.current_stream(self.device)
@@ -1040,13 +1076,13 @@ class TensorCircuit(nn.Module):
             with torch.cuda.stream(self._side_stream):
                 for layer in self.input_layer_group:
                     layer._launch_backward(data, self._nf, logspace_flows)
-            self._launch_batched_par(logspace_flows)
+            self._launch_par(logspace_flows)
             cur.wait_stream(self._side_stream)
         else:
             for layer in self.input_layer_group:
                 layer._launch_backward(data, self._nf, logspace_flows)
             if self._batched_par_pending:
-                self._launch_batched_par(logspace_flows)
+                self._launch_par(logspace_flows)
 
     # ---- data-parallel flow synchronisation overlapped with the tail of the step ---------------------------------
     def enable_flow_sync_overlap(self, group=None, dtype: Optional[torch.dtype] = None):
@@ -1431,6 +1467,12 @@ class TensorCircuit(nn.Module):
                     for t in list(f.get("fw", [])) + list(f.get("bk", [])):
                         if t is not None:
                             check("folded child rows", t, 1, self.num_nodes)
+        if self._column_program and self._nm is not None:
+            def report(what, at, extent, limit):
+                counts[what] = counts.get(what, 0) + 1
+                if at < 0 or at + extent > limit:
+                    errs.append(f"{what}: index range [{at}, {at} + {extent}) exceeds [0, {limit})")
+            self._column_program.check(self._column_program.plan(self._nm.size(1)), self, report)
         if errs:
             raise ValueError("index tables out of bounds: " + "; ".join(errs[:6]))
         return counts

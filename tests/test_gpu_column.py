@@ -1,0 +1,79 @@
+"""The column program (all levels of a circuit of small node blocks in one launch, wide levels on their own) against the CPU
+oracle and against the per-layer kernels, at the sizes where its pieces meet: batches around the 8-, 16- and 32-column
+tiles, node blocks on both sides of the fp32 / tensor-core line, levels wide enough for a launch of their own, products of
+one, two and many children, stored element values, block-sparse tables and shared leaves."""
+import pytest
+import torch
+
+import pyjuice_b200 as pj
+from helpers import check_against_oracle
+from pyjuice_b200.column import ColumnProgram
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _circuit(kind, latents):
+    torch.manual_seed(3)
+    import random
+    random.seed(3)
+    import numpy as np
+    S = pj.structures
+    if kind == "hclt":
+        tree = S.random_grid_spanning_tree(4, 5, np.random.default_rng(3))
+        return S.tree_to_hidden_circuit(tree, tree.center(), num_latents=latents, num_cats=7)
+    if kind == "pd":
+        return S.PD((9, 7), latents, split_points=[[3, 6], [3]], num_cats=5)
+    if kind == "rat":
+        return S.RAT_SPN(num_vars=40, num_latents=latents, depth=2, num_repetitions=5, num_cats=6)
+    return S.HMM(seq_length=9, num_latents=latents, num_emits=11, homogeneous=True)
+
+
+def _program(pc):
+    assert pc._column_plan() is not None
+    return pc._column_program
+
+
+@pytest.mark.parametrize("B", [1, 8, 31, 200, 257])
+@pytest.mark.parametrize("kind,latents", [("hclt", 8), ("hclt", 24), ("hclt", 64), ("hclt", 96), ("pd", 16), ("pd", 64),
+                                          ("rat", 32), ("rat", 8), ("hmm", 64), ("hmm", 320), ("hmm", 4)])
+def test_against_oracle(kind, latents, B):
+    pc = pj.compile(_circuit(kind, latents)).to(DEV)
+    cats = min(l.max_cats for l in pc.input_layer_group)
+    x = torch.randint(0, cats, (B, pc.num_vars), generator=torch.Generator().manual_seed(B))
+    errs = check_against_oracle(pc, x, step=0.2, pseudo=0.1)
+    _program(pc)
+    pc.validate_tables()
+    print(errs)
+
+
+@pytest.mark.parametrize("kind,latents", [("hclt", 64), ("hclt", 8), ("pd", 32), ("pd", 64), ("rat", 32), ("rat", 16)])
+@pytest.mark.parametrize("logspace", [True, False])
+@pytest.mark.parametrize("B", [40, 264])
+def test_wide_levels(kind, latents, logspace, B, monkeypatch):
+    """Every level on its own (as in circuits that fill the machine), against the oracle."""
+    monkeypatch.setattr(ColumnProgram, "WIDE_ITEMS", 1)
+    pc = pj.compile(_circuit(kind, latents)).to(DEV)
+    cats = min(l.max_cats for l in pc.input_layer_group)
+    x = torch.randint(0, cats, (B, pc.num_vars), generator=torch.Generator().manual_seed(B))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1, logspace_flows=logspace)
+    launches = [l for m in (0, 1) for l in _program(pc).plan(pc._nm.size(1))[m]["launches"] if not isinstance(l, list)]
+    assert any(l[2][3] > 0 for l in launches)
+    pc.validate_tables()
+
+
+@pytest.mark.parametrize("kind,latents", [("hclt", 32), ("pd", 64), ("rat", 8), ("hmm", 64)])
+def test_equals_the_per_layer_kernels(kind, latents):
+    pc = pj.compile(_circuit(kind, latents)).to(DEV)
+    cats = min(l.max_cats for l in pc.input_layer_group)
+    x = torch.randint(0, cats, (72, pc.num_vars), generator=torch.Generator().manual_seed(5)).to(DEV)
+    out = {}
+    for on in (False, True):
+        pc.use_column_program = on
+        pc.init_param_flows(flows_memory=0.0)
+        lls = pc(x)
+        pc.backward(x)
+        out[on] = (lls, pc.node_flows[pc.num_dummy_nodes:].exp().clone(), pc.param_flows.clone())
+    assert (out[True][0] - out[False][0]).abs().max().item() <= 1e-3
+    for a, b in zip(out[True][1:], out[False][1:]):
+        assert (a - b).norm() <= 1e-4 * b.norm()
