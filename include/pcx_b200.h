@@ -477,7 +477,8 @@ typedef struct {
     int32_t strip_off;  /* first record in `strips`; product task: the node row */
     int32_t n_rows;     /* MMA: strips of 16 rows (at most 2); SIMT: rows (1, 2, 4, 8 or 16); product task: rows */
     int32_t par_off;    /* MMA: first parameter fragment, [step][strip] */
-    int32_t kind;       /* 0 MMA, 1 SIMT, 2 SIMT with the contraction split over a CTA (one row), 3 product task */
+    int32_t kind;       /* 0 MMA, 1 SIMT, 2 SIMT with the contraction split over a CTA (one row), 3 product task, 4 MMA task for a whole CTA
+                         * (1, 2, 4, 8 or 16 strips) */
     int32_t sk, sr;     /* SIMT: parameter stride per child and per row; product task: sk = add to the row's flow */
     int32_t lg_entry;   /* SIMT: 3 when an entry stands for eight consecutive children, 0 for one */
     int32_t pad;
@@ -492,8 +493,14 @@ int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element
                    const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
                    const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int tiles, int cluster,
                    int wide, int logspace, int terms, void* stream);
-/* Clusters of `cluster` CTAs of that launch that the current device can hold at a time. */
-int pcx_column_clusters(int cluster);
+/* The same walk for circuits with large groups (tasks of kind 4: whole-CTA tasks, in a level's second list).  max_steps: the
+ * deepest such task (at most 64 steps: 1024 children).  cluster: up to 16.  At most 512 levels. */
+int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,
+                       const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
+                       const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int cluster, int max_steps,
+                       int logspace, int terms, void* stream);
+/* Clusters of `cluster` CTAs of those launches that the current device can hold at a time. */
+int pcx_column_clusters(int cluster, int big);
 /* Parameter fragments (1 KB each: 16 rows x 16 children, bf16 high parts then low parts in the order of the A operand of
  * mma.m16n8k16).  bases: int32 x 4: parameter of (row 0, child 0), stride per row, stride per child, unused. */
 int pcx_column_pack(void* frags, const int32_t* bases, int64_t n, const float* params, void* stream);

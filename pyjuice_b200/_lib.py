@@ -69,6 +69,7 @@ SIGNATURES = {
     "pcx_input_cat_bwd_t": [P, P, P, P, I, P, P, L, I, L, L, I, I],
     "pcx_input_cat_flush_t": [P, P, P, P, L, I],
     "pcx_column_run": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I],
+    "pcx_column_run_big": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I],
     "pcx_column_pack": [P, P, L, P],
     "pcx_column_par": [I, P, P, P, P, P, P, P, P, I, I, I, I],
     "pcx_sum_fwd_dense2": [P, P, P, P, P, P, I, P, P, I, P, L, L, I, I, I],
@@ -78,7 +79,7 @@ SIGNATURES = {
 }
 
 # entry points without a stream argument
-PLAIN = {"pcx_build_arch": [], "pcx_column_clusters": [I], "pcx_set_sum_mode": [I], "pcx_set_dependent_launch": [I], "pcx_set_stage_event": [P], "pcx_get_status": [], "pcx_clear_status": [],
+PLAIN = {"pcx_build_arch": [], "pcx_column_clusters": [I, I], "pcx_set_sum_mode": [I], "pcx_set_dependent_launch": [I], "pcx_set_stage_event": [P], "pcx_get_status": [], "pcx_clear_status": [],
          "pcx_packed_tile_count": [L, I, I, I, I], "pcx_dense_scratch_bytes": [I, I, I],
          "pcx_sm_packed_bytes": [L, I, I], "pcx_dense2_scratch_bytes": [I, I, I]}
 SUM_MODE = 1        # the process default of the arithmetic mode (see set_sum_mode / use_sum_mode)
@@ -209,7 +210,7 @@ def _invoke(lib, name, conv, args, dev) -> int:
     rc = getattr(lib, name)(*conv, stream)
     b.record()
     # launches over many layers serve two operators: tell them apart by their first argument (0 forward, 1 element flows)
-    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in ("pcx_sum_chain", "pcx_column_run") else name, a, b))
+    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in ("pcx_sum_chain", "pcx_column_run", "pcx_column_run_big") else name, a, b))
     return rc
 
 

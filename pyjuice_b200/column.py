@@ -12,7 +12,7 @@ import torch
 
 from . import _lib
 
-K_MMA, K_SIMT, K_SPLIT, K_PROD = 0, 1, 2, 3
+K_MMA, K_SIMT, K_SPLIT, K_PROD, K_CTA = 0, 1, 2, 3, 4
 WARPS = 16                   # per CTA of the column kernel
 TASK = np.dtype([(n, "<i4") for n in ("kid_off", "n_k", "n_kids", "width", "strip_off", "n_rows", "par_off", "kind", "sk",
                                       "sr", "lg_entry", "pad")])
@@ -54,7 +54,7 @@ class _Pool:
 class _Group:
     """Rows with one operand list.  ``blocks``: (first row, rows) of every node block; ``ops``: per operand block its first
     row(s) and size; ``par[b][o]``: parameter of (block b, operand block o), ``flow`` likewise (forward groups)."""
-    __slots__ = ("blocks", "ops", "par", "flow", "bs", "mma", "direct")
+    __slots__ = ("blocks", "ops", "par", "flow", "bs", "mma", "direct", "big", "depth")
 
 
 def _np(t):
@@ -71,12 +71,12 @@ def _prefix(row):
 class ColumnProgram:
     MAX_KIDS_FOLDED = 4          # elements of more children (shared leaves) keep their value for the backward pass
     MAX_FOLD_READS = 16          # child-row reads per element that folding may cost
-    MAX_BLOCK = 64
+    BIG_STRIPS, BIG_STEPS, BIG_MAX_STEPS = 8, 8, 64      # a group for CTA tasks: rows and depth (in 16) it has at least
 
     def __init__(self, pc):
         self.device = pc.device
         self.num_dummy = pc.num_dummy_nodes
-        self._by_width, self._rooms = {}, {}
+        self._by_width, self._choice, self._rooms, self._par = {}, {}, {}, None
         groups = pc.inner_layer_groups
         self.depths = []
         parents = np.zeros(pc.num_nodes + 1, dtype=np.int32)
@@ -87,7 +87,7 @@ class ColumnProgram:
                     c = _np(cids)
                     c = c[c != 0]
                     np.add.at(parents, (c[:, None] + j[None, :]).reshape(-1), 1)
-        self.em_rows = 0
+        self.em_rows = self.big_steps = 0
         for gi in range(0, len(groups), 2):
             self.depths.append(self._depth(pc, gi, parents))
         written = np.zeros(pc.num_nodes, dtype=bool)
@@ -108,6 +108,8 @@ class ColumnProgram:
                 written[p["row"]:p["row"] + p["size"]] = True
         if not written.all():
             raise Unsupported("a node without parents")
+        if self.big_steps and len(self.depths) * 2 > 512:
+            raise Unsupported("more levels than the CTA-task kernel lists")
         self._build_pack()
 
     # ---- tables of one depth ---------------------------------------------------------------------------------------
@@ -127,8 +129,6 @@ class ColumnProgram:
             direct = all(bool((parents[k:k + size] == 1).all()) for size, ks in elems.values() for k in ks)
         fw, reads = [], 0
         for layer in sgroup:
-            if layer.block_size > self.MAX_BLOCK:
-                raise Unsupported("node block too large")
             merged = {}
             for nids, cids, pids, pfids in zip(layer.partitioned_nids, layer.partitioned_cids, layer.partitioned_pids,
                                                layer.partitioned_pfids):
@@ -162,8 +162,10 @@ class ColumnProgram:
                 g.flow = np.stack([b[2] for b in blocks])
                 ebs = min(elems[e][0] for e in ids)
                 g.mma = layer.block_size >= 32 and ebs >= 32
-                strips = len(blocks) * max(1, layer.block_size // 64 if g.mma else layer.block_size // 16)
-                reads = max(reads, strips)
+                g.depth = sum(elems[e][0] for e in ids)
+                self._classify(g)
+                if not g.big:
+                    reads = max(reads, len(blocks) * max(1, layer.block_size // 64 if g.mma else layer.block_size // 16))
                 fw.append(g)
         if reads * fmax > self.MAX_FOLD_READS and reads > 1:
             raise Unsupported("products shared by too many rows to be folded")
@@ -193,6 +195,8 @@ class ColumnProgram:
                 g.flow = None
                 g.mma = cbs >= 32 and layer.block_size >= 32
                 g.direct = layer.block_size              # (parent block size)
+                g.depth = len(pars) * layer.block_size
+                self._classify(g)
                 bk.append(g)
         if direct and len(seen) != len(elems):
             raise Unsupported("a product without a sum parent")
@@ -205,6 +209,14 @@ class ColumnProgram:
                     for i in range(u.size):
                         prod_bk.append(dict(row=int(u[i]), size=layer.block_size, par=par[i][par[i] != 0], add=0))
         return dict(elems=elems, fw=fw, bk=bk, direct=direct, store=store, prod_bk=prod_bk)
+
+    def _classify(self, g):
+        steps, strips = g.depth // 16, len(g.blocks) * g.bs // 16
+        g.big = g.mma and strips >= self.BIG_STRIPS and steps >= self.BIG_STEPS
+        if g.mma and strips >= self.BIG_STRIPS and steps > self.BIG_MAX_STEPS:
+            raise Unsupported("a dense table deeper than a CTA task gathers")
+        if g.big:
+            self.big_steps = max(self.big_steps, steps)
 
     # ---- parameter fragments ---------------------------------------------------------------------------------------
     def _build_pack(self):
@@ -233,13 +245,14 @@ class ColumnProgram:
     # ---- cutting into tasks ------------------------------------------------------------------------------------------
     def _room(self, c: int) -> int:
         """Clusters of ``c`` CTAs the device holds at a time."""
-        if c not in self._rooms:
+        key = (c, bool(self.big_steps))
+        if key not in self._rooms:
             n = -1
             if self.device.type == "cuda":
                 with torch.cuda.device(self.device):
-                    n = int(_lib.load().pcx_column_clusters(c))
-            self._rooms[c] = n if n > 0 else max(1, 128 // c)
-        return self._rooms[c]
+                    n = int(_lib.load().pcx_column_clusters(*key))
+            self._rooms[key] = n if n > 0 else max(1, (128 if c < 16 else 112) // c)
+        return self._rooms[key]
 
     # A level with this many (16-row strip, 32-column) pieces gives every warp of the machine one: a launch of its own.
     WIDE_ITEMS = 148 * WARPS
@@ -251,6 +264,8 @@ class ColumnProgram:
         As many CTAs as the machine holds at a time, but no larger a cluster than a level has strips for its warps; among
         equals the widest column group, which reads longer pieces of a value row.  (A device with 148 SMs holds 74, 33
         and 15 clusters of 2, 4 and 8 CTAs.)"""
+        if self.big_steps:
+            return self._big_geometry(W)
         best = None
         for cols in (8, 16):
             n = -(-W // cols)
@@ -261,11 +276,64 @@ class ColumnProgram:
                 best = (n * c, cols // 8, 1, c)
         return best[1:]
 
+    def _piece(self, groups, nt: int, c: int):
+        """(strips per task, time) of a level's large groups on a cluster of c CTAs: rounds of tasks times what a task
+        takes in microseconds: a fixed latency, the gather and exponentials of its operand, its multiplications, and parameters
+        that neither stay in shared memory nor arrive during the gather.  (Measured per level: 512 x 512 on 8 CTAs, 8
+        columns, 5.3 us; 1024 x 1024 on 8 / 16 CTAs, 16 columns, 12.8 / 10.0.)"""
+        big = [(g.depth // 16, len(g.blocks) * g.bs // 16) for g in groups if g.big]
+        if not big:
+            return 1, 0.0
+        steps = max(s for s, _ in big)
+        best = None
+        for size in (16, 8, 4, 2, 1):
+            n = sum(-(-strips // size) for _, strips in big)
+            stream = max(0.0, size * steps - max(0, 150 - steps * nt // 2)) * 0.01
+            cost = -(-n // c) * (3.0 + 0.025 * steps * nt + 0.003 * size * steps * nt + stream)
+            if best is None or cost < best[1] - 1e-9:
+                best = (size, cost)
+        return best
+
+    def _big_cost(self, nt: int, c: int, n: int) -> float:
+        """Estimated time of a pass: all levels with their barriers, times the waves of clusters."""
+        level = 0.5 + 0.03 * c
+        return sum(level + self._piece(d["fw"], nt, c)[1] for d in self.depths) * -(-n // max(1, self._room(c)))
+
+    def suits(self, W: int) -> bool:
+        """Whether the program is the better choice at this row width.  With large groups it is while a level's CTA tasks go
+        around the cluster about once: it is then bound by the latency of a level, which is lower than that of the
+        per-layer kernels and of the tiles that wait on counters.  With several rounds per level a CTA works through its tasks
+        one latency after the other, where those keep two tiles per SM under way (784-variable tree, 128 latents, 512
+        samples: 745 us forward against 556)."""
+        if not self.big_steps:
+            return True
+        nt, _, c, _ = self.plan(W)["fused"]
+        size = [self._piece(d["fw"], nt, c)[0] for d in self.depths]
+        tasks = [sum(-(-(len(g.blocks) * g.bs // 16) // p) for g in d["fw"] if g.big) for d, p in zip(self.depths, size)]
+        waves = -(-(-(-W // (8 * nt))) // max(1, self._room(c)))
+        return waves == 1 and sum(-(-n // c) for n in tasks) <= 1.5 * sum(1 for n in tasks if n)
+
+    def _big_geometry(self, W: int):
+        best = None
+        for nt in (1, 2):
+            n = -(-W // (8 * nt))
+            for c in (1, 2, 4, 8, 16):
+                cost = self._big_cost(nt, c, n)
+                if best is None or cost < best[0] - 1e-9:
+                    best = (cost, nt, 1, c)
+        return best[1:]
+
     def plan(self, W: int):
         found = self._by_width.get(W)
         if found is None:
             found = self._by_width[W] = self._cut(W)
         return found
+
+    def choose(self, W: int):
+        """The plan for rows of W samples, or None where the per-layer kernels are the better choice."""
+        if W not in self._choice:
+            self._choice[W] = self.suits(W)
+        return self.plan(W) if self._choice[W] else None
 
     @staticmethod
     def _count(groups):
@@ -277,7 +345,7 @@ class ColumnProgram:
         tasks = {0: [], 1: []}
         levels = {0: [], 1: []}
         wide_tiles = -(-W // 32)
-        is_wide = lambda strips: W >= 32 and strips * wide_tiles >= self.WIDE_ITEMS
+        is_wide = lambda strips: not self.big_steps and W >= 32 and strips * wide_tiles >= self.WIDE_ITEMS
         counts = [self._count(d["fw"]) for d in self.depths]
         small = [n for n in counts if not is_wide(n)]
         nt, tiles, c = self.geometry(W, float(np.mean(small)) if small else 1.0)
@@ -302,15 +370,22 @@ class ColumnProgram:
             if stored:
                 before[i] = self._prod_tables(d)
             for g in d["fw"]:
+                if g.big:
+                    self._cta_tasks(d, g, 0, self._piece(d["fw"], nt, c)[0], kids, frag, strips[0], split)
+                    continue
                 self._fw_tasks(d, g, stored, self._strips_per_task(n, workers), kids, frag, strips[0], tasks[0], split)
             self._level(tasks[0], levels[0], strips[0], first, split, how)
         for d in reversed(self.depths):
             first = len(tasks[1])
             n = self._count(d["bk"])
             how, workers = shape(n)
+            split = []
             for g in d["bk"]:
+                if g.big:
+                    self._cta_tasks(d, g, 1, self._piece(d["bk"], nt, c)[0], kids, frag, strips[1], split)
+                    continue
                 self._bk_tasks(d, g, self._strips_per_task(n, workers), kids, frag, strips[1], tasks[1])
-            self._level(tasks[1], levels[1], strips[1], first, [], how)
+            self._level(tasks[1], levels[1], strips[1], first, split, how)
             if d["direct"]:
                 continue
             first = len(tasks[1])
@@ -320,7 +395,7 @@ class ColumnProgram:
                     tasks[1].append((off, p["par"].size, 0, 1, p["row"] + r, min(16, p["size"] - r), 0, K_PROD, p["add"], 0, 0, 0))
             self._level(tasks[1], levels[1], strips[1], first, [], shape(len(tasks[1]) - first)[0])
         dev = self.device
-        out = dict(kids=None, frags=torch.empty(max(frag.n, 1) * 1024, dtype=torch.uint8, device=dev),
+        out = dict(fused=fused, kids=None, frags=torch.empty(max(frag.n, 1) * 1024, dtype=torch.uint8, device=dev),
                    bases=frag.tensor(dev), n_frag=frag.n)
         for m in (0, 1):
             rec = np.array(tasks[m], dtype=TASK)
@@ -336,9 +411,15 @@ class ColumnProgram:
                 at = end
             out[m] = dict(tasks=torch.from_numpy(rec.view(np.uint8)).to(dev), strips=strips[m].tensor(dev), levels=tab,
                           launches=launches)
-        out["par"] = self._par_jobs(kids)
         out["kids"] = kids.tensor(dev)
         return out
+
+    @property
+    def par(self):
+        """Jobs of the parameter flows (the same for every row width), built when the first pass needs them."""
+        if self._par is None:
+            self._par = self._par_jobs()
+        return self._par
 
     @staticmethod
     def _level(tasks, levels, strips, first, split, how):
@@ -374,29 +455,65 @@ class ColumnProgram:
                         torch.from_numpy(cids).to(self.device), size))
         return out
 
+    def _operand(self, d, g, mode):
+        """Operand rows of an MMA group, one line per 16-deep step."""
+        if mode == 1:
+            return np.concatenate([np.arange(p, p + g.direct, 16) for p in g.ops])[:, None]
+        elems, store = d["elems"], d["store"]
+        nk = max(len(elems[e][1]) for e in g.ops)
+        rows = []
+        for e in g.ops:
+            size, ks = elems[e]
+            ks = ks + [0] * (nk - len(ks))
+            for o in range(0, size, 16):
+                # (an absent child is a dummy row: zeros, whatever the offset)
+                rows.append([k + o if k else 0 for k in ks] + ([store[e] + o] if store else []))
+        return np.asarray(rows)
+
+    def _outputs(self, d, g, mode, kids):
+        """Output records of an MMA group, one per strip."""
+        if mode == 0:
+            out = np.zeros((len(g.blocks) * (g.bs // 16), 4), dtype=np.int32)
+            out[:, 0] = np.concatenate([np.arange(b, b + g.bs, 16) for b in g.blocks])
+            return out
+        return np.asarray([self._record(d, e, o, kids) for e in g.blocks for o in range(0, g.bs, 16)], dtype=np.int32)
+
+    def _record(self, d, e, o, kids):
+        """Output record of element block e from row o on (backward)."""
+        size, ks = d["elems"][e]
+        if d["store"]:
+            return [e + o, d["store"][e] + o, 0, -1]
+        if len(ks) <= 2:
+            return [e + o, ks[0] + o, ks[1] + o if len(ks) == 2 else 0, int(d["direct"])]
+        return [e + o, kids.add([k + o for k in ks]), len(ks), 2 + int(d["direct"])]
+
+    def _cta_tasks(self, d, g, mode, per, kids, frag, strips, tasks):
+        rows = self._operand(d, g, mode)
+        out, bases = self._outputs(d, g, mode, kids), g.par[0]
+        nk = rows.shape[1] - (1 if mode == 0 and d["store"] else 0)
+        off = kids.add(rows)
+        s = 0
+        while s < len(out):
+            n = min(per, len(out) - s)
+            while n & (n - 1):                                 # powers of two divide the warps evenly
+                n &= n - 1
+            fo = frag.add(bases[s:s + n].transpose(1, 0, 2))
+            tasks.append((off, rows.shape[0], nk, rows.shape[1], strips.add(out[s:s + n]), n, fo, K_CTA, 0, 0, 0, 0))
+            s += n
+
     def _fw_tasks(self, d, g, stored, per, kids, frag, strips, tasks, split):
         elems, store = d["elems"], d["store"]
         nk = max(len(elems[e][1]) for e in g.ops)
         n_kids = -1 if stored else nk
         if g.mma:
-            rows = []
-            for e in g.ops:
-                size, ks = elems[e]
-                ks = ks + [0] * (nk - len(ks))
-                for o in range(0, size, 16):
-                    # (an absent child is a dummy row: zeros, whatever the offset)
-                    rows.append([store[e] + o] if stored else
-                                [k + o if k else 0 for k in ks] + ([store[e] + o] if store else []))
-            rows = np.asarray(rows)
-            off, width = kids.add(rows), rows.shape[1]
-            bases = g.par[0]
-            out = np.concatenate([np.arange(b, b + g.bs, 16) for b in g.blocks])
-            for s in range(0, out.size, per):
-                n = min(per, out.size - s)
-                st = np.zeros((n, 4), dtype=np.int32)
-                st[:, 0] = out[s:s + n]
+            rows = self._operand(d, g, 0)
+            if stored:
+                rows = rows[:, -1:]
+            off, out, bases = kids.add(rows), self._outputs(d, g, 0, kids), g.par[0]
+            for s in range(0, len(out), per):
+                n = min(per, len(out) - s)
                 fo = frag.add(bases[s:s + n].transpose(1, 0, 2))
-                tasks.append((off, rows.shape[0], n_kids, width, strips.add(st), n, fo, K_MMA, 0, 0, 0, 0))
+                tasks.append((off, rows.shape[0], n_kids, rows.shape[1], strips.add(out[s:s + n]), n, fo, K_MMA, 0, 0, 0, 0))
             return
         depth = sum(elems[e][0] for e in g.ops)
         lg = 3 if all(elems[e][0] % 8 == 0 for e in g.ops) else 0
@@ -418,26 +535,14 @@ class ColumnProgram:
                     (kids.add(rows), depth, n_kids, rows.shape[1], strips.add(st), n, 0, kind, g.bs, 1, lg, 0))
 
     def _bk_tasks(self, d, g, per, kids, frag, strips, tasks):
-        elems, store, pbs = d["elems"], d["store"], g.direct
-
-        def record(e, o):
-            size, ks = elems[e]
-            if store:
-                return [e + o, store[e] + o, 0, -1]
-            if len(ks) <= 2:
-                return [e + o, ks[0] + o, ks[1] + o if len(ks) == 2 else 0, int(d["direct"])]
-            return [e + o, kids.add([k + o for k in ks]), len(ks), 2 + int(d["direct"])]
-
+        pbs = g.direct
         if g.mma:
-            rows = np.concatenate([np.arange(p, p + pbs, 16) for p in g.ops])
-            off = kids.add(rows)
-            bases = g.par[0]
-            out = [(e, o) for e in g.blocks for o in range(0, g.bs, 16)]
+            rows = self._operand(d, g, 1)
+            off, out, bases = kids.add(rows), self._outputs(d, g, 1, kids), g.par[0]
             for s in range(0, len(out), per):
-                part = out[s:s + per]
-                st = np.asarray([record(e, o) for e, o in part])
-                fo = frag.add(bases[s:s + len(part)].transpose(1, 0, 2))
-                tasks.append((off, rows.size, 1, 1, strips.add(st), len(part), fo, K_MMA, 0, 0, 0, 0))
+                n = min(per, len(out) - s)
+                fo = frag.add(bases[s:s + n].transpose(1, 0, 2))
+                tasks.append((off, rows.shape[0], 1, 1, strips.add(out[s:s + n]), n, fo, K_MMA, 0, 0, 0, 0))
             return
         lg = 3 if pbs % 8 == 0 else 0
         step = 1 << lg
@@ -446,12 +551,12 @@ class ColumnProgram:
                 n = min(16, g.bs - r)
                 rows = np.asarray([[pid + r * pbs + o, p + o] for p, pid in zip(g.ops, pids.tolist())
                                    for o in range(0, pbs, step)])
-                st = np.asarray([record(e, r)])
+                st = np.asarray([self._record(d, e, r, kids)])
                 tasks.append((kids.add(rows), len(g.ops) * pbs, 1, 2, strips.add(st), n, 0, K_SIMT, 1, pbs, lg, 0))
 
     # ---- parameter flows ---------------------------------------------------------------------------------------------
-    def _par_jobs(self, kids):
-        pp = _Pool(2)
+    def _par_jobs(self):
+        pp, kids = _Pool(2), _Pool()
         jobs = {0: [], 1: [], 2: [], 3: []}
         for d in self.depths:
             elems, store = d["elems"], d["store"]
@@ -496,7 +601,7 @@ class ColumnProgram:
                             tab = [[par[b, i] + o * g.bs + r, g.flow[b, i] + o * g.bs + r] for _, o, i in ks]
                             jobs[1].append((first + r, 0, min(16, g.bs - r), off, len(ks) * step, n_kids, width, pp.add(tab),
                                             g.bs, lg, 0, 0))
-        return dict(pp=pp.tensor(self.device),
+        return dict(pp=pp.tensor(self.device), kids=kids.tensor(self.device),
                     jobs={k: (torch.from_numpy(np.array(v, dtype=PAR).view(np.uint8)).to(self.device), len(v))
                           for k, v in jobs.items() if v})
 
@@ -518,18 +623,22 @@ class ColumnProgram:
                     _lib.call("pcx_prod_fwd", em, nm, nids, cids, nids.numel(), cids.size(1), size, W)
                 continue
             levels, n, (nt, tiles, cluster, wide) = launch
+            if self.big_steps:
+                _lib.call("pcx_column_run_big", mode, nm, nf, ef, em, params, plan["frags"], p["tasks"], plan["kids"],
+                          p["strips"], levels, n, W, nt, cluster, self.big_steps, int(logspace), terms)
+                continue
             _lib.call("pcx_column_run", mode, nm, nf, ef, em, params, plan["frags"], p["tasks"], plan["kids"], p["strips"],
                       levels, n, W, nt, tiles, cluster, wide, int(logspace), terms)
 
     def param_flows(self, plan, pf, nf, nm, params, logspace: bool = True):
         W = nm.size(1)
-        for kind, (jobs, n) in plan["par"]["jobs"].items():
-            _lib.call("pcx_column_par", kind, pf, nf, nm, self.buffers(W), params, jobs, plan["kids"], plan["par"]["pp"], n,
+        for kind, (jobs, n) in self.par["jobs"].items():
+            _lib.call("pcx_column_par", kind, pf, nf, nm, self.buffers(W), params, jobs, self.par["kids"], self.par["pp"], n,
                       W, int(logspace), 1 if _lib.sum_mode() == 2 else 3)
 
     def check(self, plan, pc, report):
         """Bounds of every index the kernels form from the plan's tables; ``report(what, index, extent, limit)``."""
-        kids, pp = plan["kids"].cpu().numpy(), plan["par"]["pp"].cpu().numpy().reshape(-1, 2)
+        kids, pp = plan["kids"].cpu().numpy(), self.par["pp"].cpu().numpy().reshape(-1, 2)
         n_par, n_flow = int(pc.params.numel()), int(pc.num_param_flows)
         bases = plan["bases"].cpu().numpy().reshape(-1, 4)[:plan["n_frag"]]
         for b in bases:
@@ -550,11 +659,11 @@ class ColumnProgram:
                     for r in kids[off:off + k]:
                         report("column parent rows", int(r), int(t["n_rows"]), pc.num_elements)
                     continue
-                n_ent = k if t["kind"] == K_MMA else (k >> int(t["lg_entry"]))
-                span = 16 if t["kind"] == K_MMA else (1 << int(t["lg_entry"]))
+                n_ent = k if t["kind"] in (K_MMA, K_CTA) else (k >> int(t["lg_entry"]))
+                span = 16 if t["kind"] in (K_MMA, K_CTA) else (1 << int(t["lg_entry"]))
                 assert off + n_ent * w <= kids.size
                 ent = kids[off:off + n_ent * w].reshape(n_ent, w)
-                if t["kind"] == K_MMA:
+                if t["kind"] in (K_MMA, K_CTA):
                     assert int(t["par_off"]) + k * int(t["n_rows"]) <= plan["n_frag"]
                 else:
                     ext = (span - 1) * int(t["sk"]) + (int(t["n_rows"]) - 1) * int(t["sr"]) + 1
@@ -567,8 +676,8 @@ class ColumnProgram:
                     report("column operand rows", int(r), span, limit)
                 for r in ent[:, nk:].reshape(-1):
                     report("column stored rows", int(r), span, self.em_rows)
-                n_st = int(t["n_rows"]) if t["kind"] == K_MMA else 1
-                rows = 16 if t["kind"] == K_MMA else int(t["n_rows"])
+                n_st = int(t["n_rows"]) if t["kind"] in (K_MMA, K_CTA) else 1
+                rows = 16 if t["kind"] in (K_MMA, K_CTA) else int(t["n_rows"])
                 for st in strips[int(t["strip_off"]):int(t["strip_off"]) + n_st]:
                     if mode == 0:
                         report("column output rows", int(st[0]), rows, pc.num_nodes)
@@ -582,7 +691,8 @@ class ColumnProgram:
                     else:
                         for r in kids[int(st[1]):int(st[1]) + int(st[2])]:
                             report("column child rows", int(r), rows, pc.num_nodes)
-        for kind, (jobs, n) in plan["par"]["jobs"].items():
+        kids = self.par["kids"].cpu().numpy()
+        for kind, (jobs, n) in self.par["jobs"].items():
             for t in jobs.cpu().numpy().view(PAR):
                 mma = kind != 1
                 span = 16 if mma else (1 << int(t["lg_entry"]))

@@ -41,7 +41,7 @@ constexpr int CW = CT / 32;
 constexpr int MAX_SMEM_LEVELS = 512;
 constexpr int WT = 384;                     // of the wide launches: 12 warps, 168 registers each
 constexpr int MAX_STRIPS = 2;               // 16-row strips an MMA task may hold (accumulators and element values)
-enum ColKind { K_MMA = 0, K_SIMT = 1, K_SPLIT = 2, K_PROD = 3 };
+enum ColKind { K_MMA = 0, K_SIMT = 1, K_SPLIT = 2, K_PROD = 3, K_CTA = 4 };
 enum ColMode { C_FWD = 0, C_ELE = 1 };
 
 struct ColArgs {
@@ -176,11 +176,13 @@ __device__ __forceinline__ void load_element(const ColArgs& a, const int4& st, i
     }
 #pragma unroll
     for (int j = 0; j < 2 * NT; ++j) { e.x[0][j] = 0.0f; e.x[1][j] = 0.0f; }
-    for (int c = 0; c < st.z; ++c) {
-        float x[2 * NT];
+    for (int c = 0; c < st.z; c += 2) {
+        const bool two = c + 1 < st.z;
+        float x[2 * NT], y[2 * NT];
         ldvec<2 * NT>(a.nm + (int64_t)(__ldg(a.kids + st.y + c) + row) * a.W + co, x);
+        ldvec<2 * NT>(a.nm + (int64_t)(two ? __ldg(a.kids + st.y + c + 1) + row : 0) * a.W + co, y);
 #pragma unroll
-        for (int j = 0; j < 2 * NT; ++j) e.x[0][j] += x[j];
+        for (int j = 0; j < 2 * NT; ++j) { e.x[0][j] += x[j]; e.x[1][j] += two ? y[j] : 0.0f; }
     }
 }
 
@@ -1045,6 +1047,332 @@ __global__ void __launch_bounds__(CT, 1) column_kernel(const ColArgs a) {
     }
 }
 
+// ---- large groups: CTA tasks ---------------------------------------------------------------------------------------------
+// Where many rows share a long child list (node blocks of 128 and more: hidden trees with 128 latents and up, the dense
+// transitions of an HMM) warp tasks would each gather the list again.  A CTA task gathers, exponentiates and splits it once
+// into shared memory in the order of the B fragments, and the 16 warps multiply strips (and, where a task has fewer than 16
+// strips, parts of the contraction) from there.  What the task does not wait for is there before it starts: the parameter
+// fragments of a CTA's next task are copied to shared memory while the current one finishes, and tied layers (every
+// transition of a homogeneous HMM) find them there already -- 512 x 512 parameters over a cluster of 8 CTAs are 128 KB each.
+// tcgen05 would need 128-row tiles and a trip through tensor memory per level; with 8 or 16 columns per cluster the
+// multiplication is a tenth of a level, which is gather, two CTA barriers and the cluster barrier.
+constexpr int BIG_MAX_STEPS = 64;
+
+template <int NT>
+struct BigSmem {
+    static constexpr int MAX = CW * 8 * NT * 4;                        // column maxima per warp
+    static constexpr int RED = CW * 32 * NT * 16;                      // partial accumulators
+    static constexpr int LEVELS = MAX_SMEM_LEVELS * 16;
+    static constexpr int PART = CW * 64 * 4;                           // split tasks
+    static constexpr int FIXED = MAX + RED + LEVELS + PART;
+};
+
+struct BigState {
+    uint8_t* a_frag;            // shared: the parameter fragments of one task (its first `held` steps)
+    uint4* b_frag;              // shared: [step][tile][lane]
+    float* s_max;
+    float4* s_red;
+    int a_bytes;
+    int a_off, a_held;          // fragments now in (or on their way to) a_frag: first fragment, steps
+};
+
+struct BigParams { int par_off, n_k, n_rows; };             // whose fragments: n_k = 0: nobody's
+
+__device__ __forceinline__ void big_load_params(const ColArgs& a, const BigParams& t, BigState& b) {
+    if (t.par_off == b.a_off) return;
+    b.a_off = t.par_off;
+    b.a_held = min(t.n_k, b.a_bytes / (t.n_rows * 1024));
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(b.a_frag);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(a.frags) + (int64_t)t.par_off * 1024;
+    const int bytes = b.a_held * t.n_rows * 1024;
+    for (int i = threadIdx.x * 16; i < bytes; i += CT * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i), "l"(src + i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// What a warp needs of a CTA task before its first load of a value: fetched while the level before it closes.
+struct BigAhead {
+    int kid[4][2];              // operand rows of its first four half steps (children 0 and 1)
+    int4 st;                    // its output record
+};
+
+template <int MODE>
+__device__ __forceinline__ void big_look_ahead(const ColArgs& a, const PcxColTask& t, BigAhead& f) {
+    const int warp = threadIdx.x >> 5, halves = 2 * t.n_k;
+    const int32_t* kid = a.kids + t.kid_off;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int u = warp + CW * j, q = u < halves ? u >> 1 : 0;
+        f.kid[j][0] = __ldg(kid + q * t.width);
+        f.kid[j][1] = (MODE == C_FWD && t.n_kids > 1) ? __ldg(kid + q * t.width + 1) : 0;
+    }
+    f.st = __ldg(a.strips + t.strip_off + warp % t.n_rows);
+}
+
+// PER: half steps per warp (depth / 128, rounded up to 1, 2, 4 or 8).
+template <int MODE, int NT, int PER, typename Next>
+__device__ __forceinline__ void cta_task(const ColArgs& a, const PcxColTask& t, const BigAhead& f, int col0, BigState& b, Next next) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
+    const int W = a.W;
+    const int cl = (col0 + NT * g < W) ? col0 + NT * g : 0;
+    const int co = col0 + 2 * NT * tq;
+    const bool co_ok = co < W;
+    const int32_t* kid = a.kids + t.kid_off;
+    const int halves = 2 * t.n_k;
+
+    // operand: half step u = rows 2t, 2t+1 (+ 8) of a 16-deep step; up to four at a time, with two operand rows each
+    float v[PER][2][NT];
+#pragma unroll
+    for (int j0 = 0; j0 < PER; j0 += 4) {
+        constexpr int N = PER < 4 ? PER : 4;
+        float y[N][2][NT];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int u = warp + CW * (j0 + j), o = 2 * tq + 8 * (u & 1);
+            int r0, r1;
+            if (j0 == 0) {
+                r0 = f.kid[j][0];
+                r1 = f.kid[j][1];
+            } else {
+                const int32_t* e = kid + (u < halves ? u >> 1 : 0) * t.width;
+                r0 = __ldg(e);
+                r1 = (MODE == C_FWD && t.n_kids > 1) ? __ldg(e + 1) : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                ldvec<NT>((MODE == C_ELE ? a.nf : a.nm) + (int64_t)(r0 + o + i) * W + cl, v[j0 + j][i]);
+                ldvec<NT>(a.nm + (int64_t)((MODE == C_ELE ? r0 : r1) + o + i) * W + cl, y[j][i]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+                    v[j0 + j][i][n] = MODE == C_ELE ? flow_over_value(v[j0 + j][i][n], y[j][i][n], a.logspace) : v[j0 + j][i][n] + y[j][i][n];
+        if (MODE == C_FWD) {
+            for (int c = 2; c < t.n_kids; c += 2) {        // elements of more than two children
+                float x[N][2][NT];
+                const bool two = c + 1 < t.n_kids;
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const int u = warp + CW * (j0 + j), o = 2 * tq + 8 * (u & 1);
+                    const int32_t* e = kid + (u < halves ? u >> 1 : 0) * t.width + c;
+                    const int r0 = __ldg(e) + o, r1 = two ? __ldg(e + 1) + o : o;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        ldvec<NT>(a.nm + (int64_t)(r0 + i) * W + cl, x[j][i]);
+                        ldvec<NT>(a.nm + (int64_t)(r1 + i) * W + cl, y[j][i]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < N; ++j)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) v[j0 + j][i][n] += x[j][i][n] + (two ? y[j][i][n] : 0.0f);
+            }
+            if (t.width > t.n_kids && col0 + NT * g < W) { // keep the elements' values
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const int u = warp + CW * (j0 + j);
+                    if (u < halves) {
+                        const int r = __ldg(kid + (u >> 1) * t.width + t.n_kids) + 2 * tq + 8 * (u & 1);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) stvec<NT>(a.em + (int64_t)(r + i) * W + cl, v[j0 + j][i]);
+                    }
+                }
+            }
+        }
+    }
+    // strips and parts of the contraction (strips per task: a power of two up to 16)
+    const int parts = CW / t.n_rows, strip = warp % t.n_rows, part = warp / t.n_rows;
+    ElementValue<NT> ev[2];
+    if (MODE == C_ELE && part == 0 && co_ok) {             // (in flight until the epilogue)
+        load_element<NT>(a, f.st, g, co, ev[0]);
+        load_element<NT>(a, f.st, g + 8, co, ev[1]);
+    }
+    float m[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        m[n] = PCX_NEG_INF;
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+            if (warp + CW * j < halves) m[n] = fmaxf(m[n], fmaxf(v[j][0][n], v[j][1][n]));
+        m[n] = fmaxf(m[n], __shfl_xor_sync(0xffffffffu, m[n], 1));
+        m[n] = fmaxf(m[n], __shfl_xor_sync(0xffffffffu, m[n], 2));
+        if (tq == 0) b.s_max[(NT * g + n) * CW + warp] = m[n];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        // four lanes share a column: each takes the maxima of four warps
+        const float4 q = *reinterpret_cast<const float4*>(b.s_max + (NT * g + n) * CW + tq * 4);
+        m[n] = fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w));
+        m[n] = fmaxf(m[n], __shfl_xor_sync(0xffffffffu, m[n], 1));
+        m[n] = fmaxf(m[n], __shfl_xor_sync(0xffffffffu, m[n], 2));
+        const float sh = (m[n] == PCX_NEG_INF) ? 0.0f : m[n];
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int u = warp + CW * j;
+            if (u < halves) {
+                uint32_t hi, lo;
+                split2(fast_exp(v[j][0][n] - sh), fast_exp(v[j][1][n] - sh), hi, lo);
+                // (the two halves of a step interleave their words: see the reader)
+                *reinterpret_cast<uint2*>(reinterpret_cast<uint32_t*>(b.b_frag + ((u >> 1) * NT + n) * 32 + lane) + 2 * (u & 1)) = make_uint2(hi, lo);
+            }
+        }
+    }
+    const int k_begin = part * t.n_k / parts, k_end = (part + 1) * t.n_k / parts;
+    float acc[3][NT][4];                                    // the three products have accumulators of their own: no chain
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[x][n][c] = 0.0f;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    {
+        const uint4* as = reinterpret_cast<const uint4*>(b.a_frag) + strip * 64 + lane;
+        const uint4* ag = a.frags + ((int64_t)t.par_off + strip) * 64 + lane;
+        const int stride = t.n_rows * 64, held = b.a_held;
+        auto step = [&](int k, const uint4& ah, const uint4& al) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const uint4 w = b.b_frag[(k * NT + n) * 32 + lane];        // hi, lo of rows 2t; hi, lo of rows 2t + 8
+                mma16816(acc[0][n], ah, w.x, w.z);
+                if (a.terms == 3) {
+                    mma16816(acc[1][n], ah, w.y, w.w);
+                    mma16816(acc[2][n], al, w.x, w.z);
+                }
+            }
+        };
+        int k = k_begin;
+#pragma unroll 4
+        for (; k < min(k_end, held); ++k) step(k, as[k * stride], as[k * stride + 32]);
+#pragma unroll 4
+        for (; k < k_end; ++k) step(k, __ldg(ag + (int64_t)k * stride), __ldg(ag + (int64_t)k * stride + 32));
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[0][n][c] += acc[1][n][c] + acc[2][n][c];
+    if (part > 0) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+            b.s_red[(warp * NT + n) * 32 + lane] = make_float4(acc[0][n][0], acc[0][n][1], acc[0][n][2], acc[0][n][3]);
+    }
+    __syncthreads();
+    next();
+    if (part > 0) return;
+    for (int q = 1; q < parts; ++q)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const float4 x = b.s_red[((strip + q * t.n_rows) * NT + n) * 32 + lane];
+            acc[0][n][0] += x.x; acc[0][n][1] += x.y; acc[0][n][2] += x.z; acc[0][n][3] += x.w;
+        }
+    float m0[NT], m1[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        m0[n] = __shfl_sync(0xffffffffu, m[n], 8 * tq);
+        m1[n] = __shfl_sync(0xffffffffu, m[n], 8 * tq + 4);
+    }
+    if (!co_ok) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int row = g + 8 * h;
+        float o[2 * NT];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const float x0 = acc[0][n][2 * h], x1 = acc[0][n][2 * h + 1];
+            o[n] = fast_log_plus(MODE == C_FWD ? fmaxf(x0, 1e-24f) : x0, m0[n]);
+            o[NT + n] = fast_log_plus(MODE == C_FWD ? fmaxf(x1, 1e-24f) : x1, m1[n]);
+        }
+        if (MODE == C_FWD) {
+            stvec<2 * NT>(a.nm + (int64_t)(f.st.x + row) * W + co, o);
+            continue;
+        }
+#pragma unroll
+        for (int n = 0; n < 2 * NT; ++n) {
+            o[n] += ev[h].x[0][n] + ev[h].x[1][n];
+            if (!a.logspace) o[n] = __expf(o[n]);
+        }
+        store_flow<2 * NT>(a, f.st, row, co, o);
+    }
+}
+
+template <int MODE, int NT>
+__global__ void __launch_bounds__(CT, 1) column_big_kernel(const ColArgs a, int a_bytes, int b_bytes) {
+    using C = BigSmem<NT>;
+    extern __shared__ __align__(128) uint8_t s_pipe[];
+    BigState b;
+    b.a_frag = s_pipe;
+    b.b_frag = reinterpret_cast<uint4*>(s_pipe + a_bytes);
+    uint8_t* fixed = s_pipe + a_bytes + b_bytes;
+    b.s_max = reinterpret_cast<float*>(fixed);
+    b.s_red = reinterpret_cast<float4*>(fixed + C::MAX);
+    int4* levels = reinterpret_cast<int4*>(fixed + C::MAX + C::RED);
+    float* s_part = reinterpret_cast<float*>(fixed + C::MAX + C::RED + C::LEVELS);
+    b.a_bytes = a_bytes;
+    b.a_off = -1;
+    b.a_held = 0;
+    const int rank = blockIdx.x % a.cluster, warp = threadIdx.x >> 5;
+    const int col0 = (blockIdx.x / a.cluster) * 8 * NT;
+    const int worker = warp * a.cluster + rank, workers = CW * a.cluster;
+    for (int i = threadIdx.x; i < a.n_levels; i += CT) levels[i] = __ldg(a.levels + i);
+    __syncthreads();
+    // this CTA's CTA tasks, across levels: the record of the next one is fetched when the products of the current one are
+    // done, its parameters follow, and the rows it will read are known before the barrier opens
+    int next_l = 0, next_i = rank;
+    auto advance = [&](int& at) {
+        while (next_l < a.n_levels && next_i >= levels[next_l].w) { ++next_l; next_i = rank; }
+        at = next_l;
+        const int task = next_l < a.n_levels ? levels[next_l].z + next_i : 0;
+        next_i += a.cluster;
+        return load_record(a.tasks, task);
+    };
+    int at;
+    PcxColTask t = advance(at);
+    BigAhead f;
+    if (t.kind == K_CTA) {
+        big_load_params(a, BigParams{t.par_off, t.n_k, t.n_rows}, b);
+        big_look_ahead<MODE>(a, t, f);
+    }
+    for (int l = 0; l < a.n_levels; ++l) {
+        const int4 lv = levels[l];
+        for (int i = worker; i < lv.y; i += workers) run_task<MODE, NT>(a, load_record(a.tasks, lv.x + i), col0);
+        while (at == l) {
+            PcxColTask t1;
+            int at1;
+            auto next = [&]() {
+                t1 = advance(at1);
+                if (at1 < a.n_levels && t1.kind == K_CTA) big_load_params(a, BigParams{t1.par_off, t1.n_k, t1.n_rows}, b);
+            };
+            if (t.kind == K_CTA) {
+                if (t.n_k <= 8) cta_task<MODE, NT, 1>(a, t, f, col0, b, next);
+                else if (t.n_k <= 16) cta_task<MODE, NT, 2>(a, t, f, col0, b, next);
+                else if (t.n_k <= 32) cta_task<MODE, NT, 4>(a, t, f, col0, b, next);
+                else cta_task<MODE, NT, 8>(a, t, f, col0, b, next);
+            } else {
+                if (MODE == C_FWD) split_task<NT, CW>(a, t, col0, s_part);
+                next();
+            }
+            t = t1; at = at1;
+            if (at < a.n_levels && t.kind == K_CTA) big_look_ahead<MODE>(a, t, f);
+        }
+        if (a.cluster == 1) {
+            __syncthreads();
+        } else {
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // ---- parameter fragments -----------------------------------------------------------------------------------------------
 // Fragment f covers 16 rows x 16 children: element (row r, child k) is params[base + r * sr + k * sk].  64 words of 16
 // bytes: the high parts of the 32 lanes' A registers, then the low parts.
@@ -1560,6 +1888,36 @@ int launch_column(const ColArgs& a, cudaStream_t st) {
     return 0;
 }
 
+// Shared memory of the CTA-task kernel: operand fragments of the deepest task, the rest for parameter fragments.
+constexpr int BIG_TOTAL = 227 * 1024;
+
+template <int MODE, int NT>
+int big_setup() {
+    static PcxOnce done;
+    if (!done) {
+        cudaError_t e = cudaFuncSetAttribute(column_big_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, BIG_TOTAL);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(column_big_kernel<MODE, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return (int)e;
+        done = true;
+    }
+    return 0;
+}
+
+template <int MODE, int NT>
+int launch_big(const ColArgs& a, int max_steps, cudaStream_t st) {
+    int rc = big_setup<MODE, NT>();
+    if (rc != 0) return rc;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = column_config<MODE, NT>((int)pcx_cdiv(a.W, 8 * NT), a.cluster, &attr, st);
+    cfg.dynamicSmemBytes = BIG_TOTAL;
+    const int b_bytes = max_steps * NT * 512;
+    const int a_bytes = (BIG_TOTAL - BigSmem<NT>::FIXED - b_bytes) & ~1023;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, column_big_kernel<MODE, NT>, a, a_bytes, b_bytes);
+    if (e != cudaSuccess) return (int)e;
+    PCX_LAUNCH_CHECK();
+    return 0;
+}
+
 template <int MODE>
 int launch_column_nt(const ColArgs& a, int nt, cudaStream_t st) {
     if (a.wide == 1) {
@@ -1591,8 +1949,8 @@ int launch_column_nt(const ColArgs& a, int nt, cudaStream_t st) {
 
 extern "C" {
 
-int pcx_column_clusters(int cluster) {
-    if (cluster < 1 || cluster > 8) return -1;
+int pcx_column_clusters(int cluster, int big) {
+    if (cluster < 1 || cluster > (big ? 16 : 8)) return -1;
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = column_config<C_ELE, 2>(1, cluster, &attr, nullptr);
     int n = 0;
@@ -1601,8 +1959,35 @@ int pcx_column_clusters(int cluster) {
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
         return n;
     }
-    if (cudaOccupancyMaxActiveClusters(&n, column_kernel<C_ELE, 2>, &cfg) != cudaSuccess) { cudaGetLastError(); return -1; }
+    cudaError_t e;
+    if (big) {
+        if (big_setup<C_ELE, 2>() != 0) return -1;
+        cfg.dynamicSmemBytes = BIG_TOTAL;
+        e = cudaOccupancyMaxActiveClusters(&n, column_big_kernel<C_ELE, 2>, &cfg);
+    } else {
+        e = cudaOccupancyMaxActiveClusters(&n, column_kernel<C_ELE, 2>, &cfg);
+    }
+    if (e != cudaSuccess) { cudaGetLastError(); return -1; }
     return n;
+}
+
+int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,
+                       const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
+                       const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int cluster, int max_steps,
+                       int logspace, int terms, void* stream) {
+    if (n_levels <= 0 || W <= 0) return 0;
+    if (W % 8 != 0 || (nt != 1 && nt != 2) || cluster < 1 || cluster > 16 || (mode != 0 && mode != 1)) return -1;
+    if (n_levels > MAX_SMEM_LEVELS || max_steps < 1 || max_steps > BIG_MAX_STEPS) return -1;
+    if (((reinterpret_cast<uintptr_t>(node_mars) | reinterpret_cast<uintptr_t>(node_flows) |
+          reinterpret_cast<uintptr_t>(element_flows) | reinterpret_cast<uintptr_t>(element_values)) & 15) != 0) return -1;
+    ColArgs a{};
+    a.nm = node_mars; a.nf = node_flows; a.ef = element_flows; a.em = element_values; a.params = params;
+    a.frags = reinterpret_cast<const uint4*>(frags); a.tasks = tasks; a.kids = kids;
+    a.strips = reinterpret_cast<const int4*>(strips); a.levels = reinterpret_cast<const int4*>(levels);
+    a.n_levels = n_levels; a.W = W; a.logspace = logspace; a.terms = terms; a.cluster = cluster; a.tiles = 1;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (mode == 0) return nt == 1 ? launch_big<C_FWD, 1>(a, max_steps, st) : launch_big<C_FWD, 2>(a, max_steps, st);
+    return nt == 1 ? launch_big<C_ELE, 1>(a, max_steps, st) : launch_big<C_ELE, 2>(a, max_steps, st);
 }
 
 int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,

@@ -70,8 +70,9 @@ class ParamPacker:
     parameter tensor was replaced, modified through torch, or updated by an EM step (``invalidate``)."""
     TILE_BYTES = 32768
 
-    def __init__(self, device):
+    def __init__(self, device, owner=None):
         self.device = device
+        self.owner = owner                       # weak reference to the circuit whose ``params`` the tiles follow
         self.entries = {}
         self.sm_entries = {}
         self._stamp = None
@@ -151,6 +152,11 @@ class ParamPacker:
                 self._sm_jobs = self._sm_job_table()
             jobs, n_jobs, n_vec = self._sm_jobs
             _lib.call("pcx_pack_sm_jobs", jobs, n_jobs, n_vec, params)
+
+    def refresh_from_owner(self):
+        pc = self.owner() if self.owner is not None else None
+        if pc is not None:
+            self.refresh(pc.params.data)
 
     def refresh(self, params: torch.Tensor, plan=None):
         if self.stale(params, plan):
@@ -292,12 +298,22 @@ class InputLayer(Layer, nn.Module):
         sh["dirty"] = False
         self._arena_zero = False
 
-    def _zero_shadow(self):
+    def _launch_zero_shadow(self):
         sh = self._shadow
         if sh is not None and sh["dirty"]:
             _fill(sh["flows"], 0.0)
             sh["touched"].zero_()
-            sh["dirty"] = False
+
+    def _zero_shadow(self):
+        self._launch_zero_shadow()
+        if self._shadow is not None:
+            self._shadow["dirty"] = False
+
+    def _mark_cleared(self):
+        """What the host keeps track of when all accumulators have been cleared."""
+        if self._shadow is not None:
+            self._shadow["dirty"] = False
+        self._arena_zero = True
 
     def to(self, device):
         device = torch.device(f"cuda:{device}") if isinstance(device, int) else torch.device(device)
@@ -438,24 +454,51 @@ class InputLayer(Layer, nn.Module):
 
     def mini_batch_em(self, step_size: float, pseudocount: float = 0.0, keep_zero_params: bool = False):
         self._require_cuda()
+        state = self._em_state(keep_zero_params)
+        self._launch_em(step_size, pseudocount, keep_zero_params)
+        self._mark_em(state)
+
+    def _em_state(self, keep_zero_params: bool):
+        """What decides which launches an update takes: (straight from the transposed shadow, flows to move out of it, tied
+        replicas to fold, accumulators known to be empty)."""
         sh = self._shadow
-        if (sh is not None and sh["dirty"] and self._arena_zero and not keep_zero_params and sh["logp"] is not None
-                and self.use_fused_shadow_em):
+        dirty = sh is not None and bool(sh["dirty"])
+        direct = (dirty and bool(self._arena_zero) and not keep_zero_params and sh["logp"] is not None
+                  and bool(self.use_fused_shadow_em))
+        return (direct, dirty and not direct, not direct and not getattr(self, "_tied_folded", False), bool(self._arena_zero))
+
+    def _launch_em(self, step_size: float, pseudocount: float, keep_zero_params: bool):
+        sh = self._shadow
+        if self._em_state(keep_zero_params)[0]:
             # every flow of this update sits in the transposed shadow and the accumulators proper are empty: update
             # the parameters and the transposed log-parameter table straight from it.  The flows stay in
             # the shadow (still "dirty"): whoever reads `param_flows` later gets them moved over as usual.
-            self._param_epoch += 1
             if sh.get("totals") is None:
                 sh["totals"] = torch.zeros(16 * sh["R"], dtype=torch.float32, device=self.device)
             _lib.call("pcx_em_input_cat_t", self.params.data, sh["logp"], sh["flows"], sh["totals"], sh["R"], sh["C"],
                       float(step_size), float(pseudocount))
-            sh["stamp"] = (self.params.data_ptr(), self.params._version, self._param_epoch)
             return
-        self.fold_tied_flows()
-        self._param_epoch += 1                            # the kernel below writes the parameters behind torch's back
+        if sh is not None and sh["dirty"]:
+            _lib.call("pcx_input_cat_flush_t", self._param_flows, sh["flows"], sh["touched"], sh["row_pfid"], sh["R"], sh["C"])
+        if not getattr(self, "_tied_folded", False):
+            for start, n, ch_pfids in self.tied2source_nids:
+                _lib.call("pcx_tied_accum", self._param_flows, int(start), int(n), ch_pfids, int(ch_pfids.numel()))
         _lib.call("pcx_em_input_cat", self.params.data, self._param_flows, self._dev["source_nids"],
                   self._dev["s_pids"], self._dev["s_pfids"], self._dev["node_cats"], int(self.source_nids.numel()), self.max_cats,
                   float(step_size), float(pseudocount), int(bool(keep_zero_params)))
+
+    def _mark_em(self, state):
+        """What the host keeps track of when an update has been launched (the kernels write the parameters behind torch's
+        back: the epoch tells the tables derived from them)."""
+        direct, flushed, _, _ = state
+        self._param_epoch += 1
+        if direct:
+            self._mark_shadow()
+            return
+        if flushed:
+            self._shadow["dirty"] = False
+            self._arena_zero = False
+        self._tied_folded = True
 
     def add_missing_flows(self, node_flows: torch.Tensor, scale: float = 1.0, **kwargs):
         """``node_flows``: one LINEAR flow per node of the circuit (``[num_nodes]``).  Every leaf's flow, plus that of
@@ -589,20 +632,20 @@ class SumLayer(Layer, nn.Module):
             self._dev = dict(
                 fw=[tuple(map(c, q)) for q in zip(self.partitioned_nids, self.partitioned_cids, self.partitioned_pids, self.partitioned_pfids)],
                 bk=[tuple(map(c, q)) for q in zip(self.partitioned_chids, self.partitioned_parids, self.partitioned_parpids)])
-            self._packed_fw = [None] * self.num_fw_partitions
-            self._packed_bk = [None] * self.num_bk_partitions
+            self._tiles_fw = [None] * self.num_fw_partitions
+            self._tiles_bk = [None] * self.num_bk_partitions
             if packer is not None:
                 self._packer = packer
                 bs = self.block_size
                 if bs % 128 == 0:
                     for p, (nids, cids, pids, _) in enumerate(self._dev["fw"]):
                         key = ("fw", bs, tuple(pids.shape), cpu_tables["partitioned_pids"][p].numpy().tobytes())
-                        self._packed_fw[p] = packer.register(key, nids.numel(), cids.size(1), bs, 1, 0, cids, pids)
+                        self._tiles_fw[p] = packer.register(key, nids.numel(), cids.size(1), bs, 1, 0, cids, pids)
                 for p, ((chids, parids, parpids), cbs) in enumerate(zip(self._dev["bk"], self.cs_block_sizes)):
                     if cbs % 128 == 0 and bs % 8 == 0:
                         key = ("bk", bs, cbs, tuple(parids.shape), cpu_tables["partitioned_parpids"][p].numpy().tobytes(),
                                (cpu_tables["partitioned_parids"][p] != 0).numpy().tobytes())
-                        self._packed_bk[p] = packer.register(key, chids.numel(), parids.size(1), cbs, bs, 1, parids, parpids)
+                        self._tiles_bk[p] = packer.register(key, chids.numel(), parids.size(1), cbs, bs, 1, parids, parpids)
                 # small blocks: sample-major tiles of one block, or of two consecutive blocks that list the same children
                 def merged_rows(table, ids, block):
                     """[(nb, first_row tensor)]: pairs of consecutive, identical rows (nb = 2 * block <= 64), then singles."""
@@ -664,6 +707,18 @@ class SumLayer(Layer, nn.Module):
             self._groups_bk = [groups_of(t) for t in cpu_tables["partitioned_parids"]]
         return self
 
+    @property
+    def _packed_fw(self):
+        """Forward parameter tiles per partition, up to date.  (A pass under the column program does not use them, so they
+        are packed when a caller of the per-layer entry points asks.)"""
+        self._packer.refresh_from_owner()
+        return self._tiles_fw
+
+    @property
+    def _packed_bk(self):
+        self._packer.refresh_from_owner()
+        return self._tiles_bk
+
     # Tables at least this deep take the two-step dense path (operand pre-pass + GEMM over pre-tiled operands).
     DENSE_MIN_DEPTH = 512
 
@@ -671,8 +726,8 @@ class SumLayer(Layer, nn.Module):
         if not self.use_dense_kernels or B % 64 != 0 or _lib.sum_mode() == 0:
             return False
         if backward:
-            return self._packed_bk[p] is not None and self._dev["bk"][p][1].size(1) * self.block_size >= self.DENSE_MIN_DEPTH
-        return self._packed_fw[p] is not None and self._dev["fw"][p][1].size(1) >= self.DENSE_MIN_DEPTH
+            return self._tiles_bk[p] is not None and self._dev["bk"][p][1].size(1) * self.block_size >= self.DENSE_MIN_DEPTH
+        return self._tiles_fw[p] is not None and self._dev["fw"][p][1].size(1) >= self.DENSE_MIN_DEPTH
 
     def _dense_scratch(self, n_groups: int, depth: int, B: int) -> torch.Tensor:
         return self._packer.scratch(int(_lib.load().pcx_dense_scratch_bytes(n_groups, depth, B)))
@@ -687,9 +742,9 @@ class SumLayer(Layer, nn.Module):
             return False
         if backward:
             depth = self._dev["bk"][p][1].size(1) * self.block_size
-            return self._packed_bk[p] is not None and self.DENSE_MIN_DEPTH <= depth <= self.DENSE_WIDE_MAX_DEPTH
+            return self._tiles_bk[p] is not None and self.DENSE_MIN_DEPTH <= depth <= self.DENSE_WIDE_MAX_DEPTH
         depth = self._dev["fw"][p][1].size(1)
-        return self._packed_fw[p] is not None and self.DENSE_MIN_DEPTH <= depth <= self.DENSE_WIDE_MAX_DEPTH
+        return self._tiles_fw[p] is not None and self.DENSE_MIN_DEPTH <= depth <= self.DENSE_WIDE_MAX_DEPTH
 
     def _wide_scratch(self, n_groups: int, depth: int, B: int):
         """Operand scratch of one wide-tile launch, shared by all layers (they run one after the other)."""
@@ -701,7 +756,7 @@ class SumLayer(Layer, nn.Module):
         B = node_mars.size(1)
         row_group, group_row, n_groups = self._groups_fw[p]
         scratch, nbytes = self._wide_scratch(n_groups, cids.size(1), B)
-        _lib.call("pcx_sum_fwd_dense2", node_mars, element_mars, self._packed_fw[p], nids, cids, fkids, fc, row_group,
+        _lib.call("pcx_sum_fwd_dense2", node_mars, element_mars, self._tiles_fw[p], nids, cids, fkids, fc, row_group,
                   group_row, n_groups, scratch, nbytes, nids.numel(), cids.size(1), self.block_size, B)
 
     def _backward_ele_wide(self, p: int, node_flows, element_flows, node_mars, element_mars, fkids, fc: int, direct: bool,
@@ -711,7 +766,7 @@ class SumLayer(Layer, nn.Module):
         B = node_flows.size(1)
         row_group, group_row, n_groups = self._groups_bk[p]
         scratch, nbytes = self._wide_scratch(n_groups, parids.size(1) * self.block_size, B)
-        _lib.call("pcx_sum_bwd_ele_dense2", element_flows, element_mars, node_flows, node_mars, self._packed_bk[p], chids,
+        _lib.call("pcx_sum_bwd_ele_dense2", element_flows, element_mars, node_flows, node_mars, self._tiles_bk[p], chids,
                   parids, fkids, fc, int(bool(direct)), row_group, group_row, n_groups, scratch, nbytes,
                   chids.numel(), parids.size(1), self.block_size, cbs, B, int(bool(logspace_flows)))
 
@@ -747,10 +802,10 @@ class SumLayer(Layer, nn.Module):
             elif packed and self._dense_ok(p, B, False):
                 row_group, group_row, n_groups = self._groups_fw[p]
                 scratch = self._dense_scratch(n_groups, cids.size(1), B)
-                _lib.call("pcx_sum_fwd_dense", node_mars, element_mars, self._packed_fw[p], nids, cids, row_group,
+                _lib.call("pcx_sum_fwd_dense", node_mars, element_mars, self._tiles_fw[p], nids, cids, row_group,
                           group_row, n_groups, scratch, scratch.numel(), nids.numel(), cids.size(1), self.block_size, B)
-            elif packed and self._packed_fw[p] is not None:
-                _lib.call("pcx_sum_fwd_packed", node_mars, element_mars, self._packed_fw[p], nids, cids,
+            elif packed and self._tiles_fw[p] is not None:
+                _lib.call("pcx_sum_fwd_packed", node_mars, element_mars, self._tiles_fw[p], nids, cids,
                           nids.numel(), cids.size(1), self.block_size, B)
             elif packed and self.use_sample_major and self._sm_fw[p] is not None:
                 for nb, first_row, n_merged, buf in self._sm_fw[p]:
@@ -776,7 +831,7 @@ class SumLayer(Layer, nn.Module):
                 self._forward_wide(p, node_mars, None, f["fw"][p], f["fc"])
             return
         for p, (nids, cids, _, _) in enumerate(self._dev["fw"]):
-            _lib.call("pcx_sum_fwd_fused", node_mars, self._packed_fw[p], nids, cids, f["fw"][p], f["fc"],
+            _lib.call("pcx_sum_fwd_fused", node_mars, self._tiles_fw[p], nids, cids, f["fw"][p], f["fc"],
                       nids.numel(), cids.size(1), self.block_size, B)
 
     def backward_ele_fused(self, node_flows, element_flows, node_mars, logspace_flows: bool):
@@ -794,7 +849,7 @@ class SumLayer(Layer, nn.Module):
                                         f["bk"][p], f["fc"], f["direct"], logspace_flows)
             return
         for p, ((chids, parids, _), cbs) in enumerate(zip(self._dev["bk"], self.cs_block_sizes)):
-            _lib.call("pcx_sum_bwd_ele_fused", element_flows, node_flows, node_mars, self._packed_bk[p], chids, parids,
+            _lib.call("pcx_sum_bwd_ele_fused", element_flows, node_flows, node_mars, self._tiles_bk[p], chids, parids,
                       f["bk"][p], f["fc"], int(f["direct"]), chids.numel(), parids.size(1), self.block_size, cbs, B,
                       int(bool(logspace_flows)))
 
@@ -840,11 +895,11 @@ class SumLayer(Layer, nn.Module):
             elif packed and self._dense_ok(p, B, True):
                 row_group, group_row, n_groups = self._groups_bk[p]
                 scratch = self._dense_scratch(n_groups, parids.size(1) * self.block_size, B)
-                _lib.call("pcx_sum_bwd_ele_dense", element_flows, element_mars, node_flows, node_mars, self._packed_bk[p],
+                _lib.call("pcx_sum_bwd_ele_dense", element_flows, element_mars, node_flows, node_mars, self._tiles_bk[p],
                           chids, parids, row_group, group_row, n_groups, scratch, scratch.numel(), chids.numel(),
                           parids.size(1), self.block_size, cbs, B, ls)
-            elif packed and self._packed_bk[p] is not None:
-                _lib.call("pcx_sum_bwd_ele_packed", element_flows, element_mars, node_flows, node_mars, self._packed_bk[p],
+            elif packed and self._tiles_bk[p] is not None:
+                _lib.call("pcx_sum_bwd_ele_packed", element_flows, element_mars, node_flows, node_mars, self._tiles_bk[p],
                           chids, parids, chids.numel(), parids.size(1), self.block_size, cbs, B, ls)
             elif packed and self.use_sample_major and self._sm_bk[p] is not None:
                 for nb, first_row, n_merged, buf in self._sm_bk[p]:
@@ -859,7 +914,7 @@ class SumLayer(Layer, nn.Module):
                 if (stage is not None and packed and (self._dense_ok(p, B, False) or self._wide_ok(p, B, False))
                         and self._groups_fw[p][2] == 1 and stage(self, p, node_flows, node_mars, element_mars, ls)):
                     continue                       # this table's flows come out of one product over all staged layers
-                if (packed and self.use_sample_major and self._packed_fw[p] is None and self._sm_fw[p] is not None
+                if (packed and self.use_sample_major and self._tiles_fw[p] is None and self._sm_fw[p] is not None
                         and B % 8 == 0):
                     for nb, first_row, n_merged, _ in self._sm_fw[p]:
                         _lib.call("pcx_sum_bwd_par_sm", param_flows, node_flows, node_mars, element_mars, params,

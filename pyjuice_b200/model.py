@@ -19,6 +19,7 @@ from __future__ import annotations
 import contextlib
 import functools
 import os
+import weakref
 from functools import partial
 from typing import Optional, Sequence, Union
 
@@ -94,7 +95,7 @@ class TensorCircuit(nn.Module):
         self.use_cuda_graphs = True
         self._column_program = None
         self.use_dataflow_launch = True       # runs of folded depths as one launch (tiles wait on counters)
-        self.use_column_program = True        # circuits of small node blocks: all levels in one launch
+        self.use_column_program = True        # all levels in one launch (see column.py)
         self.use_side_stream = True           # independent kernels of a step share the device (two streams)
         self.debug_poison = False             # fill value / flow buffers with NaN before every pass (see `assert_no_poison`)
         self.use_nvtx = bool(os.environ.get("PCX_B200_NVTX"))     # NVTX ranges around the phases of a step (profilers)
@@ -327,7 +328,7 @@ class TensorCircuit(nn.Module):
             _lib.load()                                   # fail here, loudly, if the kernels are not built
         nn.Module.to(self, device)
         self.input_layer_group.to(device)
-        self._packer = ParamPacker(device) if device.type == "cuda" else None
+        self._packer = ParamPacker(device, weakref.ref(self)) if device.type == "cuda" else None
         for group in self.inner_layer_groups:
             if group.is_sum():
                 group.to(device, packer=self._packer)
@@ -379,8 +380,8 @@ class TensorCircuit(nn.Module):
                         parents.index_add_(0, rows, torch.ones_like(rows, dtype=torch.int32))
         for gi in range(1, len(self.inner_layer_groups), 2):
             pgroup, sgroup = self.inner_layer_groups[gi - 1], self.inner_layer_groups[gi]
-            big = all(l.block_size % 128 == 0 and l._packer is not None and all(b is not None for b in l._packed_fw)
-                      and all(b is not None for b in l._packed_bk) for l in sgroup)
+            big = all(l.block_size % 128 == 0 and l._packer is not None and all(b is not None for b in l._tiles_fw)
+                      and all(b is not None for b in l._tiles_bk) for l in sgroup)
             # small blocks (sample-major tiles): products of at most two children can be folded in as well
             small = (not big) and all(l._packer is not None and getattr(l, "_sm_fw", None) is not None
                                       and all(t is not None for t in l._sm_fw) and all(t is not None for t in l._sm_bk)
@@ -570,17 +571,19 @@ class TensorCircuit(nn.Module):
         return (not backward) or self._nm.size(1) % 8 == 0
 
     def _column_plan(self):
-        """The column program's plan for the current row width, or None where the per-layer kernels run: a node block of
-        more than 64 nodes (their tables fill 128-row tensor-core tiles), fp32 or rule-based passes, `reference_compat`."""
-        if (not (self.use_column_program and self.fuse_product_layers and SumLayer.use_sample_major) or self._reference_compat
-                or self._alg[0] != 0 or _lib.sum_mode() == 0):
+        """The column program's plan for the current row width, or None where the per-layer kernels run: a dense table of
+        more than 1024 children under large blocks (those fill the wide dense kernels), fp32 or rule-based passes,
+        `reference_compat`, and any switch that asks for other kernels."""
+        if (not (self.use_column_program and self.fuse_product_layers and self.use_dataflow_launch and self.chain_tile is None
+                 and SumLayer.use_sample_major and SumLayer.use_dense_kernels and SumLayer.use_wide_dense)
+                or self._reference_compat or self._alg[0] != 0 or _lib.sum_mode() == 0):
             return None
         if self._column_program is None:
             try:
                 self._column_program = ColumnProgram(self)
             except Unsupported:
                 self._column_program = False
-        return self._column_program.plan(self._nm.size(1)) if self._column_program else None
+        return self._column_program.choose(self._nm.size(1)) if self._column_program else None
 
     def _launch_cfg(self):
         """Everything that changes which kernels a pass launches (part of the key of a captured graph)."""
@@ -627,11 +630,11 @@ class TensorCircuit(nn.Module):
                         f = layer._fusion
                         if mode == 0:
                             for p, (nids, cids, _, _) in enumerate(layer._dev["fw"]):
-                                jobs.append((layer._packed_fw[p], nids, cids, f["fw"][p], cids.size(1), layer.block_size, 1,
+                                jobs.append((layer._tiles_fw[p], nids, cids, f["fw"][p], cids.size(1), layer.block_size, 1,
                                              nids.numel() * (layer.block_size // 128), level))
                         else:
                             for p, ((chids, parids, _), cbs) in enumerate(zip(layer._dev["bk"], layer.cs_block_sizes)):
-                                jobs.append((layer._packed_bk[p], chids, parids, f["bk"][p], parids.size(1), cbs,
+                                jobs.append((layer._tiles_bk[p], chids, parids, f["bk"][p], parids.size(1), cbs,
                                              layer.block_size, chids.numel() * (cbs // 128), level))
                 level_tiles = [0] * len(levels)
                 for j in jobs:
@@ -825,7 +828,7 @@ class TensorCircuit(nn.Module):
                     if not ((wide or layer._dense_ok(p, B, False)) and layer._groups_fw[p][2] == 1):
                         assert not folded, "a dense-folded table must qualify for the dense parameter-flow product"
                         continue
-                    g = groups.setdefault((layer._packed_fw[p].data_ptr(), wide),
+                    g = groups.setdefault((layer._tiles_fw[p].data_ptr(), wide),
                                           dict(members=[], tables=(cids, pids, pfids), n_blocks=nids.numel(),
                                                K=cids.size(1), block_size=layer.block_size, wide=wide))
                     where[(id(layer), p)] = (g, len(g["members"]))
@@ -1190,19 +1193,9 @@ class TensorCircuit(nn.Module):
                 layer._arena_zero = True
             self._graphs = {k: g for k, g in self._graphs.items() if k[0] != "bk"}
         elif flows_memory == 0.0:
-            # Input layers whose accumulators are known to be empty still (all their flows went to the transposed
-            # shadow and were consumed from there, nothing read or wrote the accumulators proper) need no clearing:
-            # on configs[4] that is 2.1 GB of replica accumulators per step.
-            arena, layers = self._flow_arena, list(self.input_layer_group)
-            clean = [bool(getattr(layer, "_arena_zero", False)) for layer in layers]
-            for layer in layers:
-                layer._zero_shadow()
-            if all(clean):
-                _fill(arena.buf[:arena.segment_end(0)], 0.0)
-            else:
-                _fill(arena.buf, 0.0)
-            for layer in layers:
-                layer._arena_zero = True
+            self._clear_launches()
+            for layer in self.input_layer_group:
+                layer._mark_cleared()
         elif flows_memory != 1.0:
             for layer in self.input_layer_group:
                 layer._flush_shadow()
@@ -1216,6 +1209,19 @@ class TensorCircuit(nn.Module):
                 self._cum_flow_host, self._cum_flow_dev, self._cum_flow_head = 0.0, None, None
             else:
                 self._cum_flow = self._cum_flow * flows_memory
+
+    def _clear_launches(self, em_state=None):
+        """``em_state``: the update that has just been launched (see `InputLayer._em_state`): flows it moved out of a shadow
+        are in the accumulators.  Input layers whose accumulators are known to be empty still (all their flows went to the transposed shadow and
+        were consumed from there, nothing read or wrote the accumulators proper) need no clearing: on configs[4] that is
+        2.1 GB of replica accumulators per step."""
+        arena, clean = self._flow_arena, True
+        for i, layer in enumerate(self.input_layer_group):
+            moved = em_state is not None and em_state[i][1]
+            if not moved:
+                layer._launch_zero_shadow()
+            clean = clean and layer._arena_zero and not moved
+        _fill(arena.buf[:arena.segment_end(0)] if clean else arena.buf, 0.0)
 
     def zero_param_flows(self):
         self.init_param_flows(flows_memory=0.0)
@@ -1270,6 +1276,37 @@ class TensorCircuit(nn.Module):
                 self._nm, self._em, self._nf, self._ef, self._eflow_mode = saved
         return td
 
+    def _em_step(self, step_size: float, pseudocount: float, keep_zero_params: bool):
+        """`mini_batch_em` followed by clearing the accumulators, as optimizers do after every batch: the same launches, from
+        a captured graph once the same step has been made twice (an update of a small circuit is a handful of kernels of
+        2 us each, and twice that in host work when they are launched one by one; large updates cover their launches)."""
+        assert 0.0 < step_size <= 1.0, "`step_size` should be between 0 and 1."
+        self._require_cuda()
+        layers = list(self.input_layer_group)
+        state = tuple(layer._em_state(keep_zero_params) for layer in layers)
+        if (not self.use_cuda_graphs or self._reference_compat or getattr(self, "_late_sync", None) is not None
+                or self.param_flows is None or self.num_sum_params >= self._EM_FORK_PARAMS
+                or any(layer._shadow is not None or layer.num_parameters >= 4 * self._EM_FORK_PARAMS for layer in layers)):
+            self.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
+            self.init_param_flows(flows_memory=0.0)
+            return
+        key = ("em", step_size, pseudocount, keep_zero_params, state, self.use_side_stream, self._param_ptrs(),
+               self.param_flows.data_ptr())
+        if key not in self._graphs:
+            seen = [k for k in self._graphs if k[0] == "em"]
+            if len(seen) >= 4:                               # a schedule of step sizes: keep the latest few
+                del self._graphs[seen[0]]
+        def launches():
+            self._em_launches(step_size, pseudocount, keep_zero_params)
+            self._clear_launches(state)
+        with torch.no_grad():
+            self._run_inner(key, launches)
+        self._packer.invalidate()
+        for layer, st in zip(layers, state):
+            layer._mark_em(st)
+            layer._mark_cleared()
+        self._cum_flow_host, self._cum_flow_dev, self._cum_flow_head = 0.0, None, None
+
     # Below this many sum parameters the update of either kind takes a few microseconds, less than the host spends on
     # sending work to a second stream and joining it again (35 us).
     _EM_FORK_PARAMS = 1 << 21
@@ -1293,41 +1330,45 @@ class TensorCircuit(nn.Module):
             self._cum_flow = 0.0
             step_size = 1.0
         with torch.no_grad():
-            def sum_update():
-                head = self.param_flows[:2048].clone() if (self._reference_compat and self._fusing_dev) else None
-                for start, n, chs in self._fusing_dev:
-                    _lib.call("pcx_tied_accum", self.param_flows, start, n, chs, int(chs.numel()))
-                if head is not None:
-                    for tgt, sizes, ch, G, M in self.parflow_fusing_kwargs:
-                        pads = ((ch == 0).sum(dim=1) - (ch[:, 0] == 0).long()).tolist()
-                        for t, n, pad in zip(tgt.tolist(), sizes.tolist(), pads):
-                            if pad > 0:
-                                self.param_flows[t:t + n].add_(head[:n], alpha=float(pad))
-                e = self._em_dev
-                _lib.call("pcx_em_sum", self.params.data, self.param_flows, e["par"], e["flow"], e["fan"], e["bs"],
-                          int(e["par"].numel()), e["max_bs"], float(step_size), float(pseudocount),
-                          int(bool(keep_zero_params)))
-                self._packer.invalidate()
+            self._em_launches(step_size, pseudocount, keep_zero_params)
+            self._packer.invalidate()
+            for layer in self.input_layer_group:
+                layer._mark_em(layer._em_state(keep_zero_params))
 
-            def input_update():
-                for layer in self.input_layer_group:
-                    layer.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
+    def _em_launches(self, step_size: float, pseudocount: float, keep_zero_params: bool):
+        def sum_update():
+            head = self.param_flows[:2048].clone() if (self._reference_compat and self._fusing_dev) else None
+            for start, n, chs in self._fusing_dev:
+                _lib.call("pcx_tied_accum", self.param_flows, start, n, chs, int(chs.numel()))
+            if head is not None:
+                for tgt, sizes, ch, G, M in self.parflow_fusing_kwargs:
+                    pads = ((ch == 0).sum(dim=1) - (ch[:, 0] == 0).long()).tolist()
+                    for t, n, pad in zip(tgt.tolist(), sizes.tolist(), pads):
+                        if pad > 0:
+                            self.param_flows[t:t + n].add_(head[:n], alpha=float(pad))
+            e = self._em_dev
+            _lib.call("pcx_em_sum", self.params.data, self.param_flows, e["par"], e["flow"], e["fan"], e["bs"],
+                      int(e["par"].numel()), e["max_bs"], float(step_size), float(pseudocount), int(bool(keep_zero_params)))
 
-            # sum parameters and input-layer parameters are disjoint
-            if getattr(self, "_late_sync", None) is not None:
-                input_update()                              # beside the all-reduce of the sum-layer flows
-                self._finish_late_sync()
+        def input_update():
+            for layer in self.input_layer_group:
+                layer._launch_em(step_size, pseudocount, keep_zero_params)
+
+        # sum parameters and input-layer parameters are disjoint
+        if getattr(self, "_late_sync", None) is not None:
+            input_update()                                  # beside the all-reduce of the sum-layer flows
+            self._finish_late_sync()
+            sum_update()
+        elif self.use_side_stream and self.num_sum_params >= self._EM_FORK_PARAMS:    # on two streams
+            cur = torch.cuda.current_stream(self.device)
+            self._side_stream.wait_stream(cur)
+            with torch.cuda.stream(self._side_stream):
                 sum_update()
-            elif self.use_side_stream and self.num_sum_params >= self._EM_FORK_PARAMS:    # on two streams
-                cur = torch.cuda.current_stream(self.device)
-                self._side_stream.wait_stream(cur)
-                with torch.cuda.stream(self._side_stream):
-                    sum_update()
-                input_update()
-                cur.wait_stream(self._side_stream)
-            else:
-                sum_update()
-                input_update()
+            input_update()
+            cur.wait_stream(self._side_stream)
+        else:
+            sum_update()
+            input_update()
 
     def sync_param_flows(self, dtype: Optional[torch.dtype] = None, op=None, group=None, sync_cum_flow: bool = True,
                          _lazy: bool = False):

@@ -36,13 +36,14 @@ def _program(pc):
 
 @pytest.mark.parametrize("B", [1, 8, 31, 200, 257])
 @pytest.mark.parametrize("kind,latents", [("hclt", 8), ("hclt", 24), ("hclt", 64), ("hclt", 96), ("pd", 16), ("pd", 64),
-                                          ("rat", 32), ("rat", 8), ("hmm", 64), ("hmm", 320), ("hmm", 4)])
+                                          ("rat", 32), ("rat", 8), ("hmm", 64), ("hmm", 320), ("hmm", 4),
+                                          ("hmm", 128), ("hmm", 512), ("hmm", 1024), ("hclt", 128), ("hclt", 256), ("rat", 128)])
 def test_against_oracle(kind, latents, B):
     pc = pj.compile(_circuit(kind, latents)).to(DEV)
     cats = min(l.max_cats for l in pc.input_layer_group)
     x = torch.randint(0, cats, (B, pc.num_vars), generator=torch.Generator().manual_seed(B))
     errs = check_against_oracle(pc, x, step=0.2, pseudo=0.1)
-    _program(pc)
+    assert latents >= 128 or pc._column_plan() is not None
     pc.validate_tables()
     print(errs)
 
@@ -62,7 +63,8 @@ def test_wide_levels(kind, latents, logspace, B, monkeypatch):
     pc.validate_tables()
 
 
-@pytest.mark.parametrize("kind,latents", [("hclt", 32), ("pd", 64), ("rat", 8), ("hmm", 64)])
+@pytest.mark.parametrize("kind,latents", [("hclt", 32), ("pd", 64), ("rat", 8), ("hmm", 64), ("hmm", 256), ("hmm", 1024),
+                                          ("hclt", 256)])
 def test_equals_the_per_layer_kernels(kind, latents):
     pc = pj.compile(_circuit(kind, latents)).to(DEV)
     cats = min(l.max_cats for l in pc.input_layer_group)
