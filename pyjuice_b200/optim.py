@@ -76,8 +76,7 @@ class MiniBatchEM(CircuitOptimizer):
         if self.sync_every <= 1:
             self._sync_flows()           # synchronous data parallelism: one update on the summed flows
         ss = self.step_size if step_size is None else step_size
-        self.pc.mini_batch_em(step_size=ss, pseudocount=self.pseudocount, keep_zero_params=self.keep_zero_params)
-        self.zero_flows()
+        self.pc._em_step(ss, self.pseudocount, self.keep_zero_params)
         self._post_update_sync()
 
 
@@ -92,5 +91,4 @@ class FullBatchEM(CircuitOptimizer):
     def step(self, step_size: Optional[float] = None):
         self._sync_flows()
         ss = 1.0 if step_size is None else step_size
-        self.pc.mini_batch_em(step_size=ss, pseudocount=self.pseudocount, keep_zero_params=self.keep_zero_params)
-        self.zero_flows()
+        self.pc._em_step(ss, self.pseudocount, self.keep_zero_params)
