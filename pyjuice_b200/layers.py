@@ -123,7 +123,10 @@ class ParamPacker:
 
     # ``plan``: a plan of the column program; its parameter fragments then stand in for all tiles of the per-layer kernels.
     def _stamp_of(self, params: torch.Tensor):
-        return (params.data_ptr(), params._version, self._epoch)
+        # (``.data`` of a parameter counts versions of its own: the circuit's parameter tells for both)
+        pc, ptr = self.owner() if self.owner is not None else None, params.data_ptr()
+        own = pc is not None and pc._sum_params.data_ptr() == ptr
+        return (ptr, pc._sum_params._version if own else params._version, self._epoch)
 
     def stale(self, params: torch.Tensor, plan=None) -> bool:
         """Whether the tiles lag behind ``params``."""
@@ -248,6 +251,8 @@ class InputLayer(Layer, nn.Module):
             object.__setattr__(self, name, value)
         else:
             nn.Module.__setattr__(self, name, value)
+            if name == "params":                            # reads go through `__dict__`, not `nn.Module.__getattr__`
+                object.__setattr__(self, "_leaf_params", value)
 
     def is_input(self):
         return True
@@ -375,7 +380,7 @@ class InputLayer(Layer, nn.Module):
             self._mark_shadow()
 
     def _shadow_stamp(self):
-        return (self.params.data_ptr(), self.params._version, self._param_epoch)
+        return (self._leaf_params.data_ptr(), self._leaf_params._version, self._param_epoch)
 
     def _shadow_stale(self, B: int) -> bool:
         return self._shadow_ok(B) and self._shadow["stamp"] != self._shadow_stamp()

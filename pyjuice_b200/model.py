@@ -46,6 +46,9 @@ def _pc_model_backward_hook(grad, pc, inputs, **kwargs):
     return None
 
 
+_LL = (0, 0.0)
+
+
 def _in_own_mode(fn):
     """Run a public method in the circuit's own arithmetic mode (``self.sum_mode``; None = the process default).
     A pass under another propagation rule ("MPE", "GeneralLL") runs on the plain fp32 kernels (mode 0: nothing is
@@ -57,11 +60,11 @@ def _in_own_mode(fn):
             name = kwargs.get("propagation_alg")
             if name is None:
                 name = self.default_propagation_alg if fn.__name__ == "forward" else "LL"
-                if fn.__name__ == "forward":
+                if fn.__name__ == "forward" and self.propagation_alg_kwargs:
                     kwargs = {**self.propagation_alg_kwargs, **kwargs}
             if not isinstance(name, str):
                 raise NotImplementedError("one propagation rule per layer is outside the compiled path")
-            self._alg = _alg_of(name, kwargs)
+            self._alg = _LL if name == "LL" else _alg_of(name, kwargs)
             kwargs["propagation_alg"] = name
             if self._alg[0] != 0:
                 mode = 0
@@ -108,6 +111,7 @@ class TensorCircuit(nn.Module):
         self._run_params = {}
         self._cum_flow_host = 0.0
         self._cum_flow_dev = None
+        self._late_sync = None
         self._eflow_mode = 1
         self._reference_compat = False
 
@@ -118,6 +122,10 @@ class TensorCircuit(nn.Module):
             object.__setattr__(self, name, value)
         else:
             nn.Module.__setattr__(self, name, value)
+            if name == "params":                            # reads go through `__dict__`, not `nn.Module.__getattr__`
+                object.__setattr__(self, "_sum_params", value)
+            elif name == "input_layer_group":
+                object.__setattr__(self, "_leaf_layers", tuple(value) if value is not None else ())
 
     @property
     def reference_compat(self) -> bool:
@@ -342,7 +350,7 @@ class TensorCircuit(nn.Module):
         self._fusing_dev = [(start, n, torch.tensor(accs, dtype=torch.int64, device=device))
                             for start, n, accs in self._tied_sum_groups]
         self._nm = self._em = self._nf = self._ef = self.param_flows = None
-        self._data_buf = self._root_mars = self._root_w = self._cum_buf = None
+        self._data_buf = self._root_view = self._root_w = self._cum_buf = None
         if device.type == "cuda":
             self._mask_parentless_in_device_tables()
         self._setup_fusion()
@@ -497,14 +505,17 @@ class TensorCircuit(nn.Module):
     def _ensure_buffers(self, B: int, backward: bool = False):
         """(Re)allocate the value buffers when the padded batch size changes.  Dummy rows are written here once:
         every other row is fully overwritten by the layer that owns it on each pass."""
+        changed = self._batch != B
         self._batch = B
         W = -(-B // self._PAD) * self._PAD
         if self._nm is None or self._nm.size(1) != W:
             self._nm = torch.zeros(self.num_nodes, W, device=self.device)
             self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
-            self._root_mars = self._nm[self._root_node_range[0]:self._root_node_range[1]]
+            changed = True
             self._nf = self._ef = None
             self._graphs = {}
+        if changed:
+            self._root_view = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t()
         if backward and (self._nf is None or self._nf.size(1) != W):
             self._nf = torch.empty(self.num_nodes, W, device=self.device)
             self._ef = torch.full((self.num_elements, W), NEG_INF, device=self.device)
@@ -707,7 +718,7 @@ class TensorCircuit(nn.Module):
         return self.forward(*args, propagation_alg="GeneralLL", **kwargs)
 
     def _param_ptrs(self):
-        return (self.params.data_ptr(),) + tuple(layer.params.data_ptr() for layer in self.input_layer_group)
+        return (self._sum_params.data_ptr(), *[layer._leaf_params.data_ptr() for layer in self._leaf_layers])
 
     def _forward_pass(self, data: torch.Tensor, pack: bool, shadows):
         """All launches of a forward pass on the batch in ``data``, captured as one graph.  The operand tiles of the
@@ -734,9 +745,10 @@ class TensorCircuit(nn.Module):
                 propagation_alg: Optional[str] = None, pflow_temperature: float = 1.0, **kwargs):
         """Per-sample log-likelihoods ``[B, num_roots]`` of ``inputs`` (``[B, num_vars]``, integer)."""
         self._require_cuda()
-        _unsupported(input_layer_fn=input_layer_fn is not None, cache=cache is not None, return_cache=return_cache,
-                     pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6,
-                     missing_mask=kwargs.get("missing_mask") is not None)
+        if kwargs or input_layer_fn is not None or cache is not None or return_cache or pflow_temperature != 1.0:
+            _unsupported(input_layer_fn=input_layer_fn is not None, cache=cache is not None, return_cache=return_cache,
+                         pflow_temperature=abs(pflow_temperature - 1.0) > 1e-6,
+                         missing_mask=kwargs.get("missing_mask") is not None)
         origin_inputs = inputs
         with torch.no_grad():
             B = inputs.size(0)
@@ -747,19 +759,20 @@ class TensorCircuit(nn.Module):
             if self.debug_poison:               # every row must be rewritten by the layer that owns it
                 _fill(self._nm[self.num_dummy_nodes:], float("nan"))
             plan = self._column_plan()
-            pack = _lib.sum_mode() != 0 and self._packer.stale(self.params.data, plan)
-            shadows = tuple(layer._shadow_stale(W) for layer in self.input_layer_group)
+            pack = _lib.sum_mode() != 0 and self._packer.stale(self._sum_params, plan)
+            shadows = tuple([layer._shadow_stale(W) for layer in self._leaf_layers])
             key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
             self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
             if pack:
-                self._packer.mark(self.params.data, plan)
-            for layer, stale in zip(self.input_layer_group, shadows):
+                self._packer.mark(self._sum_params, plan)
+            for layer, stale in zip(self._leaf_layers, shadows):
                 if stale:
                     layer._mark_shadow()
-            lls = self._root_mars[:, :B].t().clone()
+            lls = self._root_view.clone()
         if torch.is_grad_enabled():
-            lls.requires_grad = True
-            lls.register_hook(partial(_pc_model_backward_hook, pc=self, inputs=origin_inputs, **self._alg_kwargs()))
+            lls.requires_grad_()
+            lls.register_hook(partial(_pc_model_backward_hook, pc=self, inputs=origin_inputs,
+                                      **(self._alg_kwargs() if self._alg[0] else {})))
         return lls
 
     # ------------------------------------------------------------------------------------------
@@ -1009,8 +1022,8 @@ class TensorCircuit(nn.Module):
                 # cleared once per pass, as the reference does, and rows without a writer keep an earlier depth's flow)
                 _fill(self._ef, NEG_INF if logspace_flows else 0.0)
                 self._eflow_mode = ls
-            if compute_param_flows:                          # decay (or clear) the accumulators and the flow total first
-                self.init_param_flows(flows_memory=flows_memory)
+            if compute_param_flows and (flows_memory != 1.0 or self.param_flows is None or self._late_sync is not None):
+                self.init_param_flows(flows_memory=flows_memory)     # decay (or clear) the accumulators and the flow total
             r0, r1 = self._root_node_range
             if self._root_w is None or self._root_w.size(1) != W:
                 self._root_w = torch.empty(r1 - r0, W, device=self.device)
@@ -1029,7 +1042,7 @@ class TensorCircuit(nn.Module):
                 self._cum_flow_dev = total
 
             if _lib.sum_mode() != 0:
-                self._packer.refresh(self.params.data, self._column_plan())
+                self._packer.refresh(self._sum_params, self._column_plan())
             # The parameter flows of the sum layers and of the input layer close the pass.  They belong to the captured
             # pass too, unless data-parallel ranks overlap them with the all-reduce, or the leaves see another batch.
             tail = compute_param_flows and own and not self._overlap_ready()
@@ -1041,7 +1054,7 @@ class TensorCircuit(nn.Module):
                                              bool(logspace_flows)))
             self._bk_par_pending[key] = self._batched_par_pending
             if tail:
-                for layer in self.input_layer_group:
+                for layer in self._leaf_layers:
                     layer._mark_backward(W)
             elif compute_param_flows:
                 # the input layer first, then the all-reduce of its flows (the larger part of the arena) beside the sum
@@ -1097,9 +1110,11 @@ class TensorCircuit(nn.Module):
         self._overlap_dtype = dtype                      # e.g. bfloat16: both parts travel in reduced precision
 
     def _overlap_ready(self) -> bool:
-        import torch.distributed as dist
         g = getattr(self, "_overlap_group", None)
-        return (g is not None and self.device.type == "cuda" and dist.is_available() and dist.is_initialized()
+        if g is None:
+            return False
+        import torch.distributed as dist
+        return (self.device.type == "cuda" and dist.is_available() and dist.is_initialized()
                 and dist.get_world_size(g[0]) > 1)
 
     def _input_reduce_end(self) -> int:
@@ -1282,7 +1297,7 @@ class TensorCircuit(nn.Module):
         2 us each, and twice that in host work when they are launched one by one; large updates cover their launches)."""
         assert 0.0 < step_size <= 1.0, "`step_size` should be between 0 and 1."
         self._require_cuda()
-        layers = list(self.input_layer_group)
+        layers = self._leaf_layers
         state = tuple(layer._em_state(keep_zero_params) for layer in layers)
         if (not self.use_cuda_graphs or self._reference_compat or getattr(self, "_late_sync", None) is not None
                 or self.param_flows is None or self.num_sum_params >= self._EM_FORK_PARAMS
