@@ -274,11 +274,12 @@ int pcx_sum_bwd_ele_dense2(float* element_flows, const float* element_mars, floa
 /* Parameter flows: step 1 writes the operands of one layer at sample positions [slot * B, (slot + 1) * B) of the
  * concatenated batch (x_tiles: [row tiles][n_chunks_total] tiles of 32 KB; y_tiles: [ceil(K / 256)][n_chunks_total]
  * tiles of 64 KB; both zero-filled once by the caller; n_chunks_total = ceil(layers * B / 64)); `cids_row` / `fkids_row`
- * are the children of table row 0 (every row lists the same).  Step 2 is one product per group of tied layers. */
+ * are the children of table row 0 (every row lists the same).  `n_slots` layers of equal shape go in one call: layer y has
+ * nids[y * n_blocks ...], cids_row / fkids_row[y * K ...] and slot + y.  Step 2 is one product per group of tied layers. */
 int pcx_sum_par_dense2_stage(void* x_tiles, void* y_tiles, const float* node_flows, const float* node_mars,
                              const float* element_mars, const int32_t* nids, const int32_t* cids_row,
                              const int32_t* fkids_row, int fc, int64_t n_blocks, int K, int block_size, int B,
-                             int n_chunks_total, int slot, int logspace, void* stream);
+                             int n_chunks_total, int slot, int n_slots, int logspace, void* stream);
 int pcx_sum_par_dense2_gemm(float* param_flows, const float* params, const void* x_tiles, const void* y_tiles,
                             const int32_t* cids, const int32_t* pids, const int32_t* pfids, int64_t n_blocks, int K,
                             int block_size, int n_chunks_total, void* stream);

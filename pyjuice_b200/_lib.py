@@ -74,7 +74,7 @@ SIGNATURES = {
     "pcx_column_par": [I, P, P, P, P, P, P, P, P, I, I, I, I],
     "pcx_sum_fwd_dense2": [P, P, P, P, P, P, I, P, P, I, P, L, L, I, I, I],
     "pcx_sum_bwd_ele_dense2": [P, P, P, P, P, P, P, P, I, I, P, P, I, P, L, L, I, I, I, I, I],
-    "pcx_sum_par_dense2_stage": [P, P, P, P, P, P, P, P, I, L, I, I, I, I, I, I],
+    "pcx_sum_par_dense2_stage": [P, P, P, P, P, P, P, P, I, L, I, I, I, I, I, I, I],
     "pcx_sum_par_dense2_gemm": [P, P, P, P, P, P, P, L, I, I, I],
 }
 

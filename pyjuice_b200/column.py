@@ -76,7 +76,8 @@ class ColumnProgram:
     def __init__(self, pc):
         self.device = pc.device
         self.num_dummy = pc.num_dummy_nodes
-        self._by_width, self._choice, self._rooms, self._par = {}, {}, {}, None
+        self.dense_par_bytes = pc.dense_par_max_bytes
+        self._by_width, self._choice, self._rooms, self._par = {}, {}, {}, {}
         groups = pc.inner_layer_groups
         self.depths = []
         parents = np.zeros(pc.num_nodes + 1, dtype=np.int32)
@@ -414,12 +415,15 @@ class ColumnProgram:
         out["kids"] = kids.tensor(dev)
         return out
 
-    @property
-    def par(self):
-        """Jobs of the parameter flows (the same for every row width), built when the first pass needs them."""
-        if self._par is None:
-            self._par = self._par_jobs()
-        return self._par
+    def par(self, W: int):
+        """Tables of the parameter flows for rows of W samples, built when the first pass needs them: the groups of tied
+        tables that go through one dense product, and the jobs of all others."""
+        if "tied" not in self._par:
+            self._par["tied"] = self._tied_groups()
+        pick = tuple(g["n"] * W * g["n_blocks"] * g["bs"] * g["K"] >= self.DENSE_PAR_WORK for g in self._par["tied"])
+        if pick not in self._par:
+            self._par[pick] = self._par_jobs([g for g, p in zip(self._par["tied"], pick) if p])
+        return self._par[pick]
 
     @staticmethod
     def _level(tasks, levels, strips, first, split, how):
@@ -555,12 +559,54 @@ class ColumnProgram:
                 tasks.append((kids.add(rows), len(g.ops) * pbs, 1, 2, strips.add(st), n, 0, K_SIMT, 1, pbs, lg, 0))
 
     # ---- parameter flows ---------------------------------------------------------------------------------------------
-    def _par_jobs(self):
+    # Tied tables contract one product over all their layers' samples.  A 64 x 64 tile of a job of its own forms the
+    # exponentials of its rows and of its elements again for every tile they belong to; the product of the dense layers forms
+    # them once (`pcx_sum_par_dense2_stage`) and multiplies on the fifth-generation tensor cores, but takes two launches and
+    # two more passes over the operands.  Rows x children x samples where the two meet, from HMMs of 128 to 1024 states
+    # (microseconds, jobs / product): 256 states, 31 layers, 128 samples 64 / 59; 512, 7, 64: 47 / 51; 512, 63, 16: 82 / 52;
+    # 1024, 31, 128: 329 / 116.  Tables of 128 rows fill half a product tile and never gain.
+    DENSE_PAR_ROWS, DENSE_PAR_DEPTH, DENSE_PAR_WORK = 256, 256, 200_000_000
+
+    def _tied_groups(self):
+        """Groups of tied tables whose parameter flows may be one dense product."""
+        found = {}
+        for d in self.depths:
+            for g in d["fw"]:
+                rows = len(g.blocks) * g.bs
+                if (not g.mma or d["store"] or g.bs % 128 != 0 or not self.DENSE_PAR_ROWS <= rows <= 6144
+                        or g.depth < self.DENSE_PAR_DEPTH or max(len(d["elems"][e][1]) for e in g.ops) > 8):
+                    continue
+                sizes = tuple(d["elems"][e][0] for e in g.ops)
+                found.setdefault((g.par[1].tobytes(), g.bs, sizes), []).append((d["elems"], g))
+        tied = []
+        put = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(self.device)
+        for (_, bs, sizes), members in found.items():
+            if len(members) < 2:
+                continue
+            fc = max(len(elems[e][1]) for elems, g in members for e in g.ops)
+            fc = 2 if fc <= 2 else (4 if fc <= 4 else 8)
+            off = np.concatenate([np.arange(s) for s in sizes])
+            fk = np.zeros((len(members), off.size, fc), dtype=np.int32)
+            for m, (elems, g) in enumerate(members):
+                for j in range(fc):
+                    row = np.repeat([elems[e][1][j] if j < len(elems[e][1]) else 0 for e in g.ops], sizes)
+                    fk[m, :, j] = np.where(row != 0, row + off, 0)
+            g = members[0][1]
+            each = lambda t: np.repeat(t, sizes, axis=1) + off[None, :] * bs
+            tied.append(dict(members={id(g) for _, g in members}, n=len(members), fc=fc, K=off.size, bs=bs,
+                             n_blocks=len(g.blocks), fk=put(fk), nids=put([g.blocks for _, g in members]),
+                             cids=put(np.ones((len(g.blocks), off.size))), pids=put(each(g.par[1])), pfids=put(each(g.flow))))
+        return tied
+
+    def _par_jobs(self, dense):
         pp, kids = _Pool(2), _Pool()
         jobs = {0: [], 1: [], 2: [], 3: []}
+        covered = set().union(*[g["members"] for g in dense])
         for d in self.depths:
             elems, store = d["elems"], d["store"]
             for g in d["fw"]:
+                if id(g) in covered:
+                    continue
                 nk = max(len(elems[e][1]) for e in g.ops)
                 par = g.par[1] if isinstance(g.par, tuple) else g.par
 
@@ -601,7 +647,7 @@ class ColumnProgram:
                             tab = [[par[b, i] + o * g.bs + r, g.flow[b, i] + o * g.bs + r] for _, o, i in ks]
                             jobs[1].append((first + r, 0, min(16, g.bs - r), off, len(ks) * step, n_kids, width, pp.add(tab),
                                             g.bs, lg, 0, 0))
-        return dict(pp=pp.tensor(self.device), kids=kids.tensor(self.device),
+        return dict(pp=pp.tensor(self.device), kids=kids.tensor(self.device), dense=dense,
                     jobs={k: (torch.from_numpy(np.array(v, dtype=PAR).view(np.uint8)).to(self.device), len(v))
                           for k, v in jobs.items() if v})
 
@@ -630,15 +676,38 @@ class ColumnProgram:
             _lib.call("pcx_column_run", mode, nm, nf, ef, em, params, plan["frags"], p["tasks"], plan["kids"], p["strips"],
                       levels, n, W, nt, tiles, cluster, wide, int(logspace), terms)
 
+    def _dense_operands(self, g, n: int, W: int):
+        """Operand tiles of n layers of a group of tied tables, W samples each (zero beyond the last sample)."""
+        chunks = -(-n * W // 64)
+        if g.get("W") != W:
+            g["W"], g["tiles"] = W, {}
+        if n not in g["tiles"]:
+            make = lambda k: torch.zeros(k, dtype=torch.uint8, device=self.device)
+            g["tiles"][n] = (make(g["n_blocks"] * (g["bs"] // 128) * chunks * 32768), make(-(-g["K"] // 256) * chunks * 65536))
+        return (*g["tiles"][n], chunks)
+
     def param_flows(self, plan, pf, nf, nm, params, logspace: bool = True):
         W = nm.size(1)
-        for kind, (jobs, n) in self.par["jobs"].items():
-            _lib.call("pcx_column_par", kind, pf, nf, nm, self.buffers(W), params, jobs, self.par["kids"], self.par["pp"], n,
-                      W, int(logspace), 1 if _lib.sum_mode() == 2 else 3)
+        par = self.par(W)
+        for g in par["dense"]:
+            # (as many layers at a time as the operand buffers may take)
+            layer = 4 * W * (g["n_blocks"] * g["bs"] + -(-g["K"] // 256) * 256)
+            step = max(1, min(g["n"], self.dense_par_bytes // layer))
+            for m in range(0, g["n"], step):
+                n = min(step, g["n"] - m)
+                x, y, chunks = self._dense_operands(g, n, W)
+                _lib.call("pcx_sum_par_dense2_stage", x, y, nf, nm, None, g["nids"][m], None, g["fk"][m], g["fc"],
+                          g["n_blocks"], g["K"], g["bs"], W, chunks, 0, n, int(logspace))
+                _lib.call("pcx_sum_par_dense2_gemm", pf, params, x, y, g["cids"], g["pids"], g["pfids"], g["n_blocks"], g["K"],
+                          g["bs"], chunks)
+        for kind, (jobs, n) in par["jobs"].items():
+            _lib.call("pcx_column_par", kind, pf, nf, nm, self.buffers(W), params, jobs, par["kids"], par["pp"], n, W,
+                      int(logspace), 1 if _lib.sum_mode() == 2 else 3)
 
-    def check(self, plan, pc, report):
+    def check(self, plan, W: int, pc, report):
         """Bounds of every index the kernels form from the plan's tables; ``report(what, index, extent, limit)``."""
-        kids, pp = plan["kids"].cpu().numpy(), self.par["pp"].cpu().numpy().reshape(-1, 2)
+        par = self.par(W)
+        kids, pp = plan["kids"].cpu().numpy(), par["pp"].cpu().numpy().reshape(-1, 2)
         n_par, n_flow = int(pc.params.numel()), int(pc.num_param_flows)
         bases = plan["bases"].cpu().numpy().reshape(-1, 4)[:plan["n_frag"]]
         for b in bases:
@@ -691,8 +760,14 @@ class ColumnProgram:
                     else:
                         for r in kids[int(st[1]):int(st[1]) + int(st[2])]:
                             report("column child rows", int(r), rows, pc.num_nodes)
-        kids = self.par["kids"].cpu().numpy()
-        for kind, (jobs, n) in self.par["jobs"].items():
+        for g in par["dense"]:
+            for r in g["nids"].cpu().reshape(-1).tolist():
+                report("column flow rows", int(r), g["bs"], pc.num_nodes)
+            report("column child rows", int(g["fk"].max()), 1, pc.num_nodes)
+            report("column parameters", int(g["pids"].max()), g["bs"], n_par)
+            report("column parameter flows", int(g["pfids"].max()), g["bs"], n_flow)
+        kids = par["kids"].cpu().numpy()
+        for kind, (jobs, n) in par["jobs"].items():
             for t in jobs.cpu().numpy().view(PAR):
                 mma = kind != 1
                 span = 16 if mma else (1 << int(t["lg_entry"]))

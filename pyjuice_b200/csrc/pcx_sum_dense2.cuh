@@ -175,21 +175,52 @@ __device__ __forceinline__ void wide_gather_em(const WideArgs& a, int64_t i, int
     }
 }
 
+// Epilogue of a parameter-flow tile: parameter * product, added to the accumulators.  Latency bounds it (four warps walk 256
+// columns, each index -> parameter -> atomic), so nothing waits for what could be asked for earlier: the 32 columns of a
+// group have their indices in the 32 lanes (read while the main loop runs, handed round by shuffles) and a group's 32
+// parameters are requested before the previous group is finished.  A product of 128 x 256 tiles short enough to be all
+// epilogue (1024 x 1024, seven chunks): 33 us with eight columns at a time, 30 now.
+template <int DN>
+struct WideParEpi {
+    int pid[DN / 32], fid[DN / 32];
+    float p[32];
+    __device__ __forceinline__ void open(const WideArgs& a, int64_t i, int at, int nt) {
+#pragma unroll
+        for (int q = 0; q < DN / 32; ++q) {
+            const int e = nt * DN + q * 32 + (threadIdx.x & 31);
+            const bool in = e < a.K && a.cids[i * a.K + e] != 0;
+            pid[q] = in ? a.pids[i * a.K + e] : -1;
+            fid[q] = in ? a.pfids[i * a.K + e] : 0;
+        }
+        request(a, at, 0);
+    }
+    __device__ __forceinline__ void request(const WideArgs& a, int at, int q) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int o = __shfl_sync(0xffffffffu, pid[q], j);
+            p[j] = a.params[o < 0 ? 0 : (int64_t)o + at];
+            if (o < 0) p[j] = 0.0f;
+        }
+    }
+    // (q is a constant at every call: the loops are unrolled)
+    __device__ __forceinline__ void add(const WideArgs& a, int at, int q, const float* v) {
+        float pf[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pf[j] = p[j] != 0.0f ? p[j] * v[j] : 0.0f;
+        const int f = fid[q];
+        if (q + 1 < DN / 32) request(a, at, q + 1);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int o = __shfl_sync(0xffffffffu, f, j);
+            if (pf[j] != 0.0f) atomicAdd(a.out + ((int64_t)o + at), pf[j]);
+        }
+    }
+};
+
 // Epilogue of one row and 32 consecutive columns.
 template <int EPI, int DN>
 __device__ __forceinline__ void wide_finish(const WideArgs& a, int64_t i, int r0, int row, int nt, int cb, const float* v,
                                             const float* pre_em = nullptr, const int* pre_fk = nullptr) {
-    if (EPI == W_PAR) {
-#pragma unroll 4
-        for (int j = 0; j < 32; ++j) {
-            const int e = nt * DN + cb + j;
-            if (e >= a.K) break;
-            if (a.cids[i * a.K + e] == 0) continue;
-            const float pf = a.params[(int64_t)a.pids[i * a.K + e] + r0 + row] * v[j];
-            if (pf != 0.0f) atomicAdd(a.out + (int64_t)a.pfids[i * a.K + e] + r0 + row, pf);
-        }
-        return;
-    }
     const int b0 = nt * DN + cb;
     if (b0 >= a.B) return;
     const float* sh = a.shift + (int64_t)a.b_group[i] * a.B + b0;
@@ -268,8 +299,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) wide_gemm_kernel(const WideArgs 
     const int tiles_r = a.row_block / BM;
     const int64_t i = mt / tiles_r;
     const int r0 = (int)(mt % tiles_r) * BM;
-    const int chunks_here = a.n_chunks / a.splits;
-    const int c_begin = split * chunks_here;
+    // PAR: the parts of a split contraction are independent CTAs (their epilogues add atomically) and may be uneven
+    const int c_begin = (EPI == W_PAR) ? (int)((int64_t)a.n_chunks * split / gridDim.z) : split * (a.n_chunks / a.splits);
+    const int chunks_here = (EPI == W_PAR) ? (int)((int64_t)a.n_chunks * (split + 1) / gridDim.z) - c_begin
+                                           : a.n_chunks / a.splits;
     const int n_steps = chunks_here * (KC / W_STEP);
 
     if (tid == 0) {
@@ -372,15 +405,17 @@ __global__ void __launch_bounds__(W_THREADS, 1) wide_gemm_kernel(const WideArgs 
             if (c0 < a.B) wide_gather_em(a, i, r0, row, c0, em0, fk0);
             if (QW0 == 64 && c0 + 32 < a.B) wide_gather_em(a, i, r0, row, c0 + 32, em1, fk0);
         }
+        WideParEpi<DN> par;
+        if (EPI == W_PAR) par.open(a, i, r0 + row, nt);
         bool ok = mbar_wait(&s_done, 0u, 1u << 24);
         if (!ok) s_fail = 3;
-        ok = ok && (s_fail == 0);
+        ok = __all_sync(0xffffffffu, ok && (s_fail == 0));
         tc_fence_after_sync();
         const uint32_t tbase = tmem + ((uint32_t)(lq * 32) << 16);
         const int used = n_steps < ACCS ? n_steps : ACCS;
         if (a.splits == 1) {
             if (ok) {
-#pragma unroll 1
+#pragma unroll (EPI == W_PAR ? DN / 32 : 1)
                 for (int cb = 0; cb < DN; cb += 32) {
                     float v[32];
                     tmem_ld<32>(tbase + (uint32_t)cb, v);
@@ -390,7 +425,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) wide_gemm_kernel(const WideArgs 
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] += u[j];
                     }
-                    wide_finish<EPI, DN>(a, i, r0, row, nt, cb, v);
+                    if (EPI == W_PAR) par.add(a, r0 + row, cb / 32, v);
+                    else wide_finish<EPI, DN>(a, i, r0, row, nt, cb, v);
                 }
             }
         } else {
@@ -630,18 +666,24 @@ __global__ void __launch_bounds__(W_PREP_THREADS) wide_prep_rows_kernel(const Wi
 // Parameter-flow operands of one layer (contraction over the batch), into the columns of slot `slot`:
 // X tile (row tile mt, chunk cc): [8 sample groups][128 rows][8 samples] hi, lo; Y tile (edge tile et of 256, chunk cc):
 // [8 sample groups][256 edges][8 samples] hi, lo.  The concatenated sample index of (slot, b) is slot * B + b.
-// Grid (ceil(B / 8), 1, cs), clusters of cs along z (rows and edges are split over the cluster), 512 threads.
+// Grid (ceil(B / 8), layers, cs): layer y has its rows at kids[y * blocks], its elements at cids_row / fk_row[y * Kfw] and
+// the slot slot + y; clusters of cs along z (rows and edges are split over the cluster), 512 threads.
 template <int FC>
-__global__ void __launch_bounds__(W_PREP_THREADS) wide_prep_par_kernel(const WidePrepArgs a) {
+__global__ void __launch_bounds__(W_PREP_THREADS) wide_prep_par_kernel(const WidePrepArgs base) {
     extern __shared__ float s_dyn[];
     __shared__ float s_red[(W_PREP_THREADS / 32) * 8];
     __shared__ float s_peer[8 * 8];
     const int tid = threadIdx.x;
     const int b0 = blockIdx.x * W_PREP_SAMPLES;
-    const int rows_here = a.depth_pad / a.cs;
+    const int rows_here = base.depth_pad / base.cs;
     const int k_begin = blockIdx.z * rows_here;
     const int ld = rows_here + 4;
     float sh[8];
+    WidePrepArgs a = base;
+    a.kids += (int64_t)blockIdx.y * (a.depth / a.par_block);          // one layer of the group per grid row
+    a.slot += blockIdx.y;
+    if (FC == 0) a.cids_row += (int64_t)blockIdx.y * a.Kfw;
+    else a.fk_row += (int64_t)blockIdx.y * a.Kfw * FC;
     griddep_wait();
     griddep_launch_dependents();
     wide_prep_stage<0>(a, 0, b0, k_begin, rows_here, s_dyn, ld, s_red, s_peer, sh);   // mode 2: flow - value of the layer's rows
@@ -707,9 +749,11 @@ __global__ void __launch_bounds__(W_PREP_THREADS) wide_prep_par_kernel(const Wid
 }
 
 // CTAs per group that share the operand rows of a pre-pass (= its cluster size): whole 64-row chunks each.
-inline int wide_prep_cluster(int n_chunks) {
+// `ctas`: CTAs of the launch without a cluster; a launch that fills the machine by itself needs none (31 layers of 1024 rows,
+// 128 samples: 83 us with clusters of four, 37 without).
+inline int wide_prep_cluster(int n_chunks, int64_t ctas = 1) {
     int cs = 1;
-    while (cs < 4 && n_chunks % (cs * 2) == 0 && n_chunks / (cs * 2) >= 4) cs *= 2;
+    while (cs < 4 && ctas * cs < 2 * 148 && n_chunks % (cs * 2) == 0 && n_chunks / (cs * 2) >= 4) cs *= 2;
     return cs;
 }
 
@@ -777,7 +821,7 @@ int launch_wide_gemm(const WideArgs& a, dim3 grid, cudaStream_t st) {
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int n_attr = 0;
-    if (grid.z > 1) {
+    if (grid.z > 1 && EPI != W_PAR) {
         attr[n_attr].id = cudaLaunchAttributeClusterDimension;       // the CTAs that split one tile's contraction
         attr[n_attr].val.clusterDim.x = 1;
         attr[n_attr].val.clusterDim.y = 1;
@@ -930,11 +974,11 @@ int pcx_sum_bwd_ele_dense2(float* element_flows, const float* element_mars, floa
 int pcx_sum_par_dense2_stage(void* x_tiles, void* y_tiles, const float* node_flows, const float* node_mars,
                              const float* element_mars, const int32_t* nids, const int32_t* cids_row,
                              const int32_t* fkids_row, int fc, int64_t n_blocks, int K, int block_size, int B,
-                             int n_chunks_total, int slot, int logspace, void* stream) {
-    if (n_blocks <= 0 || B <= 0) return 0;
+                             int n_chunks_total, int slot, int n_slots, int logspace, void* stream) {
+    if (n_blocks <= 0 || B <= 0 || n_slots <= 0) return 0;
     const int64_t rows = n_blocks * block_size;
     if (block_size % BM != 0 || K <= 0 || slot < 0 || B % 8 != 0 || rows > W_MAX_DEPTH) return -1;
-    if (((int64_t)slot + 1) * B > (int64_t)n_chunks_total * KC) return -1;
+    if (n_slots > 65535 || ((int64_t)slot + n_slots) * B > (int64_t)n_chunks_total * KC) return -1;
     if (fkids_row == nullptr && element_mars == nullptr) return -1;
     if (fkids_row != nullptr && fc != 2 && fc != 4 && fc != 8) return -1;
     WidePrepArgs p{};
@@ -943,8 +987,8 @@ int pcx_sum_par_dense2_stage(void* x_tiles, void* y_tiles, const float* node_flo
     p.tiles = reinterpret_cast<uint8_t*>(x_tiles); p.y_tiles = reinterpret_cast<uint8_t*>(y_tiles);
     p.emars = element_mars; p.cids_row = cids_row; p.fk_row = fkids_row; p.fc = fc; p.Kfw = K;
     p.n_chunks_total = n_chunks_total; p.slot = slot;
-    p.cs = wide_prep_cluster(p.depth_pad / KC);
-    const dim3 grid((unsigned)(B / W_PREP_SAMPLES), 1, (unsigned)p.cs);
+    p.cs = wide_prep_cluster(p.depth_pad / KC, (int64_t)(B / W_PREP_SAMPLES) * n_slots);
+    const dim3 grid((unsigned)(B / W_PREP_SAMPLES), (unsigned)n_slots, (unsigned)p.cs);
     const size_t smem = (size_t)(p.depth_pad / p.cs + 4) * 8 * sizeof(float);
     cudaStream_t st = (cudaStream_t)stream;
     if (fkids_row == nullptr) return launch_wide_prep_par<0>(p, grid, smem, st);
@@ -962,7 +1006,11 @@ int pcx_sum_par_dense2_gemm(float* param_flows, const float* params, const void*
     a.a_tiles = reinterpret_cast<const uint8_t*>(x_tiles); a.b_tiles = reinterpret_cast<const uint8_t*>(y_tiles);
     a.n_chunks = n_chunks_total; a.splits = 1; a.row_block = block_size; a.terms = (g_sum_mode == 2) ? 1 : 3;
     a.out = param_flows; a.params = params; a.cids = cids; a.pids = pids; a.pfids = pfids; a.K = K;
-    const dim3 grid((unsigned)(n_blocks * (block_size / BM)), (unsigned)pcx_cdiv(K, 256), 1);
+    // A product of few output tiles is cut along its contraction until the parts fill the SMs, down to four chunks a part
+    // (fewer would not pay for the epilogue, which adds the whole tile).
+    const int64_t tiles = n_blocks * (block_size / BM) * pcx_cdiv(K, 256);
+    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(148 / tiles, n_chunks_total / 4));
+    const dim3 grid((unsigned)(n_blocks * (block_size / BM)), (unsigned)pcx_cdiv(K, 256), (unsigned)parts);
     return launch_wide_gemm<W_PAR, 256>(a, grid, (cudaStream_t)stream);
 }
 

@@ -25,6 +25,7 @@
 #include "pcx_common.cuh"
 #include "pcx_tc.cuh"
 #include "../../include/pcx_b200.h"
+#include <algorithm>
 #include <float.h>
 
 namespace {

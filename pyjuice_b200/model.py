@@ -892,7 +892,7 @@ class TensorCircuit(nn.Module):
                 fk = f["fw"][p] if (f is not None and f.get("dense") and element_mars is None) else None
                 _lib.call("pcx_sum_par_dense2_stage", g["x"], g["y"], node_flows, node_mars, element_mars, nids, cids,
                           fk, f["fc"] if fk is not None else 0, nids.numel(), cids.size(1), layer.block_size,
-                          node_flows.size(1), g["n_chunks"], slot, ls)
+                          node_flows.size(1), g["n_chunks"], slot, 1, ls)
             else:
                 _lib.call("pcx_sum_par_dense_stage", g["x"], g["y"], dense["work"], node_flows, node_mars, element_mars,
                           nids, cids, nids.numel(), cids.size(1), layer.block_size, node_flows.size(1), g["n_chunks"],
@@ -1528,7 +1528,7 @@ class TensorCircuit(nn.Module):
                 counts[what] = counts.get(what, 0) + 1
                 if at < 0 or at + extent > limit:
                     errs.append(f"{what}: index range [{at}, {at} + {extent}) exceeds [0, {limit})")
-            self._column_program.check(self._column_program.plan(self._nm.size(1)), self, report)
+            self._column_program.check(self._column_program.plan(self._nm.size(1)), self._nm.size(1), self, report)
         if errs:
             raise ValueError("index tables out of bounds: " + "; ".join(errs[:6]))
         return counts

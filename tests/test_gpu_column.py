@@ -63,6 +63,21 @@ def test_wide_levels(kind, latents, logspace, B, monkeypatch):
     pc.validate_tables()
 
 
+@pytest.mark.parametrize("latents", [256, 384, 640])
+@pytest.mark.parametrize("logspace", [True, False])
+@pytest.mark.parametrize("B,most", [(1, 1 << 30), (77, 1 << 30), (256, 1 << 30), (77, 1 << 19)])
+def test_tied_parameter_flows_as_one_product(latents, logspace, B, most, monkeypatch):
+    """Tied transitions contracted over all their layers' samples: one part and several, a last chunk that is partly empty,
+    output tiles that are partly empty, and (`most`) operand buffers that hold a few layers at a time."""
+    monkeypatch.setattr(ColumnProgram, "DENSE_PAR_WORK", 0)
+    pc = pj.compile(_circuit("hmm", latents)).to(DEV)
+    pc.dense_par_max_bytes = most
+    x = torch.randint(0, 11, (B, pc.num_vars), generator=torch.Generator().manual_seed(B))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1, logspace_flows=logspace)
+    assert _program(pc).par(pc._nm.size(1))["dense"]
+    pc.validate_tables()
+
+
 @pytest.mark.parametrize("kind,latents", [("hclt", 32), ("pd", 64), ("rat", 8), ("hmm", 64), ("hmm", 256), ("hmm", 1024),
                                           ("hclt", 256)])
 def test_equals_the_per_layer_kernels(kind, latents):
