@@ -366,8 +366,10 @@ class ColumnProgram:
             split = []
             # Elements of many children in a level that has the machine to itself: their values come from the product
             # kernel, whose 2048 threads per SM hide the latency of the gather better than the warp tasks (16384 elements
-            # of 24 children, 1024 samples: 155 + 25 us instead of 320).
-            stored = bool(d["store"]) and is_wide(n)
+            # of 24 children, 1024 samples: 155 + 25 us instead of 320).  A CTA of a fused level gathers some 500 child rows
+            # in a microsecond: from several microseconds' worth of rows the kernel's launch is the smaller cost.
+            reads = sum(d["elems"][e][0] * len(d["elems"][e][1]) for e in d["store"])
+            stored = bool(d["store"]) and (is_wide(n) or reads > 3000 * c)
             if stored:
                 before[i] = self._prod_tables(d)
             for g in d["fw"]:
@@ -404,7 +406,8 @@ class ColumnProgram:
             launches, at = [], 0
             while at < len(levels[m]):                        # consecutive fused levels are one launch
                 how, end = levels[m][at][1], at + 1
-                while how is fused and end < len(levels[m]) and levels[m][end][1] is fused:
+                while (how is fused and end < len(levels[m]) and levels[m][end][1] is fused
+                       and not (m == 0 and end in before)):
                     end += 1
                 if m == 0 and at in before:
                     launches.append(before[at])

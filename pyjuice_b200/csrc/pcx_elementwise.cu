@@ -199,7 +199,20 @@ input_cat_fwd_staged(float* __restrict__ node_mars, const float* __restrict__ pa
     const int64_t n0 = (int64_t)blockIdx.x * G;
     const int g_end = (int)min((int64_t)G, n_nodes - n0);
     stage_rows(s, vids, s_pids, node_cats, max_cats, n0, G, n_nodes);
-    for (int c = threadIdx.x; c < max_cats; c += kStageThreads) {
+    if (g_end < 8) {                                       // long rows: eight categories of a row per thread
+        for (int g = 0; g < g_end; ++g)
+            for (int c0 = threadIdx.x; c0 < max_cats; c0 += kStageThreads * 8) {
+                float p[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int c = c0 + u * kStageThreads;
+                    p[u] = c < s.cats[g] ? params[s.row[g] + c] : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (c0 + u * kStageThreads < max_cats) s_tab[g * max_cats + c0 + u * kStageThreads] = logf(p[u]);
+            }
+    } else for (int c = threadIdx.x; c < max_cats; c += kStageThreads) {
         for (int g0 = 0; g0 < g_end; g0 += 8) {
             float p[8];
 #pragma unroll
@@ -463,7 +476,10 @@ __device__ __forceinline__ void prod_split(const ProdDiv d, uint32_t t, uint32_t
 }
 
 // Product forward.  Thread = (row block i, ROWS nodes j (and j + block / 2) of the block, VEC consecutive samples).
-template <int VEC, int ROWS>
+// Few threads wait for one another's loads less than a thread for its own, so U children are requested at a time (row 0 exists
+// and stands in for an absent child; the sum keeps the children's order).  Leaf products of 96 children, 4608 elements, 16
+// samples, one child at a time: most of a query of 103 us.
+template <int VEC, int ROWS, int U>
 __global__ void prod_fwd_kernel(float* __restrict__ element_mars, const float* __restrict__ node_mars,
                                 const int32_t* __restrict__ nids, const int32_t* __restrict__ cids,
                                 uint32_t total, int64_t block0, ProdDiv d, int n_chs, int B) {
@@ -480,24 +496,38 @@ __global__ void prod_fwd_kernel(float* __restrict__ element_mars, const float* _
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[r][v] = 0.0f;
     const int32_t* crow = cids + i * n_chs;
-    for (int c = 0; c < n_chs; ++c) {
-        int32_t cid = crow[c];
-        if (cid == 0) continue;
-        const float* src = node_mars + ((int64_t)cid + j) * B + b;
+    for (int c0 = 0; c0 < n_chs; c0 += U) {
+        int32_t cid[U];
+        float x[U][ROWS][VEC];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            if (VEC == 4) {
-                float4 x = *reinterpret_cast<const float4*>(src + r * jstep);
-                acc[r][0] += x.x; acc[r][1] += x.y; acc[r][2] += x.z; acc[r][3] += x.w;
-            } else {
-                acc[r][0] += src[r * jstep];
+        for (int u = 0; u < U; ++u) cid[u] = c0 + u < n_chs ? crow[c0 + u] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float* src = node_mars + (cid[u] != 0 ? ((int64_t)cid[u] + j) * B : 0) + b;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                const float* at = src + (cid[u] != 0 ? r * jstep : 0);
+                if (VEC == 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(at);
+                    x[u][r][0] = q.x; x[u][r][1 % VEC] = q.y; x[u][r][2 % VEC] = q.z; x[u][r][3 % VEC] = q.w;
+                } else {
+                    x[u][r][0] = *at;
+                }
             }
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (cid[u] != 0)
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) acc[r][v] += x[u][r][v];
     }
     float* dst = element_mars + ((int64_t)nids[i] + j) * B + b;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-        if (VEC == 4) *reinterpret_cast<float4*>(dst + r * jstep) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        if (VEC == 4) *reinterpret_cast<float4*>(dst + r * jstep) =
+            make_float4(acc[r][0], acc[r][1 % VEC], acc[r][2 % VEC], acc[r][3 % VEC]);
         else dst[r * jstep] = acc[r][0];
     }
 }
@@ -758,19 +788,20 @@ int pcx_prod_fwd(float* element_mars, const float* node_mars, const int32_t* nid
                  int64_t n_blocks, int n_chs, int block_size, int B, void* stream) {
     if (n_blocks <= 0 || B <= 0) return 0;
     if (B % 4 == 0) {
-        if (block_size % 2 == 0)
+        // two nodes per thread while that leaves every SM about 1000 threads; fewer threads have more children under way
+        if (block_size % 2 == 0 && n_blocks * block_size * (B / 4) >= 2 * 148 * 1024)
             prod_launches(n_blocks, block_size / 2, B / 4, [&](int64_t b0, uint32_t total, ProdDiv d) {
-                prod_fwd_kernel<4, 2><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
+                prod_fwd_kernel<4, 2, 2><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
                     element_mars, node_mars, nids, cids, total, b0, d, n_chs, B);
             });
         else
             prod_launches(n_blocks, block_size, B / 4, [&](int64_t b0, uint32_t total, ProdDiv d) {
-                prod_fwd_kernel<4, 1><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
+                prod_fwd_kernel<4, 1, 8><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
                     element_mars, node_mars, nids, cids, total, b0, d, n_chs, B);
             });
     } else {
         prod_launches(n_blocks, block_size, B, [&](int64_t b0, uint32_t total, ProdDiv d) {
-            prod_fwd_kernel<1, 1><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
+            prod_fwd_kernel<1, 1, 4><<<grid_for(total), kThreads, 0, (cudaStream_t)stream>>>(
                 element_mars, node_mars, nids, cids, total, b0, d, n_chs, B);
         });
     }

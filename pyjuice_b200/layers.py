@@ -259,8 +259,11 @@ class InputLayer(Layer, nn.Module):
 
     # Tables with more categories than the staged kernels can hold in shared memory are looked up through a transposed
     # shadow ([category, row] instead of [row, category]); flows are accumulated in the same layout and moved into
-    # `param_flows` (the reference's layout) whenever that tensor is read.
-    SHADOW_MIN_CATS = 8193
+    # `param_flows` (the reference's layout) whenever that tensor is read.  So are tied tables (the emissions of an HMM) of a
+    # few hundred categories and more, for batches of at most that many samples: every replica has accumulators of its own
+    # (74 positions of a table of 29 MB: 2.1 GB to add to, to fold and to clear), of which the shadow needs one, and with
+    # fewer samples than categories a histogram in shared memory merges little.
+    SHADOW_MIN_CATS, SHADOW_MIN_TIED_CATS = 8193, 512
     use_fused_shadow_em = True
 
     @property
@@ -277,12 +280,14 @@ class InputLayer(Layer, nn.Module):
     def _setup_shadow(self, device):
         self._shadow = None
         C = self.max_cats
-        if device.type != "cuda" or C < self.SHADOW_MIN_CATS or int(self.node_cats.min()) != C:
+        if device.type != "cuda" or C < self.SHADOW_MIN_TIED_CATS or int(self.node_cats.min()) != C:
             return
         s_pids = self.s_pids.cpu()
         if self.num_parameters % C != 0 or bool((s_pids % C != 0).any()):
             return
         R = self.num_parameters // C
+        if C < self.SHADOW_MIN_CATS and (self.num_nodes < 2 * R or R < 32):
+            return
         src = self.source_nids.cpu()
         row_pfid = torch.full((R,), -1, dtype=torch.int64)
         row_pfid[s_pids[src] // C] = self.s_pfids.cpu()[src]
@@ -292,7 +297,7 @@ class InputLayer(Layer, nn.Module):
                             flows=None, stamp=None, dirty=False)
 
     def _shadow_ok(self, B: int) -> bool:
-        return self._shadow is not None and B % 4 == 0
+        return self._shadow is not None and B % 4 == 0 and (B <= self.max_cats or self.max_cats >= self.SHADOW_MIN_CATS)
 
     def _flush_shadow(self):
         """Move the flows accumulated in the transposed shadow into `param_flows` (source rows) and clear the shadow."""
