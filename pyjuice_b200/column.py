@@ -280,8 +280,9 @@ class ColumnProgram:
     def _piece(self, groups, nt: int, c: int):
         """(strips per task, time) of a level's large groups on a cluster of c CTAs: rounds of tasks times what a task
         takes in microseconds: a fixed latency, the gather and exponentials of its operand, its multiplications, and parameters
-        that neither stay in shared memory nor arrive during the gather.  (Measured per level: 512 x 512 on 8 CTAs, 8
-        columns, 5.3 us; 1024 x 1024 on 8 / 16 CTAs, 16 columns, 12.8 / 10.0.)"""
+        that neither stay in shared memory nor arrive during the gather.  (Measured per level, mean of the two
+        directions, CTAs x columns: 512 x 512 on 4 x 8 / 8 x 16 8.5 / 9.6 us; 1024 x 1024 on 8 x 8 / 16 x 16 / 8 x 16 / 4 x 8
+        12.4 / 13.2 / 16.2 / 16.9: sixteen columns cost the element flows two more microseconds than eight.)"""
         big = [(g.depth // 16, len(g.blocks) * g.bs // 16) for g in groups if g.big]
         if not big:
             return 1, 0.0
@@ -290,7 +291,7 @@ class ColumnProgram:
         for size in (16, 8, 4, 2, 1):
             n = sum(-(-strips // size) for _, strips in big)
             stream = max(0.0, size * steps - max(0, 150 - steps * nt // 2)) * 0.01
-            cost = -(-n // c) * (3.0 + 0.025 * steps * nt + 0.003 * size * steps * nt + stream)
+            cost = -(-n // c) * (1.2 + 1.8 * nt + 0.025 * steps * nt + 0.003 * size * steps * nt + stream)
             if best is None or cost < best[1] - 1e-9:
                 best = (size, cost)
         return best
