@@ -255,6 +255,8 @@ class ColumnProgram:
             self._rooms[key] = n if n > 0 else max(1, (128 if c < 16 else 112) // c)
         return self._rooms[key]
 
+    PROD_READS = 3000            # child rows a CTA may gather for the stored elements of a fused level (see `_cut`)
+
     # A level with this many (16-row strip, 32-column) pieces gives every warp of the machine one: a launch of its own.
     WIDE_ITEMS = 148 * WARPS
 
@@ -370,7 +372,7 @@ class ColumnProgram:
             # of 24 children, 1024 samples: 155 + 25 us instead of 320).  A CTA of a fused level gathers some 500 child rows
             # in a microsecond: from several microseconds' worth of rows the kernel's launch is the smaller cost.
             reads = sum(d["elems"][e][0] * len(d["elems"][e][1]) for e in d["store"])
-            stored = bool(d["store"]) and (is_wide(n) or reads > 3000 * c)
+            stored = bool(d["store"]) and (is_wide(n) or reads > self.PROD_READS * c)
             if stored:
                 before[i] = self._prod_tables(d)
             for g in d["fw"]:
@@ -690,10 +692,16 @@ class ColumnProgram:
             g["tiles"][n] = (make(g["n_blocks"] * (g["bs"] // 128) * chunks * 32768), make(-(-g["K"] // 256) * chunks * 65536))
         return (*g["tiles"][n], chunks)
 
-    def param_flows(self, plan, pf, nf, nm, params, logspace: bool = True):
+    def param_flows(self, pf, nf, nm, params, logspace: bool = True, beside=None):
+        """``beside``: None: all parameter flows; True: those that go beside the others on a second stream, False: the others.
+        The jobs of kinds 0 and 1 (roots, products of many children) are few and long and leave most of an SM free, which
+        the staged tiles, persistent and bound by shared memory, cannot use: 62 of 560 us of a Poon-Domingos circuit over 784
+        variables.  Without other jobs they are not split off: they then run beside the leaves' flows."""
         W = nm.size(1)
         par = self.par(W)
-        for g in par["dense"]:
+        split = bool(par["dense"]) or any(k > 1 for k in par["jobs"])
+        kinds = [k for k in par["jobs"] if beside is None or (split and k <= 1) == beside]
+        for g in par["dense"] if beside is not True else ():
             # (as many layers at a time as the operand buffers may take)
             layer = 4 * W * (g["n_blocks"] * g["bs"] + -(-g["K"] // 256) * 256)
             step = max(1, min(g["n"], self.dense_par_bytes // layer))
@@ -704,7 +712,8 @@ class ColumnProgram:
                           g["n_blocks"], g["K"], g["bs"], W, chunks, 0, n, int(logspace))
                 _lib.call("pcx_sum_par_dense2_gemm", pf, params, x, y, g["cids"], g["pids"], g["pfids"], g["n_blocks"], g["K"],
                           g["bs"], chunks)
-        for kind, (jobs, n) in par["jobs"].items():
+        for kind in kinds:
+            jobs, n = par["jobs"][kind]
             _lib.call("pcx_column_par", kind, pf, nf, nm, self.buffers(W), params, jobs, par["kids"], par["pp"], n, W,
                       int(logspace), 1 if _lib.sum_mode() == 2 else 3)
 

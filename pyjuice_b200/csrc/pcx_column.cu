@@ -943,7 +943,8 @@ __global__ void __launch_bounds__(WT, 1) column_pipe_kernel(const ColArgs a) {
 }
 
 // Wide product levels: a thread owns four columns of one row, so that an SM has 2048 rows' loads under way (a level of 2712
-// tasks of 16 rows at 512 samples, 1.5 parents each: 78 us as warp tasks).
+// tasks of 16 rows at 512 samples, 1.5 parents each: 78 us as warp tasks).  Long parent lists are taken four at a time: 25088
+// rows of 16 parents, 1024 samples: 234 us two at a time, 185 now (1.6 GB of reads, from L2).
 __global__ void __launch_bounds__(256) column_prod_kernel(const ColArgs a) {
     const int4 lv = __ldg(a.levels);
     const int W4 = a.W >> 2;
@@ -970,7 +971,22 @@ __global__ void __launch_bounds__(256) column_prod_kernel(const ColArgs a) {
         if (add && !a.logspace)
 #pragma unroll
             for (int j = 0; j < 4; ++j) sum[j] = mx[j];
-        for (int p = 0; p < n; p += 2) {
+        int p = 0;
+        for (; p + 4 <= n; p += 4) {
+            float x[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ldvec<4>(a.ef + (int64_t)(__ldg(par + p + q) + row) * a.W + co, x[q]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (!a.logspace) { sum[j] += (x[0][j] + x[1][j]) + (x[2][j] + x[3][j]); continue; }
+                const float mn = fmaxf(mx[j], fmaxf(fmaxf(x[0][j], x[1][j]), fmaxf(x[2][j], x[3][j])));
+                const float sh = (mn == PCX_NEG_INF) ? 0.0f : mn;
+                sum[j] = sum[j] * fast_exp(mx[j] - sh) + (fast_exp(x[0][j] - sh) + fast_exp(x[1][j] - sh))
+                         + (fast_exp(x[2][j] - sh) + fast_exp(x[3][j] - sh));
+                mx[j] = mn;
+            }
+        }
+        for (; p < n; p += 2) {
             float x[2][4];
             ldvec<4>(a.ef + (int64_t)(__ldg(par + p) + row) * a.W + co, x[0]);
             if (p + 1 < n) ldvec<4>(a.ef + (int64_t)(__ldg(par + p + 1) + row) * a.W + co, x[1]);

@@ -954,12 +954,12 @@ class TensorCircuit(nn.Module):
             cur.wait_stream(side)
         self._batched_par_pending = any_fused and pf is not None     # launched by `backward`, after this sweep
 
-    def _launch_par(self, logspace_flows: bool):
-        plan = self._column_plan()
-        if plan is None:
+    def _launch_par(self, logspace_flows: bool, beside=None):
+        """``beside``: see `ColumnProgram.param_flows`; the batched launch of the per-layer kernels is one piece."""
+        if self._column_plan() is not None:
+            self._column_program.param_flows(self.param_flows, self._nf, self._nm, self.params.data, logspace_flows, beside)
+        elif not beside:
             self._launch_batched_par(logspace_flows)
-        else:
-            self._column_program.param_flows(plan, self.param_flows, self._nf, self._nm, self.params.data, logspace_flows)
 
     def _launch_batched_par(self, logspace_flows: bool):
         B = self._nf.size(1)
@@ -1090,9 +1090,10 @@ class TensorCircuit(nn.Module):
         if self._batched_par_pending and self.use_side_stream:
             self._side_stream.wait_stream(cur)
             with torch.cuda.stream(self._side_stream):
+                self._launch_par(logspace_flows, beside=True)
                 for layer in self.input_layer_group:
                     layer._launch_backward(data, self._nf, logspace_flows)
-            self._launch_par(logspace_flows)
+            self._launch_par(logspace_flows, beside=False)
             cur.wait_stream(self._side_stream)
         else:
             for layer in self.input_layer_group:

@@ -94,3 +94,27 @@ def test_equals_the_per_layer_kernels(kind, latents):
     assert (out[True][0] - out[False][0]).abs().max().item() <= 1e-3
     for a, b in zip(out[True][1:], out[False][1:]):
         assert (a - b).norm() <= 1e-4 * b.norm()
+
+
+@pytest.mark.parametrize("latents,depth", [(32, 2), (8, 1), (16, 2)])
+@pytest.mark.parametrize("B", [3, 40])
+def test_products_of_many_children_ahead_of_a_fused_level(latents, depth, B, monkeypatch):
+    """Stored elements from the product kernel in the middle of the fused levels: odd numbers of children, ragged batches."""
+    monkeypatch.setattr(ColumnProgram, "PROD_READS", 0)
+    pc = pj.compile(pj.structures.RAT_SPN(num_vars=45, num_latents=latents, depth=depth, num_repetitions=3, num_cats=6)).to(DEV)
+    x = torch.randint(0, 6, (B, pc.num_vars), generator=torch.Generator().manual_seed(B))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1)
+    assert any(isinstance(launch, list) for launch in pc._column_plan()[0]["launches"])
+
+
+@pytest.mark.parametrize("cats", [511, 512, 1100, 5000])
+@pytest.mark.parametrize("homogeneous", [True, False])
+@pytest.mark.parametrize("B", [5, 530])
+def test_leaves_of_mid_size_vocabularies(cats, homogeneous, B):
+    """Staged tables of several and of few long rows, and tied tables on both sides of the transposed shadow's line."""
+    torch.manual_seed(5)
+    pc = pj.compile(pj.structures.HMM(seq_length=3, num_latents=32, num_emits=cats, homogeneous=homogeneous)).to(DEV)
+    x = torch.randint(0, cats, (B, 3), generator=torch.Generator().manual_seed(B))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1)
+    layer = pc.input_layer_group[0]
+    assert layer._shadow_ok(pc._nm.size(1)) == (homogeneous and cats >= 512 and pc._nm.size(1) <= cats)
