@@ -316,56 +316,41 @@ __global__ void __launch_bounds__(W_THREADS, 1) wide_gemm_kernel(const WideArgs 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = s_tmem;
-    const uint8_t* a_src = a.a_tiles + ((size_t)mt * a.n_chunks + c_begin) * (2 * A_TILE);
-    // The parameter tiles are older than the pre-pass that precedes this kernel in its stream (which has itself waited for its
-    // predecessor before it let this kernel start), so the first stages' are on their way while that pre-pass still runs.
-    const int early = (EPI == W_PAR) ? 0 : min(n_steps, (int)C::STAGES);
-    const uint64_t keep = l2_policy_evict_last();
-    auto copy_a = [&](int t) {
-        const int c = t / (KC / W_STEP), h = t % (KC / W_STEP);
-        uint8_t* dst = smem + (t % C::STAGES) * C::STAGE;
-        const uint8_t* a_at = a_src + (size_t)c * (2 * A_TILE) + h * W_A_HALF;
-        if (EPI == W_PAR) {                          // staged operands, shared by the CTAs of a wave only: default policy
-            if (lane == 0) bulk_copy_g2s(dst, a_at, W_A_HALF, &s_full[t % C::STAGES]);
-            if (lane == 1) bulk_copy_g2s(dst + W_A_HALF, a_at + A_TILE, W_A_HALF, &s_full[t % C::STAGES]);
-        } else {                                     // parameter tiles: keep them for the next (tied) layer
-            if (lane == 0) bulk_copy_g2s_hint(dst, a_at, W_A_HALF, &s_full[t % C::STAGES], keep);
-            if (lane == 1) bulk_copy_g2s_hint(dst + W_A_HALF, a_at + A_TILE, W_A_HALF, &s_full[t % C::STAGES], keep);
-        }
-    };
-    if (warp == 0) {
-        for (int t = 0; t < early; ++t) {
-            if (lane == 0) mbar_expect_tx(&s_full[t], C::STAGE);
-            __syncwarp();
-            copy_a(t);
-        }
-    }
     griddep_wait();                                 // everything above overlapped the previous kernel's tail
     griddep_launch_dependents();
 
     const int64_t b_row = (EPI == W_PAR) ? (int64_t)nt : (int64_t)a.b_group[i] * a.n_ct + nt;
+    const uint8_t* a_src = a.a_tiles + ((size_t)mt * a.n_chunks + c_begin) * (2 * A_TILE);
     const uint8_t* b_src = a.b_tiles + ((size_t)b_row * a.n_chunks + c_begin) * C::B_TILE;
 
     if (warp == 0) {
         // ---- copy warp: lane 0 waits for the stage and arms its barrier, four lanes move one piece each -------------
-        int armed = early;
+        int armed = 0;
+        const uint64_t keep = l2_policy_evict_last();
         for (int t = 0; t < n_steps; ++t) {
             const int s = t % C::STAGES;
             int stop = 0;
             if (lane == 0) {
                 if (t >= C::STAGES && !mbar_wait(&s_empty[s], (uint32_t)((t / C::STAGES - 1) & 1))) s_fail = 1;
                 stop = s_fail;
-                if (!stop && t >= early) mbar_expect_tx(&s_full[s], C::STAGE);
+                if (!stop) mbar_expect_tx(&s_full[s], C::STAGE);
             }
             stop = __shfl_sync(0xffffffffu, stop, 0);
             if (stop) break;
             const int c = t / (KC / W_STEP), h = t % (KC / W_STEP);
             uint8_t* dst = smem + s * C::STAGE;
+            const uint8_t* a_at = a_src + (size_t)c * (2 * A_TILE) + h * W_A_HALF;
             const uint8_t* b_at = b_src + (size_t)c * C::B_TILE + h * C::B_HALF;
-            if (t >= early) copy_a(t);
+            if (EPI == W_PAR) {                      // staged operands, shared by the CTAs of a wave only: default policy
+                if (lane == 0) bulk_copy_g2s(dst, a_at, W_A_HALF, &s_full[s]);
+                if (lane == 1) bulk_copy_g2s(dst + W_A_HALF, a_at + A_TILE, W_A_HALF, &s_full[s]);
+            } else {                                 // parameter tiles: keep them for the next (tied) layer
+                if (lane == 0) bulk_copy_g2s_hint(dst, a_at, W_A_HALF, &s_full[s], keep);
+                if (lane == 1) bulk_copy_g2s_hint(dst + W_A_HALF, a_at + A_TILE, W_A_HALF, &s_full[s], keep);
+            }
             if (lane == 2) bulk_copy_g2s(dst + 2 * W_A_HALF, b_at, C::B_HALF, &s_full[s]);
             if (lane == 3) bulk_copy_g2s(dst + 2 * W_A_HALF + C::B_HALF, b_at + C::B_TILE / 2, C::B_HALF, &s_full[s]);
-            armed = max(armed, t + 1);
+            armed = t + 1;
         }
         if (lane == 0 && s_fail) {
             // let the copies that are still in flight land before this CTA's shared memory goes away
