@@ -274,8 +274,14 @@ class InputLayer(Layer, nn.Module):
 
     @param_flows.setter
     def param_flows(self, value):
+        """A buffer handed over takes the place of the accumulators: later backward passes add to it, updates read it, and
+        it is cleared or decayed with the others."""
+        if value is not None and (value.dtype != torch.float32 or not value.is_contiguous()
+                                  or value.numel() < self.num_param_flows):
+            raise ValueError(f"`param_flows` must be a contiguous float32 tensor of {self.num_param_flows} flows")
         self._param_flows = value
         self._arena_zero = False                 # unknown content (whoever hands over a cleared buffer says so)
+        self._tied_folded = False
 
     def _setup_shadow(self, device):
         self._shadow = None

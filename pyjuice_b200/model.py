@@ -720,6 +720,9 @@ class TensorCircuit(nn.Module):
     def _param_ptrs(self):
         return (self._sum_params.data_ptr(), *[layer._leaf_params.data_ptr() for layer in self._leaf_layers])
 
+    def _flow_ptrs(self):
+        return (self.param_flows.data_ptr(), *[layer._param_flows.data_ptr() for layer in self._leaf_layers])
+
     def _forward_pass(self, data: torch.Tensor, pack: bool, shadows):
         """All launches of a forward pass on the batch in ``data``, captured as one graph.  The operand tiles of the
         tensor-core kernels are re-packed (when the parameters changed: ``pack``) on a second stream, beside the input
@@ -1024,6 +1027,10 @@ class TensorCircuit(nn.Module):
                 self._eflow_mode = ls
             if compute_param_flows and (flows_memory != 1.0 or self.param_flows is None or self._late_sync is not None):
                 self.init_param_flows(flows_memory=flows_memory)     # decay (or clear) the accumulators and the flow total
+            if compute_param_flows:
+                for layer in self._leaf_layers:
+                    if layer._param_flows is None:                   # taken away by the caller
+                        layer.init_param_flows()
             r0, r1 = self._root_node_range
             if self._root_w is None or self._root_w.size(1) != W:
                 self._root_w = torch.empty(r1 - r0, W, device=self.device)
@@ -1047,7 +1054,7 @@ class TensorCircuit(nn.Module):
             # pass too, unless data-parallel ranks overlap them with the all-reduce, or the leaves see another batch.
             tail = compute_param_flows and own and not self._overlap_ready()
             key = ("bk", W, bool(compute_param_flows), tail, ls, self._launch_cfg(), self._param_ptrs(),
-                   self.param_flows.data_ptr() if compute_param_flows else 0, data.data_ptr() if tail else 0)
+                   self._flow_ptrs() if compute_param_flows else 0, data.data_ptr() if tail else 0)
             self._batched_par_pending = self._bk_par_pending.get(key, False)
             with self._nvtx("pcx backward"):
                 self._run_inner(key, partial(self._backward_sweep, data if tail else None, compute_param_flows,
@@ -1215,7 +1222,8 @@ class TensorCircuit(nn.Module):
         elif flows_memory != 1.0:
             for layer in self.input_layer_group:
                 layer._flush_shadow()
-            _scale(self._flow_arena.buf, flows_memory)
+            for buf in (self._flow_arena.buf, *self._handed_over_flows()):
+                _scale(buf, flows_memory)
         # The running flow total decays with the flows it normalises.  (The reference only clears it when the
         # rescaled EM update consumes it, model/tensorcircuit.py:1363-1374, so that under data parallelism, where every
         # synchronisation replaces it by the sum over ranks, it doubles per step; here it stays the total of the
@@ -1238,6 +1246,13 @@ class TensorCircuit(nn.Module):
                 layer._launch_zero_shadow()
             clean = clean and layer._arena_zero and not moved
         _fill(arena.buf[:arena.segment_end(0)] if clean else arena.buf, 0.0)
+        for buf in self._handed_over_flows():
+            _fill(buf, 0.0)
+
+    def _handed_over_flows(self):
+        """Accumulators that a caller has put in the place of their part of the arena (``layer.param_flows = buffer``)."""
+        own = [self.param_flows, *[layer._param_flows for layer in self.input_layer_group]]
+        return [t for t, view in zip(own, self._flow_arena.views) if t is not None and t.data_ptr() != view.data_ptr()]
 
     def zero_param_flows(self):
         self.init_param_flows(flows_memory=0.0)
@@ -1301,13 +1316,14 @@ class TensorCircuit(nn.Module):
         layers = self._leaf_layers
         state = tuple(layer._em_state(keep_zero_params) for layer in layers)
         if (not self.use_cuda_graphs or self._reference_compat or getattr(self, "_late_sync", None) is not None
-                or self.param_flows is None or self.num_sum_params >= self._EM_FORK_PARAMS
+                or self.param_flows is None or any(layer._param_flows is None for layer in layers)
+                or self.num_sum_params >= self._EM_FORK_PARAMS
                 or any((layer._shadow is not None and layer.max_cats >= layer.SHADOW_MIN_CATS) or layer.num_parameters >= 4 * self._EM_FORK_PARAMS for layer in layers)):
             self.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
             self.init_param_flows(flows_memory=0.0)
             return
         key = ("em", step_size, pseudocount, keep_zero_params, state, self.use_side_stream, self._param_ptrs(),
-               self.param_flows.data_ptr())
+               self._flow_ptrs())
         if key not in self._graphs:
             seen = [k for k in self._graphs if k[0] == "em"]
             if len(seen) >= 4:                               # a schedule of step sizes: keep the latest few
@@ -1352,6 +1368,9 @@ class TensorCircuit(nn.Module):
                 layer._mark_em(layer._em_state(keep_zero_params))
 
     def _em_launches(self, step_size: float, pseudocount: float, keep_zero_params: bool):
+        if self.param_flows is None or any(layer._param_flows is None for layer in self.input_layer_group):
+            raise RuntimeError("there are no parameter flows to update from: run a backward pass first")
+
         def sum_update():
             head = self.param_flows[:2048].clone() if (self._reference_compat and self._fusing_dev) else None
             for start, n, chs in self._fusing_dev:

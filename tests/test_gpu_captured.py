@@ -1,0 +1,91 @@
+"""Steps that are replayed from captured graphs, against the CPU oracle: what may change between two passes of a circuit has
+to reach the replay."""
+import numpy as np
+import pytest
+import torch
+
+import pyjuice_b200 as pj
+from helpers import OracleTrainer, folded_input_flows, rel_close
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _compiled(kind, latents=8, cats=7):
+    torch.manual_seed(3)
+    S = pj.structures
+    if kind == "hclt":
+        tree = S.random_grid_spanning_tree(4, 5, np.random.default_rng(3))
+        ns = S.tree_to_hidden_circuit(tree, tree.center(), num_latents=latents, num_cats=cats)
+    else:
+        ns = S.HMM(seq_length=6, num_latents=latents, num_emits=cats, homogeneous=True)
+    return pj.compile(ns, verbose=False).to(DEV)
+
+
+def _batch(pc, B, seed=0):
+    cats = min(layer.max_cats for layer in pc.input_layer_group)
+    return torch.randint(0, cats, (B, pc.num_vars), generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+def _step(pc, opt, x):
+    lls = pc(x)
+    lls.mean().backward()
+    opt.step()
+    return lls
+
+
+# (32 states, 600 categories: leaf flows through the transposed shadow)
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 8, 7), ("hmm", 8, 7), ("hmm", 32, 600)])
+def test_leaf_flow_buffer_handed_over_between_steps(kind, latents, cats):
+    pc = _compiled(kind, latents, cats)
+    opt = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1)
+    x = _batch(pc, 40)
+    for _ in range(4):
+        _step(pc, opt, x)
+    layer, ref = pc.input_layer_group[0], OracleTrainer(pc)
+    arena_part = layer.param_flows
+    layer.param_flows = buf = torch.zeros_like(arena_part)
+    for i in range(5):
+        pc(x).mean().backward()
+        ref.accumulate(x)
+        if i == 0:
+            assert layer.param_flows is buf
+            ok, err = rel_close(folded_input_flows(layer, buf), folded_input_flows(layer, ref.ipf[0]))
+            assert ok, err
+            assert arena_part.abs().max().item() == 0.0
+        opt.step()
+        ref.update(0.3, 0.1)
+        ref.check_params(pc)
+        assert buf.abs().max().item() == 0.0                 # cleared with the others
+    pc(x).mean().backward()
+    before = layer.param_flows.clone()
+    pc.init_param_flows(flows_memory=0.5)
+    assert torch.equal(layer.param_flows, before * 0.5)
+
+
+def test_leaf_flow_buffer_that_does_not_fit_is_refused():
+    pc = _compiled("hclt")
+    pc.init_param_flows(flows_memory=0.0)
+    layer = pc.input_layer_group[0]
+    n = layer.num_param_flows
+    for bad in (torch.zeros(n - 1, device=DEV), torch.zeros(n, device=DEV, dtype=torch.float64),
+                torch.zeros(2 * n, device=DEV)[::2]):
+        with pytest.raises(ValueError, match="param_flows"):
+            layer.param_flows = bad
+
+
+def test_leaf_flow_buffer_taken_away_between_steps():
+    pc = _compiled("hclt")
+    opt = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1)
+    x = _batch(pc, 40)
+    for _ in range(4):
+        _step(pc, opt, x)
+    ref = OracleTrainer(pc)
+    pc.input_layer_group[0].param_flows = None
+    with pytest.raises(RuntimeError, match="backward pass"):
+        pc.mini_batch_em(step_size=0.3)
+    for _ in range(4):
+        _step(pc, opt, x)
+        ref.accumulate(x)
+        ref.update(0.3, 0.1)
+        ref.check_params(pc)
