@@ -76,7 +76,6 @@ class ColumnProgram:
     def __init__(self, pc):
         self.device = pc.device
         self.num_dummy = pc.num_dummy_nodes
-        self.dense_par_bytes = pc.dense_par_max_bytes
         self._by_width, self._choice, self._rooms, self._par = {}, {}, {}, {}
         groups = pc.inner_layer_groups
         self.depths = []
@@ -692,8 +691,16 @@ class ColumnProgram:
             g["tiles"][n] = (make(g["n_blocks"] * (g["bs"] // 128) * chunks * 32768), make(-(-g["K"] // 256) * chunks * 65536))
         return (*g["tiles"][n], chunks)
 
-    def param_flows(self, pf, nf, nm, params, logspace: bool = True, beside=None):
-        """``beside``: None: all parameter flows; True: those that go beside the others on a second stream, False: the others.
+    def drop_operands(self):
+        """Gives back the operand buffers of the dense products."""
+        for par in self._par.values():
+            for g in par["dense"] if isinstance(par, dict) else ():
+                g.pop("W", None)
+                g.pop("tiles", None)
+
+    def param_flows(self, pf, nf, nm, params, max_bytes: int, logspace: bool = True, beside=None):
+        """``max_bytes``: limit of a dense product's operands.  ``beside``: None: all parameter flows; True: those that go
+        beside the others on a second stream, False: the others.
         The jobs of kinds 0 and 1 (roots, products of many children) are few and long and leave most of an SM free, which
         the staged tiles, persistent and bound by shared memory, cannot use: 62 of 560 us of a Poon-Domingos circuit over 784
         variables.  Without other jobs they are not split off: they then run beside the leaves' flows."""
@@ -704,7 +711,7 @@ class ColumnProgram:
         for g in par["dense"] if beside is not True else ():
             # (as many layers at a time as the operand buffers may take)
             layer = 4 * W * (g["n_blocks"] * g["bs"] + -(-g["K"] // 256) * 256)
-            step = max(1, min(g["n"], self.dense_par_bytes // layer))
+            step = max(1, min(g["n"], max_bytes // layer))
             for m in range(0, g["n"], step):
                 n = min(step, g["n"] - m)
                 x, y, chunks = self._dense_operands(g, n, W)

@@ -90,13 +90,13 @@ class TensorCircuit(nn.Module):
 
         self._nm = self._em = self._nf = self._ef = None
         self._batch = 0
+        self._column_program = None
         self.param_flows = None
         self._init_layers(layer_sparsity_tol, max_num_partitions, max_tied_ns_per_parflow_block)
 
         self._optim_hyperparams = {"compute_param_flows": True, "flows_memory": 1.0}
         self._graphs = {}
         self.use_cuda_graphs = True
-        self._column_program = None
         self.use_dataflow_launch = True       # runs of folded depths as one launch (tiles wait on counters)
         self.use_column_program = True        # all levels in one launch (see column.py)
         self.use_side_stream = True           # independent kernels of a step share the device (two streams)
@@ -104,7 +104,7 @@ class TensorCircuit(nn.Module):
         self.use_nvtx = bool(os.environ.get("PCX_B200_NVTX"))     # NVTX ranges around the phases of a step (profilers)
         self.sum_mode = None                  # this circuit's arithmetic (0, 1 or 2 as `_lib.set_sum_mode`); None = default
         self.chain_tile = None                # tile width of that launch in samples (16 / 32 / 64); None = choose
-        self.dense_par_max_bytes = 16 << 30   # operand buffers of the dense parameter-flow product (all groups)
+        self.dense_par_max_bytes = 16 << 30
         self.default_propagation_alg = "LL"        # "LL", "MPE" or "GeneralLL" (see `set_propagation_alg`)
         self.propagation_alg_kwargs = dict()
         self._alg = (0, 0.0)                        # rule of the pass in progress: (id, alpha)
@@ -149,6 +149,18 @@ class TensorCircuit(nn.Module):
             if group.is_prod():
                 for layer in group:
                     layer._raw_backward_tables = bool(on)
+
+    @property
+    def dense_par_max_bytes(self) -> int:
+        """Bytes that the operand buffers of the dense parameter-flow products may take (all groups of a circuit)."""
+        return self._dense_par_max_bytes
+
+    @dense_par_max_bytes.setter
+    def dense_par_max_bytes(self, n: int):
+        self._dense_par_max_bytes = int(n)
+        self._graphs, self._dense_par_cache = {}, {}          # plans and graphs that hold the buffers of the old limit
+        if self._column_program:
+            self._column_program.drop_operands()
 
     # ------------------------------------------------------------------------------------------
     # construction
@@ -960,7 +972,8 @@ class TensorCircuit(nn.Module):
     def _launch_par(self, logspace_flows: bool, beside=None):
         """``beside``: see `ColumnProgram.param_flows`; the batched launch of the per-layer kernels is one piece."""
         if self._column_plan() is not None:
-            self._column_program.param_flows(self.param_flows, self._nf, self._nm, self.params.data, logspace_flows, beside)
+            self._column_program.param_flows(self.param_flows, self._nf, self._nm, self.params.data,
+                                             self.dense_par_max_bytes, logspace_flows, beside)
         elif not beside:
             self._launch_batched_par(logspace_flows)
 

@@ -6,6 +6,7 @@ import torch
 
 import pyjuice_b200 as pj
 from helpers import OracleTrainer, folded_input_flows, rel_close
+from pyjuice_b200.column import ColumnProgram
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -89,3 +90,22 @@ def test_leaf_flow_buffer_taken_away_between_steps():
         ref.accumulate(x)
         ref.update(0.3, 0.1)
         ref.check_params(pc)
+
+
+def test_limit_of_the_dense_operands_changed_between_steps(monkeypatch):
+    monkeypatch.setattr(ColumnProgram, "DENSE_PAR_WORK", 0)
+    pc = _compiled("hmm", 256, 11)
+    opt = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1)
+    x = _batch(pc, 77)
+    for _ in range(3):
+        _step(pc, opt, x)
+    group, = pc._column_program.par(pc._nm.size(1))["dense"]
+    assert list(group["tiles"]) == [group["n"]]               # all layers in one product
+    ref = OracleTrainer(pc)
+    pc.dense_par_max_bytes = 1 << 19
+    for _ in range(4):
+        _step(pc, opt, x)
+        ref.accumulate(x)
+        ref.update(0.3, 0.1)
+        ref.check_params(pc)
+    assert max(group["tiles"]) < group["n"]
