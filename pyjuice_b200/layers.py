@@ -251,8 +251,10 @@ class InputLayer(Layer, nn.Module):
             object.__setattr__(self, name, value)
         else:
             nn.Module.__setattr__(self, name, value)
-            if name == "params":                            # reads go through `__dict__`, not `nn.Module.__getattr__`
-                object.__setattr__(self, "_leaf_params", value)
+
+    @property
+    def _leaf_params(self):                      # goes round `nn.Module.__getattr__`; looked up each time (see `TensorCircuit`)
+        return self._parameters["params"]
 
     def is_input(self):
         return True

@@ -122,10 +122,16 @@ class TensorCircuit(nn.Module):
             object.__setattr__(self, name, value)
         else:
             nn.Module.__setattr__(self, name, value)
-            if name == "params":                            # reads go through `__dict__`, not `nn.Module.__getattr__`
-                object.__setattr__(self, "_sum_params", value)
-            elif name == "input_layer_group":
-                object.__setattr__(self, "_leaf_layers", tuple(value) if value is not None else ())
+
+    # Reads that go round `nn.Module.__getattr__`.  What they return is looked up each time: a parameter or module may be
+    # replaced in these tables directly (`torch.func.functional_call`, a conversion that makes new parameters).
+    @property
+    def _sum_params(self):
+        return self._parameters["params"]
+
+    @property
+    def _leaf_layers(self):
+        return self._modules["input_layer_group"].layers
 
     @property
     def reference_compat(self) -> bool:

@@ -109,3 +109,24 @@ def test_limit_of_the_dense_operands_changed_between_steps(monkeypatch):
         ref.update(0.3, 0.1)
         ref.check_params(pc)
     assert max(group["tiles"]) < group["n"]
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 32, 7), ("hmm", 32, 600)])
+def test_parameters_replaced_in_the_module_tables(kind, latents, cats):
+    """`torch.func.functional_call` puts other tensors in the place of the parameters for one call."""
+    pc, other = _compiled(kind, latents, cats), _compiled(kind, latents, cats)
+    with torch.no_grad():
+        other.params.copy_(pc.params)
+        leaf = other.input_layer_group[0].params
+        leaf.copy_(leaf[torch.randperm(leaf.numel(), device=DEV)])
+    other.params.data = other.params.data ** 1.5
+    x = _batch(pc, 24)
+    with torch.no_grad():
+        want = other(x)
+        own = [pc(x) for _ in range(4)][-1]
+        tensors = {n: p.detach().clone() for n, p in other.named_parameters()}
+        got = [torch.func.functional_call(pc, tensors, (x,)) for _ in range(4)]
+        assert torch.equal(pc(x), own)
+    assert (want - own).abs().min().item() > 1e-2
+    for g in got:
+        assert torch.equal(g, want)
