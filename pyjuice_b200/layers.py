@@ -134,11 +134,13 @@ class ParamPacker:
             return plan.get("stamp") != self._stamp_of(params)
         return bool(self.entries or self.sm_entries) and self._stamp_of(params) != self._stamp
 
+    # A stamp names the parameters by their address, so the storage is held as long as the stamp: another tensor cannot be
+    # there meanwhile.
     def mark(self, params: torch.Tensor, plan=None):
         if plan is not None:
-            plan["stamp"] = self._stamp_of(params)
+            plan["stamp"], plan["stamped"] = self._stamp_of(params), params.detach()
         else:
-            self._stamp = self._stamp_of(params)
+            self._stamp, self._stamped = self._stamp_of(params), params.detach()
 
     def launch(self, params: torch.Tensor, plan=None):
         if plan is not None:
@@ -400,6 +402,7 @@ class InputLayer(Layer, nn.Module):
 
     def _mark_shadow(self):
         self._shadow["stamp"] = self._shadow_stamp()
+        self._shadow["stamped"] = self._leaf_params.detach()         # (see `ParamPacker.mark`)
 
     def _launch_forward(self, data: torch.Tensor, node_mars: torch.Tensor, stale: bool):
         B = node_mars.size(1)

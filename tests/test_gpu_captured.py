@@ -130,3 +130,22 @@ def test_parameters_replaced_in_the_module_tables(kind, latents, cats):
     assert (want - own).abs().min().item() > 1e-2
     for g in got:
         assert torch.equal(g, want)
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 32, 7), ("hclt", 128, 7), ("hmm", 32, 600)])
+def test_parameters_at_the_address_of_freed_ones(kind, latents, cats):
+    """Tables derived from parameters that are gone do not serve others that came to lie where they were."""
+    pc, other = _compiled(kind, latents, cats), _compiled(kind, latents, cats)
+    x = _batch(pc, 24)
+    host = [{n: p.detach().cpu() ** (1.0 + 0.5 * i) for n, p in pc.named_parameters()} for i in range(5)]
+    lls, at = [], []
+    with torch.no_grad():
+        for h in host:
+            tensors = {n: p.to(DEV) for n, p in h.items()}
+            at.append([t.data_ptr() for t in tensors.values()])
+            lls.append(torch.func.functional_call(pc, tensors, (x,)).cpu())
+            del tensors
+        for h, got in zip(host, lls):
+            for n, p in other.named_parameters():
+                p.copy_(h[n])
+            assert torch.equal(got, other(x).cpu()), at
