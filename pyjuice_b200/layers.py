@@ -75,7 +75,7 @@ class ParamPacker:
         self.owner = owner                       # weak reference to the circuit whose ``params`` the tiles follow
         self.entries = {}
         self.sm_entries = {}
-        self._stamp = None
+        self._stamp = self._stamped = None
         self._epoch = 0
 
     def register(self, key, n_rows, K, row_block, par_block, mode, kids, kpar):
@@ -87,7 +87,7 @@ class ParamPacker:
             entry = dict(buf=buf, tiles=tiles, kids=kids, kpar=kpar, K=K, row_block=row_block,
                          par_block=par_block if mode == 1 else 1, n_chunks=(contraction + 63) // 64, mode=mode)
             self.entries[key] = entry
-            self._stamp = None
+            self._stamp = self._stamped = None
             self._jobs = None
         return entry["buf"]
 
@@ -117,7 +117,7 @@ class ParamPacker:
             entry = dict(buf=torch.empty(nbytes, dtype=torch.uint8, device=self.device),
                          args=(first_row, kids, kpar, n_merged, nb, block, K, par_block, mode))
             self.sm_entries[key] = entry
-            self._stamp = None
+            self._stamp = self._stamped = None
             self._sm_jobs = None
         return entry["buf"]
 
@@ -125,8 +125,9 @@ class ParamPacker:
     def _stamp_of(self, params: torch.Tensor):
         # (``.data`` of a parameter counts versions of its own: the circuit's parameter tells for both)
         pc, ptr = self.owner() if self.owner is not None else None, params.data_ptr()
-        own = pc is not None and pc._sum_params.data_ptr() == ptr
-        return (ptr, pc._sum_params._version if own else params._version, self._epoch)
+        if pc is not None and params is not pc._parameters["params"] and pc._parameters["params"].data_ptr() == ptr:
+            params = pc._parameters["params"]
+        return (ptr, params._version, self._epoch)
 
     def stale(self, params: torch.Tensor, plan=None) -> bool:
         """Whether the tiles lag behind ``params``."""
@@ -137,10 +138,13 @@ class ParamPacker:
     # A stamp names the parameters by their address, so the storage is held as long as the stamp: another tensor cannot be
     # there meanwhile.
     def mark(self, params: torch.Tensor, plan=None):
-        if plan is not None:
-            plan["stamp"], plan["stamped"] = self._stamp_of(params), params.detach()
+        stamp = self._stamp_of(params)
+        last = self._stamp if plan is None else plan.get("stamp")
+        held = params.detach() if last is None or last[0] != stamp[0] else None
+        if plan is None:
+            self._stamp, self._stamped = stamp, self._stamped if held is None else held
         else:
-            self._stamp, self._stamped = self._stamp_of(params), params.detach()
+            plan["stamp"], plan["stamped"] = stamp, plan["stamped"] if held is None else held
 
     def launch(self, params: torch.Tensor, plan=None):
         if plan is not None:
@@ -255,7 +259,7 @@ class InputLayer(Layer, nn.Module):
             nn.Module.__setattr__(self, name, value)
 
     @property
-    def _leaf_params(self):                      # goes round `nn.Module.__getattr__`; looked up each time (see `TensorCircuit`)
+    def _leaf_params(self):                      # (goes round `nn.Module.__getattr__`)
         return self._parameters["params"]
 
     def is_input(self):
