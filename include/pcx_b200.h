@@ -524,6 +524,30 @@ int pcx_column_par(int kind, float* param_flows, const float* node_flows, const 
                    const float* element_values, const float* params, const PcxColPar* jobs, const int32_t* kids,
                    const int32_t* offsets, int n_jobs, int W, int logspace, int terms, void* stream);
 
+/* The planner of the column program (host only).  Functions that may refuse return 1 when the circuit has a table the program
+ * does not cover and -1 on an error, with the reason in `why`.
+ *
+ * desc: nodes, elements, dummy nodes, first root row, row after the last, depths; per depth: 1 if products without parents
+ * exist, product layers, sum layers, each: how many, then per layer block size and twice (forward, backward tables): how many
+ * partitions, then per partition rows n, width w, child block size (backward tables of sums; else 0) and the places in `tables`
+ * of its tables: [n], then [n, w] each.  Products: elements, children; nodes, parent elements (0: none).  Sums: nodes,
+ * children, parameters, flows; elements, parents, parameters. */
+int pcx_colplan_new(const int64_t* desc, int64_t n_desc, const int32_t* tables, int64_t n_tables, void** planner, char* why,
+                    int why_len);
+int pcx_colplan_free(void* planner);
+/* Rows of stored element values; depth (in 16) of the deepest CTA task, 0 without any. */
+int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps);
+/* Whether the program is the better choice at rows of W samples; rooms: clusters of 1, 2, 4, 8 and 16 CTAs at a time. */
+int pcx_colplan_suits(const void* planner, int64_t W, const int32_t* rooms);
+/* Tables: the launches at rows of W samples; groups of tied tables; parameter-flow jobs, without the groups flagged in `dense`.
+ * Each makes a blob: one array of device tables and a description of its sections (see column.py). */
+int pcx_colplan_cut(const void* planner, int64_t W, const int32_t* rooms, int64_t wide_items, int64_t prod_reads, void** blob,
+                    char* why, int why_len);
+int pcx_colplan_tied(const void* planner, void** blob, char* why, int why_len);
+int pcx_colplan_jobs(const void* planner, const uint8_t* dense, void** blob, char* why, int why_len);
+int pcx_colplan_blob(const void* blob, const int32_t** data, int64_t* n_data, const int64_t** meta, int64_t* n_meta);
+int pcx_colplan_blob_free(void* blob);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,6 +1,6 @@
 """Builds the CUDA library in-tree: ``python -m pyjuice_b200.csrc.build``.
 
-One shared object, ``libpcx_b200.so``, from every ``.cu`` file beside this script, compiled for
+One shared object, ``libpcx_b200.so``, from every ``.cu`` and ``.cpp`` file beside this script, compiled for
 sm_100a only.  ``nvcc`` cross-compiles, so no GPU is needed to build.
 
 ``python -m pyjuice_b200.csrc.build --trace`` builds a second library, ``libpcx_b200_trace.so``, with
@@ -24,7 +24,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
 
 
 def sources():
-    return sorted(glob.glob(os.path.join(HERE, "*.cu")))
+    return sorted(glob.glob(os.path.join(HERE, "*.cu")) + glob.glob(os.path.join(HERE, "*.cpp")))
 
 
 def needs_build() -> bool:
@@ -48,7 +48,7 @@ def _build(lib: str, extra, obj_suffix: str, verbose: bool) -> str:
     from concurrent.futures import ThreadPoolExecutor
 
     def compile_one(src):
-        obj = src[:-3] + obj_suffix
+        obj = os.path.splitext(src)[0] + obj_suffix
         cmd = [NVCC, *flags, "-c", src, "-o", obj] + (["-Xptxas", "-v"] if verbose else [])
         subprocess.run(cmd, check=True)
         return obj

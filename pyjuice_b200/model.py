@@ -292,17 +292,20 @@ class TensorCircuit(nn.Module):
     def _mask_parentless_in_device_tables(self):
         """The kernels' copies of the product layers' backward tables skip parentless products (id 0 = padding), so
         the backward sweep needs no reset of the element-flow buffer; the public tables stay as compiled."""
-        for gi, (lo, hi, orphan) in self._parentless.items():
+        for gi in self._parentless:
             for layer in self.inner_layer_groups[gi]:
                 if layer._dev is None:
                     continue
-                bk = []
                 layer._dev["bk_raw"] = list(layer._dev["bk"])          # as compiled (`reference_compat`)
-                for u_cids, parids in layer._dev["bk"]:
-                    p = parids.long().cpu()
-                    dead = orphan[p.clamp(max=hi - 1)] & (p != 0)
-                    bk.append((u_cids, torch.where(dead, torch.zeros_like(p), p).to(torch.int32).to(parids.device)))
-                layer._dev["bk"] = bk
+                layer._dev["bk"] = [(u, self._without_parentless(gi, p).to(torch.int32).to(p.device)) for u, p in layer._dev["bk"]]
+
+    def _without_parentless(self, gi: int, parids: torch.Tensor) -> torch.Tensor:
+        """``parids`` (a backward table of product group ``gi``) on the host, parentless products replaced by padding."""
+        p = parids.long().cpu()
+        if gi not in self._parentless:
+            return p
+        _, hi, orphan = self._parentless[gi]
+        return torch.where(orphan[p.clamp(max=hi - 1)] & (p != 0), torch.zeros_like(p), p)
 
     def _compile_em_blocks(self):
         """Per node block of every untied sum vector: first parameter, first flow, real fan-in, block size —
@@ -736,7 +739,7 @@ class TensorCircuit(nn.Module):
         return self.forward(*args, propagation_alg="GeneralLL", **kwargs)
 
     def _param_ptrs(self):
-        return (self._sum_params.data_ptr(), *[layer._leaf_params.data_ptr() for layer in self._leaf_layers])
+        return (self._parameters["params"].data_ptr(), *[layer._parameters["params"].data_ptr() for layer in self._leaf_layers])
 
     def _flow_ptrs(self):
         return (self.param_flows.data_ptr(), *[layer._param_flows.data_ptr() for layer in self._leaf_layers])
@@ -781,12 +784,13 @@ class TensorCircuit(nn.Module):
                 _fill(self._nm[self.num_dummy_nodes:], float("nan"))
             plan = self._column_plan()
             pack = _lib.sum_mode() != 0 and self._packer.stale(self._sum_params, plan)
-            shadows = tuple([layer._shadow_stale(W) for layer in self._leaf_layers])
+            leaves = self._leaf_layers
+            shadows = tuple([layer._shadow_stale(W) for layer in leaves])
             key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
             self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
             if pack:
                 self._packer.mark(self._sum_params, plan)
-            for layer, stale in zip(self._leaf_layers, shadows):
+            for layer, stale in zip(leaves, shadows):
                 if stale:
                     layer._mark_shadow()
             lls = self._root_view.clone()
@@ -1046,8 +1050,9 @@ class TensorCircuit(nn.Module):
                 self._eflow_mode = ls
             if compute_param_flows and (flows_memory != 1.0 or self.param_flows is None or self._late_sync is not None):
                 self.init_param_flows(flows_memory=flows_memory)     # decay (or clear) the accumulators and the flow total
+            leaves = self._leaf_layers
             if compute_param_flows:
-                for layer in self._leaf_layers:
+                for layer in leaves:
                     if layer._param_flows is None:                   # taken away by the caller
                         layer.init_param_flows()
             r0, r1 = self._root_node_range
@@ -1080,7 +1085,7 @@ class TensorCircuit(nn.Module):
                                              bool(logspace_flows)))
             self._bk_par_pending[key] = self._batched_par_pending
             if tail:
-                for layer in self._leaf_layers:
+                for layer in leaves:
                     layer._mark_backward(W)
             elif compute_param_flows:
                 # the input layer first, then the all-reduce of its flows (the larger part of the arena) beside the sum
