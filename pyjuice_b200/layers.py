@@ -33,7 +33,7 @@ def _dev_i32(t: torch.Tensor, device) -> torch.Tensor:
 def _rows(*bufs):
     """Value buffers as the kernels address them.  A circuit's public buffers are views of the first B columns of rows
     padded to a multiple of eight samples; the kernels work on whole rows."""
-    return tuple(t if t is None or t.stride(0) == t.size(1) or t.size(0) <= 1
+    return tuple(t if t is None or t.stride(0) == t.size(1) or t.size(0) <= 1 or t.size(1) == 0
                  else t.as_strided((t.size(0), t.stride(0)), (t.stride(0), 1)) for t in bufs)
 
 

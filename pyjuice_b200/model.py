@@ -764,6 +764,21 @@ class TensorCircuit(nn.Module):
         with self._nvtx("pcx forward: inner layers"):
             self._forward_inner()
 
+    def _forward_launches(self, data: torch.Tensor, W: int):
+        if self.debug_poison:               # every row must be rewritten by the layer that owns it
+            _fill(self._nm[self.num_dummy_nodes:], float("nan"))
+        plan = self._column_plan()
+        pack = _lib.sum_mode() != 0 and self._packer.stale(self._sum_params, plan)
+        leaves = self._leaf_layers
+        shadows = tuple([layer._shadow_stale(W) for layer in leaves])
+        key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
+        self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
+        if pack:
+            self._packer.mark(self._sum_params, plan)
+        for layer, stale in zip(leaves, shadows):
+            if stale:
+                layer._mark_shadow()
+
     @_in_own_mode
     def forward(self, inputs: torch.Tensor, input_layer_fn=None, cache=None, return_cache: bool = False,
                 propagation_alg: Optional[str] = None, pflow_temperature: float = 1.0, **kwargs):
@@ -780,19 +795,8 @@ class TensorCircuit(nn.Module):
             W = self._nm.size(1)
             data = self._data_buf = self._prepare_inputs(inputs, out=self._data_buf)
             self._last_inputs = origin_inputs
-            if self.debug_poison:               # every row must be rewritten by the layer that owns it
-                _fill(self._nm[self.num_dummy_nodes:], float("nan"))
-            plan = self._column_plan()
-            pack = _lib.sum_mode() != 0 and self._packer.stale(self._sum_params, plan)
-            leaves = self._leaf_layers
-            shadows = tuple([layer._shadow_stale(W) for layer in leaves])
-            key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
-            self._run_inner(key, partial(self._forward_pass, data, pack, shadows))
-            if pack:
-                self._packer.mark(self._sum_params, plan)
-            for layer, stale in zip(leaves, shadows):
-                if stale:
-                    layer._mark_shadow()
+            if W > 0:                           # (an empty batch has nothing to launch)
+                self._forward_launches(data, W)
             lls = self._root_view.clone()
         if torch.is_grad_enabled():
             lls.requires_grad_()
@@ -1063,7 +1067,7 @@ class TensorCircuit(nn.Module):
             if compute_param_flows:
                 if w is None:
                     self._cum_flow_host += (r1 - r0) * B
-                else:
+                elif B > 0:
                     if self._cum_buf is None:
                         self._cum_buf = torch.zeros((), dtype=torch.float64, device=self.device)
                     total = self._cum_buf
@@ -1071,6 +1075,10 @@ class TensorCircuit(nn.Module):
                       B, r1 - r0, W, int(normalise), total, int(self._cum_flow_dev is not None))
             if total is not None:
                 self._cum_flow_dev = total
+            if W == 0:                          # (an empty batch has nothing to launch)
+                if compute_param_flows:
+                    self._start_early_flow_sync()            # (a collective: every rank takes part)
+                return
 
             if _lib.sum_mode() != 0:
                 self._packer.refresh(self._sum_params, self._column_plan())

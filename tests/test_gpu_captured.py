@@ -149,3 +149,22 @@ def test_parameters_at_the_address_of_freed_ones(kind, latents, cats):
             for n, p in other.named_parameters():
                 p.copy_(h[n])
             assert torch.equal(got, other(x).cpu()), at
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 8, 7), ("hclt", 32, 7), ("hclt", 128, 7), ("hmm", 32, 600)])
+def test_empty_batches_add_nothing(kind, latents, cats):
+    pc = _compiled(kind, latents, cats)
+    x = _batch(pc, 24)
+    pc.init_param_flows(flows_memory=0.0)
+    pc(x).mean().backward()
+    flows, total = [pc.param_flows.clone(), pc.input_layer_group[0].param_flows.clone()], pc._cum_flow
+    for _ in range(3):
+        lls = pc(x[:0])
+        assert lls.shape == (0, 1)
+        lls.sum().backward()
+        pc.backward(x[:0])
+        assert pc.node_flows.shape == (pc.num_nodes, 0)
+    assert torch.equal(pc.param_flows, flows[0]) and torch.equal(pc.input_layer_group[0].param_flows, flows[1])
+    assert pc._cum_flow == total
+    pc(x).mean().backward()
+    assert (pc.param_flows - 2 * flows[0]).norm() <= 1e-5 * flows[0].norm() and pc._cum_flow == 2 * total
