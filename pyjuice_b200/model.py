@@ -507,21 +507,21 @@ class TensorCircuit(nn.Module):
     def _columns(self, t):
         return t if t is None or t.size(1) == self._batch else t[:, :self._batch]
 
-    @property
-    def node_mars(self):
-        return self._columns(self._nm)
+    def _set_columns(self, name: str, t):
+        """The buffers are public: None gives one back (the next pass makes another), a tensor of its shape is copied into it."""
+        own = getattr(self, name)
+        if t is None:
+            setattr(self, name, None)
+            self._graphs = {k: g for k, g in self._graphs.items() if k[0] not in ("fw", "bk")}
+        elif t is not own:
+            if own is None or tuple(t.shape) != (own.size(0), self._batch):
+                raise ValueError(f"a tensor of shape {tuple(t.shape)} does not fit the buffer of the last pass")
+            self._columns(own).copy_(t)
 
-    @property
-    def element_mars(self):
-        return self._columns(self._em)
-
-    @property
-    def node_flows(self):
-        return self._columns(self._nf)
-
-    @property
-    def element_flows(self):
-        return self._columns(self._ef)
+    node_mars = property(lambda self: self._columns(self._nm), lambda self, t: self._set_columns("_nm", t))
+    element_mars = property(lambda self: self._columns(self._em), lambda self, t: self._set_columns("_em", t))
+    node_flows = property(lambda self: self._columns(self._nf), lambda self, t: self._set_columns("_nf", t))
+    element_flows = property(lambda self: self._columns(self._ef), lambda self, t: self._set_columns("_ef", t))
 
     def _ensure_buffers(self, B: int, backward: bool = False):
         """(Re)allocate the value buffers when the padded batch size changes.  Dummy rows are written here once:
@@ -529,7 +529,7 @@ class TensorCircuit(nn.Module):
         changed = self._batch != B
         self._batch = B
         W = -(-B // self._PAD) * self._PAD
-        if self._nm is None or self._nm.size(1) != W:
+        if self._nm is None or self._em is None or self._nm.size(1) != W:
             self._nm = torch.zeros(self.num_nodes, W, device=self.device)
             self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             changed = True
@@ -537,7 +537,7 @@ class TensorCircuit(nn.Module):
             self._graphs = {}
         if changed:
             self._root_view = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t()
-        if backward and (self._nf is None or self._nf.size(1) != W):
+        if backward and (self._nf is None or self._ef is None or self._nf.size(1) != W):
             self._nf = torch.empty(self.num_nodes, W, device=self.device)
             self._ef = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             self._eflow_mode = 1

@@ -168,3 +168,26 @@ def test_empty_batches_add_nothing(kind, latents, cats):
     assert pc._cum_flow == total
     pc(x).mean().backward()
     assert (pc.param_flows - 2 * flows[0]).norm() <= 1e-5 * flows[0].norm() and pc._cum_flow == 2 * total
+
+
+@pytest.mark.parametrize("B", [24, 21])
+def test_public_buffers_can_be_given_back_and_written(B):
+    pc = _compiled("hclt", 32, 7)
+    x = _batch(pc, B)
+    want = [pc(x).clone() for _ in range(3)][-1]
+    pc.backward(x)
+    own = slice(pc.num_dummy_nodes, None)                    # (nobody writes the flows of dummy rows)
+    flows = pc.node_flows.clone()
+    for name in ("node_mars", "element_mars", "node_flows", "element_flows"):
+        setattr(pc, name, None)
+        assert getattr(pc, name) is None
+        assert torch.equal(pc(x), want)
+        pc.backward(x)
+        assert torch.equal(pc.node_flows[own], flows[own])
+    pc.node_flows = torch.full_like(flows, 0.5)
+    assert torch.equal(pc.node_flows, torch.full_like(flows, 0.5))
+    with pytest.raises(ValueError, match="does not fit"):
+        pc.node_flows = flows[:, :-1]
+    pc.node_mars = None
+    with pytest.raises(AssertionError, match="forward"):
+        pc.backward(x)
