@@ -7,7 +7,6 @@ from __future__ import annotations
 
 import ctypes
 import weakref
-from collections import OrderedDict
 
 import numpy as np
 import torch
@@ -145,7 +144,7 @@ class ColumnProgram:
         em_rows, big_steps = ctypes.c_int(), ctypes.c_int()
         _lib.load().pcx_colplan_info(self._planner, ctypes.byref(em_rows), ctypes.byref(big_steps))
         self.em_rows, self.big_steps = em_rows.value, big_steps.value
-        self._by_width, self._par, self._tied, self._rooms = OrderedDict(), {}, None, None
+        self._by_width, self._par, self._tied, self._rooms = {}, {}, None, None
 
     # ---- cutting into tasks ------------------------------------------------------------------------------------------
     def _room(self):
@@ -177,6 +176,13 @@ class ColumnProgram:
             self._by_width[W] = self._cut(W) if self.suits(W) else None
         return self._by_width[W]
 
+    def keep(self, widths):
+        """Drops what belongs to other row widths."""
+        self._by_width = {W: plan for W, plan in self._by_width.items() if W in widths}
+        if self._tied is not None:
+            picks = [self._pick(W) for W in widths if W is not None]
+            self._par = {pick: par for pick, par in self._par.items() if pick in picks}
+
     def _cut(self, W: int):
         blob = _Blob(self.device, "pcx_colplan_cut", self._planner, W, self._room(), self.WIDE_ITEMS, self.PROD_READS)
         n_frag, at_bases, at_kids, n_kids = blob.next(4)
@@ -206,10 +212,14 @@ class ColumnProgram:
         tables that go through one dense product, and the jobs of all others."""
         if self._tied is None:
             self._tied = self._tied_groups()
-        pick = tuple(g["n"] * W * g["n_blocks"] * g["bs"] * g["K"] >= self.DENSE_PAR_WORK for g in self._tied)
+        pick = self._pick(W)
         if pick not in self._par:
             self._par[pick] = self._par_jobs(pick)
         return self._par[pick]
+
+    def _pick(self, W: int):
+        """Which groups of tied tables go through the dense product."""
+        return tuple(g["n"] * W * g["n_blocks"] * g["bs"] * g["K"] >= self.DENSE_PAR_WORK for g in self._tied)
 
     def _tied_groups(self):
         blob = _Blob(self.device, "pcx_colplan_tied", self._planner)

@@ -530,11 +530,13 @@ class TensorCircuit(nn.Module):
         self._batch = B
         W = -(-B // self._PAD) * self._PAD
         if self._nm is None or self._em is None or self._nm.size(1) != W:
+            last = None if self._nm is None else self._nm.size(1)
             self._nm = torch.zeros(self.num_nodes, W, device=self.device)
             self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             changed = True
             self._nf = self._ef = None
             self._graphs = {}
+            self._keep_plans((W, last))
         if changed:
             self._root_view = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t()
         if backward and (self._nf is None or self._ef is None or self._nf.size(1) != W):
@@ -542,6 +544,17 @@ class TensorCircuit(nn.Module):
             self._ef = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             self._eflow_mode = 1
             self._graphs = {k: g for k, g in self._graphs.items() if k[0] != "bk"}
+
+    def _keep_plans(self, widths):
+        """Drops the plans of all other row widths, with their operand buffers and parameter fragments (of a Poon-Domingos
+        circuit over 784 variables with 64 latents 96 MB each).  The present width and the one before it: a ragged last
+        batch comes back once per epoch.  No captured pass holds one: graphs go when the width changes."""
+        for name in ("_chain_cache", "_par_job_cache", "_dense_par_cache"):
+            cache = self.__dict__.get(name, {})
+            self.__dict__[name] = {key: plan for key, plan in cache.items() if key[0] in widths}
+        self._bk_par_pending = {}
+        if self._column_program:
+            self._column_program.keep(widths)
 
     def _init_buffer(self, name: str, shape, set_value: Optional[float] = None):
         t = getattr(self, name, None)

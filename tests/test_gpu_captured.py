@@ -191,3 +191,21 @@ def test_public_buffers_can_be_given_back_and_written(B):
     pc.node_mars = None
     with pytest.raises(AssertionError, match="forward"):
         pc.backward(x)
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 32, 7), ("hclt", 256, 7), ("hmm", 640, 11), ("hmm", 1280, 11)])
+def test_memory_does_not_grow_with_the_number_of_batch_sizes(kind, latents, cats):
+    """What a circuit holds after steps of ten sizes: at most what two circuits that saw the largest only would hold."""
+    def held(sizes):
+        pc = _compiled(kind, latents, cats)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        opt = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1)
+        for B in sizes:
+            for _ in range(3):
+                _step(pc, opt, _batch(pc, B))
+        torch.cuda.synchronize()
+        return torch.cuda.memory_allocated() - before
+    one, many = held([72]), held([72, 8, 16, 24, 32, 40, 48, 56, 64, 72])
+    # (a MB for what graphs own)
+    assert many <= 2 * one + (1 << 20), (many, one)
