@@ -77,19 +77,34 @@ class ParamPacker:
         self.sm_entries = {}
         self._stamp = self._stamped = None
         self._epoch = 0
+        self._ready = True                       # nothing registered, nothing to prepare
 
     def register(self, key, n_rows, K, row_block, par_block, mode, kids, kpar):
         entry = self.entries.get(key)
         if entry is None:
             tiles = int(_lib.load().pcx_packed_tile_count(n_rows, K, row_block, par_block, mode))
-            buf = torch.empty(tiles * self.TILE_BYTES, dtype=torch.uint8, device=self.device)
             contraction = K if mode == 0 else K * par_block
-            entry = dict(buf=buf, tiles=tiles, kids=kids, kpar=kpar, K=K, row_block=row_block,
-                         par_block=par_block if mode == 1 else 1, n_chunks=(contraction + 63) // 64, mode=mode)
+            entry = dict(buf=self._later(), nbytes=tiles * self.TILE_BYTES, tiles=tiles, kids=kids, kpar=kpar, K=K,
+                         row_block=row_block, par_block=par_block if mode == 1 else 1,
+                         n_chunks=(contraction + 63) // 64, mode=mode)
             self.entries[key] = entry
             self._stamp = self._stamped = None
-            self._jobs = None
+            self._ready = False
         return entry["buf"]
+
+    # Tiles get their memory when a pass first needs them: under the column program none does.
+    def _later(self):
+        return torch.empty(0, dtype=torch.uint8, device=self.device)
+
+    def prepare(self, plan=None):
+        """Memory and job tables of what `launch` packs, on the current stream and outside any capture."""
+        if plan is not None or self._ready:
+            return
+        for e in (*self.entries.values(), *self.sm_entries.values()):
+            if e["buf"].numel() != e["nbytes"]:
+                e["buf"].resize_(e["nbytes"])
+        self._jobs, self._sm_jobs = self._job_table(), self._sm_job_table()
+        self._ready = True
 
     def invalidate(self):
         self._epoch += 1
@@ -114,11 +129,10 @@ class ParamPacker:
         if entry is None:
             depth = K if mode == 0 else K * par_block
             nbytes = int(_lib.load().pcx_sm_packed_bytes(n_merged, depth, nb))
-            entry = dict(buf=torch.empty(nbytes, dtype=torch.uint8, device=self.device),
-                         args=(first_row, kids, kpar, n_merged, nb, block, K, par_block, mode))
+            entry = dict(buf=self._later(), nbytes=nbytes, args=(first_row, kids, kpar, n_merged, nb, block, K, par_block, mode))
             self.sm_entries[key] = entry
             self._stamp = self._stamped = None
-            self._sm_jobs = None
+            self._ready = False
         return entry["buf"]
 
     # ``plan``: a plan of the column program; its parameter fragments then stand in for all tiles of the per-layer kernels.
@@ -152,13 +166,9 @@ class ParamPacker:
                 _lib.call("pcx_column_pack", plan["frags"], plan["bases"], plan["n_frag"], params)
             return
         if self.entries:
-            if getattr(self, "_jobs", None) is None:
-                self._jobs = self._job_table()
             jobs, n_jobs, n_vec = self._jobs
             _lib.call("pcx_pack_sum_params", jobs, n_jobs, n_vec, params)
         if self.sm_entries:
-            if getattr(self, "_sm_jobs", None) is None:
-                self._sm_jobs = self._sm_job_table()
             jobs, n_jobs, n_vec = self._sm_jobs
             _lib.call("pcx_pack_sm_jobs", jobs, n_jobs, n_vec, params)
 
@@ -169,6 +179,7 @@ class ParamPacker:
 
     def refresh(self, params: torch.Tensor, plan=None):
         if self.stale(params, plan):
+            self.prepare(plan)
             self.launch(params, plan)
             self.mark(params, plan)
 
@@ -187,10 +198,6 @@ class ParamPacker:
             vec += n_merged * n_chunks * 8 * nb
         jobs = torch.from_numpy(rec.view(np.uint8).copy()).to(self.device)
         return jobs, len(self.sm_entries), vec
-
-    @property
-    def nbytes(self):
-        return sum(e["buf"].numel() for e in self.entries.values())
 
     def scratch(self, nbytes: int) -> torch.Tensor:
         """Operand scratch of the dense sum kernels: one buffer, shared by all layers (they run one after the other);

@@ -782,6 +782,8 @@ class TensorCircuit(nn.Module):
             _fill(self._nm[self.num_dummy_nodes:], float("nan"))
         plan = self._column_plan()
         pack = _lib.sum_mode() != 0 and self._packer.stale(self._sum_params, plan)
+        if pack:
+            self._packer.prepare(plan)
         leaves = self._leaf_layers
         shadows = tuple([layer._shadow_stale(W) for layer in leaves])
         key = ("fw", W, self._launch_cfg(), pack, shadows, data.data_ptr(), self._param_ptrs())
@@ -883,7 +885,7 @@ class TensorCircuit(nn.Module):
                     if not ((wide or layer._dense_ok(p, B, False)) and layer._groups_fw[p][2] == 1):
                         assert not folded, "a dense-folded table must qualify for the dense parameter-flow product"
                         continue
-                    g = groups.setdefault((layer._tiles_fw[p].data_ptr(), wide),
+                    g = groups.setdefault((id(layer._tiles_fw[p]), wide),
                                           dict(members=[], tables=(cids, pids, pfids), n_blocks=nids.numel(),
                                                K=cids.size(1), block_size=layer.block_size, wide=wide))
                     where[(id(layer), p)] = (g, len(g["members"]))

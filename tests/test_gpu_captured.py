@@ -209,3 +209,22 @@ def test_memory_does_not_grow_with_the_number_of_batch_sizes(kind, latents, cats
     one, many = held([72]), held([72, 8, 16, 24, 32, 40, 48, 56, 64, 72])
     # (a MB for what graphs own)
     assert many <= 2 * one + (1 << 20), (many, one)
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 64, 7), ("hclt", 256, 7), ("hmm", 640, 11)])
+def test_parameter_tiles_have_memory_once_a_pass_needs_them(kind, latents, cats):
+    pc = _compiled(kind, latents, cats)
+    opt = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1)
+    x = _batch(pc, 40)
+    for _ in range(3):
+        _step(pc, opt, x)
+    tiles = [e["buf"] for e in (*pc._packer.entries.values(), *pc._packer.sm_entries.values())]
+    assert tiles and all(t.numel() == 0 for t in tiles)       # the column program ran
+    ref = OracleTrainer(pc)
+    pc.use_column_program = False
+    for _ in range(3):
+        _step(pc, opt, x)
+        ref.accumulate(x)
+        ref.update(0.3, 0.1)
+    ref.check_params(pc)
+    assert all(t.numel() > 0 for t in tiles)
