@@ -535,7 +535,7 @@ class TensorCircuit(nn.Module):
             self._em = torch.full((self.num_elements, W), NEG_INF, device=self.device)
             changed = True
             self._nf = self._ef = None
-            self._graphs = {}
+            self._graphs = {k: g for k, g in self._graphs.items() if k[0] == "em"}     # (an update reads no batch)
             self._keep_plans((W, last))
         if changed:
             self._root_view = self._nm[self._root_node_range[0]:self._root_node_range[1], :B].t()

@@ -228,3 +228,23 @@ def test_parameter_tiles_have_memory_once_a_pass_needs_them(kind, latents, cats)
         ref.update(0.3, 0.1)
     ref.check_params(pc)
     assert all(t.numel() > 0 for t in tiles)
+
+
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 8, 7), ("hclt", 64, 7), ("hclt", 128, 7), ("hmm", 32, 600), ("hmm", 640, 11)])
+def test_batch_sizes_change_between_steps(kind, latents, cats):
+    """An epoch's ragged last batch and the full batches around it, other padded columns of one row width, and (600
+    categories) both sides of the line up to which leaf flows go through the transposed shadow."""
+    pc = _compiled(kind, latents, cats)
+    opt, ref = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1), OracleTrainer(pc)
+    sizes = [72] * 4 + [37] + [72] * 4 + [37, 72, 69, 66, 72] + ([608] * 3 + [72] if cats == 600 else [])
+    updates = set()
+    for i, B in enumerate(sizes):
+        x = _batch(pc, B, seed=i)
+        lls = _step(pc, opt, x)
+        want = ref.accumulate(x)
+        assert (lls.detach().double().cpu() - want).abs().max().item() <= 1e-3
+        ref.update(0.3, 0.1)
+        ref.check_params(pc)
+        updates.add(tuple(id(g) for k, g in pc._graphs.items() if k[0] == "em" and g != "warm"))
+    if cats == 7:                                             # captured once, and kept when the width changed
+        assert len(updates - {()}) == 1
