@@ -248,3 +248,50 @@ def test_batch_sizes_change_between_steps(kind, latents, cats):
         updates.add(tuple(id(g) for k, g in pc._graphs.items() if k[0] == "em" and g != "warm"))
     if cats == 7:                                             # captured once, and kept when the width changed
         assert len(updates - {()}) == 1
+
+
+def _structured(kind, latents):
+    import random
+    torch.manual_seed(3)
+    random.seed(3)
+    S = pj.structures
+    ns = (S.PD((9, 7), latents, split_points=[[3, 6], [3]], num_cats=5) if kind == "pd" else
+          S.RAT_SPN(num_vars=40, num_latents=latents, depth=2, num_repetitions=5, num_cats=6))
+    return pj.compile(ns, verbose=False).to(DEV)
+
+
+@pytest.mark.parametrize("kind,latents", [("pd", 64), ("pd", 16), ("rat", 32), ("rat", 8)])
+@pytest.mark.parametrize("attr,value", [("WIDE_ITEMS", 1), ("PROD_READS", 0)])
+@pytest.mark.parametrize("B", [40, 203])
+def test_replayed_launches_of_single_levels(kind, latents, attr, value, B, monkeypatch):
+    """Wide levels, products ahead of a level, and parameter flows on two streams, in their captured form."""
+    monkeypatch.setattr(ColumnProgram, attr, value)
+    pc = _structured(kind, latents)
+    opt, ref = pj.optim.MiniBatchEM(pc, step_size=0.3, pseudocount=0.1), OracleTrainer(pc)
+    for i in range(4):
+        x = _batch(pc, B, seed=i)
+        lls = _step(pc, opt, x)
+        assert (lls.detach().double().cpu() - ref.accumulate(x)).abs().max().item() <= 1e-3
+        ref.update(0.3, 0.1)
+        ref.check_params(pc)
+    assert all(g != "warm" for k, g in pc._graphs.items() if k[0] == "bk")
+
+
+@pytest.mark.parametrize("homogeneous", [True, False])
+def test_flows_accumulate_across_the_line_of_the_transposed_shadow(homogeneous):
+    """Batches of at most as many samples as categories go through the shadow of tied tables, larger ones do not."""
+    torch.manual_seed(3)
+    pc = pj.compile(pj.structures.HMM(seq_length=5, num_latents=32, num_emits=600, homogeneous=homogeneous), verbose=False).to(DEV)
+    opt, ref = pj.optim.FullBatchEM(pc, pseudocount=0.1), OracleTrainer(pc)
+    layer = pc.input_layer_group[0]
+    for sizes in ([40, 608, 600, 616, 40], [608, 40], [40, 40, 40], [608, 608]):
+        for i, B in enumerate(sizes):
+            x = _batch(pc, B, seed=i)
+            pc(x).mean().backward()
+            ref.accumulate(x)
+            assert layer._shadow_ok(pc._nm.size(1)) == (homogeneous and B <= 600)
+        ok, err = rel_close(folded_input_flows(layer, layer.param_flows), folded_input_flows(layer, ref.ipf[0]))
+        assert ok, err
+        opt.step()
+        ref.update(1.0, 0.1)
+        ref.check_params(pc)
