@@ -295,3 +295,28 @@ def test_flows_accumulate_across_the_line_of_the_transposed_shadow(homogeneous):
         opt.step()
         ref.update(1.0, 0.1)
         ref.check_params(pc)
+
+
+@pytest.mark.parametrize("logspace", [True, False])
+@pytest.mark.parametrize("kind,latents,cats", [("hclt", 8, 7), ("hclt", 64, 7), ("hclt", 128, 7), ("hclt", 256, 7), ("hmm", 32, 600),
+                                               ("hmm", 640, 11), ("hmm", 1280, 11), ("pd", 32, 5), ("rat", 8, 6)])
+def test_padding_columns_of_probability_zero(kind, latents, cats, logspace):
+    """Rows are padded with samples of category 0; where that category has probability zero they are worth nothing."""
+    pc = _structured(kind, latents) if kind in ("pd", "rat") else _compiled(kind, latents, cats)
+    layer = pc.input_layer_group[0]
+    with torch.no_grad():
+        table = layer.params.view(-1, layer.max_cats)
+        table[:, 0] = 0.0
+        table /= table.sum(dim=1, keepdim=True)
+    x = _batch(pc, 21).clamp(min=1)
+    ref = OracleTrainer(pc)
+    ref.accumulate(x)
+    for i in range(3):
+        pc.init_param_flows(flows_memory=0.0)
+        lls = pc(x)
+        pc.backward(x if i else None, logspace_flows=logspace)
+        assert torch.isfinite(lls).all()
+        ok, err = rel_close(pc.param_flows, ref.pf)
+        assert ok, err
+        ok, err = rel_close(folded_input_flows(layer, layer.param_flows), folded_input_flows(layer, ref.ipf[0]))
+        assert ok, err
