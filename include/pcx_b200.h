@@ -489,13 +489,14 @@ typedef struct {
  * 3: the flow goes to the children's rows, else to element_flows.
  * wide > 0: ONE level over the whole machine (cluster 1, nt 4, tiles = all column tiles of the row): 1 any tasks, 2 MMA
  * tasks of at most 32 operand entries and two children per element (operands staged through shared memory), 3 (element flows) product tasks only.
- * levels: int32 x 4: first warp task, how many, first split task, how many.  terms: 3 (bf16 hi / lo) or 1. */
+ * levels: int32 x 4: first warp task, how many, first split task, how many; at most PCX_COLUMN_MAX_LEVELS.  terms: 3 (bf16 hi / lo) or 1. */
+#define PCX_COLUMN_MAX_LEVELS 512
 int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,
                    const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
                    const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int tiles, int cluster,
                    int wide, int logspace, int terms, void* stream);
 /* The same walk for circuits with large groups (tasks of kind 4: whole-CTA tasks, in a level's second list).  max_steps: the
- * deepest such task (at most 64 steps: 1024 children).  cluster: up to 16.  At most 512 levels. */
+ * deepest such task (at most 64 steps: 1024 children).  cluster: up to 16. */
 int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* element_flows, float* element_values,
                        const float* params, const void* frags, const PcxColTask* tasks, const int32_t* kids,
                        const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int cluster, int max_steps,

@@ -38,7 +38,7 @@ namespace {
 
 constexpr int CT = 512;                     // threads per CTA (16 warps, 128 registers each)
 constexpr int CW = CT / 32;
-constexpr int MAX_SMEM_LEVELS = 512;
+constexpr int MAX_LEVELS = PCX_COLUMN_MAX_LEVELS;          // of one launch: the level table sits in shared memory
 constexpr int WT = 384;                     // of the wide launches: 12 warps, 168 registers each
 constexpr int MAX_STRIPS = 2;               // 16-row strips an MMA task may hold (accumulators and element values)
 enum ColKind { K_MMA = 0, K_SIMT = 1, K_SPLIT = 2, K_PROD = 3, K_CTA = 4 };
@@ -1011,7 +1011,7 @@ __global__ void __launch_bounds__(256) column_prod_kernel(const ColArgs a) {
 template <int MODE, int NT>
 __global__ void __launch_bounds__(CT, 1) column_kernel(const ColArgs a) {
     __shared__ float s_part[CW * 64];
-    __shared__ int4 s_levels[MAX_SMEM_LEVELS];
+    __shared__ int4 levels[MAX_LEVELS];
     const int warp = threadIdx.x >> 5;
     const int rank = blockIdx.x % a.cluster;
     const int tile = warp % a.tiles;
@@ -1020,10 +1020,8 @@ __global__ void __launch_bounds__(CT, 1) column_kernel(const ColArgs a) {
     const int worker = (warp / a.tiles) * a.cluster + rank, workers = (CW / a.tiles) * a.cluster;
     // The level table sits in shared memory; the record of the warp's next task is in registers and the lines of its tables
     // are on their way to L1, across levels: a level opens with the loads of its values.
-    const bool in_smem = a.n_levels <= MAX_SMEM_LEVELS;
-    for (int i = threadIdx.x; i < a.n_levels && in_smem; i += CT) s_levels[i] = __ldg(a.levels + i);
+    for (int i = threadIdx.x; i < a.n_levels; i += CT) levels[i] = __ldg(a.levels + i);
     __syncthreads();
-    const int4* levels = in_smem ? s_levels : a.levels;
     int next_l = 0, next_i = worker;                       // the task after the fetched ones
     auto advance = [&](int& task, int& at) {
         while (next_l < a.n_levels && next_i >= levels[next_l].y) { ++next_l; next_i = worker; }
@@ -1078,7 +1076,7 @@ template <int NT>
 struct BigSmem {
     static constexpr int MAX = CW * 8 * NT * 4;                        // column maxima per warp
     static constexpr int RED = CW * 32 * NT * 16;                      // partial accumulators
-    static constexpr int LEVELS = MAX_SMEM_LEVELS * 16;
+    static constexpr int LEVELS = MAX_LEVELS * 16;
     static constexpr int PART = CW * 64 * 4;                           // split tasks
     static constexpr int FIXED = MAX + RED + LEVELS + PART;
 };
@@ -1993,7 +1991,7 @@ int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* ele
                        int logspace, int terms, void* stream) {
     if (n_levels <= 0 || W <= 0) return 0;
     if (W % 8 != 0 || (nt != 1 && nt != 2) || cluster < 1 || cluster > 16 || (mode != 0 && mode != 1)) return -1;
-    if (n_levels > MAX_SMEM_LEVELS || max_steps < 1 || max_steps > BIG_MAX_STEPS) return -1;
+    if (n_levels > MAX_LEVELS || max_steps < 1 || max_steps > BIG_MAX_STEPS) return -1;
     if (((reinterpret_cast<uintptr_t>(node_mars) | reinterpret_cast<uintptr_t>(node_flows) |
           reinterpret_cast<uintptr_t>(element_flows) | reinterpret_cast<uintptr_t>(element_values)) & 15) != 0) return -1;
     ColArgs a{};
@@ -2011,6 +2009,7 @@ int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element
                    const int32_t* strips, const int32_t* levels, int n_levels, int W, int nt, int tiles, int cluster,
                    int wide, int logspace, int terms, void* stream) {
     if (n_levels <= 0 || W <= 0) return 0;
+    if (n_levels > MAX_LEVELS) return -1;
     if (wide < 0 || wide > 3 || (wide == 3 && mode == 0) || (wide > 0 && (n_levels != 1 || nt != 4 || tiles != (int)pcx_cdiv(W, 8 * nt)))) return -1;
     if (W % 8 != 0 || (nt != 1 && nt != 2 && !(nt == 4 && wide > 0)) || cluster < 1 || cluster > 8 || (mode != 0 && mode != 1)) return -1;
     if (tiles < 1 || (wide == 0 && (tiles > CW || (tiles & (tiles - 1)) != 0))) return -1;

@@ -805,9 +805,8 @@ struct Cutter {
             int64_t n = 0;
             for (size_t at = 0, end; at < levels[mode].size(); at = end) {      // consecutive fused levels are one launch
                 const Shape how = levels[mode][at].how;
-                for (end = at + 1; how.wide == 0 && end < levels[mode].size() && levels[mode][end].how.wide == 0
-                                   && !(mode == 0 && before[end]);)
-                    ++end;
+                const size_t last = std::min(levels[mode].size(), at + PCX_COLUMN_MAX_LEVELS);
+                for (end = at + 1; how.wide == 0 && end < last && levels[mode][end].how.wide == 0 && !(mode == 0 && before[end]);) ++end;
                 if (mode == 0 && before[at]) n += products(pc.depths[at], blob, launches);
                 launches.insert(launches.end(), {0, (int64_t)at, (int64_t)(end - at), how.nt, how.tiles, how.cluster, how.wide});
                 ++n;

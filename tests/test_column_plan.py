@@ -207,6 +207,14 @@ def test_walk_with_tied_tables_in_one_product(work, monkeypatch):
     assert bool(program.par(8)["dense"]) == (work == 0)
 
 
+@pytest.mark.parametrize("latents", [4, 128])
+def test_walk_of_more_levels_than_one_launch_takes(latents):
+    torch.manual_seed(3)
+    ns = pj.structures.HMM(seq_length=600, num_latents=latents, num_emits=3, homogeneous=True)
+    _, plan = _check(pj.compile(ns, verbose=False), 8)
+    assert all(n <= 512 for m in (0, 1) for _, n, _ in plan[m]["launches"]) and len(plan[0]["launches"]) == 2
+
+
 def test_deep_tables_are_refused():
     S = pj.structures
     with pytest.raises(Unsupported):

@@ -118,3 +118,15 @@ def test_leaves_of_mid_size_vocabularies(cats, homogeneous, B):
     check_against_oracle(pc, x, step=0.2, pseudo=0.1)
     layer = pc.input_layer_group[0]
     assert layer._shadow_ok(pc._nm.size(1)) == (homogeneous and cats >= 512 and pc._nm.size(1) <= cats)
+
+
+@pytest.mark.parametrize("tokens", [512, 513, 600])
+def test_more_levels_than_one_launch_takes(tokens):
+    """(Two categories: the log-likelihood of 600 tokens stays near 400, one fp32 rounding there is 3e-5.)"""
+    torch.manual_seed(5)
+    pc = pj.compile(pj.structures.HMM(seq_length=tokens, num_latents=128, num_emits=2, homogeneous=True)).to(DEV)
+    x = torch.randint(0, 2, (5, tokens), generator=torch.Generator().manual_seed(1))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1)
+    plan = pc._column_plan()
+    assert plan is not None and pc._column_program.big_steps > 0
+    assert len(plan[0]["launches"]) == (1 if tokens <= 512 else 2) and sum(n for _, n, _ in plan[0]["launches"]) == tokens
