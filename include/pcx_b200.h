@@ -465,8 +465,8 @@ int pcx_input_cat_missing(float* param_flows, const float* params, const float* 
                           const int32_t* node_cats, int64_t n_source, float scale, void* stream);
 
 /* ---- column program: all levels of a circuit of small node blocks in one launch --------------------------------
- * A cluster of `cluster` CTAs owns 8 * nt * tiles columns (nt 1 or 2; tiles a power of two) of the value buffers ([rows, W], W % 8 == 0) and walks the levels; a level is a
- * list of tasks without dependencies among them.  Takes the place of the per-layer launches of
+ * A cluster of `cluster` CTAs owns 8 * nt columns (nt 1 or 2; tiles 1) of the value buffers ([rows, W], W % 8 == 0) and
+ * walks the levels; a level is a list of tasks without dependencies among them.  Takes the place of the per-layer launches of
  * model/tensorcircuit.py:377-441 (forward) and 556-674 (backward). */
 typedef struct {
     int32_t kid_off;    /* first entry of the task in `kids` */
@@ -508,10 +508,10 @@ int pcx_column_clusters(int cluster, int big);
 int pcx_column_pack(void* frags, const int32_t* bases, int64_t n, const float* params, void* stream);
 
 /* Parameter flows of all levels.  kind 0: tensor-core tiles of up to 32 nodes (strips of 16 from row0 and row1) x n_k
- * (at most 2) steps of 16 edges; kind 1: fp32 tiles of n_strips nodes (1, 2, 4, 8 or 16) x n_k
- * edges; kinds 2 and 3: as kind 0 for elements of at most two children (or stored values), up to 2 x 2 / 4 x 4 strips x
- * steps, operands staged through shared memory.  offsets: int32 x 2: (parameter,
- * flow) of the first (node, edge) of every (step, strip) / entry; the next edge is bs further. */
+ * (at most 2) steps of 16 edges, elements with their children's rows (any number); kind 1: fp32 tiles of n_strips nodes (1, 2,
+ * 4, 8 or 16) x n_k edges; kinds 2 and 3: as kind 0 for elements of at most two children or stored values, up to 2 x 2 /
+ * 4 x 4 strips x steps, operands staged through shared memory.  offsets: int32 x 2: (parameter, flow) of the first
+ * (node, edge) of every (step, strip) / entry; the next edge is bs further. */
 typedef struct {
     int32_t row0, row1;
     int32_t n_strips;

@@ -60,7 +60,7 @@ struct ColArgs {
     int logspace;
     int terms;
     int cluster;                // CTAs per cluster
-    int tiles;                  // column tiles of 8 * NT per cluster
+    int tiles;                  // column tiles of 32 (wide launches)
     int wide;                   // one level, spread over the whole grid
 };
 
@@ -679,23 +679,25 @@ __device__ void prod_task(const ColArgs& a, const PcxColTask& t, int col0) {
 template <int MODE, int NT>
 __device__ __forceinline__ void run_task(const ColArgs& a, const PcxColTask& t, int col0) {
     if (t.kind == K_MMA) {
-        if (NT == 4 || t.n_k <= 2 || (MODE == C_FWD && t.n_kids > 2)) mma_task<MODE, NT, 2>(a, t, col0);
-        else mma_task<MODE, NT, NT == 4 ? 2 : 4>(a, t, col0);
-    } else if (MODE == C_ELE && t.kind == K_PROD) {
-        prod_task<NT>(a, t, col0);
+        if constexpr (NT < 4) {
+            if (t.n_k > 2 && !(MODE == C_FWD && t.n_kids > 2)) {
+                mma_task<MODE, NT, 4>(a, t, col0);
+                return;
+            }
+        }
+        mma_task<MODE, NT, 2>(a, t, col0);
+    } else if (MODE == C_ELE && NT < 4 && t.kind == K_PROD) {              // (wide product levels: column_prod_kernel)
+        prod_task<NT < 4 ? NT : 2>(a, t, col0);
     } else {
         simt_task<MODE, NT>(a, t, col0);
     }
 }
 
-// A cluster's columns may be several tiles: neighbouring warps of a CTA then take the tiles of one task, so that a
-// parameter fragment is fetched once per SM and the pieces of a value row that are requested at about the same time are
-// neighbours (256 bytes of a DRAM page instead of 64: with 16 columns per cluster, the levels of a 784-variable
-// Poon-Domingos circuit that outgrow the L2 ran at 0.8 TB/s).
-//
 // A level with work for every warp of the machine gains nothing from sharing a launch, and loses the SMs that the
-// clusters leave idle: it is a launch of its own (`wide`), all warps of the grid over (task, column tile) with the tiles
-// of a task next to one another.
+// clusters leave idle: it is a launch of its own (`wide`), all warps of the grid over (task, tile of 32 columns) with the
+// tiles of a task next to one another: a parameter fragment is then fetched once per SM, and the pieces of a value row that
+// are requested at about the same time are neighbours (256 bytes of a DRAM page instead of 64: with 16 columns per
+// cluster, the levels of a 784-variable Poon-Domingos circuit that outgrow the L2 ran at 0.8 TB/s).
 template <int MODE>
 __global__ void __launch_bounds__(WT, 1) column_wide_kernel(const ColArgs a) {
     constexpr int NT = 4, NW = WT / 32;
@@ -1014,10 +1016,8 @@ __global__ void __launch_bounds__(CT, 1) column_kernel(const ColArgs a) {
     __shared__ int4 levels[MAX_LEVELS];
     const int warp = threadIdx.x >> 5;
     const int rank = blockIdx.x % a.cluster;
-    const int tile = warp % a.tiles;
-    const int col_base = (blockIdx.x / a.cluster) * 8 * NT * a.tiles;
-    const int col0 = col_base + tile * 8 * NT;
-    const int worker = (warp / a.tiles) * a.cluster + rank, workers = (CW / a.tiles) * a.cluster;
+    const int col0 = (blockIdx.x / a.cluster) * 8 * NT;
+    const int worker = warp * a.cluster + rank, workers = CW * a.cluster;
     // The level table sits in shared memory; the record of the warp's next task is in registers and the lines of its tables
     // are on their way to L1, across levels: a level opens with the loads of its values.
     for (int i = threadIdx.x; i < a.n_levels; i += CT) levels[i] = __ldg(a.levels + i);
@@ -1043,14 +1043,13 @@ __global__ void __launch_bounds__(CT, 1) column_kernel(const ColArgs a) {
                 touch(a.frags + (int64_t)t1.par_off * 64 + (threadIdx.x & 31) * 8);
             int task2, at2;
             advance(task2, at2);
-            if (col0 < a.W) run_task<MODE, NT>(a, t, col0);
+            run_task<MODE, NT>(a, t, col0);
             t = t1; at = at1;
             task1 = task2; at1 = at2;
         }
         const int4 lv = levels[l];
         if (MODE == C_FWD)
-            for (int i = rank; i < lv.w * a.tiles; i += a.cluster)
-                split_task<NT, CW>(a, a.tasks[lv.z + i / a.tiles], col_base + (i % a.tiles) * 8 * NT, s_part);
+            for (int i = rank; i < lv.w; i += a.cluster) split_task<NT, CW>(a, a.tasks[lv.z + i], col0, s_part);
         if (a.cluster == 1) {
             __syncthreads();
         } else {
@@ -1432,10 +1431,9 @@ struct ColParArgs {
     int terms;
 };
 
-// Tensor-core tiles: a warp owns 32 nodes (two strips) x 32 edges, the batch in steps of 16.  All operands of a step (flow
-// and value of 32 rows, the children's rows of 32 edges) are requested together; the row numbers stay in registers.  The
-// eight warps of a CTA take neighbouring tiles, which share one side's rows.
-template <int NK>
+// Tensor-core tiles of elements of more than two children (up to two, and stored values: column_par_pipe_kernel): a warp owns
+// 32 nodes (two strips) x 32 edges, the batch in steps of 16.  Flow and value of 32 rows are requested together, then the rows
+// of 32 edges child by child.  The eight warps of a CTA take neighbouring tiles, which share one side's rows.
 __device__ __forceinline__ void par_mma_tile(const ColParArgs& a, const PcxColPar& t, int b_begin, int b_end) {
     const int lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int64_t W = a.W;
@@ -1446,14 +1444,6 @@ __device__ __forceinline__ void par_mma_tile(const ColParArgs& a, const PcxColPa
         for (int e = 0; e < 4; ++e)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[s][e][c] = 0.0f;
-    const float* ysrc = t.n_kids < 0 ? a.em : a.nm;
-    int kid[2][NK > 0 ? NK : 1];
-    if (NK > 0) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-            for (int c = 0; c < NK; ++c) kid[q][c] = __ldg(a.kids + t.kid_off + (q < t.n_k ? q : 0) * t.width + c) + g;
-    }
     const int64_t r0 = (int64_t)(t.row0 + g) * W, r1 = (int64_t)(t.row1 + g) * W;
     for (int b0 = b_begin; b0 < b_end; b0 += 16) {
         // lane t holds samples 4t .. 4t+3 where the fragments have 2t, 2t+1, 2t+8, 2t+9: the order of a sum's terms is free,
@@ -1470,39 +1460,21 @@ __device__ __forceinline__ void par_mma_tile(const ColParArgs& a, const PcxColPa
                 ldvec<4>(a.nm + at + c0, v[s][h]);
             }
         float y[4][4];
-        if (NK > 0) {
-            float z[4][NK > 1 ? 4 : 1];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[e][i] = 0.0f;
+        for (int c = 0; c < t.n_kids; ++c) {
+            float z[4][4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float* p = ysrc + (int64_t)(kid[e >> 1][0] + 8 * (e & 1)) * W;
-                ldvec<4>(p + c0, y[e]);
-                if (NK > 1) {
-                    const float* p2 = ysrc + (int64_t)(kid[e >> 1][NK > 1 ? 1 : 0] + 8 * (e & 1)) * W;
-                    ldvec<4>(p2 + c0, z[e]);
-                }
+                const int k = __ldg(a.kids + t.kid_off + ((e >> 1) < t.n_k ? (e >> 1) : 0) * t.width + c) + g + 8 * (e & 1);
+                ldvec<4>(a.nm + k * W + c0, z[e]);
             }
-            if (NK > 1)
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) y[e][i] += z[e][i];
-        } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) y[e][i] = 0.0f;
-            for (int c = 0; c < t.n_kids; ++c) {
-                float z[4][4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int k = __ldg(a.kids + t.kid_off + ((e >> 1) < t.n_k ? (e >> 1) : 0) * t.width + c) + g + 8 * (e & 1);
-                    ldvec<4>(a.nm + k * W + c0, z[e]);
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) y[e][i] += z[e][i];
-            }
+                for (int i = 0; i < 4; ++i) y[e][i] += z[e][i];
         }
         float sh[4];
 #pragma unroll
@@ -1574,9 +1546,7 @@ __global__ void __launch_bounds__(256, 2) column_par_mma_kernel(const ColParArgs
     const int split = item / a.n_jobs, job = item - split * a.n_jobs;
     const PcxColPar t = a.jobs[job];
     const int b_begin = split * a.per_split, b_end = min(a.W, b_begin + a.per_split);
-    if (t.n_kids == -1 || t.n_kids == 1) par_mma_tile<1>(a, t, b_begin, b_end);
-    else if (t.n_kids == 2) par_mma_tile<2>(a, t, b_begin, b_end);
-    else par_mma_tile<0>(a, t, b_begin, b_end);
+    par_mma_tile(a, t, b_begin, b_end);
 }
 
 // The same tiles with their operands copied ahead through shared memory (see column_pipe_kernel): MS strips of 16 nodes x NE
@@ -1895,7 +1865,7 @@ cudaLaunchConfig_t column_config(int n_clusters, int cluster, cudaLaunchAttribut
 template <int MODE, int NT>
 int launch_column(const ColArgs& a, cudaStream_t st) {
     cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = column_config<MODE, NT>((int)pcx_cdiv(a.W, 8 * NT * a.tiles), a.cluster, &attr, st);
+    cudaLaunchConfig_t cfg = column_config<MODE, NT>((int)pcx_cdiv(a.W, 8 * NT), a.cluster, &attr, st);
     cudaError_t e = cudaLaunchKernelEx(&cfg, column_kernel<MODE, NT>, a);
     if (e != cudaSuccess) return (int)e;
     PCX_LAUNCH_CHECK();
@@ -2012,7 +1982,7 @@ int pcx_column_run(int mode, float* node_mars, float* node_flows, float* element
     if (n_levels > MAX_LEVELS) return -1;
     if (wide < 0 || wide > 3 || (wide == 3 && mode == 0) || (wide > 0 && (n_levels != 1 || nt != 4 || tiles != (int)pcx_cdiv(W, 8 * nt)))) return -1;
     if (W % 8 != 0 || (nt != 1 && nt != 2 && !(nt == 4 && wide > 0)) || cluster < 1 || cluster > 8 || (mode != 0 && mode != 1)) return -1;
-    if (tiles < 1 || (wide == 0 && (tiles > CW || (tiles & (tiles - 1)) != 0))) return -1;
+    if (wide == 0 && tiles != 1) return -1;
     if (((reinterpret_cast<uintptr_t>(node_mars) | reinterpret_cast<uintptr_t>(node_flows) |
           reinterpret_cast<uintptr_t>(element_flows) | reinterpret_cast<uintptr_t>(element_values)) & 15) != 0) return -1;
     ColArgs a{};
