@@ -4,7 +4,7 @@
                     [--impl ours|reference|triton]
 
 One "step" is one mini-batch of the named configuration through ``pc(x)``, ``lls.mean().backward()`` and
-``MiniBatchEM.step()``.  The headline workload is configs[4] (the homogeneous HMM: the largest single-GPU
+``MiniBatchEM.step()``.  The headline workload is ``cfg4`` (the homogeneous HMM: the largest single-GPU
 configuration and the one whose sum layers are bound by the tensor cores); the other benchmark configurations
 are measured in the same run and reported under ``other_configs``.  Rank 0 prints ONE JSON line:
 
@@ -247,21 +247,21 @@ def family_work(stats, B, elsize):
 # Sources: profiles/ncu_full_cfg1_chain_par.md, profiles/ncu_full_cfg4_wide_gemm.md, profiles/launch_list_cfg2_pd_b512.md,
 # profiles/traffic_cfg3_rat_spn_b1024.md
 TRAFFIC_PER_LAUNCH = {
-    # configs[1], B = 512: one dataflow launch each for the forward pass and the element flows, one batched launch
+    # 784-variable tree, B = 512: one dataflow launch each for the forward pass and the element flows, one batched launch
     # for the parameter flows
     ("cfg1", "pcx_sum_fwd"): 389.0e6,
     ("cfg1", "pcx_sum_bwd_ele"): 801.4e6,
     ("cfg1", "pcx_sum_bwd_par"): 636.3e6,
-    # configs[4], B = 256: the GEMM of one 4096 x 4096 transition layer (captured without cache flushes between
+    # HMM, B = 256: the GEMM of one 4096 x 4096 transition layer (captured without cache flushes between
     # kernels: the tied parameter tiles stay in L2 from layer to layer); parameter flows: the capture of a 7-layer
     # circuit scaled to the 127 layers of the one product (traffic grows with the contraction depth)
     ("cfg4", "pcx_sum_fwd"): 31.7e6,
     ("cfg4", "pcx_sum_bwd_ele"): 51.0e6,
     ("cfg4", "pcx_sum_bwd_par"): 449.2e6 * 127 / 7,
-    # configs[2], B = 512: mean over the 29 parameter-flow launches of a step, captured at B = 128 and scaled by 4
+    # Poon-Domingos, B = 512: mean over the 29 parameter-flow launches of a step, captured at B = 128 and scaled by 4
     # (every operand is a row of B samples)
     ("cfg2", "pcx_sum_bwd_par"): 1536.0e6 * 4 / 29,
-    # configs[3], B = 1024: mean over the product-backward launches of the capture
+    # random tensorised network, B = 1024: mean over the product-backward launches of the capture
     ("cfg3", "pcx_prod_bwd"): (2569.6e6 + 503.2e6) / 29,
 }
 
@@ -343,7 +343,7 @@ def oracle_step_time(pc, x_cpu: torch.Tensor, repeats: int = 1):
 
 
 def cpu_sample_size(config: str, B: int, requested: int) -> int:
-    """Samples per CPU step (configs[4] is 12.8 GFLOP per sample plus half a minute of per-step table work on the host)."""
+    """Samples per CPU step (the HMM is 12.8 GFLOP per sample plus half a minute of per-step table work on the host)."""
     return min(B, requested, 128 if config.startswith("cfg4") else requested)
 
 

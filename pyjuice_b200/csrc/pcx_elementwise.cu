@@ -155,8 +155,8 @@ __global__ void input_cat_bwd_kernel(float* __restrict__ param_flows, const floa
 // atomics and adds every non-zero bin to the flow accumulators once -- G * num_cats global atomics instead of
 // G * B.  Category ids are clamped to the staged table so that invalid data cannot address outside it.
 // What bounds them is latency, so every phase has several independent loads per thread under way: eight parameter rows while
-// staging, four nodes' flows while counting.  (784 variables x 128 nodes x 256 categories, 512 samples: see the table of the
-// design notes.)
+// staging, four nodes' flows while counting.  (784 variables x 128 nodes x 256 categories, 512 samples, 103 MB of parameters and
+// 205 MB of values or flows: forward 69 us, backward 123 us = 4.5 and 3.3 TB/s with the flow table read and written.)
 constexpr int kStageThreads = 128;
 constexpr int kStageMax = 16;
 

@@ -10,10 +10,11 @@
 // reproducible bit for bit) -- no global scratch, no counters, and the epilogue runs on every SM.  The only waits
 // between CTAs are the hardware's cluster barriers (the CTAs of a cluster are resident together by construction).
 //
-//   operand pre-pass   ONE kernel per layer and pass: a CTA owns 8 samples and ALL operand rows; it gathers the
-//                      log-domain values (the product layer is folded in: a product's value is the sum of its
-//                      children's rows), keeps them in shared memory, reduces the per-sample maximum, and writes
-//                      exp(value - max) as bf16 hi / lo operand tiles.  No element_mars, no separate maximum pass.
+//   operand pre-pass   ONE kernel per layer and pass: a cluster of up to four CTAs owns 8 samples, each CTA its part
+//                      of the operand rows; it gathers the log-domain values (the product layer is folded in: a product's
+//                      value is the sum of its children's rows), keeps them in shared memory, reduces the per-sample
+//                      maximum (across the cluster through distributed shared memory), and writes exp(value - max)
+//                      as bf16 hi / lo operand tiles.  No element_mars, no separate maximum pass.
 //   GEMM               warp 0 streams 32-deep operand slices with bulk copies into a ring of 4-8 stages, one thread
 //                      of warp 1 issues three tcgen05.mma per 16-deep step (hi x hi, hi x lo, lo x hi; N = 64, 128
 //                      or 256) into a TMEM accumulator, warps 2-5 finish: log + shift (forward), + element value and
@@ -36,7 +37,7 @@ constexpr int W_STEP = 32;                          // contraction depth per pip
 constexpr int W_A_HALF = (W_STEP / 8) * BM * 16;    // 8 KB: hi (or lo) part of the A operand of one stage
 constexpr int W_THREADS = 192;                      // warp 0 copies, warp 1 multiplies, warps 2-5 finish
 constexpr int W_PREP_THREADS = 512;
-constexpr int W_PREP_SAMPLES = 8;                   // samples per pre-pass CTA (one 32-byte sector per row)
+constexpr int W_PREP_SAMPLES = 8;                   // samples per pre-pass cluster (one 32-byte sector per row)
 constexpr int W_MAX_DEPTH = 6144;                   // operand rows the pre-pass can hold in shared memory
 
 template <int DN>

@@ -500,8 +500,9 @@ class TensorCircuit(nn.Module):
     # The buffers hold a multiple of eight columns (`_PAD`): eight fp32 samples are one 32-byte sector, and every fast
     # kernel (vector loads, folded products, dense operands, tensor-core parameter flows) reads whole groups of them.  A
     # ragged batch used to fall back to the general kernels as a whole (an HMM with 512 states, 64 tokens and 77
-    # samples: 3.87 ms per training step, 2.78 ms padded to 80; 196-variable tree, 256 states, 100 samples: 1.85, 1.34 ms).  Padding columns evaluate category 0 and get the
-    # root flow 0, so they add nothing to any parameter flow.  The public attributes are views of the first B columns.
+    # samples: 3.87 ms per training step, 2.78 ms padded to 80; 196-variable tree, 256 states, 100 samples: 1.85, 1.34 ms).
+    # Padding columns evaluate category 0 and get the root flow 0, so they add nothing to any parameter flow.  The public
+    # attributes are views of the first B columns.
     _PAD = 8
 
     def _columns(self, t):
@@ -1283,9 +1284,9 @@ class TensorCircuit(nn.Module):
 
     def _clear_launches(self, em_state=None):
         """``em_state``: the update that has just been launched (see `InputLayer._em_state`): flows it moved out of a shadow
-        are in the accumulators.  Input layers whose accumulators are known to be empty still (all their flows went to the transposed shadow and
-        were consumed from there, nothing read or wrote the accumulators proper) need no clearing: on configs[4] that is
-        2.1 GB of replica accumulators per step."""
+        are in the accumulators.  Input layers whose accumulators are known to be empty still (all their flows went to the
+        transposed shadow and were consumed from there, nothing read or wrote the accumulators proper) need no clearing: 2.1 GB
+        of replica accumulators per step of a homogeneous HMM of 4096 states and 32768 categories."""
         arena, clean = self._flow_arena, True
         for i, layer in enumerate(self.input_layer_group):
             moved = em_state is not None and em_state[i][1]
