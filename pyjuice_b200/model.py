@@ -1364,9 +1364,9 @@ class TensorCircuit(nn.Module):
         layers = self._leaf_layers
         state = tuple(layer._em_state(keep_zero_params) for layer in layers)
         if (not self.use_cuda_graphs or self._reference_compat or getattr(self, "_late_sync", None) is not None
-                or self.param_flows is None or any(layer._param_flows is None for layer in layers)
-                or self.num_sum_params >= self._EM_FORK_PARAMS
-                or any((layer._shadow is not None and layer.max_cats >= layer.SHADOW_MIN_CATS) or layer.num_parameters >= 4 * self._EM_FORK_PARAMS for layer in layers)):
+                or self.param_flows is None or self.num_sum_params >= self._EM_FORK_PARAMS
+                or any(layer._param_flows is None or (layer._shadow is not None and layer.max_cats >= layer.SHADOW_MIN_CATS)
+                       or layer.num_parameters >= 4 * self._EM_FORK_PARAMS for layer in layers)):
             self.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
             self.init_param_flows(flows_memory=0.0)
             return
