@@ -1480,6 +1480,7 @@ class TensorCircuit(nn.Module):
             self._late_sync = arena.all_reduce_range_async(0, arena.segment_end(0), group=group,
                                                            dtype=getattr(self, "_overlap_dtype", None))
             self._late_head = bool(sync_cum_flow)
+            self._reduce_handed_over(group, getattr(self, "_overlap_dtype", None))
             early.wait()
             if not _lazy:
                 self._finish_late_sync()
@@ -1491,9 +1492,20 @@ class TensorCircuit(nn.Module):
             _ = self._cum_flow                              # fold a pending total of an earlier sync into the host part
         total = self._cum_flow_host if self._cum_flow_dev is None else self._cum_flow_dev + self._cum_flow_host
         head = arena.all_reduce(total, group=group, dtype=dtype, reduce_len=reduce_len, op=op)
+        self._reduce_handed_over(group, dtype, op)
         if sync_cum_flow:
             self._cum_flow_host, self._cum_flow_dev, self._cum_flow_head = 0.0, None, head
         return None
+
+    def _reduce_handed_over(self, group, dtype: Optional[torch.dtype], op=None):
+        """The exchange of accumulators that lie outside the arena (every rank has to have handed over the same ones)."""
+        import torch.distributed as dist
+        op = dist.ReduceOp.SUM if op is None else op
+        for buf in self._handed_over_flows():
+            low = buf if dtype is None or dtype == buf.dtype else buf.to(dtype)
+            dist.all_reduce(low, op=op, group=group)
+            if low is not buf:
+                buf.copy_(low)
 
     def average_params(self, dtype: Optional[torch.dtype] = None, group=None):
         """Replace the sum parameters and every input layer's parameters by their mean over the data-parallel ranks

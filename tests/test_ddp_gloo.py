@@ -85,6 +85,34 @@ def test_local_sgd_parameter_average_world2(tmp_path):
         assert open(tmp_path / f"rank{r}.txt").read() == "ok"
 
 
+def _handed_over_worker(rank, world, port, out_dir):
+    sys.path.insert(0, ROOT)
+    import pyjuice_b200 as pj
+    from pyjuice_b200.flows import FlowArena
+    dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{port}", rank=rank, world_size=world)
+    try:
+        pc = pj.compile(pj.structures.HMM(seq_length=5, num_latents=8, num_emits=11), verbose=False)
+        layer = pc.input_layer_group[0]
+        ok = True
+        for dtype in (None, torch.bfloat16):
+            pc._flow_arena = FlowArena([pc.num_param_flows, layer.num_param_flows], "cpu")
+            pc.param_flows = pc._flow_arena.views[0]
+            layer.param_flows = buf = torch.full((layer.num_param_flows,), float(rank + 1))
+            pc.param_flows.fill_(10.0 * (rank + 1))
+            pc.sync_param_flows(dtype=dtype)
+            ok = ok and layer.param_flows is buf and bool((buf == 3.0).all()) and bool((pc.param_flows == 30.0).all())
+        open(os.path.join(out_dir, f"rank{rank}.txt"), "w").write("ok" if ok else "bad")
+    finally:
+        dist.destroy_process_group()
+
+
+def test_leaf_flow_buffers_handed_over_are_exchanged_too_world2(tmp_path):
+    port = 33500 + (os.getpid() % 2000)
+    mp.spawn(_handed_over_worker, args=(2, port, str(tmp_path)), nprocs=2, join=True)
+    for r in range(2):
+        assert open(tmp_path / f"rank{r}.txt").read() == "ok"
+
+
 def test_sync_is_noop_without_process_group():
     import pyjuice_b200 as pj
     ns = pj.structures.HMM(seq_length=4, num_latents=4, num_emits=5)
