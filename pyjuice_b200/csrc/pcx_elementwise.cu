@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(256)
 load_inputs_kernel(int32_t* __restrict__ data, const void* __restrict__ x, int elsize, int64_t B, int64_t V,
                    int64_t stride_b, int64_t stride_v, int64_t W) {
     __shared__ int32_t tile[32][33];
-    const int64_t b0 = (int64_t)blockIdx.x * 32, v0 = (int64_t)blockIdx.y * 32;
+    const uint32_t wide = (uint32_t)((W + 31) / 32);       // tiles of one row of tiles (one-dimensional grid: any V and W)
+    const int64_t b0 = (int64_t)(blockIdx.x % wide) * 32, v0 = (int64_t)(blockIdx.x / wide) * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int k = ty; k < 32; k += 8) {
         const int64_t b = b0 + k, v = v0 + tx;
@@ -670,9 +671,9 @@ int pcx_load_inputs(int32_t* data, const void* x, int elsize, int64_t B, int64_t
                     int64_t W, void* stream) {
     if (elsize != 1 && elsize != 2 && elsize != 4 && elsize != 8) return -1;
     if (B <= 0 || V <= 0) return 0;
-    if (W < B || pcx_cdiv(V, 32) > 65535) return -1;
-    dim3 grid((unsigned)pcx_cdiv(W, 32), (unsigned)pcx_cdiv(V, 32));
-    load_inputs_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(data, x, elsize, B, V, stride_b, stride_v, W);
+    const int64_t tiles = pcx_cdiv(W, 32) * pcx_cdiv(V, 32);
+    if (W < B || tiles > INT32_MAX) return -1;
+    load_inputs_kernel<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(data, x, elsize, B, V, stride_b, stride_v, W);
     PCX_LAUNCH_CHECK();
     return 0;
 }

@@ -320,3 +320,15 @@ def test_padding_columns_of_probability_zero(kind, latents, cats, logspace):
         assert ok, err
         ok, err = rel_close(folded_input_flows(layer, layer.param_flows), folded_input_flows(layer, ref.ipf[0]))
         assert ok, err
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.int64])
+@pytest.mark.parametrize("B,V", [(3, 1), (1, 33), (70, 31), (5, 2_100_000), (2_100_000, 5)])
+def test_inputs_of_any_number_of_variables_and_samples(B, V, dtype):
+    from pyjuice_b200 import _lib
+    x = torch.randint(0, 200, (B, V), generator=torch.Generator().manual_seed(B), dtype=dtype).to(DEV)
+    W = -(-B // 8) * 8
+    for src in (x, x.t().contiguous().t()):
+        out = torch.full((V, W), -1, dtype=torch.int32, device=DEV)
+        _lib.call("pcx_load_inputs", out, src, src.element_size(), B, V, src.stride(0), src.stride(1), W)
+        assert torch.equal(out[:, :B], x.t().to(torch.int32)) and not out[:, B:].any()
