@@ -478,7 +478,7 @@ class InputLayer(Layer, nn.Module):
         (The reference leaves the replicas in place, so that with `flows_memory` in (0, 1) their decayed content is
         added to the source again at the next update; that double count is not reproduced.)"""
         self._flush_shadow()
-        if getattr(self, "_tied_folded", False):
+        if self._tied_folded:
             return
         for start, n, ch_pfids in self.tied2source_nids:
             _lib.call("pcx_tied_accum", self._param_flows, int(start), int(n), ch_pfids, int(ch_pfids.numel()))
@@ -497,7 +497,7 @@ class InputLayer(Layer, nn.Module):
         dirty = sh is not None and bool(sh["dirty"])
         direct = (dirty and bool(self._arena_zero) and not keep_zero_params and sh["logp"] is not None
                   and bool(self.use_fused_shadow_em))
-        return (direct, dirty and not direct, not direct and not getattr(self, "_tied_folded", False), bool(self._arena_zero))
+        return (direct, dirty and not direct, not direct and not self._tied_folded, bool(self._arena_zero))
 
     def _launch_em(self, step_size: float, pseudocount: float, keep_zero_params: bool):
         sh = self._shadow
@@ -512,7 +512,7 @@ class InputLayer(Layer, nn.Module):
             return
         if sh is not None and sh["dirty"]:
             _lib.call("pcx_input_cat_flush_t", self._param_flows, sh["flows"], sh["touched"], sh["row_pfid"], sh["R"], sh["C"])
-        if not getattr(self, "_tied_folded", False):
+        if not self._tied_folded:
             for start, n, ch_pfids in self.tied2source_nids:
                 _lib.call("pcx_tied_accum", self._param_flows, int(start), int(n), ch_pfids, int(ch_pfids.numel()))
         _lib.call("pcx_em_input_cat", self.params.data, self._param_flows, self._dev["source_nids"],

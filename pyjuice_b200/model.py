@@ -755,8 +755,12 @@ class TensorCircuit(nn.Module):
     def _param_ptrs(self):
         return (self._parameters["params"].data_ptr(), *[layer._parameters["params"].data_ptr() for layer in self._leaf_layers])
 
-    def _flow_ptrs(self):
-        return (self.param_flows.data_ptr(), *[layer._param_flows.data_ptr() for layer in self._leaf_layers])
+    def _all_ptrs(self):
+        """Addresses of all parameters and flow accumulators."""
+        ptrs = [self._parameters["params"].data_ptr(), self.param_flows.data_ptr()]
+        for layer in self._leaf_layers:
+            ptrs += (layer._parameters["params"].data_ptr(), layer._param_flows.data_ptr())
+        return tuple(ptrs)
 
     def _forward_pass(self, data: torch.Tensor, pack: bool, shadows):
         """All launches of a forward pass on the batch in ``data``, captured as one graph.  The operand tiles of the
@@ -1101,8 +1105,8 @@ class TensorCircuit(nn.Module):
             # The parameter flows of the sum layers and of the input layer close the pass.  They belong to the captured
             # pass too, unless data-parallel ranks overlap them with the all-reduce, or the leaves see another batch.
             tail = compute_param_flows and own and not self._overlap_ready()
-            key = ("bk", W, bool(compute_param_flows), tail, ls, self._launch_cfg(), self._param_ptrs(),
-                   self._flow_ptrs() if compute_param_flows else 0, data.data_ptr() if tail else 0)
+            key = ("bk", W, bool(compute_param_flows), tail, ls, self._launch_cfg(),
+                   self._all_ptrs() if compute_param_flows else self._param_ptrs(), data.data_ptr() if tail else 0)
             self._batched_par_pending = self._bk_par_pending.get(key, False)
             with self._nvtx("pcx backward"):
                 self._run_inner(key, partial(self._backward_sweep, data if tail else None, compute_param_flows,
@@ -1361,17 +1365,18 @@ class TensorCircuit(nn.Module):
         2 us each, and twice that in host work when they are launched one by one; large updates cover their launches)."""
         assert 0.0 < step_size <= 1.0, "`step_size` should be between 0 and 1."
         self._require_cuda()
-        layers = self._leaf_layers
-        state = tuple(layer._em_state(keep_zero_params) for layer in layers)
-        if (not self.use_cuda_graphs or self._reference_compat or getattr(self, "_late_sync", None) is not None
-                or self.param_flows is None or self.num_sum_params >= self._EM_FORK_PARAMS
-                or any(layer._param_flows is None or (layer._shadow is not None and layer.max_cats >= layer.SHADOW_MIN_CATS)
-                       or layer.num_parameters >= 4 * self._EM_FORK_PARAMS for layer in layers)):
+        layers, fork = self._leaf_layers, self._EM_FORK_PARAMS
+        state = tuple([layer._em_state(keep_zero_params) for layer in layers])
+        direct = (not self.use_cuda_graphs or self._reference_compat or self._late_sync is not None
+                  or self.param_flows is None or self.num_sum_params >= fork)
+        for layer in layers:
+            direct = (direct or layer._param_flows is None or layer.num_parameters >= 4 * fork
+                      or (layer._shadow is not None and layer.max_cats >= layer.SHADOW_MIN_CATS))
+        if direct:
             self.mini_batch_em(step_size=step_size, pseudocount=pseudocount, keep_zero_params=keep_zero_params)
             self.init_param_flows(flows_memory=0.0)
             return
-        key = ("em", step_size, pseudocount, keep_zero_params, state, self.use_side_stream, self._param_ptrs(),
-               self._flow_ptrs())
+        key = ("em", step_size, pseudocount, keep_zero_params, state, self.use_side_stream, self._all_ptrs())
         if key not in self._graphs:
             seen = [k for k in self._graphs if k[0] == "em"]
             if len(seen) >= 4:                               # a schedule of step sizes: keep the latest few
