@@ -503,6 +503,19 @@ int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* ele
                        int logspace, int terms, void* stream);
 /* Clusters of `cluster` CTAs of those launches that the current device can hold at a time. */
 int pcx_column_clusters(int cluster, int big);
+/* A chain: consecutive levels of one group of n_strips * 16 rows (at most 1024) and as many children, all with the same
+ * fragments, each reading the level before it.  A cluster of ceil(n_strips / per) CTAs (at most 16; at most 8 where per > 4) owns
+ * 8 * nt columns (nt 1 - 3, per * nt at most 16), a CTA `per` strips (at most 8).  Flows are logarithms.
+ * rows: int32 x 2, [n_levels + 1][n_strips].  Forward: first the two child rows of the elements of every 16-deep step (0: none),
+ * then per level the output row of a strip and the other child row of the element that the next level makes of it.  Element
+ * flows: first the parent rows of every step, then per level the two child rows of the strip's elements, of which the first is
+ * the parent row of the next level's step.  strips: int32 x 2 per strip: its first fragment, fragments per step.
+ * work: pcx_column_chain_bytes bytes, 16-byte aligned, of one launch at a time. */
+int pcx_column_chain(int mode, float* node_mars, float* node_flows, const void* frags, void* work, const int32_t* rows,
+                     const int32_t* strips, int n_levels, int n_strips, int W, int nt, int per, int terms, void* stream);
+int64_t pcx_column_chain_bytes(int n_strips, int W, int nt, int per);
+/* Clusters of `cluster` CTAs (1 - 16) of a chain that the current device can hold at a time. */
+int pcx_column_chain_clusters(int cluster);
 /* Parameter fragments (1 KB each: 16 rows x 16 children, bf16 high parts then low parts in the order of the A operand of
  * mma.m16n8k16).  bases: int32 x 4: parameter of (row 0, child 0), stride per row, stride per child, unused. */
 int pcx_column_pack(void* frags, const int32_t* bases, int64_t n, const float* params, void* stream);
@@ -538,7 +551,8 @@ int pcx_colplan_new(const int64_t* desc, int64_t n_desc, const int32_t* tables, 
 int pcx_colplan_free(void* planner);
 /* Rows of stored element values; depth (in 16) of the deepest CTA task, 0 without any. */
 int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps);
-/* Whether the program is the better choice at rows of W samples; rooms: clusters of 1, 2, 4, 8 and 16 CTAs at a time. */
+/* Whether the program is the better choice at rows of W samples; rooms: clusters of 1, 2, 4, 8 and 16 CTAs at a time, then
+ * clusters of 1 ... 16 CTAs of a chain. */
 int pcx_colplan_suits(const void* planner, int64_t W, const int32_t* rooms);
 /* Tables: the launches at rows of W samples; groups of tied tables; parameter-flow jobs, without the groups flagged in `dense`.
  * Each makes a blob: one array of device tables and a description of its sections (see column.py). */

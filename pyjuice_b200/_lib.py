@@ -70,6 +70,7 @@ SIGNATURES = {
     "pcx_input_cat_flush_t": [P, P, P, P, L, I],
     "pcx_column_run": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I],
     "pcx_column_run_big": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I],
+    "pcx_column_chain": [I, P, P, P, P, P, P, I, I, I, I, I, I],
     "pcx_column_pack": [P, P, L, P],
     "pcx_column_par": [I, P, P, P, P, P, P, P, P, I, I, I, I],
     "pcx_sum_fwd_dense2": [P, P, P, P, P, P, I, P, P, I, P, L, L, I, I, I],
@@ -79,7 +80,7 @@ SIGNATURES = {
 }
 
 # entry points without a stream argument
-PLAIN = {"pcx_build_arch": [], "pcx_column_clusters": [I, I], "pcx_set_sum_mode": [I], "pcx_set_dependent_launch": [I], "pcx_set_stage_event": [P], "pcx_get_status": [], "pcx_clear_status": [],
+PLAIN = {"pcx_build_arch": [], "pcx_column_clusters": [I, I], "pcx_column_chain_clusters": [I], "pcx_column_chain_bytes": [I, I, I, I], "pcx_set_sum_mode": [I], "pcx_set_dependent_launch": [I], "pcx_set_stage_event": [P], "pcx_get_status": [], "pcx_clear_status": [],
          "pcx_packed_tile_count": [L, I, I, I, I], "pcx_dense_scratch_bytes": [I, I, I],
          "pcx_sm_packed_bytes": [L, I, I], "pcx_dense2_scratch_bytes": [I, I, I]}
 # the planner of the column program (host only; the last two arguments of those that may refuse: a text buffer and its size)
@@ -146,7 +147,7 @@ def load() -> ctypes.CDLL:
     for name, args in PLAIN.items():
         fn = getattr(lib, name)
         fn.restype = c_int64 if name in ("pcx_packed_tile_count", "pcx_dense_scratch_bytes", "pcx_sm_packed_bytes",
-                                        "pcx_dense2_scratch_bytes") else c_int
+                                        "pcx_dense2_scratch_bytes", "pcx_column_chain_bytes") else c_int
         fn.argtypes = list(args)
     for name, args in SIGNATURES.items():
         fn = getattr(lib, name)
@@ -214,7 +215,7 @@ def _invoke(lib, name, conv, args, dev) -> int:
     rc = getattr(lib, name)(*conv, stream)
     b.record()
     # launches over many layers serve two operators: tell them apart by their first argument (0 forward, 1 element flows)
-    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in ("pcx_sum_chain", "pcx_column_run", "pcx_column_run_big") else name, a, b))
+    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in ("pcx_sum_chain", "pcx_column_run", "pcx_column_run_big", "pcx_column_chain") else name, a, b))
     return rc
 
 

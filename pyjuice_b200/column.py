@@ -116,6 +116,14 @@ def _refuse_deep_tables(pc):
                         raise Unsupported("a dense table deeper than a CTA task gathers")
 
 
+class _Chain:
+    """A launch of ``n`` levels of one tied group of ``S`` strips (see `pcx_column_chain`), and its exchange buffer."""
+
+    def __init__(self, rows, strips, n, S, W, nt, per):
+        self.rows, self.strips, self.n, self.S, self.nt, self.per = rows, strips, n, S, nt, per
+        self.work = torch.empty(_lib.load().pcx_column_chain_bytes(S, W, nt, per), dtype=torch.uint8, device=rows.device)
+
+
 def _pointer(a):
     return a.ctypes.data_as(ctypes.c_void_p)
 
@@ -148,14 +156,15 @@ class ColumnProgram:
 
     # ---- cutting into tasks ------------------------------------------------------------------------------------------
     def _room(self):
-        """Clusters of 1, 2, 4, 8 and 16 CTAs the device holds at a time."""
+        """Clusters of 1, 2, 4, 8 and 16 CTAs the device holds at a time, then clusters of 1 ... 16 CTAs of a chain."""
         if self._rooms is None:
-            rooms = []
-            for c in (1, 2, 4, 8, 16):
+            rooms, lib = [], _lib.load()
+            for c, count in ([(c, lambda c: lib.pcx_column_clusters(c, bool(self.big_steps))) for c in (1, 2, 4, 8, 16)]
+                             + [(c, lib.pcx_column_chain_clusters) for c in range(1, 17)]):
                 n = -1
                 if self.device.type == "cuda":
                     with torch.cuda.device(self.device):
-                        n = int(_lib.load().pcx_column_clusters(c, bool(self.big_steps)))
+                        n = int(count(c))
                 rooms.append(n if n > 0 else max(1, (128 if c < 16 else 112) // c))
             self._rooms = np.asarray(rooms, dtype=np.int32)
         return _pointer(self._rooms)
@@ -191,14 +200,18 @@ class ColumnProgram:
         for mode in (0, 1):
             tasks, n_tasks, strips, n_strips, levels, n_levels = blob.next(6)
             out[mode] = dict(tasks=blob.take(tasks, 12 * n_tasks), strips=blob.take(strips, n_strips),
-                             levels=blob.take(levels, n_levels, 4), launches=[])
-        for mode in (0, 1):
-            launches = out[mode]["launches"]
+                             levels=blob.take(levels, n_levels, 4), launches=[], chained=[])
+        for mode, form in ((0, "launches"), (1, "launches"), (0, "chained"), (1, "chained")):
+            launches = out[mode][form]
             for _ in range(blob.next()):
                 kind, *words = blob.next(7)
                 if kind == 0:                                # (levels, how many, (column groups, tiles, CTAs, wide))
                     first, n, *how = words
                     launches.append((out[mode]["levels"][first:first + n], n, tuple(how)))
+                    continue
+                if kind == 3:
+                    rows, strips, n, S, nt, per = words
+                    launches.append(_Chain(blob.take(rows, n + 1, S, 2), blob.take(strips, S, 2), n, S, W, nt, per))
                     continue
                 rows, cids, n, width, size, _ = words        # products ahead of the next level, one set per block size
                 if kind == 1:
@@ -254,10 +267,14 @@ class ColumnProgram:
         p = plan[mode]
         W = nm.size(1)
         em, terms = self.buffers(W), 1 if _lib.sum_mode() == 2 else 3
-        for launch in p["launches"]:
+        for launch in p["chained" if logspace else "launches"]:     # (a chain keeps its flows as logarithms)
             if isinstance(launch, list):
                 for nids, cids, size in launch:
                     _lib.call("pcx_prod_fwd", em, nm, nids, cids, nids.numel(), cids.size(1), size, W)
+                continue
+            if isinstance(launch, _Chain):
+                c = launch
+                _lib.call("pcx_column_chain", mode, nm, nf, plan["frags"], c.work, c.rows, c.strips, c.n, c.S, W, c.nt, c.per, terms)
                 continue
             levels, n, (nt, tiles, cluster, wide) = launch
             if self.big_steps:
@@ -326,6 +343,12 @@ class ColumnProgram:
                 assert t0 == seen and s0 == t0 + n, "column levels do not follow one another"
                 seen = s0 + ns
             assert seen == tasks.size
+            for c in p["chained"]:
+                if isinstance(c, _Chain):
+                    for r in c.rows.cpu().reshape(-1).tolist():
+                        report("column chain rows", int(r), 16, pc.num_nodes)
+                    for first, step in c.strips.cpu().tolist():
+                        assert 0 <= first and first + (c.S - 1) * step < plan["n_frag"]
             for t in tasks:
                 k, w, off = int(t["n_k"]), int(t["width"]), int(t["kid_off"])
                 if t["kind"] == K_PROD:

@@ -419,6 +419,90 @@ struct PcxColPlanner {
             }
     }
 
+    // ---- chains: see pcx_column_chain.cu -------------------------------------------------------------------------------
+    // Runs of depths of one group each, with the same parameters, where the operand of a depth is the output of the one below
+    // and at most one other row per element.  From three levels on: the launch costs about what two levels gain.
+    static constexpr int CHAIN_LEVELS = 3, CHAIN_MIN_STRIPS = 4, CHAIN_MAX_STRIPS = 64;
+    struct Chain { int first, n, strips; };     // depths first .. first + n - 1
+    std::vector<Chain> chains;
+
+    struct Pair { int x, y; };
+    // Child rows of 16-row pieces of the elements `ids`.
+    static std::vector<Pair> pieces(const Depth& d, const Ints& ids) {
+        std::vector<Pair> out;
+        for (int id : ids) {
+            const Elem& e = *d.find(id);
+            for (int o = 0; o < e.size; o += 16)
+                out.push_back({e.n > 0 ? d.kids[e.first] + o : 0, e.n > 1 ? d.kids[e.first + 1] + o : 0});
+        }
+        return out;
+    }
+    static Ints rows_of(const Ints& blocks, int size) {
+        Ints out;
+        for (int b : blocks)
+            for (int o = 0; o < size; o += 16) out.push_back(b + o);
+        return out;
+    }
+    // Puts the child that is the row of `own` first; false where there is none.
+    static bool order(std::vector<Pair>& p, const Ints& own) {
+        if (p.size() != own.size()) return false;
+        for (size_t i = 0; i < p.size(); ++i) {
+            if (p[i].y == own[i] && p[i].y != 0) std::swap(p[i].x, p[i].y);
+            if (p[i].x != own[i] || p[i].x == p[i].y) return false;
+        }
+        return true;
+    }
+    static bool chain_depth(const Depth& d) {
+        if (d.fw.size() != 1 || d.bk.size() != 1 || !d.direct || d.stored || !d.fw[0].mma || !d.bk[0].mma || d.max_kids > 2) return false;
+        const Group &f = d.fw[0], &b = d.bk[0];
+        const int S = f.strips();
+        if (S < CHAIN_MIN_STRIPS || S > CHAIN_MAX_STRIPS || f.depth != 16 * S || b.depth != 16 * S || b.strips() != S) return false;
+        for (auto& e : d.elems)
+            if (e.n < 1) return false;
+        return true;
+    }
+    bool follows(const Depth& d, const Depth& below) const {
+        if (d.fw[0].cls != below.fw[0].cls || d.bk[0].cls != below.bk[0].cls) return false;
+        auto f = pieces(d, d.fw[0].ops), b = pieces(d, d.bk[0].blocks);
+        return order(f, rows_of(below.fw[0].blocks, below.fw[0].bs)) && order(b, rows_of(below.bk[0].ops, below.bk[0].pbs));
+    }
+    void find_chains() {
+        const int n = (int)depths.size();
+        for (int i = 0, end; i < n; i = end) {
+            end = i + 1;
+            if (!chain_depth(depths[i])) continue;
+            while (end < n && end - i < PCX_COLUMN_MAX_LEVELS && chain_depth(depths[end]) && follows(depths[end], depths[end - 1])) ++end;
+            if (end - i >= CHAIN_LEVELS) chains.push_back({i, end - i, depths[i].fw[0].strips()});
+        }
+    }
+    // Tables of a chain: see pcx_column_chain.
+    Ints chain_rows(const Chain& c, int mode) const {
+        std::vector<Pair> t;
+        const Depth &low = depths[c.first], &top = depths[c.first + c.n - 1];
+        if (mode == 0) {
+            t = pieces(low, low.fw[0].ops);
+            for (int i = c.first; i < c.first + c.n; ++i) {
+                const Ints out = rows_of(depths[i].fw[0].blocks, depths[i].fw[0].bs);
+                std::vector<Pair> next(out.size());
+                if (i + 1 < c.first + c.n) {
+                    next = pieces(depths[i + 1], depths[i + 1].fw[0].ops);
+                    order(next, out);
+                }
+                for (size_t k = 0; k < out.size(); ++k) t.push_back({out[k], next[k].y});
+            }
+        } else {
+            for (int r : rows_of(top.bk[0].ops, top.bk[0].pbs)) t.push_back({r, 0});
+            for (int i = c.first + c.n - 1; i >= c.first; --i) {
+                auto p = pieces(depths[i], depths[i].bk[0].blocks);
+                if (i > c.first) order(p, rows_of(depths[i - 1].bk[0].ops, depths[i - 1].bk[0].pbs));
+                t.insert(t.end(), p.begin(), p.end());
+            }
+        }
+        Ints out;
+        for (const Pair& p : t) out.insert(out.end(), {p.x, p.y});
+        return out;
+    }
+
     // Per group: members, children per element, depth, block size, blocks, then where child rows [members, depth, children],
     // node rows [members, blocks], ones, parameters and flows [blocks, depth] lie.
     void tied_tables(Blob& out) const {
@@ -454,10 +538,38 @@ struct PcxColPlanner {
     }
 
     // ---- launch geometry ---------------------------------------------------------------------------------------------
-    struct Room {                               // clusters of 1, 2, 4, 8 and 16 CTAs that the device holds at a time
-        const int32_t* n;
+    struct Room {                               // clusters of 1, 2, 4, 8 and 16 CTAs that the device holds at a time, then
+        const int32_t* n;                       // clusters of 1 ... 16 CTAs of a chain
         int operator()(int c) const { return std::max(1, (int)n[c == 1 ? 0 : c == 2 ? 1 : c == 4 ? 2 : c == 8 ? 3 : 4]); }
+        int chain(int c) const { return std::max(1, (int)n[4 + c]); }
     };
+
+    // Strips per CTA and columns per cluster of a chain of groups of S strips: the cheapest estimate of a level, in cycles, times
+    // the waves of clusters.  `mma`: the products of a CTA's busiest scheduler, 8 cycles each (four warps share one); what else
+    // grows with the rows and columns of a CTA (partial products, epilogue) grows with it.  `stream`: fragments that neither
+    // tensor memory nor shared memory hold.  Measured, cycles a level, states / columns a cluster x strips a CTA: 128 / 8 x 1 3160;
+    // 256 / 8 x 2 3870, 8 x 4 4260; 512 / 8 x 4 5350, 8 x 8 7350; 1024 / 8 x 4 7660, 16 x 4 12 200, 8 x 8 13 000, 24 x 4 17 900,
+    // 16 x 8 20 600.
+    struct ChainShape { int nt, per, waves; double cost; };
+    static ChainShape chain_shape(int64_t W, int S, const Room& room) {
+        ChainShape best{0, 0, 0, 0.0};
+        for (int nt : {1, 2, 3})
+            for (int per : {1, 2, 3, 4, 6, 8}) {
+                const int C = cdiv(S, per), halves = per > 1 && C <= 8 ? 2 : 1, kparts = 16 / halves;
+                if (per > S || per * nt > 16 || C > kparts || cdiv(per, halves) > 4) continue;
+                const int steps = cdiv(per, std::min(per, kparts / C)), q = cdiv(per, steps), strips = cdiv(per, halves);
+                const int left = 231424 - 8960 - 2 * C * q * per * nt * 512;       // shared memory for fragments, as the launcher has it
+                if (left < 0) continue;
+                const int waves = cdiv(cdiv(W, 8 * nt), room.chain(C));
+                const int slots = strips <= 1 ? 1 : strips <= 2 ? 2 : 4;
+                const int held = 16 / slots + left / (16 * 1024 * slots);
+                const double mma = 8.1 * 3 * nt * steps * strips * cdiv(C * q * halves, 4);
+                const double stream = 1024.0 * C * q * halves * strips * std::max(0, steps - held) / 50.0;
+                const double cost = waves * (2900.0 + 2.95 * mma + 0.25 * stream);
+                if (best.nt == 0 || cost < best.cost - 1e-9) best = ChainShape{nt, per, waves, cost};
+            }
+        return best;
+    }
 
     // (strips per task, time) of a level's large groups on a cluster of c CTAs: rounds of tasks times what a task takes in
     // microseconds: a fixed latency, the gather and exponentials of its operand, its multiplications, and parameters that
@@ -522,6 +634,19 @@ struct PcxColPlanner {
     // forward against 556).
     bool suits(int64_t W, const Room& room) const {
         if (big_steps == 0) return true;
+        // (or where every level of large groups belongs to a chain whose clusters fit at once)
+        int64_t chained = 0, large = 0;
+        bool fits = true;
+        for (auto& c : chains) {
+            chained += c.n;
+            fits = fits && chain_shape(W, c.strips, room).waves == 1;
+        }
+        for (auto& d : depths) {
+            bool any = false;
+            for (auto& g : d.fw) any = any || g.big;
+            large += any;
+        }
+        if (fits && chained >= large) return true;
         const Shape s = big_shape(W, room);
         int64_t rounds = 0, levels = 0;
         for (auto& d : depths) {
@@ -547,7 +672,7 @@ struct Cutter {
     const int64_t prod_reads;                   // child rows a CTA may gather for the stored elements of a fused level
     Pool kids{1}, strips[2] = {Pool(4), Pool(4)};
     std::vector<PcxColTask> tasks[2], split;
-    struct Level { int first, n, split_first, n_split; Shape how; };
+    struct Level { int first, n, split_first, n_split; Shape how; int depth; };
     std::vector<Level> levels[2];
     Shape fused{};
     int wide_tiles;
@@ -717,7 +842,7 @@ struct Cutter {
     }
 
     // Closes a level; a wide one: which of the three kernels can take it.
-    void level(int mode, size_t first, Shape how) {
+    void level(int mode, size_t first, Shape how, int depth) {
         auto& list = tasks[mode];
         const int n = (int)(list.size() - first);
         if (how.wide != 0 && split.empty()) {
@@ -731,12 +856,13 @@ struct Cutter {
             how.wide = products ? 3 : (plain ? 2 : 1);
         }
         list.insert(list.end(), split.begin(), split.end());
-        levels[mode].push_back(Level{(int)first, n, (int)first + n, (int)split.size(), how});
+        levels[mode].push_back(Level{(int)first, n, (int)first + n, (int)split.size(), how, depth});
         split.clear();
     }
 
     // Sections: fragments, then per direction tasks, strips, levels; launches: (0, first level, levels, shape) or, a product
-    // launch, (1, node rows, child rows, how many, children, block size).
+    // launch, (1, node rows, child rows, how many, children, block size) or, a chain, (3, rows, strips, levels, strips per
+    // level, nt, strips per CTA).
     void run(Blob& blob) {
         int64_t total = 0, n_small = 0;
         for (auto& d : pc.depths)
@@ -762,7 +888,7 @@ struct Cutter {
                 else if (g.mma) mma_tasks(d, g, 0, stored, per);
                 else simt_forward(d, g, stored);
             }
-            level(0, first, shape(n));
+            level(0, first, shape(n), (int)i);
         }
         for (size_t i = pc.depths.size(); i-- > 0;) {
             const Depth& d = pc.depths[i];
@@ -774,7 +900,7 @@ struct Cutter {
                 else if (g.mma) mma_tasks(d, g, 1, false, per);
                 else simt_backward(d, g);
             }
-            level(1, first, shape(n));
+            level(1, first, shape(n), (int)i);
             if (d.direct) continue;
             first = tasks[1].size();
             for (auto& p : d.prod_bk)
@@ -783,7 +909,7 @@ struct Cutter {
                     for (int& x : rows) x += r;
                     tasks[1].push_back(task(p.n ? kids.add(rows) : 0, p.n, 0, 1, p.row + r, std::min(16, p.size - r), 0, K_PROD, p.add));
                 }
-            level(1, first, shape((int64_t)(tasks[1].size() - first)));
+            level(1, first, shape((int64_t)(tasks[1].size() - first)), -1);
         }
         auto& m = blob.meta;
         blob.data.reserve(frag.size() + kids.data.size() + 12 * (tasks[0].size() + tasks[1].size()) + strips[0].data.size() +
@@ -800,20 +926,51 @@ struct Cutter {
             m.push_back(blob.section(lv));
             m.push_back((int64_t)levels[mode].size());
         }
-        for (int mode = 0; mode < 2; ++mode) {
+        // twice: the levels by their tasks, and with chains in their places
+        for (int i = 0; i < 4; ++i) {
+            const int mode = i & 1;
+            const bool chained = i >= 2;
             std::vector<int64_t> launches;
             int64_t n = 0;
-            for (size_t at = 0, end; at < levels[mode].size(); at = end) {      // consecutive fused levels are one launch
+            for (size_t at = 0, end; at < levels[mode].size(); at = end, ++n) { // consecutive fused levels are one launch
                 const Shape how = levels[mode][at].how;
                 const size_t last = std::min(levels[mode].size(), at + PCX_COLUMN_MAX_LEVELS);
-                for (end = at + 1; how.wide == 0 && end < last && levels[mode][end].how.wide == 0 && !(mode == 0 && before[end]);) ++end;
+                if (const auto* c = chained ? starts(mode, at) : nullptr) {
+                    const auto shape = PcxColPlanner::chain_shape(W, c->strips, room);
+                    launches.insert(launches.end(), {3, blob.section(pc.chain_rows(*c, mode)), blob.section(chain_strips(mode, at)), c->n,
+                                                     c->strips, shape.nt, shape.per});
+                    end = at + c->n;
+                    continue;
+                }
+                for (end = at + 1; how.wide == 0 && end < last && levels[mode][end].how.wide == 0 && !(mode == 0 && before[end]) &&
+                                   !(chained && starts(mode, end)); ++end) {}
                 if (mode == 0 && before[at]) n += products(pc.depths[at], blob, launches);
                 launches.insert(launches.end(), {0, (int64_t)at, (int64_t)(end - at), how.nt, how.tiles, how.cluster, how.wide});
-                ++n;
             }
             m.push_back(n);
             m.insert(m.end(), launches.begin(), launches.end());
         }
+    }
+    // The chain whose first level is `at`, if its clusters fit at once: where they do not, the tasks, which take more columns in
+    // fewer CTAs, are faster (1024 states, 256 columns, 31 levels of a training step: 1384 us by tasks, 1443 in two waves).
+    const PcxColPlanner::Chain* starts(int mode, size_t at) const {
+        for (auto& c : pc.chains)
+            if (levels[mode][at].depth == (mode == 0 ? c.first : c.first + c.n - 1)) {
+                for (size_t l = at; l < at + c.n; ++l)
+                    if (levels[mode][l].how.wide != 0) return nullptr;
+                return PcxColPlanner::chain_shape(W, c.strips, room).waves == 1 ? &c : nullptr;
+            }
+        return nullptr;
+    }
+    // First fragment and fragments per step of every strip of a level's group.
+    Ints chain_strips(int mode, size_t at) const {
+        const Level& l = levels[mode][at];
+        Ints t;
+        for (int i = l.first; i < l.split_first + l.n_split; ++i) {
+            const PcxColTask& k = tasks[mode][i];
+            for (int r = 0; r < k.n_rows; ++r) t.insert(t.end(), {k.par_off + r, k.n_rows});
+        }
+        return t;
     }
     // Arguments of the product kernel that fills the stored values of a depth, one set per block size.
     static int64_t products(const Depth& d, Blob& blob, std::vector<int64_t>& launches) {
@@ -959,6 +1116,7 @@ int pcx_colplan_new(const int64_t* desc, int64_t n_desc, const int32_t* tables, 
         Reader in{desc, desc + n_desc, tables, n_tables};
         p->build(in);
         p->find_tied();
+        p->find_chains();
         *out = p.release();
     });
 }

@@ -29,6 +29,9 @@ struct PcxOnce {
     bool* operator&() { return &here(); }
 };
 
+// Address of the status word of the bounded waits on the current device (pcx_get_status); null on an error.
+int* pcx_status_word();
+
 // log(exp(a) + exp(b)) with -inf handled (no NaN from inf - inf).
 __device__ __forceinline__ float pcx_logaddexp(float a, float b) {
     float hi = fmaxf(a, b), lo = fminf(a, b);

@@ -1281,6 +1281,18 @@ int pcx_tc_try_sum_par(float* param_flows, const float* node_flows, const float*
     return 1;
 }
 
+int* pcx_status_word() {
+    static int* at[64];
+    int d = 0;
+    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 64) return nullptr;
+    if (at[d] == nullptr) {
+        void* p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_tc_status) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        at[d] = static_cast<int*>(p);
+    }
+    return at[d];
+}
+
 extern "C" {
 
 int pcx_set_sum_mode(int mode) {

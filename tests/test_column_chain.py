@@ -1,0 +1,139 @@
+"""Chains of the column program (runs of tied levels in one launch): their tables, walked in float64 on the host, and the kernel
+against the same levels by their tasks, at the sizes where its shapes meet: strips per CTA that do not divide the rows, one to
+three column tiles per cluster, parameters beyond tensor memory, chains of odd and even length."""
+import numpy as np
+import pytest
+import torch
+
+import pyjuice_b200 as pj
+from helpers import check_against_oracle
+from pyjuice_b200.column import ColumnProgram, _Chain
+
+DEV = "cuda:0"
+
+
+def _hmm(latents, tokens, banded=False, homogeneous=True):
+    torch.manual_seed(3)
+    alpha = None
+    if banded:                                             # most transitions are impossible
+        i = torch.arange(latents)
+        alpha = torch.rand(latents, latents) * ((i[:, None] - i[None, :]).abs() < 5)
+        alpha = alpha / alpha.sum(dim=1, keepdim=True)
+    return pj.compile(pj.structures.HMM(seq_length=tokens, num_latents=latents, num_emits=7, homogeneous=homogeneous, alpha=alpha),
+                      verbose=False)
+
+
+def _lse(x, axis):
+    m = x.max(axis=axis, keepdims=True)
+    m = np.where(np.isinf(m), 0.0, m)
+    return np.log(np.exp(x - m).sum(axis=axis)) + m.squeeze(axis)
+
+
+def _chains(plan, mode):
+    return [c for c in plan[mode]["chained"] if isinstance(c, _Chain)]
+
+
+@pytest.mark.parametrize("latents,tokens", [(64, 5), (96, 6), (320, 4)])
+def test_tables(latents, tokens):
+    pc = _hmm(latents, tokens)
+    program = ColumnProgram(pc)
+    plan = program.plan(16)
+    bases, params = plan["bases"].numpy().reshape(-1, 4), pc.params.data.double().numpy()
+    rng = np.random.default_rng(1)
+    nm, nf = rng.normal(size=(pc.num_nodes, 2)), rng.normal(size=(pc.num_nodes, 2))
+    nm[:pc.num_dummy_nodes] = 0.0
+    want_nm, want_nf = nm.copy(), nf.copy()
+    for mode, want in ((0, want_nm), (1, want_nf)):        # the same levels by their tasks
+        from test_column_plan import _Walk
+        walk = _Walk(pc, program, plan, want_nm)
+        walk.nf = want_nf
+        chain, = _chains(plan, mode)
+        assert chain.n == tokens - 1 and chain.S == latents // 16
+        tasks = list(walk.levels(mode))
+        for t in (tasks[:-1] if mode == 0 else tasks[1:]):
+            if t["n_rows"] == 1 and t["kind"] not in (0, 4):
+                continue                                   # the root's level
+            v, walk.first = walk.operand(t, mode)
+            for st, n, theta in walk.outputs(t, mode):
+                o = _lse(np.log(theta)[:, :, None] + v[None], 1)
+                if mode == 0:
+                    want_nm[st[0]:st[0] + n] = o
+                else:
+                    kids = [k for k in st[1:3].tolist() if k]
+                    for k in kids:
+                        want_nf[k:k + n] = o + sum(want_nm[j:j + n] for j in kids)
+    for mode in (0, 1):
+        chain, = _chains(plan, mode)
+        rows, strips = chain.rows.numpy(), chain.strips.numpy()
+        at = np.arange(16)
+        of = lambda r: (r[:, None] + at).reshape(-1)
+        theta = np.empty((16 * chain.S, 16 * chain.S))
+        for s, (first, step) in enumerate(strips):
+            for k in range(chain.S):
+                b, sr, sk, _ = bases[first + k * step]
+                theta[16 * s:16 * s + 16, 16 * k:16 * k + 16] = params[b + at[:, None] * sr + at[None, :] * sk]
+        x, y = of(rows[0, :, 0]), of(np.where(rows[0, :, 1] > 0, rows[0, :, 1], 0))
+        if mode == 0:
+            v = nm[x] + np.where(np.repeat(rows[0, :, 1] > 0, 16)[:, None], nm[y], 0.0)
+        else:
+            v = want_nf[x] - want_nm[x]
+        for l in range(chain.n):
+            o = _lse(np.log(theta)[:, :, None] + v[None], 1)
+            x, has = of(rows[l + 1, :, 0]), np.repeat(rows[l + 1, :, 1] > 0, 16)[:, None]
+            y = of(rows[l + 1, :, 1])
+            other = np.where(has, want_nm[y], 0.0)
+            if mode == 0:
+                np.testing.assert_allclose(o, want_nm[x], rtol=1e-12)
+                v = o + other
+            else:
+                o = o + want_nm[x] + other
+                np.testing.assert_allclose(o, want_nf[x], rtol=1e-9, atol=1e-9)
+                assert not has.any() or np.allclose(o[has[:, 0]], want_nf[y][has[:, 0]])
+                v = o - want_nm[x]
+
+
+def test_what_is_no_chain():
+    assert not _chains(ColumnProgram(_hmm(64, 3)).plan(8), 0)                       # two levels
+    assert not _chains(ColumnProgram(_hmm(64, 6, homogeneous=False)).plan(8), 0)    # every level its own parameters
+    assert not _chains(ColumnProgram(_hmm(32, 6)).plan(8), 0)                       # two strips
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 50, 130, 256])
+@pytest.mark.parametrize("latents,tokens,banded", [(64, 4, False), (96, 5, False), (128, 9, True), (320, 6, False), (512, 7, False),
+                                                   (768, 4, False), (1024, 5, False), (1024, 6, True)])
+def test_against_the_tasks(latents, tokens, banded, B, monkeypatch):
+    """Two bf16 parts per factor leave a relative error of about 3 * 2^-16 a level in either form, hence in a logarithm: 1e-4 for the
+    two together; the float32 rounding of values near -20 is far below."""
+    x = torch.randint(0, 7, (B, tokens), generator=torch.Generator().manual_seed(B)).to(DEV)
+    got = []
+    for tasks in (False, True):
+        pc = _hmm(latents, tokens, banded).to(DEV)
+        if tasks:
+            cut = ColumnProgram._cut
+            def without(self, W):
+                plan = cut(self, W)
+                for mode in (0, 1):
+                    plan[mode]["chained"] = plan[mode]["launches"]
+                return plan
+            monkeypatch.setattr(ColumnProgram, "_cut", without)
+        lls = pc(x)
+        lls.mean().backward()
+        plan = pc._column_plan()
+        assert plan is not None and len(_chains(plan, 0)) == len(_chains(plan, 1))
+        assert len(_chains(plan, 0)) == (0 if tasks or (latents == 1024 and B == 256) else 1)
+        d = pc.num_dummy_nodes
+        got.append((lls.detach(), pc.node_mars[d:].clone(), pc.node_flows[d:].exp(), pc.param_flows.clone()))
+    for a, b in zip(got[0][:2], got[1][:2]):
+        assert not torch.isnan(a).any() and (a - b).abs().nan_to_num().max() <= 1e-4 * tokens
+        assert torch.equal(torch.isinf(a), torch.isinf(b))
+    for a, b in zip(got[0][2:], got[1][2:]):
+        assert (a - b).abs().max() <= 1e-4 * tokens * b.abs().max()
+    assert pj._lib.get_status(DEV) == 0
+
+
+@pytest.mark.gpu
+def test_linear_flows_go_by_the_tasks():
+    pc = _hmm(128, 6).to(DEV)
+    x = torch.randint(0, 7, (40, 6), generator=torch.Generator().manual_seed(1))
+    check_against_oracle(pc, x, step=0.2, pseudo=0.1, logspace_flows=False)
