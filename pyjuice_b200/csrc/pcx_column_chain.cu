@@ -65,9 +65,30 @@ constexpr int CHAIN_SCALE = CHAIN_WARPS * 16 * 8 * 4;
 constexpr int CHAIN_MAX = 3 * 8 * 8 * 4;
 constexpr int CHAIN_FIXED = CHAIN_SCALE + CHAIN_MAX;
 
-__device__ __forceinline__ void tmem_store8(uint32_t addr, const uint4& h, const uint4& l) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(h.x), "r"(h.y),
-                 "r"(h.z), "r"(h.w), "r"(l.x), "r"(l.y), "r"(l.z), "r"(l.w) : "memory");
+// Four registers per lane (the high or low part of a fragment) to tensor memory, and N such parts back.
+__device__ __forceinline__ void tmem_store(uint32_t addr, const uint4& v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tmem_load(uint32_t addr, uint4* v) {
+    static_assert(N == 2 || N == 4 || N == 8, "parts of fragments");
+    if constexpr (N == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                     "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                     : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w),
+                       "=r"(v[2].x), "=r"(v[2].y), "=r"(v[2].z), "=r"(v[2].w), "=r"(v[3].x), "=r"(v[3].y), "=r"(v[3].z), "=r"(v[3].w),
+                       "=r"(v[4].x), "=r"(v[4].y), "=r"(v[4].z), "=r"(v[4].w), "=r"(v[5].x), "=r"(v[5].y), "=r"(v[5].z), "=r"(v[5].w),
+                       "=r"(v[6].x), "=r"(v[6].y), "=r"(v[6].z), "=r"(v[6].w), "=r"(v[7].x), "=r"(v[7].y), "=r"(v[7].z), "=r"(v[7].w) : "r"(addr));
+    else if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w) : "r"(addr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w),
+                       "=r"(v[2].x), "=r"(v[2].y), "=r"(v[2].z), "=r"(v[2].w), "=r"(v[3].x), "=r"(v[3].y), "=r"(v[3].z), "=r"(v[3].w) : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i].x), "+r"(v[i].y), "+r"(v[i].z), "+r"(v[i].w));
 }
 
 // ---- words that say whether they are there -------------------------------------------------------------------------------
@@ -101,6 +122,7 @@ template <int MODE, int NT, int PS>
 __global__ void __launch_bounds__(CHAIN_THREADS, 1) column_chain_kernel(const ChainArgs a) {
     constexpr int KT = CHAIN_TMEM / PS;                   // steps with fragments in tensor memory
     constexpr int AC = PS * NT <= 2 ? 3 : 1;              // accumulators of a strip and tile: short tables wait for the latency of a product
+    constexpr bool SPLIT = PS * NT >= 8;                  // low parts fetched once the high ones are done with: registers
     constexpr int KB = NT == 1 ? (PS == 4 ? 2 : 4) : (NT == 2 && PS < 4 ? 2 : 1);   // steps whose operands are requested together
     extern __shared__ __align__(128) uint8_t s_chain[];
     __shared__ uint32_t s_tmem;
@@ -147,7 +169,8 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) column_chain_kernel(const Ch
             const uint4* f = fragment(k, p);
             const uint4 h = __ldg(f), l = __ldg(f + 32);
             if (k < KT) {
-                tmem_store8(tmem + (k * PS + p) * 8, h, l);
+                tmem_store(tmem + (2 * k * PS + p) * 4, h);       // [step][part][strip]
+                tmem_store(tmem + ((2 * k + 1) * PS + p) * 4, l);
             } else {
                 s_frag[((k - KT) * PS + p) * 64 + lane] = h;
                 s_frag[((k - KT) * PS + p) * 64 + 32 + lane] = l;
@@ -312,42 +335,35 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) column_chain_kernel(const Ch
             for (int kk = 0; kk < KB; ++kk) {
                 const int k = k0 + kk;
                 if (k < n_k) {
-                    uint4 ah[PS], al[PS];
-                    if (k < KT) {
-                        float r[8 * PS];
-                        tmem_ld<8 * PS>(tmem + k * PS * 8, r);
-#pragma unroll
-                        for (int p = 0; p < PS; ++p) {
-                            const uint32_t* u = reinterpret_cast<const uint32_t*>(r) + 8 * p;
-                            ah[p] = make_uint4(u[0], u[1], u[2], u[3]);
-                            al[p] = make_uint4(u[4], u[5], u[6], u[7]);
+                    uint4 f[SPLIT ? 1 : 2][PS];            // high and low parts
+                    auto fetch = [&](int lo) {
+                        if (k < KT) {
+                            tmem_load<SPLIT ? PS : 2 * PS>(tmem + (2 * k + lo) * PS * 4, f[0]);
+                            return;
                         }
-                    } else if (k < KT + a.smem_steps) {
 #pragma unroll
-                        for (int p = 0; p < PS; ++p) {
-                            ah[p] = s_frag[((k - KT) * PS + p) * 64 + lane];
-                            al[p] = s_frag[((k - KT) * PS + p) * 64 + 32 + lane];
-                        }
-                    } else {
+                        for (int i = 0; i < (SPLIT ? 1 : 2); ++i)
 #pragma unroll
-                        for (int p = 0; p < PS; ++p) {
-                            const uint4* f = fragment(k, p);
-                            ah[p] = __ldg(f);
-                            al[p] = __ldg(f + 32);
-                        }
-                    }
+                            for (int p = 0; p < PS; ++p)
+                                f[i][p] = k < KT + a.smem_steps ? s_frag[((k - KT) * PS + p) * 64 + 32 * (lo + i) + lane]
+                                                                : __ldg(fragment(k, p) + 32 * (lo + i));
+                    };
+                    fetch(0);
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
                         const uint4 w = b[kk][n];          // hi, lo of rows 2t; hi, lo of rows 2t + 8
-                        const uint32_t wx = w.x ^ round;
 #pragma unroll
-                        for (int p = 0; p < PS; ++p) mma16816(acc[0][p][n], ah[p], wx, w.z);
-                        if (a.terms == 3) {
+                        for (int p = 0; p < PS; ++p) mma16816(acc[0][p][n], f[0][p], w.x ^ round, w.z);
+                        if (a.terms == 3)
 #pragma unroll
-                            for (int p = 0; p < PS; ++p) mma16816(acc[AC == 3 ? 1 : 0][p][n], ah[p], w.y, w.w);
+                            for (int p = 0; p < PS; ++p) mma16816(acc[AC == 3 ? 1 : 0][p][n], f[0][p], w.y, w.w);
+                    }
+                    if (a.terms == 3) {
+                        if (SPLIT) fetch(1);
 #pragma unroll
-                            for (int p = 0; p < PS; ++p) mma16816(acc[AC == 3 ? 2 : 0][p][n], al[p], wx, w.z);
-                        }
+                        for (int n = 0; n < NT; ++n)
+#pragma unroll
+                            for (int p = 0; p < PS; ++p) mma16816(acc[AC == 3 ? 2 : 0][p][n], f[SPLIT ? 0 : 1][p], b[kk][n].x ^ round, b[kk][n].z);
                     }
                 }
             }
