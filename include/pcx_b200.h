@@ -503,6 +503,15 @@ int pcx_column_run_big(int mode, float* node_mars, float* node_flows, float* ele
                        int logspace, int terms, void* stream);
 /* Clusters of `cluster` CTAs of those launches that the current device can hold at a time. */
 int pcx_column_clusters(int cluster, int big);
+/* Products whose source rows are read many times over, through shared memory.  mode 0: out (stored element values) = sum of rows
+ * of src (node_mars); mode 1: out (node_flows) = log-sum-exp (logspace), or sum, of rows of src (element_flows), added to what is
+ * there where an item says so.  sources: first row of every source block (at most PCX_STAGED_SOURCES).  items: int32 x 4: first
+ * output row, first chunk of its list, sources in the list, add.  lists: chunks of eight uint16 places in `sources`, filled up
+ * with n_sources.  All blocks have block_size rows. */
+#define PCX_STAGED_COLUMNS 32
+#define PCX_STAGED_SOURCES 880
+int pcx_prod_staged(int mode, float* out, const float* src, const int32_t* sources, const int32_t* items, const int32_t* lists,
+                    int n_sources, int n_items, int block_size, int W, int logspace, void* stream);
 /* A chain: consecutive levels of one group of n_strips * 16 rows (at most 1024) and as many children, all with the same
  * fragments, each reading the level before it.  A cluster of ceil(n_strips / per) CTAs (at most 16; at most 8 where per > 4) owns
  * 8 * nt columns (nt 1 - 3, per * nt at most 16), a CTA `per` strips (at most 8).  Flows are logarithms.

@@ -70,6 +70,7 @@ SIGNATURES = {
     "pcx_input_cat_flush_t": [P, P, P, P, L, I],
     "pcx_column_run": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I],
     "pcx_column_run_big": [I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I],
+    "pcx_prod_staged": [I, P, P, P, P, P, I, I, I, I, I],
     "pcx_column_chain": [I, P, P, P, P, P, P, I, I, I, I, I, I],
     "pcx_column_pack": [P, P, L, P],
     "pcx_column_par": [I, P, P, P, P, P, P, P, P, I, I, I, I],

@@ -124,6 +124,28 @@ class _Chain:
         self.work = torch.empty(_lib.load().pcx_column_chain_bytes(S, W, nt, per), dtype=torch.uint8, device=rows.device)
 
 
+class _Staged:
+    """Tables of `pcx_prod_staged`: products of one block size, their sources through shared memory."""
+
+    def __init__(self, sources, items, lists, size):
+        self.sources, self.items, self.lists, self.size = sources, items, lists, size
+
+    def run(self, mode, out, src, logspace):
+        _lib.call("pcx_prod_staged", mode, out, src, self.sources, self.items, self.lists, self.sources.numel(), self.items.size(0),
+                  self.size, src.size(1), int(logspace))
+
+    def check(self, report, mode, pc, em_rows):
+        """Bounds of every index the kernel forms (see `ColumnProgram.check`)."""
+        lists, n = self.lists.cpu().numpy().view(np.uint16).reshape(-1, 8), self.sources.numel()
+        limits = (em_rows, pc.num_nodes) if mode == 0 else (pc.num_nodes, pc.num_elements)
+        for row, at, k, _ in self.items.cpu().tolist():
+            report("column product rows", row, self.size, limits[0])
+            places = lists[at:at + -(-k // 8)].reshape(-1)
+            assert 0 <= at and places.size >= k and (places[:k] < n).all() and (places[k:] == n).all()
+        for r in self.sources.cpu().tolist():
+            report("column product sources", r, self.size, limits[1])
+
+
 def _pointer(a):
     return a.ctypes.data_as(ctypes.c_void_p)
 
@@ -200,11 +222,17 @@ class ColumnProgram:
         for mode in (0, 1):
             tasks, n_tasks, strips, n_strips, levels, n_levels = blob.next(6)
             out[mode] = dict(tasks=blob.take(tasks, 12 * n_tasks), strips=blob.take(strips, n_strips),
-                             levels=blob.take(levels, n_levels, 4), launches=[], chained=[])
+                             levels=blob.take(levels, n_levels, 4), launches=[], chained=[], staged={})
         for mode, form in ((0, "launches"), (1, "launches"), (0, "chained"), (1, "chained")):
-            launches = out[mode][form]
+            launches, staged = out[mode][form], out[mode]["staged"]
             for _ in range(blob.next()):
                 kind, *words = blob.next(7)
+                if kind == 4:                                # the launch before this one, staged
+                    sources, n_sources, items, n_items, n_chunks, size = words
+                    at = launches[-1]
+                    staged[form, len(launches) - 1, len(at) - 1 if isinstance(at, list) else 0] = _Staged(
+                        blob.take(sources, n_sources), blob.take(items, n_items, 4), blob.take(items + 4 * n_items, n_chunks, 4), size)
+                    continue
                 if kind == 0:                                # (levels, how many, (column groups, tiles, CTAs, wide))
                     first, n, *how = words
                     launches.append((out[mode]["levels"][first:first + n], n, tuple(how)))
@@ -267,9 +295,13 @@ class ColumnProgram:
         p = plan[mode]
         W = nm.size(1)
         em, terms = self.buffers(W), 1 if _lib.sum_mode() == 2 else 3
-        for launch in p["chained" if logspace else "launches"]:     # (a chain keeps its flows as logarithms)
+        form = "chained" if logspace else "launches"         # (a chain keeps its flows as logarithms)
+        for i, launch in enumerate(p[form]):
             if isinstance(launch, list):
-                for nids, cids, size in launch:
+                for q, (nids, cids, size) in enumerate(launch):
+                    if (form, i, q) in p["staged"]:
+                        p["staged"][form, i, q].run(mode, em, nm, logspace)
+                        continue
                     _lib.call("pcx_prod_fwd", em, nm, nids, cids, nids.numel(), cids.size(1), size, W)
                 continue
             if isinstance(launch, _Chain):
@@ -277,6 +309,9 @@ class ColumnProgram:
                 _lib.call("pcx_column_chain", mode, nm, nf, plan["frags"], c.work, c.rows, c.strips, c.n, c.S, W, c.nt, c.per, terms)
                 continue
             levels, n, (nt, tiles, cluster, wide) = launch
+            if (form, i, 0) in p["staged"]:
+                p["staged"][form, i, 0].run(mode, nf, ef, logspace)
+                continue
             if self.big_steps:
                 _lib.call("pcx_column_run_big", mode, nm, nf, ef, em, params, plan["frags"], p["tasks"], plan["kids"],
                           p["strips"], levels, n, W, nt, cluster, self.big_steps, int(logspace), terms)
@@ -349,6 +384,8 @@ class ColumnProgram:
                         report("column chain rows", int(r), 16, pc.num_nodes)
                     for first, step in c.strips.cpu().tolist():
                         assert 0 <= first and first + (c.S - 1) * step < plan["n_frag"]
+            for staged in p["staged"].values():
+                staged.check(report, mode, pc, self.em_rows)
             for t in tasks:
                 k, w, off = int(t["n_k"]), int(t["width"]), int(t["kid_off"])
                 if t["kind"] == K_PROD:

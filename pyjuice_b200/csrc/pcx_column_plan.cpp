@@ -946,6 +946,7 @@ struct Cutter {
                                    !(chained && starts(mode, end)); ++end) {}
                 if (mode == 0 && before[at]) n += products(pc.depths[at], blob, launches);
                 launches.insert(launches.end(), {0, (int64_t)at, (int64_t)(end - at), how.nt, how.tiles, how.cluster, how.wide});
+                if (how.wide == 3) n += product_flows(pc.depths[levels[mode][at - 1].depth], blob, launches);
             }
             m.push_back(n);
             m.insert(m.end(), launches.begin(), launches.end());
@@ -973,7 +974,8 @@ struct Cutter {
         return t;
     }
     // Arguments of the product kernel that fills the stored values of a depth, one set per block size.
-    static int64_t products(const Depth& d, Blob& blob, std::vector<int64_t>& launches) {
+    int64_t products(const Depth& d, Blob& blob, std::vector<int64_t>& launches) const {
+        int64_t made = 0;
         Ints sizes;
         for (auto& e : d.elems)
             if (std::find(sizes.begin(), sizes.end(), e.size) == sizes.end()) sizes.push_back(e.size);
@@ -988,9 +990,60 @@ struct Cutter {
                     for (int c = 0; c < n; ++c) cids.push_back(c < e.n ? d.kids[e.first + c] : 0);
                 }
             launches.insert(launches.end(), {q == 0 ? 1 : 2, blob.section(rows), blob.section(cids), (int64_t)rows.size(), n, sizes[q], 0});
+            std::vector<Item> readers;
+            for (auto& e : d.elems)
+                if (e.size == sizes[q]) readers.push_back({e.store, 0, d.kids.data() + e.first, e.n});
+            made += 1 + staged(readers, sizes[q], blob, launches);
         }
-        return (int64_t)sizes.size();
+        return made;
     }
+    // The flows of a product level, if all of it can be staged.
+    int64_t product_flows(const Depth& d, Blob& blob, std::vector<int64_t>& launches) const {
+        std::vector<Item> readers;
+        for (auto& p : d.prod_bk) {
+            if (p.size != d.prod_bk[0].size) return 0;
+            readers.push_back({p.row, p.add, d.parents.data() + p.first, p.n});
+        }
+        return readers.empty() ? 0 : staged(readers, d.prod_bk[0].size, blob, launches);
+    }
+
+    // Tables of `pcx_prod_staged` for the rows of one block size, as a launch record that replaces the one before it: (4, sources,
+    // how many, items, how many, chunks of their lists behind them, block size).
+    struct Item { int row, add; const int32_t* from; int n; };
+    int64_t staged(std::vector<Item>& readers, int size, Blob& blob, std::vector<int64_t>& launches) const {
+        if (W < PCX_STAGED_COLUMNS || (int64_t)size * cdiv(W, PCX_STAGED_COLUMNS) < STAGED_CTAS) return 0;
+        int lo = INT32_MAX, hi = -1;
+        for (auto& r : readers)
+            for (int k = 0; k < r.n; ++k) { lo = std::min(lo, r.from[k]); hi = std::max(hi, r.from[k]); }
+        if (hi < lo) return 0;
+        Ints sources, items, place((size_t)(hi - lo) + 1, -1);
+        int64_t reads = 0;
+        for (auto& r : readers) {
+            reads += r.n;
+            for (int k = 0; k < r.n; ++k)
+                if (place[r.from[k] - lo] < 0) {
+                    place[r.from[k] - lo] = (int)sources.size();
+                    sources.push_back(r.from[k]);
+                }
+            if (sources.size() > PCX_STAGED_SOURCES) return 0;
+        }
+        if (reads < STAGED_READS * (int64_t)sources.size()) return 0;
+        std::stable_sort(readers.begin(), readers.end(), [](const Item& x, const Item& y) { return x.n > y.n; });
+        std::vector<uint16_t> words;
+        for (auto& r : readers) {
+            items.insert(items.end(), {r.row, (int)(words.size() / 8), r.n, r.add});
+            for (int k = 0; k < r.n; ++k) words.push_back((uint16_t)place[r.from[k] - lo]);
+            while (words.size() % 8 != 0) words.push_back((uint16_t)sources.size());
+        }
+        items.resize(items.size() + words.size() / 2);       // (the lists, behind the items)
+        std::memcpy(items.data() + items.size() - words.size() / 2, words.data(), words.size() * 2);
+        launches.insert(launches.end(), {4, blob.section(sources), (int64_t)sources.size(), blob.section(items), (int64_t)readers.size(),
+                                         (int64_t)words.size() / 8, size});
+        return 1;
+    }
+    // A staged source is copied once and read from shared memory: below STAGED_READS readers a source, or with fewer CTAs than
+    // SMs, the general kernels stay.
+    static constexpr int64_t STAGED_READS = 4, STAGED_CTAS = 148;
 };
 
 // ---- parameter-flow jobs (no row width in them) --------------------------------------------------------------------------
