@@ -90,35 +90,47 @@ em_sum_kernel(float* __restrict__ params, const float* __restrict__ flows,
     }
 }
 
-// One group of G threads per source node; the group strides over the node's categories.
+constexpr int EM_U = 8;
+
+// One group of G threads per source node; the group strides over the node's categories.  The first EM_U of a thread stay in
+// registers over the sum, with their parameters.  (784 variables x 128 nodes x 256 categories: 72 -> 64 us.)
 template <int G>
 __global__ void __launch_bounds__(NT)
 em_input_cat_kernel(float* __restrict__ params, const float* __restrict__ flows,
                     const int32_t* __restrict__ source_nids, const int32_t* __restrict__ s_pids,
                     const int32_t* __restrict__ s_pfids, const int32_t* __restrict__ node_cats,
                     int64_t n_source, float step, float pseudo, int keep_zero) {
-    constexpr int GROUPS = NT / G;
+    constexpr int GROUPS = NT / G, U = EM_U;
     __shared__ float s_red[NT / 32];
     const int g = threadIdx.x / G, l = threadIdx.x % G;
     const int64_t sidx = (int64_t)blockIdx.x * GROUPS + g;
-    const bool live = sidx < n_source;
-    int64_t poff = 0, foff = 0;
-    int num_cats = 1;
-    if (live) {
-        int n = source_nids[sidx];
-        poff = s_pids[n];
-        foff = s_pfids[n];
+    const float* f = flows;
+    float* p = params;
+    int num_cats = 0;
+    if (sidx < n_source) {
+        const int n = source_nids[sidx];
+        p += s_pids[n];
+        f += s_pfids[n];
         num_cats = node_cats[n];
     }
     const float add = pseudo / (float)num_cats;
-    float tot = 0.0f;
-    if (live) {
-        for (int c = l; c < num_cats; c += G) {
-            float fl = flows[foff + c];
-            if (keep_zero) tot += (params[poff + c] < 1e-12f) ? 0.0f : fl + add;
-            else tot += fl;
+    float fl[U], old[U], tot = 0.0f;
+    auto load = [&](int c0, bool with_params) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * G;
+            fl[u] = (c < num_cats) ? f[c] : 0.0f;
+            old[u] = (with_params && c < num_cats) ? p[c] : 0.0f;
         }
-    }
+    };
+    auto count = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c0 + u * G < num_cats) tot += !keep_zero ? fl[u] : (old[u] < 1e-12f) ? 0.0f : fl[u] + add;
+    };
+    for (int c0 = l + G * U; c0 < num_cats; c0 += G * U) { load(c0, keep_zero != 0); count(c0); }
+    load(l, true);
+    count(l);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     if (G > 32) {                       // G == NT: one node per CTA, combine the warps
@@ -128,13 +140,17 @@ em_input_cat_kernel(float* __restrict__ params, const float* __restrict__ flows,
 #pragma unroll
         for (int q = 0; q < NT / 32; ++q) tot += s_red[q];
     }
-    if (!live) return;
     const float denom = keep_zero ? tot : tot + pseudo;
-    for (int c = l; c < num_cats; c += G) {
-        float old = params[poff + c];
-        float upd = (1.0f - step) * old + step * (flows[foff + c] + add) / denom;
-        if (keep_zero && old < 1e-12f) upd = 0.0f;
-        params[poff + c] = upd;
+    for (int c0 = l; c0 < num_cats; c0 += G * U) {
+        if (c0 != l) load(c0, true);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + u * G;
+            if (c >= num_cats) continue;
+            float upd = (1.0f - step) * old[u] + step * (fl[u] + add) / denom;
+            if (keep_zero && old[u] < 1e-12f) upd = 0.0f;
+            p[c] = upd;
+        }
     }
 }
 
@@ -146,8 +162,9 @@ em_input_cat_kernel(float* __restrict__ params, const float* __restrict__ flows,
 // both layouts are read and written with full-width coalesced accesses.  The flows are left as they are (the caller
 // clears or moves them later).  (Tiles of 32 x 32, one CTA per 32 rows, ran at 3.1 TB/s: 128-byte runs strided by
 // 16 KB and 128 KB.)
-constexpr int EMT = 128;                                 // tile edge
-constexpr int EMT_LD = EMT + 1;                          // row pitch of the shared tile: odd, see emt_update_kernel
+// Where such tiles are fewer than the SMs, tiles of 128 rows x 32 categories: what counts is then the chain of a CTA (512 rows x
+// 1000 categories, 32 tiles: 25 us, 128 narrow ones: 18).
+constexpr int EMT = 128;                                 // rows of a tile
 
 // part[share, r] = sum over this CTA's categories of flows_t[c, r].  Grid (ceil(R / 128), shares of the categories).
 // (No atomics: the row totals are added up in a fixed order, so that data-parallel ranks, which hold bit-identical
@@ -192,29 +209,37 @@ __global__ void __launch_bounds__(256) emt_totals_kernel(float* __restrict__ tot
     }
 }
 
-// One tile of 128 rows x 128 categories per CTA (256 threads).  Lane l owns rows l, l + 32, l + 64, l + 96 on the
+// One tile of 128 rows x EC categories per CTA (256 threads).  Lane l owns rows l, l + 32, l + 64, l + 96 on the
 // transposed side and categories l, l + 32, ... on the parameter side: every global access of a warp is 128 contiguous
-// bytes (four of them make up the 512-byte run of the tile), and with a row pitch of 129 floats neither side has a
-// shared-memory bank conflict.
+// bytes (at EC = 128 four of them make up the 512-byte run of the tile), and with a row pitch of EC + 1 floats, an odd number,
+// neither side has a shared-memory bank conflict.
+template <int EC>
 __global__ void __launch_bounds__(256) emt_update_kernel(float* __restrict__ params, float* __restrict__ logp_t,
                                                           const float* __restrict__ flows_t, const float* __restrict__ totals,
                                                           int shares, int64_t R, int C, float step, float pseudo) {
-    extern __shared__ float s_p[];                       // [128 rows][EMT_LD]
+    constexpr int LD = EC + 1, J = EC / 32, V = EC == 128 ? 2 : 4;
+    extern __shared__ float s_p[];                       // [128 rows][LD]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r0 = (int64_t)blockIdx.x * EMT;
-    const int c0 = blockIdx.y * EMT;
+    const int c0 = blockIdx.y * EC;
     const float add = pseudo / (float)C;
-    // parameter tile in: warp -> rows warp, warp + 8, ...
-    for (int rr = warp; rr < EMT; rr += 8) {
-        const int64_t r = r0 + rr;
-        float v[4];
+    // parameter tile in: warp -> rows warp, warp + 8, ..., eight loads at a time
+    constexpr int ROUND = 8 / J;
+#pragma unroll 1
+    for (int rr0 = warp; rr0 < EMT; rr0 += 8 * ROUND) {
+        float v[ROUND][J];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + lane + 32 * j;
-            v[j] = (r < R && c < C) ? params[r * C + c] : 0.0f;
-        }
+        for (int q = 0; q < ROUND; ++q)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s_p[rr * EMT_LD + lane + 32 * j] = v[j];
+            for (int j = 0; j < J; ++j) {
+                const int64_t r = r0 + rr0 + 8 * q;
+                const int c = c0 + lane + 32 * j;
+                v[q][j] = (r < R && c < C) ? params[r * C + c] : 0.0f;
+            }
+#pragma unroll
+        for (int q = 0; q < ROUND; ++q)
+#pragma unroll
+            for (int j = 0; j < J; ++j) s_p[(rr0 + 8 * q) * LD + lane + 32 * j] = v[q][j];
     }
     float inv[4];
 #pragma unroll
@@ -226,11 +251,11 @@ __global__ void __launch_bounds__(256) emt_update_kernel(float* __restrict__ par
         inv[i] = (r < R) ? 1.0f / (tot + pseudo) : 0.0f;
     }
     __syncthreads();
-    // transposed side: warp -> categories warp, warp + 8, ...; two categories per round (eight loads in flight)
-    for (int cc0 = warp; cc0 < EMT; cc0 += 16) {
-        float f[2][4];
+    // transposed side: warp -> categories warp, warp + 8, ...; V categories per round (4 V loads in flight)
+    for (int cc0 = warp; cc0 < EC; cc0 += 8 * V) {
+        float f[V][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < V; ++u) {
             const int c = c0 + cc0 + 8 * u;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -239,14 +264,14 @@ __global__ void __launch_bounds__(256) emt_update_kernel(float* __restrict__ par
             }
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < V; ++u) {
             const int cc = cc0 + 8 * u;
             const int c = c0 + cc;
             if (c >= C) continue;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int64_t r = r0 + lane + 32 * i;
-                float* cell = s_p + (lane + 32 * i) * EMT_LD + cc;
+                float* cell = s_p + (lane + 32 * i) * LD + cc;
                 const float upd = (1.0f - step) * (*cell) + step * (f[u][i] + add) * inv[i];
                 *cell = upd;
                 if (r < R) logp_t[(int64_t)c * R + r] = logf(upd);
@@ -259,9 +284,9 @@ __global__ void __launch_bounds__(256) emt_update_kernel(float* __restrict__ par
         const int64_t r = r0 + rr;
         if (r >= R) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < J; ++j) {
             const int c = c0 + lane + 32 * j;
-            if (c < C) params[r * C + c] = s_p[rr * EMT_LD + lane + 32 * j];
+            if (c < C) params[r * C + c] = s_p[rr * LD + lane + 32 * j];
         }
     }
 }
@@ -310,7 +335,9 @@ int pcx_em_sum(float* params, const float* param_flows, const int64_t* blk_par, 
     if (n_blocks <= 0) return 0;
     if (max_bs <= 0) return -1;
     cudaStream_t st = (cudaStream_t)stream;
-    if (max_bs >= 32) {
+    // tiles of 32 nodes read 128 bytes of an edge, tiles of eight one sector: where the former are fewer than two a SM, four times
+    // as many CTAs with a quarter of the rounds (one 512 x 512 table: @S0@ us in 16 CTAs of 32 nodes, @S1@ in 64)
+    if (max_bs >= 32 && n_blocks * pcx_cdiv(max_bs, 32) >= 2 * 148) {
         int tiles = (int)pcx_cdiv(max_bs, 32);
         em_sum_kernel<32><<<(unsigned)(n_blocks * tiles), NT, 0, st>>>(params, param_flows, blk_par, blk_flow, blk_fan, blk_bs, tiles, step, pseudo, keep_zero);
     } else if (max_bs >= 8) {
@@ -351,15 +378,22 @@ int pcx_em_input_cat_t(float* params, float* logp_t, const float* flows_t, float
     if (shares > EMT_MAX_SHARES) shares = EMT_MAX_SHARES;
     if (shares < 1) shares = 1;
     emt_totals_kernel<<<dim3((unsigned)row_tiles, (unsigned)shares), 256, 0, st>>>(totals, flows_t, n_rows, num_cats);
-    const int smem = EMT * EMT_LD * (int)sizeof(float);
-    static PcxOnce done;
-    if (!done) {
-        e = cudaFuncSetAttribute(emt_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return (int)e;
-        done = true;
-    }
-    emt_update_kernel<<<dim3((unsigned)row_tiles, (unsigned)pcx_cdiv(num_cats, EMT)), 256, smem, st>>>(
-        params, logp_t, flows_t, totals, (int)shares, n_rows, num_cats, step, pseudo);
+    auto update = [&](auto kernel, int ec) -> int {
+        const int smem = EMT * (ec + 1) * (int)sizeof(float);
+        if (smem > 48 * 1024) {
+            static PcxOnce done;                                    // (of the wide tiles: the only ones that need it)
+            if (!done) {
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                if (e != cudaSuccess) return (int)e;
+                done = true;
+            }
+        }
+        kernel<<<dim3((unsigned)row_tiles, (unsigned)pcx_cdiv(num_cats, ec)), 256, smem, st>>>(
+            params, logp_t, flows_t, totals, (int)shares, n_rows, num_cats, step, pseudo);
+        return 0;
+    };
+    const int rc = row_tiles * pcx_cdiv(num_cats, EMT) < 148 ? update(emt_update_kernel<32>, 32) : update(emt_update_kernel<128>, 128);
+    if (rc != 0) return rc;
     PCX_LAUNCH_CHECK();
     return 0;
 }
