@@ -188,7 +188,10 @@ def family_of(name: str) -> str:
         return "pcx_sum_bwd_par"
     if name == "pcx_column_pack":
         return "pcx_pack_sum_params"
-    if name.startswith(("pcx_sum_chain", "pcx_column_run")):     # one launch: forward or element flows of many layers
+    if name == "pcx_prod_staged_fwd":
+        return "pcx_prod_fwd"
+    # one launch: forward or element flows of many layers (product levels of the column program's flows count among them)
+    if name.startswith(("pcx_sum_chain", "pcx_column_run", "pcx_column_chain", "pcx_prod_staged")):
         return "pcx_sum_fwd" if name.endswith("_fwd") else "pcx_sum_bwd_ele"
     if name.endswith("_dense2_prep"):                     # operand pre-pass of the wide dense kernels (fwd and element flows)
         return "pcx_sum_dense_prep"

@@ -216,7 +216,8 @@ def _invoke(lib, name, conv, args, dev) -> int:
     rc = getattr(lib, name)(*conv, stream)
     b.record()
     # launches over many layers serve two operators: tell them apart by their first argument (0 forward, 1 element flows)
-    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in ("pcx_sum_chain", "pcx_column_run", "pcx_column_run_big", "pcx_column_chain") else name, a, b))
+    both = ("pcx_sum_chain", "pcx_column_run", "pcx_column_run_big", "pcx_column_chain", "pcx_prod_staged")
+    PROFILE.append((name + ("_fwd", "_ele")[args[0]] if name in both else name, a, b))
     return rc
 
 
