@@ -558,10 +558,10 @@ int pcx_column_par(int kind, float* param_flows, const float* node_flows, const 
 int pcx_colplan_new(const int64_t* desc, int64_t n_desc, const int32_t* tables, int64_t n_tables, void** planner, char* why,
                     int why_len);
 int pcx_colplan_free(void* planner);
-/* Rows of stored element values; depth (in 16) of the deepest CTA task, 0 without any. */
-int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps);
-/* Whether the program is the better choice at rows of W samples; rooms: clusters of 1, 2, 4, 8 and 16 CTAs at a time, then
- * clusters of 1 ... 16 CTAs of a chain. */
+/* Rows of stored element values; depth (in 16) of the deepest CTA task, 0 without any; chains. */
+int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps, int* n_chains);
+/* Whether the program is the better choice at rows of W samples; rooms: clusters of 1, 2, 4, 8 and 16 CTAs at a time, then,
+ * for a circuit with chains, clusters of 1 ... 16 CTAs of a chain. */
 int pcx_colplan_suits(const void* planner, int64_t W, const int32_t* rooms);
 /* Tables: the launches at rows of W samples; groups of tied tables; parameter-flow jobs, without the groups flagged in `dense`.
  * Each makes a blob: one array of device tables and a description of its sections (see column.py). */

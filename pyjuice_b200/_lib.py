@@ -85,7 +85,7 @@ PLAIN = {"pcx_build_arch": [], "pcx_column_clusters": [I, I], "pcx_column_chain_
          "pcx_packed_tile_count": [L, I, I, I, I], "pcx_dense_scratch_bytes": [I, I, I],
          "pcx_sm_packed_bytes": [L, I, I], "pcx_dense2_scratch_bytes": [I, I, I]}
 # the planner of the column program (host only; the last two arguments of those that may refuse: a text buffer and its size)
-PLAIN.update({"pcx_colplan_new": [P, L, P, L, P, P, I], "pcx_colplan_free": [P], "pcx_colplan_info": [P, P, P],
+PLAIN.update({"pcx_colplan_new": [P, L, P, L, P, P, I], "pcx_colplan_free": [P], "pcx_colplan_info": [P, P, P, P],
               "pcx_colplan_suits": [P, L, P], "pcx_colplan_cut": [P, L, P, L, L, P, P, I], "pcx_colplan_tied": [P, P, P, I],
               "pcx_colplan_jobs": [P, P, P, P, I], "pcx_colplan_blob": [P, P, P, P, P], "pcx_colplan_blob_free": [P]})
 SUM_MODE = 1        # the process default of the arithmetic mode (see set_sum_mode / use_sum_mode)

@@ -150,6 +150,23 @@ def _pointer(a):
     return a.ctypes.data_as(ctypes.c_void_p)
 
 
+# {(question, device, its other arguments): answers}: what a device holds at a time does not change, and one answer costs the driver
+# some microseconds of a first pass
+_ROOMS = {}
+
+
+def _clusters(device, name, sizes, *args):
+    """How many clusters of each of ``sizes`` CTAs of a kernel the device holds at a time."""
+    found = [-1] * len(sizes)
+    if device.type == "cuda":
+        with torch.cuda.device(device):
+            key = (name, torch.cuda.current_device() if device.index is None else device.index, *args)
+            found = _ROOMS.get(key) or [int(getattr(_lib.load(), name)(c, *args)) for c in sizes]
+            if min(found) > 0:
+                _ROOMS[key] = found
+    return [n if n > 0 else max(1, (128 if c < 16 else 112) // c) for c, n in zip(sizes, found)]
+
+
 class ColumnProgram:
     PROD_READS = 3000            # child rows a CTA may gather for the stored elements of a fused level
 
@@ -171,23 +188,19 @@ class ColumnProgram:
         self._planner = ctypes.c_void_p()
         _native("pcx_colplan_new", _pointer(desc), desc.size, _pointer(tables), tables.size, ctypes.byref(self._planner))
         weakref.finalize(self, _lib.load().pcx_colplan_free, self._planner)
-        em_rows, big_steps = ctypes.c_int(), ctypes.c_int()
-        _lib.load().pcx_colplan_info(self._planner, ctypes.byref(em_rows), ctypes.byref(big_steps))
-        self.em_rows, self.big_steps = em_rows.value, big_steps.value
+        info = [ctypes.c_int() for _ in range(3)]
+        _lib.load().pcx_colplan_info(self._planner, *map(ctypes.byref, info))
+        self.em_rows, self.big_steps, self.n_chains = (v.value for v in info)
         self._by_width, self._par, self._tied, self._rooms = {}, {}, None, None
 
     # ---- cutting into tasks ------------------------------------------------------------------------------------------
     def _room(self):
-        """Clusters of 1, 2, 4, 8 and 16 CTAs the device holds at a time, then clusters of 1 ... 16 CTAs of a chain."""
+        """Clusters of 1, 2, 4, 8 and 16 CTAs the device holds at a time, then clusters of 1 ... 16 CTAs of a chain where the
+        circuit has one."""
         if self._rooms is None:
-            rooms, lib = [], _lib.load()
-            for c, count in ([(c, lambda c: lib.pcx_column_clusters(c, bool(self.big_steps))) for c in (1, 2, 4, 8, 16)]
-                             + [(c, lib.pcx_column_chain_clusters) for c in range(1, 17)]):
-                n = -1
-                if self.device.type == "cuda":
-                    with torch.cuda.device(self.device):
-                        n = int(count(c))
-                rooms.append(n if n > 0 else max(1, (128 if c < 16 else 112) // c))
+            rooms = _clusters(self.device, "pcx_column_clusters", (1, 2, 4, 8, 16), bool(self.big_steps))
+            if self.n_chains:
+                rooms += _clusters(self.device, "pcx_column_chain_clusters", range(1, 17))
             self._rooms = np.asarray(rooms, dtype=np.int32)
         return _pointer(self._rooms)
 

@@ -538,8 +538,8 @@ struct PcxColPlanner {
     }
 
     // ---- launch geometry ---------------------------------------------------------------------------------------------
-    struct Room {                               // clusters of 1, 2, 4, 8 and 16 CTAs that the device holds at a time, then
-        const int32_t* n;                       // clusters of 1 ... 16 CTAs of a chain
+    struct Room {                               // clusters of 1, 2, 4, 8 and 16 CTAs that the device holds at a time, then, for a
+        const int32_t* n;                       // circuit with chains, clusters of 1 ... 16 CTAs of a chain
         int operator()(int c) const { return std::max(1, (int)n[c == 1 ? 0 : c == 2 ? 1 : c == 4 ? 2 : c == 8 ? 3 : 4]); }
         int chain(int c) const { return std::max(1, (int)n[4 + c]); }
     };
@@ -1177,10 +1177,11 @@ int pcx_colplan_free(void* planner) {
     delete static_cast<PcxColPlanner*>(planner);
     return 0;
 }
-int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps) {
+int pcx_colplan_info(const void* planner, int* em_rows, int* big_steps, int* n_chains) {
     const auto* p = static_cast<const PcxColPlanner*>(planner);
     *em_rows = p->em_rows;
     *big_steps = p->big_steps;
+    *n_chains = (int)p->chains.size();
     return 0;
 }
 int pcx_colplan_suits(const void* planner, int64_t W, const int32_t* rooms) {

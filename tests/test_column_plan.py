@@ -233,3 +233,26 @@ def test_description_is_checked():
     with pytest.raises(pj._lib.PcxError, match="too short"):
         make(desc[:-1].copy(), tables.size)
     assert not handle.value
+
+
+@pytest.mark.parametrize("kind,latents,chains", [("hclt", 4, 0), ("hmm", 96, 1)])
+def test_a_device_is_asked_once(kind, latents, chains, monkeypatch):
+    """What a device holds at a time is asked for by the first circuit, not by every one, and about chains only where there is one."""
+    from contextlib import nullcontext
+    from types import SimpleNamespace
+    from pyjuice_b200 import _lib, column
+    programs = [ColumnProgram(_circuit(kind, latents)) for _ in range(2)]
+    asked, lib = [], _lib.load()
+
+    class Device:
+        def __getattr__(self, name):
+            if not name.endswith("_clusters"):
+                return getattr(lib, name)
+            return lambda c, *args: asked.append((name, c, *args)) or 1
+    monkeypatch.setattr(column, "_ROOMS", {}, raising=False)
+    monkeypatch.setattr(_lib, "load", Device)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: nullcontext())
+    for program in programs:
+        program.device = SimpleNamespace(type="cuda", index=3)
+        program._room()
+    assert len(asked) == len(set(asked)) == 5 + 16 * chains
