@@ -236,9 +236,13 @@ class ColumnProgram:
             tasks, n_tasks, strips, n_strips, levels, n_levels = blob.next(6)
             out[mode] = dict(tasks=blob.take(tasks, 12 * n_tasks), strips=blob.take(strips, n_strips),
                              levels=blob.take(levels, n_levels, 4), launches=[], chained=[], staged={})
-        for mode, form in ((0, "launches"), (1, "launches"), (0, "chained"), (1, "chained")):
+        for mode, form in ((0, "chained"), (0, "launches"), (1, "chained"), (1, "launches")):
+            n_launches = blob.next()
+            if n_launches < 0:                               # (no chain: the same list)
+                out[mode]["launches"] = out[mode]["chained"]
+                continue
             launches, staged = out[mode][form], out[mode]["staged"]
-            for _ in range(blob.next()):
+            for _ in range(n_launches):
                 kind, *words = blob.next(7)
                 if kind == 4:                                # the launch before this one, staged
                     sources, n_sources, items, n_items, n_chunks, size = words
@@ -308,7 +312,7 @@ class ColumnProgram:
         p = plan[mode]
         W = nm.size(1)
         em, terms = self.buffers(W), 1 if _lib.sum_mode() == 2 else 3
-        form = "chained" if logspace else "launches"         # (a chain keeps its flows as logarithms)
+        form = "chained" if logspace or p["launches"] is p["chained"] else "launches"    # (a chain keeps its flows as logarithms)
         for i, launch in enumerate(p[form]):
             if isinstance(launch, list):
                 for q, (nids, cids, size) in enumerate(launch):

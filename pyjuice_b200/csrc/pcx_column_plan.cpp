@@ -860,9 +860,9 @@ struct Cutter {
         split.clear();
     }
 
-    // Sections: fragments, then per direction tasks, strips, levels; launches: (0, first level, levels, shape) or, a product
-    // launch, (1, node rows, child rows, how many, children, block size) or, a chain, (3, rows, strips, levels, strips per
-    // level, nt, strips per CTA).
+    // Sections: fragments, then per direction tasks, strips, levels; then per direction two lists of launches, the second (by tasks
+    // alone) only where it differs (-1: it does not).  A launch: (0, first level, levels, shape) or, a product launch, (1, node
+    // rows, child rows, how many, children, block size) or, a chain, (3, rows, strips, levels, strips per level, nt, strips per CTA).
     void run(Blob& blob) {
         int64_t total = 0, n_small = 0;
         for (auto& d : pc.depths)
@@ -926,30 +926,51 @@ struct Cutter {
             m.push_back(blob.section(lv));
             m.push_back((int64_t)levels[mode].size());
         }
-        // twice: the levels by their tasks, and with chains in their places
-        for (int i = 0; i < 4; ++i) {
-            const int mode = i & 1;
-            const bool chained = i >= 2;
-            std::vector<int64_t> launches;
-            int64_t n = 0;
-            for (size_t at = 0, end; at < levels[mode].size(); at = end, ++n) { // consecutive fused levels are one launch
-                const Shape how = levels[mode][at].how;
-                const size_t last = std::min(levels[mode].size(), at + PCX_COLUMN_MAX_LEVELS);
-                if (const auto* c = chained ? starts(mode, at) : nullptr) {
-                    const auto shape = PcxColPlanner::chain_shape(W, c->strips, room);
-                    launches.insert(launches.end(), {3, blob.section(pc.chain_rows(*c, mode)), blob.section(chain_strips(mode, at)), c->n,
-                                                     c->strips, shape.nt, shape.per});
-                    end = at + c->n;
-                    continue;
+        // With chains in the places of their levels; then, where there is a chain, by tasks alone.  What goes with a level is made
+        // once for both.
+        for (int mode = 0; mode < 2; ++mode) {
+            const size_t n_levels = levels[mode].size();
+            std::vector<const PcxColPlanner::Chain*> chain(n_levels);
+            bool any = false;
+            for (size_t at = 0; at < n_levels; ++at) any = (chain[at] = starts(mode, at)) != nullptr || any;
+            std::vector<std::pair<int64_t, std::vector<int64_t>>> ahead(n_levels), staged(n_levels);    // launch records, how many
+            for (int chained = 1; chained >= 0; --chained) {
+                if (!chained && !any) {
+                    m.push_back(-1);
+                    break;
                 }
-                for (end = at + 1; how.wide == 0 && end < last && levels[mode][end].how.wide == 0 && !(mode == 0 && before[end]) &&
-                                   !(chained && starts(mode, end)); ++end) {}
-                if (mode == 0 && before[at]) n += products(pc.depths[at], blob, launches);
-                launches.insert(launches.end(), {0, (int64_t)at, (int64_t)(end - at), how.nt, how.tiles, how.cluster, how.wide});
-                if (how.wide == 3) n += product_flows(pc.depths[levels[mode][at - 1].depth], blob, launches);
+                std::vector<int64_t> launches;
+                int64_t n = 0;
+                auto add = [&](const std::pair<int64_t, std::vector<int64_t>>& records) {
+                    n += records.first;
+                    launches.insert(launches.end(), records.second.begin(), records.second.end());
+                };
+                for (size_t at = 0, end; at < n_levels; at = end, ++n) {            // consecutive fused levels are one launch
+                    const Shape how = levels[mode][at].how;
+                    const size_t last = std::min(n_levels, at + PCX_COLUMN_MAX_LEVELS);
+                    if (const auto* c = chained ? chain[at] : nullptr) {
+                        const auto shape = PcxColPlanner::chain_shape(W, c->strips, room);
+                        launches.insert(launches.end(), {3, blob.section(pc.chain_rows(*c, mode)), blob.section(chain_strips(mode, at)),
+                                                         c->n, c->strips, shape.nt, shape.per});
+                        end = at + c->n;
+                        continue;
+                    }
+                    for (end = at + 1; how.wide == 0 && end < last && levels[mode][end].how.wide == 0 && !(mode == 0 && before[end]) &&
+                                       !(chained && chain[end]); ++end) {}
+                    if (mode == 0 && before[at]) {
+                        if (ahead[at].first == 0) ahead[at].first = products(pc.depths[at], blob, ahead[at].second);
+                        add(ahead[at]);
+                    }
+                    launches.insert(launches.end(), {0, (int64_t)at, (int64_t)(end - at), how.nt, how.tiles, how.cluster, how.wide});
+                    if (how.wide == 3) {
+                        if (staged[at].first == 0)
+                            staged[at].first = product_flows(pc.depths[levels[mode][at - 1].depth], blob, staged[at].second);
+                        add(staged[at]);
+                    }
+                }
+                m.push_back(n);
+                m.insert(m.end(), launches.begin(), launches.end());
             }
-            m.push_back(n);
-            m.insert(m.end(), launches.begin(), launches.end());
         }
     }
     // The chain whose first level is `at`, if its clusters fit at once: where they do not, the tasks, which take more columns in

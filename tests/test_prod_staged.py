@@ -57,6 +57,16 @@ def test_tables_name_the_rows_of_the_general_kernels(num_vars, latents, depth, r
     assert not program.plan(24)[0]["staged"]               # narrower than a column tile
 
 
+def test_tables_are_made_once(monkeypatch):
+    """Without a chain both kinds of flows have one list of launches, and every table is in the blob once."""
+    monkeypatch.setattr(ColumnProgram, "WIDE_ITEMS", 1)
+    plan = ColumnProgram(_rat(61, 16, 3, 9)).plan(1024)
+    for mode in (0, 1):
+        assert plan[mode]["launches"] is plan[mode]["chained"]
+        held = list(plan[mode]["staged"].values())
+        assert held and len({s.items.data_ptr() for s in held}) == len({i for _, i, _ in plan[mode]["staged"]}) == len(held)
+
+
 def _tables(rng, size, n_sources, counts, device):
     sources, items, lists = rng.sample(range(n_sources + 7), n_sources), [], []
     for i, n in enumerate(counts):
