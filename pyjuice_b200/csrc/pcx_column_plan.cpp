@@ -423,34 +423,36 @@ struct PcxColPlanner {
     // Runs of depths of one group each, with the same parameters, where the operand of a depth is the output of the one below
     // and at most one other row per element.  From three levels on: the launch costs about what two levels gain.
     static constexpr int CHAIN_LEVELS = 3, CHAIN_MIN_STRIPS = 4, CHAIN_MAX_STRIPS = 64;
-    struct Chain { int first, n, strips; };     // depths first .. first + n - 1
+    struct Chain {
+        int first, n, strips;                   // depths first .. first + n - 1
+        Ints rows[2];                           // tables of the two directions: see pcx_column_chain
+    };
     std::vector<Chain> chains;
 
-    struct Pair { int x, y; };
-    // Child rows of 16-row pieces of the elements `ids`.
-    static std::vector<Pair> pieces(const Depth& d, const Ints& ids) {
-        std::vector<Pair> out;
+    // Child rows of 16-row pieces of the elements `ids`, two words each.
+    static Ints pieces(const Depth& d, const Ints& ids, int strips) {
+        Ints out;
+        out.reserve(2 * (size_t)strips);
         for (int id : ids) {
             const Elem& e = *d.find(id);
-            for (int o = 0; o < e.size; o += 16)
-                out.push_back({e.n > 0 ? d.kids[e.first] + o : 0, e.n > 1 ? d.kids[e.first + 1] + o : 0});
+            const int x = e.n > 0 ? d.kids[e.first] : 0, y = e.n > 1 ? d.kids[e.first + 1] : 0;
+            for (int o = 0; o < e.size; o += 16) {
+                out.push_back(x != 0 ? x + o : 0);
+                out.push_back(y != 0 ? y + o : 0);
+            }
         }
         return out;
     }
-    static Ints rows_of(const Ints& blocks, int size) {
-        Ints out;
+    // Puts the child first that is the row of the blocks' piece; false where there is none.
+    static bool order(Ints& p, const Ints& blocks, int size) {
+        size_t at = 0;
         for (int b : blocks)
-            for (int o = 0; o < size; o += 16) out.push_back(b + o);
-        return out;
-    }
-    // Puts the child that is the row of `own` first; false where there is none.
-    static bool order(std::vector<Pair>& p, const Ints& own) {
-        if (p.size() != own.size()) return false;
-        for (size_t i = 0; i < p.size(); ++i) {
-            if (p[i].y == own[i] && p[i].y != 0) std::swap(p[i].x, p[i].y);
-            if (p[i].x != own[i] || p[i].x == p[i].y) return false;
-        }
-        return true;
+            for (int r = b; r < b + size; r += 16, at += 2) {
+                if (at + 2 > p.size()) return false;
+                if (p[at + 1] == r) std::swap(p[at], p[at + 1]);
+                if (p[at] != r || p[at + 1] == r) return false;
+            }
+        return at == p.size();
     }
     static bool chain_depth(const Depth& d) {
         if (d.fw.size() != 1 || d.bk.size() != 1 || !d.direct || d.stored || !d.fw[0].mma || !d.bk[0].mma || d.max_kids > 2) return false;
@@ -461,46 +463,39 @@ struct PcxColPlanner {
             if (e.n < 1) return false;
         return true;
     }
-    bool follows(const Depth& d, const Depth& below) const {
+    // Extends the pieces of a run of depths (operands forward, outputs backward) by those of `d`, if it follows.
+    static bool follows(const Depth& d, const Depth& below, std::vector<Ints> (&sides)[2]) {
         if (d.fw[0].cls != below.fw[0].cls || d.bk[0].cls != below.bk[0].cls) return false;
-        auto f = pieces(d, d.fw[0].ops), b = pieces(d, d.bk[0].blocks);
-        return order(f, rows_of(below.fw[0].blocks, below.fw[0].bs)) && order(b, rows_of(below.bk[0].ops, below.bk[0].pbs));
+        Ints f = pieces(d, d.fw[0].ops, d.fw[0].strips()), b = pieces(d, d.bk[0].blocks, d.fw[0].strips());
+        if (!order(f, below.fw[0].blocks, below.fw[0].bs) || !order(b, below.bk[0].ops, below.bk[0].pbs)) return false;
+        sides[0].push_back(std::move(f));
+        sides[1].push_back(std::move(b));
+        return true;
     }
     void find_chains() {
         const int n = (int)depths.size();
         for (int i = 0, end; i < n; i = end) {
             end = i + 1;
-            if (!chain_depth(depths[i])) continue;
-            while (end < n && end - i < PCX_COLUMN_MAX_LEVELS && chain_depth(depths[end]) && follows(depths[end], depths[end - 1])) ++end;
-            if (end - i >= CHAIN_LEVELS) chains.push_back({i, end - i, depths[i].fw[0].strips()});
+            const Depth& low = depths[i];
+            if (!chain_depth(low)) continue;
+            const int strips = low.fw[0].strips();
+            std::vector<Ints> sides[2] = {{pieces(low, low.fw[0].ops, strips)}, {pieces(low, low.bk[0].blocks, strips)}};
+            while (end < n && end - i < PCX_COLUMN_MAX_LEVELS && chain_depth(depths[end]) && follows(depths[end], depths[end - 1], sides)) ++end;
+            if (end - i < CHAIN_LEVELS) continue;
+            const Depth& top = depths[end - 1];
+            Chain c{i, end - i, strips, {}};
+            for (Ints& t : c.rows) t.reserve(2 * (size_t)strips * (size_t)(c.n + 1));
+            auto add = [](Ints& to, const Ints& p) { to.insert(to.end(), p.begin(), p.end()); };
+            auto rows_of = [](Ints& to, const Ints& blocks, int size) {
+                for (int b : blocks)
+                    for (int r = b; r < b + size; r += 16) to.insert(to.end(), {r, 0});
+            };
+            for (const Ints& p : sides[0]) add(c.rows[0], p);       // a level's outputs are the first children of the next one's operand
+            rows_of(c.rows[0], top.fw[0].blocks, top.fw[0].bs);
+            rows_of(c.rows[1], top.bk[0].ops, top.bk[0].pbs);
+            for (size_t k = sides[1].size(); k-- > 0;) add(c.rows[1], sides[1][k]);
+            chains.push_back(std::move(c));
         }
-    }
-    // Tables of a chain: see pcx_column_chain.
-    Ints chain_rows(const Chain& c, int mode) const {
-        std::vector<Pair> t;
-        const Depth &low = depths[c.first], &top = depths[c.first + c.n - 1];
-        if (mode == 0) {
-            t = pieces(low, low.fw[0].ops);
-            for (int i = c.first; i < c.first + c.n; ++i) {
-                const Ints out = rows_of(depths[i].fw[0].blocks, depths[i].fw[0].bs);
-                std::vector<Pair> next(out.size());
-                if (i + 1 < c.first + c.n) {
-                    next = pieces(depths[i + 1], depths[i + 1].fw[0].ops);
-                    order(next, out);
-                }
-                for (size_t k = 0; k < out.size(); ++k) t.push_back({out[k], next[k].y});
-            }
-        } else {
-            for (int r : rows_of(top.bk[0].ops, top.bk[0].pbs)) t.push_back({r, 0});
-            for (int i = c.first + c.n - 1; i >= c.first; --i) {
-                auto p = pieces(depths[i], depths[i].bk[0].blocks);
-                if (i > c.first) order(p, rows_of(depths[i - 1].bk[0].ops, depths[i - 1].bk[0].pbs));
-                t.insert(t.end(), p.begin(), p.end());
-            }
-        }
-        Ints out;
-        for (const Pair& p : t) out.insert(out.end(), {p.x, p.y});
-        return out;
     }
 
     // Per group: members, children per element, depth, block size, blocks, then where child rows [members, depth, children],
@@ -912,8 +907,10 @@ struct Cutter {
             level(1, first, shape((int64_t)(tasks[1].size() - first)), -1);
         }
         auto& m = blob.meta;
+        size_t chain_words = 0;
+        for (auto& c : pc.chains) chain_words += c.rows[0].size() + c.rows[1].size();
         blob.data.reserve(frag.size() + kids.data.size() + 12 * (tasks[0].size() + tasks[1].size()) + strips[0].data.size() +
-                          strips[1].data.size() + 4096);
+                          strips[1].data.size() + chain_words + 8192);
         m = {(int64_t)frag.size() / 4, blob.section(frag), blob.section(kids.data), (int64_t)kids.data.size()};
         for (int mode = 0; mode < 2; ++mode) {
             static_assert(sizeof(PcxColTask) == 48, "task records are twelve words");
@@ -950,7 +947,7 @@ struct Cutter {
                     const size_t last = std::min(n_levels, at + PCX_COLUMN_MAX_LEVELS);
                     if (const auto* c = chained ? chain[at] : nullptr) {
                         const auto shape = PcxColPlanner::chain_shape(W, c->strips, room);
-                        launches.insert(launches.end(), {3, blob.section(pc.chain_rows(*c, mode)), blob.section(chain_strips(mode, at)),
+                        launches.insert(launches.end(), {3, blob.section(c->rows[mode]), blob.section(chain_strips(mode, at)),
                                                          c->n, c->strips, shape.nt, shape.per});
                         end = at + c->n;
                         continue;
