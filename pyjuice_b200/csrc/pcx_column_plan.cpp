@@ -629,19 +629,14 @@ struct PcxColPlanner {
     // forward against 556).
     bool suits(int64_t W, const Room& room) const {
         if (big_steps == 0) return true;
-        // (or where every level of large groups belongs to a chain whose clusters fit at once)
-        int64_t chained = 0, large = 0;
-        bool fits = true;
-        for (auto& c : chains) {
-            chained += c.n;
-            fits = fits && chain_shape(W, c.strips, room).waves == 1;
-        }
-        for (auto& d : depths) {
-            bool any = false;
-            for (auto& g : d.fw) any = any || g.big;
-            large += any;
-        }
-        if (fits && chained >= large) return true;
+        // (or where every level of large groups lies inside a chain whose clusters fit at once)
+        std::vector<char> chained(depths.size(), 0);
+        for (auto& c : chains)
+            if (chain_shape(W, c.strips, room).waves == 1) std::fill_n(chained.begin() + c.first, c.n, 1);
+        bool all = true;
+        for (size_t i = 0; i < depths.size(); ++i)
+            for (auto& g : depths[i].fw) all = all && (!g.big || chained[i]);
+        if (all) return true;
         const Shape s = big_shape(W, room);
         int64_t rounds = 0, levels = 0;
         for (auto& d : depths) {

@@ -98,6 +98,33 @@ def test_what_is_no_chain():
     assert not _chains(ColumnProgram(_hmm(32, 6)).plan(8), 0)                       # two strips
 
 
+def _chain_below_wide_levels(length):
+    """``length`` tied levels of 64 states under three levels of 1024 with parameters of their own."""
+    torch.manual_seed(3)
+    dist = pj.nodes.Categorical(num_cats=3)
+    with pj.set_block_size(64):
+        leaf = lambda v, n: pj.inputs(v, num_nodes=n, dist=dist)
+        ns, tied = leaf(0, 64), None
+        for v in range(1, length + 1):
+            p = pj.multiply(ns, leaf(v, 64))
+            ns = tied = pj.summate(p, num_nodes=64) if tied is None else tied.duplicate(p, tie_params=True)
+        below = 64
+        for v, n in enumerate((256, 1024, 1024, 1024), length + 1):
+            ns, below = pj.summate(pj.multiply(ns, leaf(v, below)), num_nodes=n), n
+        ns = pj.summate(pj.multiply(ns, leaf(length + 5, below)), num_nodes=1, block_size=1)
+    ns.init_parameters()
+    return pj.compile(ns, verbose=False)
+
+
+def test_a_chain_elsewhere_does_not_excuse_large_levels():
+    """Large levels outside a chain are judged as without one, however long the chain below them is."""
+    alone, below = ColumnProgram(_chain_below_wide_levels(2)), ColumnProgram(_chain_below_wide_levels(9))
+    assert alone.n_chains == 0 and below.n_chains == 1
+    assert alone.suits(64) and below.suits(64)
+    assert not alone.suits(1024) and not below.suits(1024)
+    assert ColumnProgram(_hmm(256, 5)).suits(64)           # the large levels are the chain
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B", [1, 50, 130, 256])
 @pytest.mark.parametrize("latents,tokens,banded", [(64, 4, False), (96, 5, False), (128, 9, True), (320, 6, False), (512, 7, False),
