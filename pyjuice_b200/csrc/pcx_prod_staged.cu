@@ -111,9 +111,10 @@ __global__ void __launch_bounds__(ST, 1) prod_staged_kernel(const StagedArgs a) 
                 if (k + 4 < now.z) take_rows<LOGS, 8>(mine, q, m, acc);
                 else take_rows<LOGS, 4>(mine, q, m, acc);
             }
-            if (LOGS && (now.z != 1 || add))                 // (one parent: its flow as it is)
+            if (LOGS)                                        // (one parent: its flow as it is; a maximum passes over NaN, the sum does not)
 #pragma unroll
-                for (int v = 0; v < 4; ++v) m[v] = fast_log_plus(acc[v], m[v] == PCX_NEG_INF ? 0.0f : m[v]);
+                for (int v = 0; v < 4; ++v)
+                    if (now.z != 1 || add || acc[v] != acc[v]) m[v] = fast_log_plus(acc[v], m[v] == PCX_NEG_INF ? 0.0f : m[v]);
             if (ok) stvec<4>(dst, LOGS ? m : acc);
         }
         __syncthreads();

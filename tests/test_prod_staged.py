@@ -119,6 +119,26 @@ def test_kernel(mode, logspace, W, size, n_sources):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode,logspace", [(0, True), (1, True), (1, False)])
+def test_nan_comes_through(mode, logspace):
+    """A NaN source reaches every row that reads it (also the only one of a row, whose value is passed on as it is), and no other."""
+    staged, n_out = _tables(random.Random(1), 4, 40, [0, 1, 1, 2, 9] * 13, "cuda:0")
+    g = torch.Generator(device="cuda:0").manual_seed(5)
+    src = -torch.rand(4 * 47, 40, device="cuda:0", generator=g) - 1.0
+    src[torch.rand(4 * 47, 40, device="cuda:0", generator=g) < 0.2] = float("nan")
+    out = -torch.rand(n_out, 40, device="cuda:0", generator=g)
+    out[torch.rand(n_out, 40, device="cuda:0", generator=g) < 0.2] = float("nan")
+    was = out.isnan().cpu()
+    staged.run(mode, out, src, logspace)
+    x = src.isnan().cpu()
+    for row, (sources, add) in _readers(staged).items():
+        want = was[row:row + 4].clone() if mode == 1 and add else torch.zeros(4, 40, dtype=torch.bool)
+        for s in sources:
+            want |= x[s:s + 4]
+        assert torch.equal(out[row:row + 4].isnan().cpu(), want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("W", [33, 256])
 @pytest.mark.parametrize("logspace", [True, False])
 def test_circuit_against_oracle(W, logspace, monkeypatch):
