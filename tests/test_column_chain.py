@@ -1,12 +1,15 @@
 """Chains of the column program (runs of tied levels in one launch): their tables, walked in float64 on the host, and the kernel
 against the same levels by their tasks, at the sizes where its shapes meet: strips per CTA that do not divide the rows, one to
-three column tiles per cluster, parameters beyond tensor memory, chains of odd and even length."""
+three column tiles per cluster, parameters beyond tensor memory, chains of odd and even length; then every shape of the kernel
+against float64."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import pyjuice_b200 as pj
-from helpers import check_against_oracle
+from helpers import check_against_oracle, oracle_step
 from pyjuice_b200.column import ColumnProgram, _Chain
 
 DEV = "cuda:0"
@@ -157,6 +160,65 @@ def test_against_the_tasks(latents, tokens, banded, B, monkeypatch):
     for a, b in zip(got[0][2:], got[1][2:]):
         assert (a - b).abs().max() <= 1e-4 * tokens * b.abs().max()
     assert pj._lib.get_status(DEV) == 0
+
+
+# States, column tiles a cluster, strips a CTA: every kernel of the launcher (column tiles x strips a warp, see `_kernel`), each with
+# warps that share a part of the contraction and that do not where both exist, and a last CTA of fewer strips.
+SHAPES = ([(192, nt, per) for nt in (1, 2, 3) for per in (1, 2, 3)] + [(224, 3, 5), (224, 1, 6), (192, 2, 8), (224, 1, 8)]
+          + [(320, nt, 2) for nt in (1, 2, 3)] + [(640, nt, 4) for nt in (1, 2, 3)] + [(640, 3, 3), (1024, 1, 8), (1024, 2, 4)])
+
+
+def _kernel(states, nt, per):
+    """(column tiles, strips a warp) of the kernel that the launcher takes for a chain."""
+    strips = states // 16
+    at_once = -(-per // (2 if per > 1 and -(-strips // per) <= 8 else 1))
+    return nt, (1 if at_once == 1 else 2 if at_once == 2 else 4)
+
+
+def test_the_shapes_are_all_there_are():
+    assert {_kernel(*shape) for shape in SHAPES} == {(nt, ps) for nt in (1, 2, 3) for ps in (1, 2, 4)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("B", [5, 136, 520])
+@pytest.mark.parametrize("states,nt,per", SHAPES)
+def test_shapes_against_float64(states, nt, per, B, mode, monkeypatch):
+    """Relative error of a level, hence absolute of a logarithm.  Two bf16 parts a factor (mode 1): 2^-18 for each factor's third
+    part and 2^-18 for the product of the second parts, the exponential and the logarithm 2^-22 each, and the additions: three per
+    16 children in the tensor core, 2^-23 each, some 2^-16 at 1024 states: 3 * 2^-16 with room for what they meet in.  One part
+    (mode 2): 2^-9 for each factor.  A flow has gone up and down the chain; a parameter flow has one more product in it."""
+    tokens, level = 6, (3 * 2.0 ** -16 if mode == 1 else 2.0 ** -8 + 3 * 2.0 ** -16)
+    pc = _hmm(states, tokens).to(DEV)
+    x = torch.randint(0, 7, (B, tokens), generator=torch.Generator().manual_seed(B))
+    cut = ColumnProgram._cut
+
+    def shaped(self, W):
+        plan = cut(self, W)
+        for m in (0, 1):
+            assert len(_chains(plan, m)) == 1
+            plan[m]["chained"] = [_Chain(c.rows, c.strips, c.n, c.S, W, nt, per) if isinstance(c, _Chain) else c
+                                  for c in plan[m]["chained"]]
+        return plan
+    rooms = np.full(21, 1 << 20, dtype=np.int32)           # (clusters wait for one another's place, not for one another)
+    monkeypatch.setattr(ColumnProgram, "_room", lambda self: rooms.ctypes.data_as(ctypes.c_void_p))
+    monkeypatch.setattr(ColumnProgram, "_cut", shaped)
+    ref, st, _ = oracle_step(pc, x)
+    pc.sum_mode = mode
+    pc.init_param_flows(flows_memory=0.0)
+    lls = pc(x.to(DEV))
+    pc.backward(x.to(DEV))
+    assert pj._lib.get_status(DEV) == 0
+    assert [(c.nt, c.per) for m in (0, 1) for c in _chains(pc._column_program.plan(pc._nm.size(1)), m)] == [(nt, per)] * 2
+    d = pc.num_dummy_nodes
+    rounding = lambda t: 2.0 ** -22 * t.abs()
+    for got, want in ((lls, ref), (pc.node_mars[d:], st.node_mars[d:])):
+        got = got.detach().double().cpu()
+        assert bool(((got - want).abs() <= level * tokens + rounding(want)).all())
+    flows, want = pc.node_flows[d:].double().cpu().exp(), st.node_flows[d:].exp()
+    assert bool(((flows - want).abs() <= 2.1 * level * tokens * want + 1e-30).all())
+    flows, want = pc.param_flows.double().cpu(), st.param_flows
+    assert bool(((flows - want).abs() <= 2.1 * level * (tokens + 1) * want + 1e-30).all())
 
 
 @pytest.mark.gpu
