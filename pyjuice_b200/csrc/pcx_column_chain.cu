@@ -14,10 +14,12 @@
 // that owns a row adds the value of the element's other child to it, forms the exponential, splits it and stores it in the
 // order of the B fragment; a warp of the next level reads 16-byte words that ARE its operand.  Exponentials are relative to
 // the maximum of the CTA's own rows (nobody waits for a maximum over all CTAs), and the partial products of a CTA's rows are
-// scaled where the parts of the contraction are added up.  4300 cycles a level now: operands from the other CTAs 1500,
-// multiplications 1100, scales and parts 800, logarithm to store 800.
-// Microseconds a level, before / now (forward passes of tied HMMs, leaves and launches included): 128 states, 64 columns 4.1 /
-// 2.6; 256, 64 5.0 / 2.9; 512, 77 6.5 / 3.7; 512, 256 8.2 / 5.6; 1024, 64 11.2 / 6.7; 1024, 128 14.8 / 11.1.
+// scaled where the parts of the contraction are added up.  4450 cycles a level now (512 x 512, eight columns, eight CTAs of four
+// strips): from a CTA's stores to the operands in the others' registers 1600, scales of the parts 300, multiplications 1200, parts
+// through shared memory and their sum 650, maximum over the CTA's strips, exponential, split and store 700.  With more columns
+// and rows a CTA the multiplications take over: 1024 x 1024, 24 columns, 16 CTAs of four strips 7000 of 15 400.
+// Microseconds a level, before / now (forward passes over 64 tokens, leaves and launches included): 128 states, 64 columns 3.5 /
+// 2.0; 256, 64 4.3 / 2.3; 512, 77 5.6 / 2.8; 512, 256 6.9 / 3.9; 1024, 64 10.0 / 5.2; 1024, 128 12.9 / 8.8.
 //
 //   warp (kp, ws)   strips ws * strips_w .. of the CTA, children of part kp of the contraction (parts never cross the rows of
 //                   two CTAs, so each has one scale).  Two warps share a part where the CTAs are few: half the partial products.

@@ -542,9 +542,11 @@ struct PcxColPlanner {
     // Strips per CTA and columns per cluster of a chain of groups of S strips: the cheapest estimate of a level, in cycles, times
     // the waves of clusters.  `mma`: the products of a CTA's busiest scheduler, 8 cycles each (four warps share one); what else
     // grows with the rows and columns of a CTA (partial products, epilogue) grows with it.  `stream`: fragments that neither
-    // tensor memory nor shared memory hold.  Measured, cycles a level, states / columns a cluster x strips a CTA: 128 / 8 x 1 3160;
-    // 256 / 8 x 2 3870, 8 x 4 4260; 512 / 8 x 4 5350, 8 x 8 7350; 1024 / 8 x 4 7660, 16 x 4 12 200, 8 x 8 13 000, 24 x 4 17 900,
-    // 16 x 8 20 600.
+    // tensor memory nor shared memory hold.  Cycles a level, measured forward / flows and estimated, states / columns a cluster x
+    // strips a CTA, four clusters on the machine: 128 / 8 x 1 3140 / 3210, 3040; 256 / 8 x 2 3640 / 3770, 3470; 8 x 4 4020 / 4050, 4050;
+    // 512 / 8 x 4 4460 / 4460, 5190; 8 x 8 5910 / 6110, 7490; 1024 / 8 x 4 5600 / 5720, 7490; 16 x 4 8770 / 9740, 12 080; 8 x 8 12 530 /
+    // 12 550, 12 730; 24 x 4 15 970 / 17 200, 16 660; 16 x 8 22 010 / 22 920, 22 230.  Between the ends the estimate is up to 40 % high
+    // (it was fitted when four strips of a warp cost more); the order of the shapes of one size, which is all it is for, is right.
     struct ChainShape { int nt, per, waves; double cost; };
     static ChainShape chain_shape(int64_t W, int S, const Room& room) {
         ChainShape best{0, 0, 0, 0.0};
@@ -965,8 +967,10 @@ struct Cutter {
             }
         }
     }
-    // The chain whose first level is `at`, if its clusters fit at once: where they do not, the tasks, which take more columns in
-    // fewer CTAs, are faster (1024 states, 256 columns, 31 levels of a training step: 1384 us by tasks, 1443 in two waves).
+    // The chain whose first level is `at`, if its clusters fit at once.  Where they do not, the tasks, which take more columns in
+    // fewer CTAs, are about as fast (1024 states, 256 columns, 31 levels forward and back: 445 + 576 us by tasks, 512 + 556 in
+    // two waves of 24 columns x 4 strips, which the estimate prefers; three of 16 x 4 take 453 + 488).  Where they do, the chain
+    // is faster throughout (1024 states, 192 columns: 385 + 570 by tasks, 365 + 391; 512, 512: 268 + 370, 177 + 201).
     const PcxColPlanner::Chain* starts(int mode, size_t at) const {
         for (auto& c : pc.chains)
             if (levels[mode][at].depth == (mode == 0 ? c.first : c.first + c.n - 1)) {

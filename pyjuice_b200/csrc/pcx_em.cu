@@ -93,7 +93,7 @@ em_sum_kernel(float* __restrict__ params, const float* __restrict__ flows,
 constexpr int EM_U = 8;
 
 // One group of G threads per source node; the group strides over the node's categories.  The first EM_U of a thread stay in
-// registers over the sum, with their parameters.  (784 variables x 128 nodes x 256 categories: 72 -> 64 us.)
+// registers over the sum, with their parameters.  (784 variables x 128 nodes x 256 categories: 67 -> 58 us.)
 template <int G>
 __global__ void __launch_bounds__(NT)
 em_input_cat_kernel(float* __restrict__ params, const float* __restrict__ flows,
@@ -163,7 +163,7 @@ em_input_cat_kernel(float* __restrict__ params, const float* __restrict__ flows,
 // clears or moves them later).  (Tiles of 32 x 32, one CTA per 32 rows, ran at 3.1 TB/s: 128-byte runs strided by
 // 16 KB and 128 KB.)
 // Where such tiles are fewer than the SMs, tiles of 128 rows x 32 categories: what counts is then the chain of a CTA (512 rows x
-// 1000 categories, 32 tiles: 25 us, 128 narrow ones: 11.5).
+// 1000 categories, totals included, 32 tiles: 17 us, 128 narrow ones: 9.5).
 constexpr int EMT = 128;                                 // rows of a tile
 
 // part[share, r] = sum over this CTA's categories of flows_t[c, r].  Grid (ceil(R / 128), shares of the categories).
@@ -336,7 +336,7 @@ int pcx_em_sum(float* params, const float* param_flows, const int64_t* blk_par, 
     if (max_bs <= 0) return -1;
     cudaStream_t st = (cudaStream_t)stream;
     // tiles of 32 nodes read 128 bytes of an edge, tiles of eight one sector: where the former are fewer than two a SM, four times
-    // as many CTAs with a quarter of the rounds (512 x 512 parameters: 19 us with 16 CTAs of 32 nodes, 7.6 with 64 of eight)
+    // as many CTAs with a quarter of the rounds (512 x 512 parameters: 11.1 us with 16 CTAs of 32 nodes, 4.6 with 64 of eight)
     if (max_bs >= 32 && n_blocks * pcx_cdiv(max_bs, 32) >= 2 * 148) {
         int tiles = (int)pcx_cdiv(max_bs, 32);
         em_sum_kernel<32><<<(unsigned)(n_blocks * tiles), NT, 0, st>>>(params, param_flows, blk_par, blk_flow, blk_fan, blk_bs, tiles, step, pseudo, keep_zero);
