@@ -36,9 +36,24 @@ def _chains(plan, mode):
     return [c for c in plan[mode]["chained"] if isinstance(c, _Chain)]
 
 
-@pytest.mark.parametrize("latents,tokens", [(64, 5), (96, 6), (320, 4)])
-def test_tables(latents, tokens):
-    pc = _hmm(latents, tokens)
+def _value_first(latents, tokens):
+    """The same chain, with the value of the level before as the first child of every product."""
+    torch.manual_seed(3)
+    with pj.set_block_size(32):
+        leaf = lambda v: pj.inputs(v, num_nodes=latents, dist=pj.nodes.Categorical(num_cats=7))
+        ns, tied = leaf(0), None
+        for v in range(1, tokens):
+            ns = pj.summate(ns, num_nodes=latents) if tied is None else tied.duplicate(ns, tie_params=True)
+            tied = tied or ns
+            ns = pj.multiply(ns, leaf(v))
+        ns = pj.summate(ns, num_nodes=1, block_size=1)
+    ns.init_parameters()
+    return pj.compile(ns, verbose=False)
+
+
+@pytest.mark.parametrize("latents,tokens,make", [(64, 5, _hmm), (96, 6, _hmm), (320, 4, _hmm), (96, 5, _value_first)])
+def test_tables(latents, tokens, make):
+    pc = make(latents, tokens)
     program = ColumnProgram(pc)
     plan = program.plan(16)
     bases, params = plan["bases"].numpy().reshape(-1, 4), pc.params.data.double().numpy()
